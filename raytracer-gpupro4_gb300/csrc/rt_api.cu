@@ -67,6 +67,7 @@ extern "C" rt_status rt_ctx_destroy(rt_ctx* ctx) {
     if (ctx->d_words) cudaFree(ctx->d_words);
     if (ctx->d_spill) cudaFree(ctx->d_spill);
     if (ctx->d_order) cudaFree(ctx->d_order);
+    if (ctx->d_terms) cudaFree(ctx->d_terms);
     delete ctx;
     return RT_OK;
 }

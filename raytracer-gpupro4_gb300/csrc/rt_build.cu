@@ -43,7 +43,9 @@
 #include <atomic>
 #include <mutex>
 
-#include "rt_internal.cuh"
+#include "rt_records.cuh"
+
+using namespace rt;
 
 namespace {
 
@@ -118,7 +120,7 @@ __global__ void __launch_bounds__(256) k_bounds(const float* __restrict__ tris, 
     // counters: [0] bounds ticket (reset by the last block), [1..4] sort tile
     // tickets, [5] leaf count, [6] refit epoch (advanced once per build, so a
     // replayed CUDA graph of the build still tags every arrival afresh), [7]
-    // spine-node count
+    // whether the trace records are those of this tree
     if ((gtid >= 1 && gtid < 6) || gtid == 7) counters[gtid] = 0u;
     if (gtid == 0) {
         uint32_t e = counters[6] + 1u;
@@ -1284,7 +1286,8 @@ __global__ void __launch_bounds__(THREADS) k_emit_units(const uint32_t* __restri
                                                         const float* __restrict__ tris, uint32_t n, uint32_t depth,
                                                         const uint32_t* __restrict__ scan, rt_node* nodes,
                                                         float4* __restrict__ sorted_tris, uint2* units,
-                                                        uint32_t* unit_counts, uint32_t* err) {
+                                                        uint32_t* unit_counts, uint32_t* err,
+                                                        uint32_t* __restrict__ leaf_of) {
     __shared__ uint32_t s_f[THREADS / 32], s_b[THREADS / 32], s_tmp[THREADS / 32];
     __shared__ uint32_t s_first_head, s_first_tail, s_last_head, s_last_tail, s_cont_tail;
     __shared__ float s_red[THREADS / 32][6];
@@ -1303,7 +1306,6 @@ __global__ void __launch_bounds__(THREADS) k_emit_units(const uint32_t* __restri
         s_first_head = s_first_tail = kEmitTile;
         s_last_head = s_last_tail = 0u;
     }
-
     // 0. pre-gather in sorted order (A.xyz,id | B.xyz,0 | C.xyz,0): element
     // tbase + b * THREADS + t, a batch of loads in flight per thread; the
     // warp's 32 triangles are staged and stored as three 512-byte runs
@@ -1459,6 +1461,7 @@ __global__ void __launch_bounds__(THREADS) k_emit_units(const uint32_t* __restri
             if (seen_head) {  // a leaf with head and tail in this thread
                 const int32_t count = (int32_t)k - run_pos + 1;
                 store_node(nodes, run_h, run.lo, run.hi, (count << 3) | 4 | leaf_axis_of(run_m, count, depth), run_pos);
+                leaf_of[run_pos] = run_h;
                 seen_head = false;  // the next element is a head
             } else {
                 first_tail_q = q;
@@ -1521,6 +1524,7 @@ __global__ void __launch_bounds__(THREADS) k_emit_units(const uint32_t* __restri
         if (x.head >= 0) {  // its head is in an earlier thread of this tile
             const int32_t count = (int32_t)(tbase + j) - x.head + 1;
             store_node(nodes, ft_h, fin.lo, fin.hi, (count << 3) | 4 | leaf_axis_of(ft_m, count, depth), x.head);
+            leaf_of[x.head] = ft_h;
         } else {  // it began before the tile: finished in step 3
             for (int c = 0; c < 3; ++c) { s_cont_box[c] = fin.lo[c]; s_cont_box[3 + c] = fin.hi[c]; }
             s_cont_tail = tbase + j;
@@ -1588,6 +1592,7 @@ __global__ void __launch_bounds__(THREADS) k_emit_units(const uint32_t* __restri
             const int32_t count = (int32_t)s_cont_tail - start + 1;
             const uint2 u0 = my_units[0];
             store_node(nodes, u0.x, fin.lo, fin.hi, (count << 3) | 4 | leaf_axis_of(u0.y, count, depth), start);
+            leaf_of[start] = u0.x;
         }
     }
     if (t == THREADS - 1) {  // units: cont + heads, less an open last leaf
@@ -1678,7 +1683,8 @@ __global__ void __launch_bounds__(THREADS) k_emit_chunks(const uint2* __restrict
     __shared__ uint2 s_items[kItemCap];
     __shared__ int32_t s_ipos[kItemCap];
     grid_dep_wait();
-    const uint32_t c = blockIdx.x, tile = c / kTileChunks, chunk = c % kTileChunks;
+    const uint32_t tiles = gridDim.x / kTileChunks, tile = blockIdx.x % tiles, chunk = blockIdx.x / tiles,
+                   c = tile * kTileChunks + chunk;
     const uint32_t tc = min(__ldcg(tile_counts + tile), (uint32_t)kUnitCap);
     const int cnt = (int)min((uint32_t)kChunkUnits, tc > chunk * kChunkUnits ? tc - chunk * kChunkUnits : 0u);
     if (cnt == 0) {
@@ -1823,6 +1829,36 @@ __global__ void k_gather_tris(const uint32_t* __restrict__ ids, const float* __r
     }
 }
 
+// Trace records of an imported tree: every internal node that the root reaches.
+__global__ void __launch_bounds__(256) k_trace_nodes(const rt_node* __restrict__ nodes, uint32_t num_nodes,
+                                                     TraceNode* __restrict__ tnodes, uint32_t* __restrict__ leaf_of,
+                                                     uint32_t n) {
+    const uint32_t h = blockIdx.x * blockDim.x + threadIdx.x;
+    if (h >= num_nodes) return;
+    const rt_node root = nodes[1];
+    const float4 g = trace_grid(root.min, root.max);
+    const int pc = nodes[h].prim_count, pos = nodes[h].prim_pos;
+    if (h == 0) {
+        store_trace_grid(tnodes, g, (root.prim_count & 4) ? leaf_word(1u, (uint32_t)root.prim_pos,
+                                                                      (uint32_t)(root.prim_count >> 3)) : 0u);
+        return;
+    }
+    for (int k = 31 - __clz(h); k > 0; --k)
+        if (__ldg(&nodes[h >> k].prim_count) & 4) return;  // below a leaf
+    if (pc & 4) {
+        if (pos >= 0 && (uint32_t)pos < n) leaf_of[pos] = h;
+        return;
+    }
+    if (2 * h + 1 >= num_nodes) return;  // a corrupt tree
+    const rt_node l = nodes[2 * h], r = nodes[2 * h + 1];
+    auto word = [](const rt_node& c, uint32_t ch) {
+        return (c.prim_count & 4) ? leaf_word(ch, (uint32_t)c.prim_pos, (uint32_t)(c.prim_count >> 3)) : 0u;
+    };
+    const int field = pc & 3;  // one axis past the split axis
+    store_trace_node(tnodes, h, l.min, l.max, r.min, r.max, word(l, 2 * h), word(r, 2 * h + 1),
+                     field == 0 ? 2 : field - 1, g);
+}
+
 uint32_t ceil_div(uint64_t a, uint64_t b) { return (uint32_t)((a + b - 1) / b); }
 
 }  // namespace
@@ -1850,6 +1886,7 @@ extern "C" rt_status rt_lbvh_create(rt_ctx* ctx, uint32_t max_tris, uint32_t dep
         if (e == cudaSuccess) e = cudaMalloc(p, bytes);
     };
     alloc((void**)&l->nodes, sizeof(rt_node) * l->num_nodes);
+    alloc((void**)&l->tnodes, sizeof(TraceNode) * (size_t)std::max(1u, l->num_nodes / 2));
     alloc((void**)&l->keys, 4 * cap);
     alloc((void**)&l->ids, 4 * cap);
     // one block for both ping-pong buffers: after the sort it holds the
@@ -1870,7 +1907,7 @@ extern "C" rt_status rt_lbvh_create(rt_ctx* ctx, uint32_t max_tris, uint32_t dep
     alloc((void**)&l->lookback,
           sizeof(uint32_t) * kSortPasses * 256 * ((size_t)l->sort_tiles_cap + look_groups(l->sort_tiles_cap)));
     alloc((void**)&l->scan, sizeof(uint32_t) * 4 * (size_t)l->emit_tiles_cap);
-    alloc((void**)&l->leaf_list, 4 * cap);
+    alloc((void**)&l->leaf_of, 4 * cap);
     alloc((void**)&l->arrive, sizeof(uint32_t) * std::max(1u, l->num_nodes >> 1));
     // items and item counts of every merge level (chunk slots = 4 x tiles, then
     // the groups above: < 6 x tiles in all), the tiles' unit counts (tiles),
@@ -1902,9 +1939,9 @@ extern "C" rt_status rt_lbvh_destroy(rt_lbvh* l) {
 void free_lbvh(rt_lbvh* l) {
     void* ptrs[] = {l->nodes,    l->keys,     l->ids,      l->keys_alt,  nullptr,    l->sorted_tris,
                     l->tris,     l->scene,    l->partials, l->counters,  l->hist,    l->lookback,
-                    l->scan,     l->leaf_list, l->arrive,  l->f_primary, l->f_mirror, l->f_vis,
+                    l->scan,     l->leaf_of,  l->arrive,  l->f_primary, l->f_mirror, l->f_vis,
                     l->s_lists,  l->cnodes,   l->inner,    l->inner_rank, l->w_buf, l->s_rays,
-                    l->items,    l->item_counts};
+                    l->items,    l->item_counts, l->tnodes};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     delete l;
@@ -1956,7 +1993,7 @@ static rt_status launch_build(rt_ctx* ctx, rt_lbvh* l, const float* d_tris, uint
     uint32_t* tile_counts = l->item_counts + 6 * cap;
     launch_pdl(k_emit_units<kEmitThreads>, emit_tiles, kEmitThreads, kEmitUnitsSmem, st, (const uint32_t*)l->keys,
                (const uint32_t*)l->ids, d_tris, n, l->depth, (const uint32_t*)l->scan, l->nodes, l->sorted_tris,
-               tile_units, tile_counts, ctx->d_err);
+               tile_units, tile_counts, ctx->d_err, l->leaf_of);
     RT_CHECK_LAUNCH(ctx, "k_emit_units");
     const uint32_t chunks = emit_tiles * kTileChunks;
     launch_pdl(k_emit_chunks<kEmitThreads>, chunks, kEmitThreads, kChunkSmem, st, (const uint2*)tile_units,
@@ -1976,6 +2013,7 @@ static rt_status launch_build(rt_ctx* ctx, rt_lbvh* l, const float* d_tris, uint
     }
     l->built_keys = true;
     l->compact_valid = compact;
+    l->rec_tiles = emit_tiles;  // the next trace makes the records (Records in rt_records.cuh)
     return RT_OK;
 }
 
@@ -2007,9 +2045,12 @@ extern "C" rt_status rt_lbvh_import_host(rt_ctx* ctx, rt_lbvh* l, const rt_node*
     const uint32_t blocks = std::max(1u, std::min(ceil_div(n, 256), (uint32_t)ctx->num_sms * 8));
     k_gather_tris<<<blocks, 256, 0, st>>>(l->ids, l->tris, n, l->sorted_tris);
     RT_CHECK_LAUNCH(ctx, "k_gather_tris");
+    k_trace_nodes<<<ceil_div(l->num_nodes, 256), 256, 0, st>>>(l->nodes, l->num_nodes, l->tnodes, l->leaf_of, n);
+    RT_CHECK_LAUNCH(ctx, "k_trace_nodes");
     l->n = n;
     l->src_tris = l->tris;
     l->built_keys = false;
+    l->rec_tiles = 0;          // its records are made
     l->compact_valid = false;  // an imported tree is traversed in its heap layout
     return RT_OK;
 }

@@ -13,6 +13,7 @@
 
 #include <algorithm>
 #include <cstdarg>
+#include <cstddef>
 #include <cstdio>
 #include <string>
 #include <vector>
@@ -70,6 +71,39 @@ struct SceneInfo {
     uint32_t pad[3];
 };
 
+// Trace records: an internal node (index: its heap slot) as the walks read it,
+// both children's boxes in 32 bytes, one load.
+//   box[child][axis]  centre and half-extent of the child's box, padded so
+//     that the walk's test admits every ray that box_enter admits (Walk in
+//     rt_traverse.cuh).  Centres lie on a grid of 32768 steps of E / 32768 above
+//     G + E, half-extents are fractions of E.  The high 16 bits are a float's
+//     (rounded up: the whole word read as a float is at least the half-extent);
+//     the low 16 are 0x8000 | grid step, which under 0x3f00 make the float
+//     1 + step / 32768.  The lowest bits of box[0][0] and box[0][1] are the
+//     node's split axis.
+//   word[child]  0: an internal node; a leaf is the word that the walk keeps
+//     for it (leaf_word).
+// Slot 0 holds the tree's grid and, as word[1], a root that is a leaf.
+struct __align__(32) TraceNode {
+    uint32_t box[2][3];
+    uint32_t word[2];
+};
+struct __align__(32) TraceGrid {
+    float G[3], E;
+    uint32_t pad[3];
+    uint32_t root_word;
+};
+static_assert(sizeof(TraceNode) == 32 && sizeof(TraceGrid) == 32 && offsetof(TraceGrid, root_word) == 28, "");
+
+// A leaf in one word: bit 31; then, for fewer than 32 triangles that begin
+// below position 2^25, the count in bits 29 .. 25 and the position (its heap
+// slot is leaf_of[position]); else bit 30 and the heap slot.
+constexpr uint32_t kLeafFlag = 1u << 31;
+constexpr uint32_t kBigLeaf = 1u << 30;
+__host__ __device__ inline uint32_t leaf_word(uint32_t h, uint32_t pos, uint32_t cnt) {
+    return (cnt < 32u && pos < (1u << 25)) ? kLeafFlag | (cnt << 25) | pos : kLeafFlag | kBigLeaf | h;
+}
+
 // Tiling constants
 constexpr int kSortThreads = 256;
 constexpr int kSortItems = 16;
@@ -104,6 +138,8 @@ struct rt_ctx {
     uint32_t* d_spill_count = nullptr;  // heavy-ray list length (d_words[32]; shading rays: [33], claims [34])
     uint32_t* d_words = nullptr; // 64 device words
     uint32_t* d_spill = nullptr; // heavy-ray list, kSpillCap entries
+    float* d_terms = nullptr;    // radiance terms of a path-traced image (rt_pathtrace.cu), grown on demand
+    size_t terms_bytes = 0;
     uint32_t* d_order = nullptr; // heavy-first tile order, kOrderKinds x kOrderWords (parity / counts: d_words[40..])
     // hand-over budget per trace kind (0 primary, 1 shading, 2 generic rays); 0: no hand-over
     uint32_t trace_budget[3] = {kDefaultTraceBudget, kDefaultShadeBudget, kDefaultTraceBudget};
@@ -126,6 +162,9 @@ struct rt_lbvh {
     // compact layout used by the traversal: slot 1 = root, the children of
     // internal node x at slots 2 r + 2, 2 r + 3 with r = the rank of x among
     // the reachable internal nodes in heap order (its PrimPos holds 2 r + 2)
+    TraceNode* tnodes = nullptr;    // trace records, 1 << (depth - 1)
+    uint32_t rec_tiles = 0;         // emission tiles of the last build (0: the records were made by an import)
+    uint32_t* leaf_of = nullptr;    // heap slot of the leaf whose first triangle is at a sorted position
     rt_node* cnodes = nullptr;
     uint32_t ccap = 0;              // slots of cnodes
     uint32_t* inner = nullptr;      // bitmap of reachable internal heap slots (num_nodes / 32 words, >= 1)
@@ -140,7 +179,6 @@ struct rt_lbvh {
     uint32_t* hist = nullptr;        // 4 x 256 digit histograms
     uint32_t* lookback = nullptr;    // 4 passes x sort tiles x 256 status words
     uint32_t* scan = nullptr;        // emission tiles x 4 (fwd agg, bwd agg, fwd prefix, bwd suffix)
-    uint32_t* leaf_list = nullptr;   // cap
     uint32_t* arrive = nullptr;      // 1 << (depth-1) refit arrival words (epoch-tagged)
     uint2* items = nullptr;          // emission items (heap index, mask) of every merge level: 6 x emit tiles x 64
     uint32_t* item_counts = nullptr; // 8 x emit tiles: item counts of every level (6x), tile unit counts, merge tickets
@@ -259,9 +297,9 @@ constexpr uint32_t kSpinLimit = 1u << 20;
 // Grid of a persistent kernel: as many blocks as fit on every SM at once,
 // capped by the number of 32-item tiles.
 template <typename K>
-inline uint32_t persistent_blocks(const rt_ctx* ctx, K kernel, int threads, uint32_t tiles) {
+inline uint32_t persistent_blocks(const rt_ctx* ctx, K kernel, int threads, uint32_t tiles, size_t smem = 0) {
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0) != cudaSuccess || per_sm < 1)
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) != cudaSuccess || per_sm < 1)
         per_sm = 1;
     const uint64_t full = (uint64_t)per_sm * (uint64_t)ctx->num_sms;
     const uint64_t need = ((uint64_t)tiles * 32 + threads - 1) / threads;
@@ -296,4 +334,6 @@ inline rt_status reset_work(rt_ctx* ctx, int slot) {
     RT_CHECK_CUDA(ctx, cudaMemsetAsync(ctx->d_work + slot, 0, sizeof(uint32_t), ctx->stream));
     return RT_OK;
 }
+// The same, and the trace records of l if they are not valid.
+rt_status reset_work_and_records(rt_ctx* ctx, int slot, const rt_lbvh* l);
 

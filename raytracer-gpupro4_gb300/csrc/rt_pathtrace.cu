@@ -100,20 +100,24 @@ struct PathCounts {
     uint32_t segments = 0, boxes = 0, tris = 0, hits = 0;
 };
 
-// Path regeneration.  A warp's lanes each hold one pixel and trace its
-// samples one segment at a time; every segment of every lane is one
-// warp-wide traversal (trace_ray), whatever bounce each lane is at.  A lane
-// whose sample ends begins the pixel's next sample, and a lane whose pixel
-// is done takes the next pixel from the work counter as soon as
-// kPtRefillLanes lanes of its warp are idle (the last pixels of the image
-// leave lanes idle).  The pixels are handed out in 8 x 4 tiles, lanes of
-// one grab taking consecutive pixels.  A pixel's samples stay on one lane
-// and in order, so its progressive mean is the same sequence of fp32
-// operations as a sample-by-sample loop.
-constexpr int kPtRefillLanes = 16;
+// Path regeneration.  A warp's lanes each hold one path (a sample of a
+// pixel, or a pixel whose samples follow one another, see launch_pathtrace)
+// and trace it one segment at a time.  A lane whose walk has ended waits until
+// kPtShadeLanes of the warp's have; those then shade, bounce or take the next
+// path from the work counter, and start their next walks together while the
+// other lanes keep theirs, so no lane waits for the longest walk of its warp.
+// Of 2 to 16 lanes 10 was best (shading and the walk's start cost about 1,100
+// instructions whatever the lanes).  Paths are handed out in 8 x 4 pixel
+// tiles, lanes of one grab taking consecutive pixels.
+constexpr int kPtShadeLanes = 10;
+constexpr int kPtSteps = 8;  // expansions between two leaf phases (5: 26.1 ms, 7: 23.5, 8: 23.5, 10: 24.1)
+// Blocks per SM: 64 registers and eight blocks where the paths fill the GPU
+// (23.5 ms; seven: 25.5), 128 and four where they don't (0.72 ms a 256 x 256
+// image; eight: 0.76).
+constexpr int kPtBlocks = 8, kPtSmallBlocks = 4;
 
 struct PathLane {
-    bool live = false;           // holds a pixel
+    bool live = false;           // holds a path
     uint32_t i = 0, j = 0;       // the pixel
     uint32_t n = 0;              // the sample being traced
     uint32_t s = 0;              // its segment
@@ -122,6 +126,7 @@ struct PathLane {
     int exclude = -1;
     uint32_t start = 1u;         // restart node of the segment's walk
     float fact = 0.0f;           // 1 / (n + 1)
+    float keep = 0.0f;           // n / (n + 1)
     float beta[3];
 };
 
@@ -140,6 +145,8 @@ __device__ __forceinline__ void begin_sample(PathLane& L, const PathParams& P) {
     L.start = 1u;
     L.s = 0;
     L.beta[0] = L.beta[1] = L.beta[2] = 1.0f;
+    L.keep = fdiv((float)L.n, (float)(L.n + 1));
+    L.fact = fdiv(1.0f, (float)(L.n + 1));
 }
 
 // Next ray of a path that hit triangle `id` at t (not its last segment):
@@ -154,39 +161,159 @@ __device__ __forceinline__ void bounce(PathLane& L, const float* __restrict__ so
     ++L.s;
 }
 
-// Warp-aggregated grab of pixels for the idle lanes (all lanes call).
+// Warp-aggregated grab of paths for the idle lanes (all lanes call): path
+// p is sample first + (p / 32) % per of pixel p % 32 of tile p / (32 per).
 // Returns true for a lane that took a pixel inside the image.
-__device__ __forceinline__ bool grab_pixel(PathLane& L, const PathParams& P, uint32_t* work, uint32_t total,
-                                           bool& drained) {
+__device__ __forceinline__ bool grab_path(PathLane& L, const PathParams& P, uint32_t first, uint32_t per, uint32_t* work,
+                                          uint32_t total, bool& drained) {
     constexpr uint32_t kFull = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const uint32_t idle = __ballot_sync(kFull, !L.live);
-    if (drained || !(idle == kFull || __popc(idle) >= kPtRefillLanes)) return false;
+    if (drained || idle == 0u) return false;
     uint32_t base = 0;
     if (lane == 0) base = atomicAdd(work, (uint32_t)__popc(idle));
     base = __shfl_sync(kFull, base, 0);
-    if (base + (uint32_t)__popc(idle) >= total) drained = true;
+    if (base >= total || total - base <= (uint32_t)__popc(idle)) drained = true;
     const uint32_t k = base + __popc(idle & ((1u << lane) - 1u));
-    if (L.live || k >= total) return false;
+    if (!((idle >> lane) & 1u) || base >= total || k >= total) return false;
+    const uint32_t tile = (k >> 5) / per;
     uint32_t i, j;
-    if (!tile_pixel(k >> 5, k & 31u, P.cam.width, P.cam.height, &i, &j)) return false;
+    if (!tile_pixel(tile, k & 31u, P.cam.width, P.cam.height, &i, &j)) return false;
     L.i = i;
     L.j = j;
-    L.n = P.n0;
+    L.n = first + ((k >> 5) - tile * per);
     L.live = true;
     return true;
 }
 
-// At most 72 registers (seven blocks per SM).  Per segment: closest hit; on
-// a hit acc += (1/(n+1) * beta) * Le, beta *= albedo; on a miss
-// acc += (1/(n+1) * beta) * sky.  STATS: the counting variant, which also
-// sums the walk counts into counts[4] (64-bit).
-template <bool STATS>
-__global__ void __launch_bounds__(kPtThreads, 7) k_pathtrace(TreeRef tr, const float* __restrict__ soup,
-                                                          const float* __restrict__ albedo,
-                                                          const float* __restrict__ emission, PathParams P,
-                                                          float4* __restrict__ image, uint32_t* work,
-                                                          uint32_t num_tiles, unsigned long long* counts) {
+// Whether the lanes whose walks have ended go on now (uniform): enough of
+// them, or nobody left walking.
+__device__ __forceinline__ bool shade_now(bool walking, bool live, bool drained) {
+    constexpr uint32_t kFull = 0xffffffffu;
+    const uint32_t w = __ballot_sync(kFull, walking);
+    const uint32_t held = drained ? __ballot_sync(kFull, live) : kFull;
+    return w == 0u || __popc(held & ~w) * 32 >= __popc(held) * kPtShadeLanes;
+}
+
+// The radiance terms of samples traced apart: term (sample, segment, pixel)
+// = (1 / (n + 1) * beta) * Le, and how many segments each sample has.
+struct PathTerms {
+    float* terms;       // [spp][segments][pixels][3]
+    uint8_t* segments;  // [spp][pixels]
+};
+
+// Per segment: closest hit; on a hit acc += (1/(n+1) * beta) * Le, beta *=
+// albedo; on a miss acc += (1/(n+1) * beta) * sky.  TERMS: a path is one
+// sample, and its terms are stored for k_fold_terms; otherwise a path is a
+// pixel with all its samples.
+template <bool TERMS, int BLOCKS>
+__global__ void __launch_bounds__(kPtThreads, BLOCKS) k_pathtrace(
+    TreeRef tr, const float* __restrict__ soup, const float* __restrict__ albedo, const float* __restrict__ emission,
+    PathParams P, float4* __restrict__ image, uint32_t* work, uint32_t num_tiles, PathTerms T) {
+    constexpr uint32_t kFull = 0xffffffffu;
+    const uint32_t per = TERMS ? P.spp : 1u, total = num_tiles * 32u * per;
+    const size_t px = (size_t)P.cam.width * P.cam.height;
+    mark_records(tr);
+    PathLane L;
+    L.o = mk3(0.f, 0.f, 0.f);
+    L.d = mk3(0.f, 0.f, 1.f);
+    Walk w;
+    w.clear();
+    uint2 stack[kStackSize];
+    float acc[3] = {0.0f, 0.0f, 0.0f};
+    bool drained = false;
+    for (;;) {
+        if (shade_now(w.have, L.live, drained)) {
+            bool fresh = false;  // a new segment to walk
+            if (L.live && !w.have) {
+                bool ended = w.b.id < 0;
+                float le[3] = {P.sky[0], P.sky[1], P.sky[2]};
+                if (!ended)
+                    for (int c = 0; c < 3; ++c) le[c] = __ldg(emission + 3 * (size_t)w.b.id + c);
+                const size_t p = (size_t)L.j * P.cam.width + L.i;
+                float* term = TERMS ? T.terms + 3 * (((size_t)(L.n - P.n0) * (P.bounces + 1u) + L.s) * px + p) : nullptr;
+                for (int c = 0; c < 3; ++c) {
+                    const float x = fmul(fmul(L.fact, L.beta[c]), le[c]);
+                    if (TERMS) term[c] = x;
+                    else acc[c] = fadd(acc[c], x);
+                }
+                if (!ended) {
+                    for (int c = 0; c < 3; ++c)
+                        L.beta[c] = fmul(L.beta[c], __ldg(albedo + 3 * (size_t)w.b.id + c));
+                    ended = L.s == P.bounces;
+                    if (!ended) bounce(L, soup, w.b.id, w.b.t, tr.compact ? 1u : w.b.leaf);
+                }
+                fresh = !ended;
+                if (ended) {
+                    if (TERMS) {
+                        T.segments[(size_t)(L.n - P.n0) * px + p] = (uint8_t)(L.s + 1u);
+                        L.live = false;
+                    } else if (++L.n == P.n0 + P.spp) {
+                        image[p] = make_float4(acc[0], acc[1], acc[2], 1.0f);
+                        L.live = false;
+                    } else {
+                        begin_sample(L, P);
+                        for (int c = 0; c < 3; ++c) acc[c] = fmul(acc[c], L.keep);
+                        fresh = true;
+                    }
+                }
+            }
+            if (grab_path(L, P, P.n0, per, work, total, drained)) {
+                begin_sample(L, P);
+                if (!TERMS) {
+                    acc[0] = acc[1] = acc[2] = 0.0f;
+                    if (P.n0 > 0) {  // continue the progressive mean the image holds
+                        const float4 prev = image[(size_t)L.j * P.cam.width + L.i];
+                        acc[0] = prev.x;
+                        acc[1] = prev.y;
+                        acc[2] = prev.z;
+                    }
+                    for (int c = 0; c < 3; ++c) acc[c] = fmul(acc[c], L.keep);
+                }
+                fresh = true;
+            }
+            w.start(fresh, make_ray(L.o, L.d, 1e16f, L.exclude), tr, L.start, stack);
+            if (!__any_sync(kFull, L.live)) {
+                if (drained) break;
+                continue;
+            }
+        }
+        w.round(tr, kPtSteps, stack);
+    }
+}
+
+// The progressive mean over samples n0 .. n0 + spp - 1 from their terms: the
+// same sequence of fp32 operations as tracing them one after another.
+__global__ void __launch_bounds__(256) k_fold_terms(PathTerms T, uint32_t px, uint32_t segs, uint32_t n0, uint32_t spp,
+                                                    float4* __restrict__ image) {
+    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= px) return;
+    float acc[3] = {0.0f, 0.0f, 0.0f};
+    if (n0 > 0) {
+        const float4 prev = image[p];
+        acc[0] = prev.x;
+        acc[1] = prev.y;
+        acc[2] = prev.z;
+    }
+    for (uint32_t m = 0; m < spp; ++m) {
+        const uint32_t n = n0 + m;
+        const float keep = fdiv((float)n, (float)(n + 1));
+        for (int c = 0; c < 3; ++c) acc[c] = fmul(acc[c], keep);
+        const uint32_t ns = T.segments[(size_t)m * px + p];
+        for (uint32_t s = 0; s < ns; ++s) {
+            const float* term = T.terms + 3 * (((size_t)m * segs + s) * px + p);
+            for (int c = 0; c < 3; ++c) acc[c] = fadd(acc[c], __ldg(term + c));
+        }
+    }
+    image[p] = make_float4(acc[0], acc[1], acc[2], 1.0f);
+}
+
+// The counting variant: each walk in the order whose box and triangle tests
+// are counted (traverse), a warp's lanes together; sums the walk counts into
+// counts[4] (64-bit).
+__global__ void __launch_bounds__(kPtThreads) k_pathtrace_counted(
+    TreeRef tr, const float* __restrict__ soup, const float* __restrict__ albedo, const float* __restrict__ emission,
+    PathParams P, float4* __restrict__ image, uint32_t* work, uint32_t num_tiles, unsigned long long* counts) {
     constexpr uint32_t kFull = 0xffffffffu;
     const uint32_t total = num_tiles * 32u;
     PathCounts cnt;
@@ -196,18 +323,16 @@ __global__ void __launch_bounds__(kPtThreads, 7) k_pathtrace(TreeRef tr, const f
     float acc[3] = {0.0f, 0.0f, 0.0f};
     bool drained = false;
     for (;;) {
-        if (grab_pixel(L, P, work, total, drained)) {
+        if (grab_path(L, P, P.n0, 1u, work, total, drained)) {
+            begin_sample(L, P);
             acc[0] = acc[1] = acc[2] = 0.0f;
-            if (P.n0 > 0) {  // continue the progressive mean the image holds
+            if (P.n0 > 0) {
                 const float4 prev = image[(size_t)L.j * P.cam.width + L.i];
                 acc[0] = prev.x;
                 acc[1] = prev.y;
                 acc[2] = prev.z;
             }
-            const float fant = fdiv((float)L.n, (float)(L.n + 1));
-            L.fact = fdiv(1.0f, (float)(L.n + 1));
-            for (int c = 0; c < 3; ++c) acc[c] = fmul(acc[c], fant);
-            begin_sample(L, P);
+            for (int c = 0; c < 3; ++c) acc[c] = fmul(acc[c], L.keep);
         }
         if (!__any_sync(kFull, L.live)) {
             if (drained) break;
@@ -215,25 +340,19 @@ __global__ void __launch_bounds__(kPtThreads, 7) k_pathtrace(TreeRef tr, const f
         }
         const RayState r = make_ray(L.o, L.d, 1e16f, L.exclude);
         uint32_t nb = 0, nt = 0, leaf = 1u;
-        const Hit h = trace_ray<STATS>(r, L.live, tr, false, &nb, &nt, nullptr, nullptr, L.start, &leaf);
+        const Hit h = trace_ray<true>(r, L.live, tr, false, &nb, &nt, nullptr, nullptr, L.start, &leaf);
         if (!L.live) continue;
-        if (STATS) {
-            cnt.segments += 1;
-            cnt.boxes += nb;
-            cnt.tris += nt;
-            cnt.hits += (h.id >= 0) ? 1u : 0u;
-        }
-        bool ended;
-        if (h.id < 0) {
-            for (int c = 0; c < 3; ++c) acc[c] = fadd(acc[c], fmul(fmul(L.fact, L.beta[c]), P.sky[c]));
-            ended = true;
-        } else {
-            const float* le = emission + 3 * (size_t)h.id;
-            const float* al = albedo + 3 * (size_t)h.id;
-            for (int c = 0; c < 3; ++c) {
-                acc[c] = fadd(acc[c], fmul(fmul(L.fact, L.beta[c]), __ldg(le + c)));
-                L.beta[c] = fmul(L.beta[c], __ldg(al + c));
-            }
+        cnt.segments += 1;
+        cnt.boxes += nb;
+        cnt.tris += nt;
+        cnt.hits += (h.id >= 0) ? 1u : 0u;
+        bool ended = h.id < 0;
+        float le[3] = {P.sky[0], P.sky[1], P.sky[2]};
+        if (!ended)
+            for (int c = 0; c < 3; ++c) le[c] = __ldg(emission + 3 * (size_t)h.id + c);
+        for (int c = 0; c < 3; ++c) acc[c] = fadd(acc[c], fmul(fmul(L.fact, L.beta[c]), le[c]));
+        if (!ended) {
+            for (int c = 0; c < 3; ++c) L.beta[c] = fmul(L.beta[c], __ldg(albedo + 3 * (size_t)h.id + c));
             ended = L.s == P.bounces;
             if (!ended) bounce(L, soup, h.id, h.t, leaf);
         }
@@ -242,97 +361,97 @@ __global__ void __launch_bounds__(kPtThreads, 7) k_pathtrace(TreeRef tr, const f
                 image[(size_t)L.j * P.cam.width + L.i] = make_float4(acc[0], acc[1], acc[2], 1.0f);
                 L.live = false;
             } else {
-                const float fant = fdiv((float)L.n, (float)(L.n + 1));
-                L.fact = fdiv(1.0f, (float)(L.n + 1));
-                for (int c = 0; c < 3; ++c) acc[c] = fmul(acc[c], fant);
                 begin_sample(L, P);
+                for (int c = 0; c < 3; ++c) acc[c] = fmul(acc[c], L.keep);
             }
         }
     }
-    if (STATS) {
-        unsigned long long v[4] = {cnt.segments, cnt.boxes, cnt.tris, cnt.hits};
-        for (int q = 0; q < 4; ++q) {
-            for (int off = 16; off > 0; off >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], off);
-            if ((threadIdx.x & 31) == 0 && v[q]) atomicAdd(counts + q, v[q]);
-        }
+    unsigned long long v[4] = {cnt.segments, cnt.boxes, cnt.tris, cnt.hits};
+    for (int q = 0; q < 4; ++q) {
+        for (int off = 16; off > 0; off >>= 1) v[q] += __shfl_xor_sync(kFull, v[q], off);
+        if ((threadIdx.x & 31) == 0 && v[q]) atomicAdd(counts + q, v[q]);
     }
 }
 
 // Adjoint by path replay: the same paths as k_pathtrace (same streams, same
-// walks); a lane records the triangles its sample hits, and when the sample
-// ends runs the backward recurrence G_j = E_{j+1} + a_{j+1} G_{j+1} over
-// them with the sample's weight in the final mean.
-__global__ void __launch_bounds__(kPtThreads) k_pathtrace_adjoint(
+// hits), one sample a path; a lane records the triangles its sample hits, and
+// when the sample ends runs the backward recurrence G_j = E_{j+1} + a_{j+1}
+// G_{j+1} over them with the sample's weight in the final mean.
+__global__ void __launch_bounds__(kPtThreads, kPtBlocks) k_pathtrace_adjoint(
     TreeRef tr, const float* __restrict__ soup,
     const float* __restrict__ albedo, const float* __restrict__ emission, PathParams P,
     const float4* __restrict__ dimage, float* __restrict__ dalbedo, float* __restrict__ demission, uint32_t* work,
-    uint32_t num_tiles) {
+    uint32_t num_tiles, uint32_t first, uint32_t per) {
     constexpr uint32_t kFull = 0xffffffffu;
-    const uint32_t total = num_tiles * 32u;
+    const uint32_t total = num_tiles * 32u * per;
     PathLane L;
     L.o = mk3(0.f, 0.f, 0.f);
     L.d = mk3(0.f, 0.f, 1.f);
     float dle[3] = {0.0f, 0.0f, 0.0f};
-    float gimg[3] = {0.0f, 0.0f, 0.0f};
     int seg[kMaxSeg];
     int ns = 0;
+    mark_records(tr);
+    Walk w;
+    w.clear();
+    uint2 stack[kStackSize];
     bool drained = false;
     for (;;) {
-        if (grab_pixel(L, P, work, total, drained)) {
-            const float4 g4 = __ldg(dimage + (size_t)L.j * P.cam.width + L.i);
-            gimg[0] = g4.x;
-            gimg[1] = g4.y;
-            gimg[2] = g4.z;
-            ns = 0;
-            begin_sample(L, P);
-        }
-        if (!__any_sync(kFull, L.live)) {
-            if (drained) break;
-            continue;
-        }
-        const RayState r = make_ray(L.o, L.d, 1e16f, L.exclude);
-        uint32_t nb = 0, nt = 0, leaf = 1u;
-        const Hit h = trace_ray<false>(r, L.live, tr, false, &nb, &nt, nullptr, nullptr, L.start, &leaf);
-        if (!L.live) continue;
-        const bool missed = h.id < 0;
-        if (!missed) seg[ns++] = h.id;
-        const bool ended = missed || L.s == P.bounces;
-        if (!ended) {
-            bounce(L, soup, h.id, h.t, leaf);
-            continue;
-        }
-        // weight of sample n in the progressive mean after the call
-        float w = 1.0f / (float)(L.n + 1);
-        for (uint32_t m = L.n + 1; m < P.n0 + P.spp; ++m) w *= (float)m / (float)(m + 1);
-        float beta[kMaxSeg][3];
-        beta[0][0] = beta[0][1] = beta[0][2] = 1.0f;
-        for (int q = 0; q + 1 < ns; ++q)
-            for (int c = 0; c < 3; ++c) beta[q + 1][c] = beta[q][c] * __ldg(albedo + 3 * (size_t)seg[q] + c);
-        float G[3] = {0.0f, 0.0f, 0.0f};
-        if (missed)
-            for (int c = 0; c < 3; ++c) G[c] = P.sky[c];
-        for (int q = ns - 1; q >= 0; --q) {
-            const float* al = albedo + 3 * (size_t)seg[q];
-            const float* le = emission + 3 * (size_t)seg[q];
-            const float l0 = __ldg(le), l1 = __ldg(le + 1), l2 = __ldg(le + 2);
-            const bool emitter = (l0 != 0.0f) || (l1 != 0.0f) || (l2 != 0.0f);
-            const float lev[3] = {l0, l1, l2};
-            for (int c = 0; c < 3; ++c) {
-                const float gw = gimg[c] * w;
-                const float da = gw * beta[q][c] * G[c];
-                if (da != 0.0f) atomicAdd(dalbedo + 3 * (size_t)seg[q] + c, da);
-                if (emitter) dle[c] += gw * beta[q][c];
-                G[c] = lev[c] + __ldg(al + c) * G[c];
+        if (shade_now(w.have, L.live, drained)) {
+            bool fresh = false;
+            if (L.live && !w.have) {
+                const bool missed = w.b.id < 0;
+                if (!missed) seg[ns++] = w.b.id;
+                if (!missed && L.s != P.bounces) {
+                    bounce(L, soup, w.b.id, w.b.t, tr.compact ? 1u : w.b.leaf);
+                    fresh = true;
+                } else {
+                    const float4 g4 = __ldg(dimage + (size_t)L.j * P.cam.width + L.i);
+                    const float gimg[3] = {g4.x, g4.y, g4.z};
+                    // weight of sample n in the progressive mean after the call
+                    float wn = 1.0f / (float)(L.n + 1);
+                    for (uint32_t m = L.n + 1; m < P.n0 + P.spp; ++m) wn *= (float)m / (float)(m + 1);
+                    float beta[kMaxSeg][3];
+                    beta[0][0] = beta[0][1] = beta[0][2] = 1.0f;
+                    for (int q = 0; q + 1 < ns; ++q)
+                        for (int c = 0; c < 3; ++c) beta[q + 1][c] = beta[q][c] * __ldg(albedo + 3 * (size_t)seg[q] + c);
+                    float G[3] = {0.0f, 0.0f, 0.0f};
+                    if (missed)
+                        for (int c = 0; c < 3; ++c) G[c] = P.sky[c];
+                    for (int q = ns - 1; q >= 0; --q) {
+                        const float* al = albedo + 3 * (size_t)seg[q];
+                        const float* le = emission + 3 * (size_t)seg[q];
+                        const float l0 = __ldg(le), l1 = __ldg(le + 1), l2 = __ldg(le + 2);
+                        const bool emitter = (l0 != 0.0f) || (l1 != 0.0f) || (l2 != 0.0f);
+                        const float lev[3] = {l0, l1, l2};
+                        for (int c = 0; c < 3; ++c) {
+                            const float gw = gimg[c] * wn;
+                            const float da = gw * beta[q][c] * G[c];
+                            if (da != 0.0f) atomicAdd(dalbedo + 3 * (size_t)seg[q] + c, da);
+                            if (emitter) dle[c] += gw * beta[q][c];
+                            G[c] = lev[c] + __ldg(al + c) * G[c];
+                        }
+                    }
+                    ns = 0;
+                    L.live = false;
+                }
+            }
+            if (grab_path(L, P, first, per, work, total, drained)) {
+                ns = 0;
+                begin_sample(L, P);
+                fresh = true;
+            }
+            w.start(fresh, make_ray(L.o, L.d, 1e16f, L.exclude), tr, L.start, stack);
+            if (!__any_sync(kFull, L.live)) {
+                if (drained) break;
+                continue;
             }
         }
-        ns = 0;
-        if (++L.n == P.n0 + P.spp) L.live = false;
-        else begin_sample(L, P);
+        w.round(tr, kPtSteps, stack);
     }
     // emitter gradient: warp reduction, one atomic per warp and channel
     for (int c = 0; c < 3; ++c) {
         float v = dle[c];
-        for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+        for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(kFull, v, off);
         if ((threadIdx.x & 31) == 0 && v != 0.0f) atomicAdd(demission + c, v);
     }
 }
@@ -364,6 +483,38 @@ uint32_t px_tiles(const rt_camera* cam) {
 
 TreeRef tree_ref(const rt_ctx* ctx, const rt_lbvh* l);
 
+// Bytes of radiance terms a context keeps at most.
+constexpr size_t kTermBytes = (size_t)512 << 20;
+
+// The term buffers for as many of the call's samples as fit (0: trace each
+// pixel's samples one after another).  Never in a stream capture: a graph must
+// not hold a buffer that a later call may replace.
+static uint32_t ensure_terms(rt_ctx* ctx, size_t px, uint32_t segs, uint32_t spp, PathTerms* T) {
+    const size_t sample = px * ((size_t)segs * 12 + 1);
+    const uint32_t m = (uint32_t)std::min<size_t>(spp, kTermBytes / sample);
+    if (m < 2) return 0;  // so px < 2^25, and a launch has at most 2^31 paths
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(ctx->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return 0;
+    }
+    const size_t need = m * sample;
+    if (need > ctx->terms_bytes) {
+        if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) return 0;
+        if (ctx->d_terms) cudaFree(ctx->d_terms);
+        ctx->d_terms = nullptr;
+        ctx->terms_bytes = 0;
+        if (cudaMalloc((void**)&ctx->d_terms, need) != cudaSuccess) {
+            cudaGetLastError();
+            return 0;
+        }
+        ctx->terms_bytes = need;
+    }
+    T->terms = ctx->d_terms;
+    T->segments = reinterpret_cast<uint8_t*>(ctx->d_terms + 3 * (size_t)m * segs * px);
+    return m;
+}
+
 static rt_status launch_pathtrace(rt_ctx* ctx, const rt_lbvh* l, const float* d_albedo, const float* d_emission,
                                   const rt_camera* cam, const rt_pt_params* p, float* d_image,
                                   unsigned long long* d_counts, const char* who) {
@@ -371,20 +522,48 @@ static rt_status launch_pathtrace(rt_ctx* ctx, const rt_lbvh* l, const float* d_
     rt_status s = pt_args(ctx, l, d_albedo, d_emission, cam, p, &P, who);
     if (s != RT_OK) return s;
     if (!d_image) return rt_fail(ctx, RT_ERR_INVALID, "%s: null image", who);
-    if ((s = reset_work(ctx, kWorkPath)) != RT_OK) return s;
     const uint32_t tiles = px_tiles(cam);
+    const size_t px = (size_t)cam->width * cam->height;
+    float4* image = reinterpret_cast<float4*>(d_image);
+    uint32_t* work = ctx->d_work + kWorkPath;
     if (d_counts) {
-        k_pathtrace<true><<<persistent_blocks(ctx, k_pathtrace<true>, kPtThreads, tiles), kPtThreads, 0,
-                            ctx->stream>>>(tree_ref(ctx, l), l->src_tris, d_albedo, d_emission, P,
-                                           reinterpret_cast<float4*>(d_image), ctx->d_work + kWorkPath, tiles,
-                                           d_counts);
-    } else {
-        k_pathtrace<false><<<persistent_blocks(ctx, k_pathtrace<false>, kPtThreads, tiles), kPtThreads, 0,
-                             ctx->stream>>>(tree_ref(ctx, l), l->src_tris, d_albedo, d_emission, P,
-                                            reinterpret_cast<float4*>(d_image), ctx->d_work + kWorkPath, tiles,
-                                            nullptr);
+        if ((s = reset_work(ctx, kWorkPath)) != RT_OK) return s;
+        k_pathtrace_counted<<<persistent_blocks(ctx, k_pathtrace_counted, kPtThreads, tiles), kPtThreads, 0,
+                              ctx->stream>>>(tree_ref(ctx, l), l->src_tris, d_albedo, d_emission, P, image, work, tiles,
+                                             d_counts);
+        RT_CHECK_LAUNCH(ctx, "k_pathtrace_counted");
+        return RT_OK;
     }
-    RT_CHECK_LAUNCH(ctx, "k_pathtrace");
+    // Several samples a pixel: each traced as a path of its own, their terms
+    // folded in order afterwards.  With a pixel's samples on one lane the last
+    // pixels of a 1024 x 1024 x 4 image kept single lanes busy for 15 % of the time,
+    // and a smaller image could not fill the GPU.
+    const uint32_t segs = P.bounces + 1u;
+    PathTerms T = {nullptr, nullptr};
+    const uint32_t chunk = P.spp > 1 ? ensure_terms(ctx, px, segs, P.spp, &T) : 0u;
+    auto launch = [&](auto kernel, uint32_t per) {
+        kernel<<<persistent_blocks(ctx, kernel, kPtThreads, tiles * per), kPtThreads, 0, ctx->stream>>>(
+            tree_ref(ctx, l), l->src_tris, d_albedo, d_emission, P, image, work, tiles, T);
+    };
+    if (chunk == 0u) {
+        if ((s = reset_work_and_records(ctx, kWorkPath, l)) != RT_OK) return s;
+        if ((uint64_t)tiles * 32u <= (uint64_t)ctx->num_sms * kPtSmallBlocks * kPtThreads) launch(k_pathtrace<false, kPtSmallBlocks>, 1u);
+        else launch(k_pathtrace<false, kPtBlocks>, 1u);
+        RT_CHECK_LAUNCH(ctx, "k_pathtrace");
+        return RT_OK;
+    }
+    for (uint32_t done = 0; done < p->spp; done += P.spp) {
+        P.n0 = p->first_sample + done;
+        P.spp = std::min(chunk, p->spp - done);
+        if ((s = reset_work_and_records(ctx, kWorkPath, l)) != RT_OK) return s;
+        if ((uint64_t)tiles * 32u * P.spp <= (uint64_t)ctx->num_sms * kPtSmallBlocks * kPtThreads)
+            launch(k_pathtrace<true, kPtSmallBlocks>, P.spp);
+        else
+            launch(k_pathtrace<true, kPtBlocks>, P.spp);
+        RT_CHECK_LAUNCH(ctx, "k_pathtrace");
+        k_fold_terms<<<(uint32_t)((px + 255) / 256), 256, 0, ctx->stream>>>(T, (uint32_t)px, segs, P.n0, P.spp, image);
+        RT_CHECK_LAUNCH(ctx, "k_fold_terms");
+    }
     return RT_OK;
 }
 
@@ -407,12 +586,17 @@ extern "C" rt_status rt_pathtrace_adjoint(rt_ctx* ctx, const rt_lbvh* l, const f
     rt_status s = pt_args(ctx, l, d_albedo, d_emission, cam, p, &P, "rt_pathtrace_adjoint");
     if (s != RT_OK) return s;
     if (!d_dimage || !d_dalbedo || !d_demission) return rt_fail(ctx, RT_ERR_INVALID, "rt_pathtrace_adjoint: null buffer");
-    if ((s = reset_work(ctx, kWorkAdjoint)) != RT_OK) return s;
     const uint32_t tiles = px_tiles(cam);
-    k_pathtrace_adjoint<<<persistent_blocks(ctx, k_pathtrace_adjoint, kPtThreads, tiles), kPtThreads, 0,
-                          ctx->stream>>>(tree_ref(ctx, l), l->src_tris, d_albedo, d_emission, P,
-                                         reinterpret_cast<const float4*>(d_dimage), d_dalbedo, d_demission,
-                                         ctx->d_work + kWorkAdjoint, tiles);
-    RT_CHECK_LAUNCH(ctx, "k_pathtrace_adjoint");
+    // a sample of a pixel is a path; the path counter holds 2^31 of them a launch
+    const uint32_t most = std::max(1u, (1u << 31) / std::max(32u, tiles * 32u));
+    for (uint32_t done = 0; done < P.spp; done += most) {
+        const uint32_t per = std::min(most, P.spp - done);
+        if ((s = reset_work_and_records(ctx, kWorkAdjoint, l)) != RT_OK) return s;
+        k_pathtrace_adjoint<<<persistent_blocks(ctx, k_pathtrace_adjoint, kPtThreads, tiles * per), kPtThreads, 0,
+                              ctx->stream>>>(tree_ref(ctx, l), l->src_tris, d_albedo, d_emission, P,
+                                             reinterpret_cast<const float4*>(d_dimage), d_dalbedo, d_demission,
+                                             ctx->d_work + kWorkAdjoint, tiles, P.n0 + done, per);
+        RT_CHECK_LAUNCH(ctx, "k_pathtrace_adjoint");
+    }
     return RT_OK;
 }

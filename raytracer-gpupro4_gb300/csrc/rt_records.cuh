@@ -1,0 +1,120 @@
+// rt_records.cuh -- the trace records (TraceNode in rt_internal.cuh).
+//
+// Walk (rt_traverse.cuh) reads the tree through them.  A build leaves them
+// invalid (counters[7] = 0) and a trace call makes them before its first
+// pass, in the kernel that zeroes the call's counters: callers that only build
+// do not pay for them (10 us of 312 at 2.1 M triangles, wherever in the build
+// they were written).  The trace kernel that follows on the stream marks them
+// valid, so a mark always means complete records; two streams that trace a
+// fresh tree at once both write the same values.
+#pragma once
+#include "rt_internal.cuh"
+
+namespace rt {
+
+// The grid of a tree with bounds [mn, mx]: G, E.
+__device__ __forceinline__ float4 trace_grid(const float mn[3], const float mx[3]) {
+    const float E = fmaxf(fsub(mx[0], mn[0]), fmaxf(fsub(mx[1], mn[1]), fsub(mx[2], mn[2])));
+    return make_float4(fsub(mn[0], E), fsub(mn[1], E), fsub(mn[2], E), E);
+}
+__device__ __forceinline__ void store_trace_grid(TraceNode* tnodes, float4 g, uint32_t root_word) {
+    float4* p = reinterpret_cast<float4*>(tnodes);
+    p[0] = g;
+    p[1] = make_float4(0.f, 0.f, 0.f, __uint_as_float(root_word));
+}
+
+// One axis of a child's box; rE = 1 / E.  The lowest bit of the grid step is
+// `bit` when bit >= 0.
+__device__ __forceinline__ uint32_t trace_box_word(float mn, float mx, float G, float E, float rE, int bit) {
+    const float q = fminf(fmaxf(rintf((0.5f * mn + 0.5f * mx - (G + E)) * rE * 32768.0f), 0.0f), 32767.0f);
+    uint32_t step = (uint32_t)q;
+    if (bit >= 0) step = (step & ~1u) | (uint32_t)bit;
+    const float X = fmaf(E, 1.0f + (float)step * (1.0f / 32768.0f), G);  // the centre, within 2^-24 |X|
+    float e = fmaxf(__fsub_ru(mx, X), __fsub_ru(X, mn));
+    e = __fadd_ru(e, __fmaf_ru(fabsf(X), 1.0f / 4194304.0f, E * (1.0f / 65536.0f)));  // 256 u E, and X's own error
+    e = __fmul_ru(__fmul_ru(e, rE), 1.0f + 1.0f / 1048576.0f);                        // rE and k are rounded
+    const uint32_t bits = __float_as_uint(fmaxf(e, 0.0f));
+    uint32_t w = (bits & 0xffff0000u) | 0x8000u | step;
+    if (w < bits) w += 0x10000u;
+    return w;
+}
+
+// Record of internal node h split on `axis` (0 x, 1 y, 2 z) with children of
+// boxes [llo, lhi], [rlo, rhi] and words lw, rw.
+__device__ __forceinline__ void store_trace_node(TraceNode* tnodes, uint32_t h, const float* llo, const float* lhi,
+                                                 const float* rlo, const float* rhi, uint32_t lw, uint32_t rw, int axis,
+                                                 float4 g) {
+    const float rE = fdiv(1.0f, g.w);
+    uint4* p = reinterpret_cast<uint4*>(tnodes + h);
+    p[0] = make_uint4(trace_box_word(llo[0], lhi[0], g.x, g.w, rE, axis & 1),
+                      trace_box_word(llo[1], lhi[1], g.y, g.w, rE, axis >> 1),
+                      trace_box_word(llo[2], lhi[2], g.z, g.w, rE, -1), trace_box_word(rlo[0], rhi[0], g.x, g.w, rE, -1));
+    p[1] = make_uint4(trace_box_word(rlo[1], rhi[1], g.y, g.w, rE, -1), trace_box_word(rlo[2], rhi[2], g.z, g.w, rE, -1),
+                      lw, rw);
+}
+
+// Trace record of internal node h from its children's heap records.
+__device__ __forceinline__ void trace_node_of(uint32_t h, const rt_node* nodes, uint32_t num_nodes, TraceNode* tnodes,
+                                              float4 g) {
+    const float4* p = reinterpret_cast<const float4*>(nodes + 2u * h);
+    const float4 l0 = __ldg(p), l1 = __ldg(p + 1), r0 = __ldg(p + 2), r1 = __ldg(p + 3);
+    const int lpc = __float_as_int(l1.z), rpc = __float_as_int(r1.z), field = __ldg(&nodes[h].prim_count) & 3;
+    const float llo[3] = {l0.x, l0.y, l0.z}, lhi[3] = {l0.w, l1.x, l1.y}, rlo[3] = {r0.x, r0.y, r0.z},
+                rhi[3] = {r0.w, r1.x, r1.y};
+    store_trace_node(tnodes, h, llo, lhi, rlo, rhi,
+                     (lpc & 4) ? leaf_word(2u * h, (uint32_t)__float_as_int(l1.w), (uint32_t)(lpc >> 3)) : 0u,
+                     (rpc & 4) ? leaf_word(2u * h + 1u, (uint32_t)__float_as_int(r1.w), (uint32_t)(rpc >> 3)) : 0u,
+                     field == 0 ? 2 : field - 1, g);  // the field is one past the split axis
+}
+
+// What make_records needs of a tree (tiles = 0: its records are made).
+struct Records {
+    const uint32_t* valid;
+    const uint2* units;      // the emission's leaves, kEmitTile slots per tile
+    const uint32_t* counts;  // leaves of each tile
+    uint32_t tiles;
+    const rt_node* nodes;
+    uint32_t num_nodes;
+    TraceNode* tnodes;
+};
+
+inline Records records_of(const rt_lbvh* l) {
+    return Records{l->counters + 7, reinterpret_cast<const uint2*>(l->keys_alt),
+                   l->item_counts + 6 * (size_t)l->emit_tiles_cap, l->rec_tiles, l->nodes, l->num_nodes, l->tnodes};
+}
+
+// The records of one tile's leaves (a block).  There is one internal node per
+// two neighbouring leaves, their lowest common ancestor: a thread takes a
+// leaf and the one before it.
+__device__ __forceinline__ void make_records(const Records& R, uint32_t tile) {
+    __shared__ uint32_t s_prev;  // the last leaf of the tiles before
+    if (*R.valid) return;        // uniform
+    const uint32_t cnt = min(__ldg(R.counts + tile), (uint32_t)kEmitTile);
+    if (cnt == 0u) return;
+    const rt_node root = R.nodes[1];
+    const float4 g = trace_grid(root.min, root.max);
+    if (threadIdx.x == 0) {
+        uint32_t h = 0u;
+        for (uint32_t q = tile; q-- > 0u && h == 0u;) {
+            const uint32_t c = min(__ldg(R.counts + q), (uint32_t)kEmitTile);
+            if (c) h = __ldg(&R.units[(size_t)q * kEmitTile + c - 1].x);
+        }
+        s_prev = h;
+        if (h == 0u)  // the tree's first leaf
+            store_trace_grid(R.tnodes, g, (root.prim_count & 4) ? leaf_word(1u, (uint32_t)root.prim_pos,
+                                                                            (uint32_t)(root.prim_count >> 3)) : 0u);
+    }
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < cnt; i += blockDim.x) {
+        const uint32_t b = __ldg(&R.units[(size_t)tile * kEmitTile + i].x);
+        const uint32_t a = i ? __ldg(&R.units[(size_t)tile * kEmitTile + i - 1].x) : s_prev;
+        if (a == 0u || b == 0u) continue;
+        const int da = 31 - __clz(a), db = 31 - __clz(b), dm = min(da, db);
+        const uint32_t x = (a >> (da - dm)) ^ (b >> (db - dm));
+        if (x == 0u) continue;  // only after a failed sort
+        const uint32_t h = (a >> (da - dm)) >> (32 - __clz(x));
+        if (h != 0u && 2u * h + 1u < R.num_nodes) trace_node_of(h, R.nodes, R.num_nodes, R.tnodes, g);
+    }
+}
+
+}  // namespace rt

@@ -15,6 +15,7 @@
 #include <algorithm>
 #include <cstring>
 
+#include "rt_records.cuh"
 #include "rt_traverse.cuh"
 
 using namespace rt;
@@ -616,6 +617,12 @@ TreeRef tree_ref(const rt_ctx* ctx, const rt_lbvh* l) {
     t.tris = l->sorted_tris;
     t.n = l->n;
     t.err = ctx->d_err;
+    t.heap = l->nodes;
+    t.num_heap = l->num_nodes;
+    t.tnodes = l->tnodes;
+    t.leaf_of = l->leaf_of;
+    t.num_tnodes = l->num_nodes / 2;
+    t.records_valid = l->counters + 7;
     return t;
 }
 
@@ -657,14 +664,22 @@ __device__ __forceinline__ void zero_words(uint32_t* words, unsigned long long m
     if (threadIdx.x < 64 && ((mask >> threadIdx.x) & 1ull)) words[threadIdx.x] = 0u;
 }
 
-__global__ void k_reset_words(uint32_t* words, unsigned long long mask) {
+// Blocks past the first make the trace records of a tile each.
+__global__ void __launch_bounds__(256) k_reset_words(uint32_t* words, unsigned long long mask, Records rec) {
     grid_dep_wait();
+    if (blockIdx.x > 0) {
+        make_records(rec, blockIdx.x - 1u);
+        return;
+    }
     zero_words(words, mask);
 }
 
-rt_status reset_words(rt_ctx* ctx, uint64_t mask) {
-    if (!mask) return RT_OK;
-    launch_pdl(k_reset_words, 1, 64, 0, ctx->stream, ctx->d_words, (unsigned long long)mask);
+rt_status reset_words(rt_ctx* ctx, uint64_t mask, const rt_lbvh* l = nullptr) {
+    if (!mask && !l) return RT_OK;
+    Records rec;
+    memset(&rec, 0, sizeof(rec));
+    if (l) rec = records_of(l);
+    launch_pdl(k_reset_words, 1u + rec.tiles, l ? 256 : 64, 0, ctx->stream, ctx->d_words, (unsigned long long)mask, rec);
     RT_CHECK_LAUNCH(ctx, "k_reset_words");
     return RT_OK;
 }
@@ -699,8 +714,12 @@ rt_status launch_heavy(rt_ctx* ctx, const Spill& sp, HeavyArgs a, int kind) {
     return RT_OK;
 }
 
-__global__ void k_order_begin(TileOrder o, uint32_t* words, unsigned long long reset) {
+__global__ void __launch_bounds__(256) k_order_begin(TileOrder o, uint32_t* words, unsigned long long reset, Records rec) {
     grid_dep_wait();
+    if (blockIdx.x > 0) {
+        make_records(rec, blockIdx.x - 1u);
+        return;
+    }
     zero_words(words, reset);
     __shared__ uint32_t s_w;
     if (threadIdx.x == 0) {
@@ -724,7 +743,9 @@ __global__ void k_order_begin(TileOrder o, uint32_t* words, unsigned long long r
 // Tile order of one trace kind (0 primary, 1 shading, 2 generic rays),
 // advanced to this call; enabled == false gives image order (cap 0: no list
 // is read or written).  reset: the call's counters to zero (word_bit mask).
-rt_status order_begin(rt_ctx* ctx, int kind, bool enabled, TileOrder* out, uint64_t reset = 0) {
+// l (nullable): the tree whose trace records the call needs.
+rt_status order_begin(rt_ctx* ctx, int kind, bool enabled, TileOrder* out, uint64_t reset = 0,
+                      const rt_lbvh* l = nullptr) {
     TileOrder o;
     o.cap = enabled ? kOrderCap : 0u;
     o.parity = ctx->d_words + 40 + 4 * kind;
@@ -732,10 +753,13 @@ rt_status order_begin(rt_ctx* ctx, int kind, bool enabled, TileOrder* out, uint6
     o.lists = ctx->d_order + (size_t)kind * kOrderWords;
     o.bits = o.lists + 2 * (size_t)kOrderCap;
     if (enabled) {
-        launch_pdl(k_order_begin, 1, 256, 0, ctx->stream, o, ctx->d_words, (unsigned long long)reset);
+        Records rec;
+        memset(&rec, 0, sizeof(rec));
+        if (l) rec = records_of(l);
+        launch_pdl(k_order_begin, 1u + rec.tiles, 256, 0, ctx->stream, o, ctx->d_words, (unsigned long long)reset, rec);
         RT_CHECK_LAUNCH(ctx, "k_order_begin");
     } else {
-        rt_status s = reset_words(ctx, reset);
+        rt_status s = reset_words(ctx, reset, l);
         if (s != RT_OK) return s;
     }
     *out = o;
@@ -893,6 +917,10 @@ rt_status trace_rays(rt_ctx* ctx, const rt_lbvh* l, const rt_ray* d_rays, uint32
 }
 
 }  // namespace
+
+rt_status reset_work_and_records(rt_ctx* ctx, int slot, const rt_lbvh* l) {
+    return reset_words(ctx, word_bit(ctx, ctx->d_work + slot), l);
+}
 
 extern "C" rt_status rt_trace_primary(rt_ctx* ctx, const rt_lbvh* l, const rt_camera* cam, rt_hit* d_hits,
                                       uint32_t* d_stats) {

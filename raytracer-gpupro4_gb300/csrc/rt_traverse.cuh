@@ -42,6 +42,14 @@ struct TreeRef {
     // triangles are [tri_base, n)); 0 otherwise, and 0 for the warp- and
     // block-per-ray walks
     uint32_t tri_base;
+    // the tree as Walk reads it: the heap, its trace records and leaf_of
+    // (indexed with tri_base)
+    const rt_node* __restrict__ heap;
+    uint32_t num_heap;
+    const TraceNode* __restrict__ tnodes;
+    const uint32_t* __restrict__ leaf_of;
+    uint32_t num_tnodes;
+    uint32_t* records_valid;
 };
 
 // First slot of the children pair of internal node `node` whose record's
@@ -536,6 +544,302 @@ __device__ __forceinline__ Hit traverse(const RayState& r, bool active, const Tr
     h.t = b.t;
     return h;
 }
+
+// ---------------------------------------------------------------------------
+// The walk of the kernels that count nothing.
+//
+// One lane's walk over the trace records (TraceNode): start() gives some lanes
+// a new ray, round() moves every walking lane on, so that the lanes of a warp
+// trace one ray after another without waiting for each other's walks (dynamic
+// ray fetch, Aila and Laine 2009).
+//
+// Result.  The trace records' boxes contain the heap's, padded for the
+// rounding of their own test, so every node that box_enter admits is entered
+// here too; a few more are.  A triangle is accepted only if its leaf's heap box
+// passes box_enter, and box tests are monotone in the box while every 1 / d is
+// finite, so the accepted triangles are those of the leaves that traverse()
+// reaches; the tie rule makes their order irrelevant.  The pad, in units of
+// u |1/d|, u = 2^-24: with c, e, G, E exact in the record, k = E / d and
+// n = (G - o) / d carry errors 2 E and 2 |G - o|, the three multiply-adds at
+// most |x| each for their results, at most |G - o| + 3 E, and box_enter itself
+// 2 |m - o| for a plane m: with |G - o| <= 16 E under 130 E in all; the pad is
+// 256 E.  The other rays (a zero direction component, an origin far outside the
+// scene) expand the heap records with box_enter.
+//
+// Cost.  A step reads one 32-byte record and issues about half of the
+// instructions of a step over two heap records with box_enter: centre and
+// half-extent need no minimum / maximum per axis (the half-rate pipe), and the
+// leaf flag and position come with the parent.  Every step and leaf iteration is
+// entered by the whole warp again (a loop that each lane leaves by itself
+// lets the compiler keep its lanes apart: 6.5 of 32 lanes active instead of
+// 15, 80 ms instead of 37 ms for 21 M path segments).
+__device__ __forceinline__ float min3(float a, float b, float c) {
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+// 32 bytes in one load.
+__device__ __forceinline__ void ldg32(const void* p, uint32_t w[8]) {
+    uint64_t a, b, c, d;
+    asm("ld.global.nc.v4.u64 {%0, %1, %2, %3}, [%4];" : "=l"(a), "=l"(b), "=l"(c), "=l"(d) : "l"(p));
+    w[0] = (uint32_t)a; w[1] = (uint32_t)(a >> 32);
+    w[2] = (uint32_t)b; w[3] = (uint32_t)(b >> 32);
+    w[4] = (uint32_t)c; w[5] = (uint32_t)(c >> 32);
+    w[6] = (uint32_t)d; w[7] = (uint32_t)(d >> 32);
+}
+__device__ __forceinline__ float grid_centre(uint32_t w) { return __uint_as_float(__byte_perm(w, 0x3f000000u, 0x7104)); }
+
+// First statement of a kernel that walks the records (after the wait for the
+// kernel that made them).
+__device__ __forceinline__ void mark_records(const TreeRef& tr) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *tr.records_valid = 1u;
+}
+
+constexpr uint32_t kGeneral = 8u;
+
+struct Walk {
+    f3 o, d, k, n;  // k = E / d, n = (G - o) / d
+    uint32_t sgn;   // RayState::sgn; kGeneral: the records do not serve this ray
+    int exclude;
+    Best b;         // key: the acceptance bound
+    uint32_t cur;   // internal heap slot or leaf word; 0: pop the next one
+    uint32_t pend;  // the leaf put aside (0: none)
+    uint32_t sp;
+    uint32_t tests;
+    bool have;      // the walk goes on
+
+    __device__ __forceinline__ void clear() {
+        o = d = k = n = mk3(0.f, 0.f, 0.f);
+        sgn = 0u;
+        exclude = -1;
+        b.key = 0;
+        b.t = 0.f;
+        b.u = b.v = -1.f;
+        b.id = -1;
+        b.leaf = 1u;
+        cur = pend = sp = tests = 0u;
+        have = false;
+    }
+
+    __device__ __forceinline__ void push(uint2* stack, uint32_t node, float t) {
+        stack[sp & (kStackSize - 1)] = make_uint2(node, __float_as_uint(t));
+        ++sp;
+    }
+
+    // The top of the stack, unless the bound now prunes it (cur = 0).
+    __device__ __forceinline__ void pop(const uint2* stack) {
+        --sp;
+        const uint2 e = stack[sp & (kStackSize - 1)];
+        cur = __uint_as_float(e.y) > b.t ? 0u : e.x;
+    }
+
+    static __device__ __forceinline__ bool enter(const RayState& r, const NodeBox& nb, float bt, float* t0, bool gen) {
+        return gen ? box_enter<true>(r, nb.a.x, nb.a.y, nb.a.z, nb.a.w, nb.b.x, nb.b.y, bt, t0)
+                   : box_enter<false>(r, nb.a.x, nb.a.y, nb.a.z, nb.a.w, nb.b.x, nb.b.y, bt, t0);
+    }
+
+    // Lanes with take begin ray r at heap node `first` (<= 1: the root; see
+    // traverse).
+    __device__ __forceinline__ void start(bool take, const RayState& r, const TreeRef& tr, uint32_t first, uint2* stack) {
+        if (!take) return;
+        o = r.o;
+        d = r.d;
+        sgn = r.sgn;
+        exclude = r.exclude;
+        b.key = hit_key(r.tmax, 0);
+        b.id = -1;
+        b.u = b.v = -1.0f;
+        b.t = r.tmax;
+        b.leaf = 1u;
+        cur = pend = sp = tests = 0u;
+        have = false;
+        if (!(r.tmax > 0.0f)) return;
+        const float4 g = __ldg(reinterpret_cast<const float4*>(tr.tnodes));  // G, E
+        k = mk3(fmul(g.w, r.inv.x), fmul(g.w, r.inv.y), fmul(g.w, r.inv.z));
+        const f3 q = mk3(fsub(g.x, o.x), fsub(g.y, o.y), fsub(g.z, o.z));
+        n = mk3(fmul(q.x, r.inv.x), fmul(q.y, r.inv.y), fmul(q.z, r.inv.z));
+        const float kmax = max3(fabsf(k.x), fabsf(k.y), fabsf(k.z)), kmin = min3(fabsf(k.x), fabsf(k.y), fabsf(k.z));
+        const bool gen = !(max3(fabsf(q.x), fabsf(q.y), fabsf(q.z)) <= 16.0f * g.w && kmax < 1e30f && kmin > 1e-30f);
+        if (gen) sgn |= kGeneral;
+        uint32_t node = 1u;
+        float t0;
+        if (first > 1u && !tr.compact) {
+            if (first >= tr.num_heap) {
+                atomicOr(tr.err, RT_DEVERR_BOUNDS);
+            } else {
+                const int D = 31 - __clz(first);
+#pragma unroll 2
+                for (int q = 1; q <= D; ++q) {
+                    const uint32_t sib = (first >> (D - q)) ^ 1u;
+                    const NodeBox sb = load_node(tr.heap, sib);
+                    if (enter(r, sb, b.t, &t0, gen)) push(stack, heap_item(sib, sb), t0);
+                }
+                node = first;
+            }
+        }
+        const NodeBox nb = load_node(tr.heap, node);
+        if (enter(r, nb, b.t, &t0, gen)) cur = heap_item(node, nb);
+        have = cur != 0u || sp != 0u;
+    }
+
+    // expand() of a ray that the records do not serve, over the heap.
+    __device__ __forceinline__ void expand_heap(const TreeRef& tr, uint2* stack) {
+        const uint32_t c0 = cur << 1;
+        if (c0 + 1u >= tr.num_heap) {
+            atomicOr(tr.err, RT_DEVERR_BOUNDS);
+            cur = sp = 0u;
+            return;
+        }
+        RayState r;
+        r.o = o;
+        r.inv = mk3(fdiv(1.0f, d.x), fdiv(1.0f, d.y), fdiv(1.0f, d.z));
+        const NodeBox nl = load_node(tr.heap, c0), nr = load_node(tr.heap, c0 + 1u);
+        float tl, tr_;
+        const bool hl = enter(r, nl, b.t, &tl, true), hr = enter(r, nr, b.t, &tr_, true);
+        tests += 2;
+        const int field = __ldg(&tr.heap[cur].prim_count) & 3;  // one axis past the split axis
+        const bool near_right = (sgn >> (field == 0 ? 2 : field - 1)) & 1u;
+        const bool go_right = near_right ? hr : !hl;
+        const uint32_t l = heap_item(c0, nl), r_ = heap_item(c0 + 1u, nr);
+        if (hl && hr) push(stack, near_right ? l : r_, near_right ? tl : tr_);
+        cur = (hl || hr) ? (go_right ? r_ : l) : 0u;
+    }
+
+    static __device__ __forceinline__ uint32_t heap_item(uint32_t h, const NodeBox& nb) {
+        const int pc = __float_as_int(nb.b.z);
+        return (pc & 4) ? leaf_word(h, (uint32_t)__float_as_int(nb.b.w), (uint32_t)(pc >> 3)) : h;
+    }
+
+    // One expansion of a lane that holds an internal node: cur = the near
+    // child that is hit (0: neither is).
+    __device__ __forceinline__ void expand(const TreeRef& tr, uint2* stack) {
+        if (cur >= tr.num_tnodes) {
+            atomicOr(tr.err, RT_DEVERR_BOUNDS);
+            cur = sp = 0u;
+            return;
+        }
+        uint32_t w[8];
+        ldg32(tr.tnodes + cur, w);
+        const float x0 = fmaf(grid_centre(w[0]), k.x, n.x), x1 = fmaf(grid_centre(w[3]), k.x, n.x);
+        const float y0 = fmaf(grid_centre(w[1]), k.y, n.y), y1 = fmaf(grid_centre(w[4]), k.y, n.y);
+        const float z0 = fmaf(grid_centre(w[2]), k.z, n.z), z1 = fmaf(grid_centre(w[5]), k.z, n.z);
+        const float ax = fabsf(k.x), ay = fabsf(k.y), az = fabsf(k.z);
+        float e[6];
+#pragma unroll
+        for (int q = 0; q < 6; ++q) e[q] = __uint_as_float(w[q]);
+        const float tl = max3(fmaf(-e[0], ax, x0), fmaf(-e[1], ay, y0), fmaxf(fmaf(-e[2], az, z0), 0.0f));
+        const float tr_ = max3(fmaf(-e[3], ax, x1), fmaf(-e[4], ay, y1), fmaxf(fmaf(-e[5], az, z1), 0.0f));
+        const float fl = min3(fmaf(e[0], ax, x0), fmaf(e[1], ay, y0), fminf(fmaf(e[2], az, z0), b.t));
+        const float fr = min3(fmaf(e[3], ax, x1), fmaf(e[4], ay, y1), fminf(fmaf(e[5], az, z1), b.t));
+        const bool hl = tl <= fl, hr = tr_ <= fr;
+        tests += 2;
+        const bool near_right = (sgn >> ((w[0] & 1u) | ((w[1] & 1u) << 1))) & 1u;
+        const bool go_right = near_right ? hr : !hl;  // the near child if it is hit, else the far one
+        const uint32_t l = (int)w[6] < 0 ? w[6] : cur << 1, r = (int)w[7] < 0 ? w[7] : (cur << 1) | 1u;
+        if (hl && hr) push(stack, near_right ? l : r, near_right ? tl : tr_);
+        cur = (hl || hr) ? (go_right ? r : l) : 0u;
+    }
+
+    // Moves every walking lane on: at most `steps` expansions (a lane puts its
+    // first leaf aside and goes on; with two or three leaves set aside no
+    // faster), then the leaves, a triangle of each lane at a time.  All 32
+    // lanes call.
+    __device__ __forceinline__ void round(const TreeRef& tr, int steps, uint2* stack, bool any_hit = false) {
+        constexpr uint32_t kFull = 0xffffffffu;
+        for (int s = 0; s < steps; ++s) {
+            const bool go = cur ? !((int)cur < 0 && pend) : sp != 0u;
+            if (!__any_sync(kFull, go)) break;
+            if (go) {
+                if (cur == 0u) pop(stack);
+                if ((int)cur < 0 && !pend) {
+                    pend = cur;
+                    cur = 0u;
+                }
+                if ((int)cur > 0) {
+                    if (sgn & kGeneral) expand_heap(tr, stack);
+                    else expand(tr, stack);
+                }
+            }
+            __syncwarp();
+        }
+        if ((int)cur < 0 && !pend) {
+            pend = cur;
+            cur = 0u;
+        }
+        uint32_t cnt = 0u, pos = 0u;
+        const uint32_t leaf = pend;
+        pend = 0u;
+        if (leaf) {
+            pos = leaf & 0x1ffffffu;
+            cnt = (leaf >> 25) & 31u;
+            if (leaf & kBigLeaf) {
+                const int2 z = __ldg(reinterpret_cast<const int2*>(tr.heap + (leaf & 0x3ffffffu)) + 3);
+                pos = (uint32_t)z.y;
+                cnt = (uint32_t)(z.x >> 3);
+            }
+            pos += tr.tri_base;
+            if (pos + cnt > tr.n) {
+                atomicOr(tr.err, RT_DEVERR_BOUNDS);
+                cnt = 0u;
+            }
+            tests += cnt;
+        }
+        bool inside = false;
+        while (__any_sync(kFull, cnt != 0u)) {
+            if (cnt != 0u) {
+                const float4* tp = tr.tris + 3 * (size_t)pos;
+                const float4 a = __ldg(tp), bb = __ldg(tp + 1), c = __ldg(tp + 2);
+                ++pos;
+                --cnt;
+                const int id = __float_as_int(a.w);
+                float u, v, t;
+                RayState r;
+                r.o = o;
+                r.d = d;
+                if (id != exclude && tri_test(r, a, bb, c, &u, &v, &t)) {
+                    const uint64_t key = hit_key(t, id);
+                    if (key < b.key) {
+                        const uint32_t h = (leaf & kBigLeaf) ? leaf & 0x3ffffffu
+                                                             : __ldg(tr.leaf_of + tr.tri_base + (leaf & 0x1ffffffu));
+                        if (inside || (sgn & kGeneral) || leaf_entered(tr, h)) {
+                            inside = true;
+                            b.key = key;
+                            b.t = t;
+                            b.u = u;
+                            b.v = v;
+                            b.id = id;
+                            b.leaf = h;
+                        } else {
+                            cnt = 0u;
+                        }
+                    }
+                }
+            }
+            __syncwarp();
+        }
+        if (any_hit && b.id >= 0) cur = sp = 0u;
+        have = cur != 0u || sp != 0u;
+    }
+
+    // box_enter of the heap box of leaf h.
+    __device__ __forceinline__ bool leaf_entered(const TreeRef& tr, uint32_t h) const {
+        if (h >= tr.num_heap) {
+            atomicOr(tr.err, RT_DEVERR_BOUNDS);
+            return false;
+        }
+        const NodeBox nb = load_node(tr.heap, h);
+        RayState r;
+        r.o = o;
+        r.inv = mk3(fdiv(1.0f, d.x), fdiv(1.0f, d.y), fdiv(1.0f, d.z));
+        float t0;
+        return box_enter<false>(r, nb.a.x, nb.a.y, nb.a.z, nb.a.w, nb.b.x, nb.b.y, b.t, &t0);
+    }
+};
 
 __device__ __forceinline__ uint64_t warp_min_u64(uint64_t v) {
 #pragma unroll
