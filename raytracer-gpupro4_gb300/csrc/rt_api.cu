@@ -46,7 +46,7 @@ extern "C" rt_status rt_ctx_create(int device, void* stream, rt_ctx** out) {
     if (cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
         cudaMalloc((void**)&c->d_words, 64 * sizeof(uint32_t)) != cudaSuccess ||
         cudaMemset(c->d_words, 0, 64 * sizeof(uint32_t)) != cudaSuccess ||
-        cudaMalloc((void**)&c->d_spill, sizeof(uint32_t) * kSpillCap) != cudaSuccess ||
+        cudaMalloc((void**)&c->d_spill, sizeof(uint32_t) * 2 * kSpillCap) != cudaSuccess ||
         cudaMalloc((void**)&c->d_order, sizeof(uint32_t) * kOrderKinds * kOrderWords) != cudaSuccess ||
         cudaMemset(c->d_order, 0, sizeof(uint32_t) * kOrderKinds * kOrderWords) != cudaSuccess) {
         if (c->d_words) cudaFree(c->d_words);

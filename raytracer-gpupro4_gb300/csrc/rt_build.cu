@@ -636,6 +636,36 @@ __device__ __forceinline__ void load_chunk(const uint32_t* __restrict__ keys, ui
     }
 }
 
+constexpr int kSepBit = 31;  // a batch's separator record, above every code bit
+
+// Boundary deltas of a thread's chunk with a separator record at each
+// scene boundary (off: S + 1 scene offsets in shared memory).
+__device__ __forceinline__ void load_chunk_b(const uint32_t* __restrict__ keys, uint32_t n, uint32_t s,
+                                             const uint32_t* off, uint32_t S, EmitChunk& e) {
+    const uint32_t prev = (s >= 1 && s - 1 < n) ? __ldg(keys + s - 1) : 0u;
+#pragma unroll
+    for (int q = 0; q <= kEmitItems; ++q) e.c[q] = (s + q < n) ? __ldg(keys + s + q) : 0u;
+    uint32_t sc = scene_of(off, S, s < n ? s : n - 1);
+    e.dl[0] = (s >= 1 && s < n) ? (s == off[sc] ? kSepBit : delta_of(prev, e.c[0])) : -1;
+    uint32_t nb = off[sc + 1];
+#pragma unroll
+    for (int q = 0; q < kEmitItems; ++q) {
+        const uint32_t i = s + q;
+        int d = -1;
+        if (i + 1 < n) {
+            if (i + 1 == nb) {
+                d = kSepBit;
+                ++sc;
+                nb = off[sc + 1];
+            } else {
+                d = delta_of(e.c[q], e.c[q + 1]);
+            }
+        }
+        e.dl[q + 1] = d;
+        e.r[q] = (d >= 0) ? (1u << d) : 0u;
+    }
+}
+
 // k_emit_tiles: per-tile fwd/bwd aggregates of the boundary record masks.
 __global__ void __launch_bounds__(kEmitThreads) k_emit_tiles(const uint32_t* __restrict__ keys, uint32_t n,
                                                              uint32_t* scan, uint32_t* arrive, uint32_t arrive_words,
@@ -1091,9 +1121,9 @@ __device__ __forceinline__ int leaf_axis_of(uint32_t m, int32_t count, uint32_t 
     return 1;
 }
 
-__device__ __forceinline__ void store_node(rt_node* nodes, uint32_t h, const float mn[3], const float mx[3],
-                                           int32_t prim_count, int32_t prim_pos) {
-    float4* p = reinterpret_cast<float4*>(nodes + h);
+__device__ __forceinline__ void store_node(rt_node* node, const float mn[3], const float mx[3], int32_t prim_count,
+                                           int32_t prim_pos) {
+    float4* p = reinterpret_cast<float4*>(node);
     p[0] = make_float4(mn[0], mn[1], mn[2], mx[0]);
     p[1] = make_float4(mx[1], mx[2], __int_as_float(prim_count), __int_as_float(prim_pos));
 }
@@ -1139,6 +1169,27 @@ __device__ __forceinline__ Box shfl_up_box(const Box& b, int off) {
     }
     return r;
 }
+
+// Where the emission finds its nodes.  One tree: node h is nodes[h].  A batch: a
+// node is named by scene << 23 | heap slot (depth <= 23), scene s's heap is at
+// nodes + (s << depth), and its records' positions count from its first
+// triangle off[s].
+constexpr uint32_t kSlotBits = 23;
+template <bool BATCH>
+struct Heap {
+    rt_node* nodes;
+    const uint32_t* off;
+    uint32_t depth;
+    __device__ __forceinline__ static uint32_t slot(uint32_t h) { return BATCH ? h & ((1u << kSlotBits) - 1u) : h; }
+    __device__ __forceinline__ rt_node* node(uint32_t h) const {
+        return BATCH ? nodes + ((size_t)(h >> kSlotBits) << depth) + slot(h) : nodes + h;
+    }
+    __device__ __forceinline__ int32_t first(uint32_t h) const { return BATCH ? (int32_t)__ldg(off + (h >> kSlotBits)) : 0; }
+    // the ancestor k levels up
+    __device__ __forceinline__ static uint32_t up(uint32_t h, int k) {
+        return BATCH ? (h & ~((1u << kSlotBits) - 1u)) | (slot(h) >> k) : h >> k;
+    }
+};
 
 // Shared-memory view of a CTA's units (capacity cap): unit i covers elements
 // [pos[i], pos[i + 1]) and is the node (h[i], m[i]) with box lo/hi[i];
@@ -1199,15 +1250,15 @@ __device__ __forceinline__ void push_item(const Units& u, uint2* items, uint32_t
 // child at its first unit's slot, then sets its bit; the second arrival
 // forms the parent and carries on.  Nodes whose parent boundary lies outside
 // the units, and arrivals whose sibling never came, become items.
-template <int THREADS>
-__device__ void unit_bottom_up(const Units& u, int U, rt_node* nodes, uint2* items, uint32_t* err,
+template <int THREADS, bool BATCH>
+__device__ void unit_bottom_up(const Units& u, int U, const Heap<BATCH>& heap, uint2* items, uint32_t* err,
                                uint32_t* inner) {
 #pragma unroll 1
     for (int i = threadIdx.x; i < U; i += THREADS) {
         Box b = get_box(u, i);
         uint32_t h = u.h[i], m = u.m[i];
         int li = i, ri = i;
-        while (h > 1) {
+        while (heap.slot(h) > 1) {
             const bool left = (h & 1u) == 0;
             const int k = left ? ri : li - 1;  // the parent's split boundary, after unit k
             if (k < 0 || k + 1 >= U) {
@@ -1228,9 +1279,11 @@ __device__ void unit_bottom_up(const Units& u, int U, rt_node* nodes, uint2* ite
             if (left) ri = u.aext[sarea]; else li = u.aext[sarea];
             const int d = __ffs(m) - 1;  // the parent's split bit
             m &= m - 1u;
-            h >>= 1;
-            const int32_t pos = u.pos[li], end = u.pos[ri + 1] - 1;
-            store_node(nodes, h, b.lo, b.hi, ((end - pos + 1) << 3) | ((30 - d) % 3), pos);
+            h = heap.up(h, 1);
+            // a batch: whole scenes between two units are done and not among them
+            const bool scene_end = BATCH && ri + 1 < U && (u.h[ri + 1] >> kSlotBits) != (h >> kSlotBits);
+            const int32_t pos = u.pos[li], end = (scene_end ? (int32_t)__ldg(heap.off + (h >> kSlotBits) + 1) : u.pos[ri + 1]) - 1;
+            store_node(heap.node(h), b.lo, b.hi, ((end - pos + 1) << 3) | ((30 - d) % 3), pos - heap.first(h));
             if (inner) atomicOr(inner + (h >> 5), 1u << (h & 31));
         }
     }
@@ -1247,7 +1300,7 @@ __device__ void unit_bottom_up(const Units& u, int U, rt_node* nodes, uint2* ite
             atomicOr(err, RT_DEVERR_BOUNDS);
             continue;
         }
-        push_item(u, items, u.h[li] >> up, m, err);
+        push_item(u, items, heap.up(u.h[li], up), m, err);
     }
 }
 
@@ -1280,14 +1333,16 @@ struct Seg {
     int32_t head;
 };
 
-template <int THREADS>
+template <int THREADS, bool BATCH>
 __global__ void __launch_bounds__(THREADS) k_emit_units(const uint32_t* __restrict__ keys,
                                                         const uint32_t* __restrict__ ids,
                                                         const float* __restrict__ tris, uint32_t n, uint32_t depth,
                                                         const uint32_t* __restrict__ scan, rt_node* nodes,
                                                         float4* __restrict__ sorted_tris, uint2* units,
                                                         uint32_t* unit_counts, uint32_t* err,
-                                                        uint32_t* __restrict__ leaf_of) {
+                                                        uint32_t* __restrict__ leaf_of,
+                                                        const uint32_t* __restrict__ scene_off, uint32_t S,
+                                                        uint32_t* __restrict__ ids_local) {
     __shared__ uint32_t s_f[THREADS / 32], s_b[THREADS / 32], s_tmp[THREADS / 32];
     __shared__ uint32_t s_first_head, s_first_tail, s_last_head, s_last_tail, s_cont_tail;
     __shared__ float s_red[THREADS / 32][6];
@@ -1298,7 +1353,14 @@ __global__ void __launch_bounds__(THREADS) k_emit_units(const uint32_t* __restri
     extern __shared__ float4 emit_smem[];
     float* s_box = reinterpret_cast<float*>(emit_smem);  // [6][kBoxStride]: lo xyz, hi xyz
 
+    __shared__ uint32_t s_off[BATCH ? kMaxBatchScenes + 1 : 1];
+
     grid_dep_wait();
+    if (BATCH) {
+        for (uint32_t q = threadIdx.x; q <= S; q += THREADS) s_off[q] = scene_off[q];
+        __syncthreads();
+    }
+    const Heap<BATCH> heap{nodes, scene_off, depth};
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
     const uint32_t tbase = blockIdx.x * (uint32_t)kEmitTile;
     uint2* my_units = units + (size_t)blockIdx.x * kUnitCap;
@@ -1314,17 +1376,26 @@ __global__ void __launch_bounds__(THREADS) k_emit_units(const uint32_t* __restri
         const bool soup_aligned = (reinterpret_cast<uintptr_t>(tris) & 15u) == 0;
 #pragma unroll 1
         for (int g = 0; g < kEmitItems; g += kGatherBatch) {
-            uint32_t idv[kGatherBatch];
+            uint32_t idv[kGatherBatch], loc[kGatherBatch];  // the triangle, and its id in its own tree
             float v[kGatherBatch][9];
 #pragma unroll
             for (int b = 0; b < kGatherBatch; ++b) {
                 const uint32_t k = tbase + (uint32_t)((g + b) * THREADS + t);
                 uint32_t id = k < n ? __ldg(ids + k) : 0u;
-                if (id >= n) {  // only after a failed sort (look-back timeout)
+                if (BATCH) {
+                    const uint32_t sk = scene_of(s_off, S, min(k, n - 1u));
+                    if (k < n && (id < s_off[sk] || id >= s_off[sk + 1])) {  // only after a failed sort
+                        atomicOr(err, RT_DEVERR_BOUNDS);
+                        id = s_off[sk];
+                    }
+                    loc[b] = id - s_off[sk];
+                    if (k < n) ids_local[k] = loc[b];
+                } else if (id >= n) {  // only after a failed sort (look-back timeout)
                     atomicOr(err, RT_DEVERR_BOUNDS);
                     id = 0;
                 }
                 idv[b] = id;
+                if (!BATCH) loc[b] = id;
             }
 #pragma unroll
             for (int b = 0; b < kGatherBatch; ++b) load_tri(tris, idv[b], n, soup_aligned, v[b]);
@@ -1339,7 +1410,7 @@ __global__ void __launch_bounds__(THREADS) k_emit_units(const uint32_t* __restri
                     s_box[c * kBoxStride + pb] = tb.lo[c];
                     s_box[(3 + c) * kBoxStride + pb] = tb.hi[c];
                 }
-                stage[3 * lane + 0] = make_float4(v[b][0], v[b][1], v[b][2], __int_as_float((int)idv[b]));
+                stage[3 * lane + 0] = make_float4(v[b][0], v[b][1], v[b][2], __int_as_float((int)loc[b]));
                 stage[3 * lane + 1] = make_float4(v[b][3], v[b][4], v[b][5], 0.0f);
                 stage[3 * lane + 2] = make_float4(v[b][6], v[b][7], v[b][8], 0.0f);
                 __syncwarp();
@@ -1359,7 +1430,8 @@ __global__ void __launch_bounds__(THREADS) k_emit_units(const uint32_t* __restri
     // heads and tails (the elements between them share their leaf's)
     const uint32_t s = tbase + (uint32_t)t * kEmitItems;
     EmitChunk e;
-    load_chunk(keys, n, s, e);
+    if constexpr (BATCH) load_chunk_b(keys, n, s, s_off, S, e);
+    else load_chunk(keys, n, s, e);
     uint32_t af = 0, ab = 0;
 #pragma unroll
     for (int q = 0; q < kEmitItems; ++q) af = rec_fwd(af, e.r[q]);
@@ -1377,22 +1449,29 @@ __global__ void __launch_bounds__(THREADS) k_emit_units(const uint32_t* __restri
     const int leaf_depth = (int)depth - 1;
     uint32_t hm[kEmitItems], hh[kEmitItems];  // capped mask | head | tail; heap index (heads, tails)
     uint32_t heads = 0u, tails = 0u;
+    uint32_t sc = BATCH ? scene_of(s_off, S, min(s, n - 1u)) : 0u;
 #pragma unroll
     for (int q = 0; q < kEmitItems; ++q) {
         const uint32_t k = s + q;
         hm[q] = 0u;
         hh[q] = 0u;
         if (k < n) {
-            const uint32_t anc = L[q] | R[q];
+            uint32_t first = 0u, last = n - 1u;
+            if (BATCH) {
+                while (k >= s_off[sc + 1]) ++sc;
+                first = s_off[sc];
+                last = s_off[sc + 1] - 1u;
+            }
+            const uint32_t anc = (L[q] | R[q]) & kMaskBits;  // without a batch's separator record
             const int dprev = e.dl[q], dcur = e.dl[q + 1];
-            const bool head = (k == 0) || (dprev >= 0 && __popc(keep_above(anc, dprev)) < leaf_depth);
-            const bool tail = (k == n - 1) || (dcur >= 0 && __popc(keep_above(anc, dcur)) < leaf_depth);
+            const bool head = (k == first) || (dprev >= 0 && __popc(keep_above(anc, dprev)) < leaf_depth);
+            const bool tail = (k == last) || (dcur >= 0 && __popc(keep_above(anc, dcur)) < leaf_depth);
             if (head || tail) {
                 // the capped mask and heap index: at heads, and at a tail that
                 // may close a leaf whose head is in an earlier thread (a tail
                 // after a head of this thread shares that head's)
                 uint32_t m = 0u;
-                if (head || heads == 0u) hh[q] = heap_index_capped(e.c[q], anc, leaf_depth, &m);
+                if (head || heads == 0u) hh[q] = heap_index_capped(e.c[q], anc, leaf_depth, &m) | (sc << kSlotBits);
                 hm[q] = m | (head ? kHeadBit : 0u) | (tail ? kTailBit : 0u);
                 if (head) heads |= 1u << q;
                 if (tail) tails |= 1u << q;
@@ -1460,8 +1539,9 @@ __global__ void __launch_bounds__(THREADS) k_emit_units(const uint32_t* __restri
         if (tail) {
             if (seen_head) {  // a leaf with head and tail in this thread
                 const int32_t count = (int32_t)k - run_pos + 1;
-                store_node(nodes, run_h, run.lo, run.hi, (count << 3) | 4 | leaf_axis_of(run_m, count, depth), run_pos);
-                leaf_of[run_pos] = run_h;
+                store_node(heap.node(run_h), run.lo, run.hi, (count << 3) | 4 | leaf_axis_of(run_m, count, depth),
+                           run_pos - heap.first(run_h));
+                leaf_of[run_pos] = heap.slot(run_h);
                 seen_head = false;  // the next element is a head
             } else {
                 first_tail_q = q;
@@ -1523,8 +1603,9 @@ __global__ void __launch_bounds__(THREADS) k_emit_units(const uint32_t* __restri
         const uint32_t j = t * kEmitItems + first_tail_q;
         if (x.head >= 0) {  // its head is in an earlier thread of this tile
             const int32_t count = (int32_t)(tbase + j) - x.head + 1;
-            store_node(nodes, ft_h, fin.lo, fin.hi, (count << 3) | 4 | leaf_axis_of(ft_m, count, depth), x.head);
-            leaf_of[x.head] = ft_h;
+            store_node(heap.node(ft_h), fin.lo, fin.hi, (count << 3) | 4 | leaf_axis_of(ft_m, count, depth),
+                       x.head - heap.first(ft_h));
+            leaf_of[x.head] = heap.slot(ft_h);
         } else {  // it began before the tile: finished in step 3
             for (int c = 0; c < 3; ++c) { s_cont_box[c] = fin.lo[c]; s_cont_box[3 + c] = fin.hi[c]; }
             s_cont_tail = tbase + j;
@@ -1538,14 +1619,15 @@ __global__ void __launch_bounds__(THREADS) k_emit_units(const uint32_t* __restri
     // the boxes of its triangles before this tile, folded in order with the rest
     if (cont) {
         const uint32_t m0 = my_units[0].y;
-        const int dpar = m0 ? __ffs(m0) - 1 : 31;  // a root leaf starts at 0
+        const int dpar = m0 ? __ffs(m0) - 1 : 31;  // a root leaf starts at its tree's first triangle
+        const int32_t first = heap.first(my_units[0].x);
         if (t == 0) s_found = 0;
         __syncthreads();
-        int32_t start = 0;
-        for (int64_t hi = (int64_t)tbase; hi > 0; hi -= THREADS) {
+        int32_t start = first;
+        for (int64_t hi = (int64_t)tbase; hi > first; hi -= THREADS) {
             const int64_t q = hi - t;  // candidate start: boundary (q - 1, q)
             bool hit = false;
-            if (q >= 1) {
+            if (q > first) {
                 const uint32_t a = __ldg(keys + q - 1), c = __ldg(keys + q);
                 hit = a != c && hb(a ^ c) >= dpar;
             }
@@ -1591,8 +1673,9 @@ __global__ void __launch_bounds__(THREADS) k_emit_units(const uint32_t* __restri
             const Box fin = box_union(before, in_tile);
             const int32_t count = (int32_t)s_cont_tail - start + 1;
             const uint2 u0 = my_units[0];
-            store_node(nodes, u0.x, fin.lo, fin.hi, (count << 3) | 4 | leaf_axis_of(u0.y, count, depth), start);
-            leaf_of[start] = u0.x;
+            store_node(heap.node(u0.x), fin.lo, fin.hi, (count << 3) | 4 | leaf_axis_of(u0.y, count, depth),
+                       start - first);
+            leaf_of[start] = heap.slot(u0.x);
         }
     }
     if (t == THREADS - 1) {  // units: cont + heads, less an open last leaf
@@ -1607,9 +1690,9 @@ __global__ void __launch_bounds__(THREADS) k_emit_units(const uint32_t* __restri
 // kMergeGroup groups (their items, each group's sorted by first element).
 // The nodes that cannot be formed here are written to `out` sorted by first
 // element, their number to *out_count.
-template <int THREADS>
+template <int THREADS, bool BATCH>
 __device__ void merge_group(const Units& u, const uint2* in_items, const uint32_t* in_counts, int fixed_count,
-                            uint32_t in_stride, uint32_t ng, uint32_t depth, rt_node* nodes, uint2* out,
+                            uint32_t in_stride, uint32_t ng, const Heap<BATCH>& heap, uint2* out,
                             uint32_t* out_count, uint32_t* err, uint32_t* inner, uint32_t* s_off, uint2* s_items,
                             int32_t* s_ipos) {
     const int t = threadIdx.x;
@@ -1635,12 +1718,12 @@ __device__ void merge_group(const Units& u, const uint2* in_items, const uint32_
         uint32_t g = 0;
         while (g + 1 < ng && s_off[g + 1] <= (uint32_t)i) ++g;
         uint2 it = __ldcg(in_items + (size_t)g * in_stride + (i - s_off[g]));
-        if (it.x < 1u || it.x >= (1u << depth)) {
+        if (heap.slot(it.x) < 1u || heap.slot(it.x) >= (1u << heap.depth)) {
             atomicOr(err, RT_DEVERR_BOUNDS);
             it = make_uint2(1u, 0u);  // a root stops the walk
         }
-        const float4 a = __ldcg(reinterpret_cast<const float4*>(nodes + it.x));
-        const float4 b = __ldcg(reinterpret_cast<const float4*>(nodes + it.x) + 1);
+        const float4 a = __ldcg(reinterpret_cast<const float4*>(heap.node(it.x)));
+        const float4 b = __ldcg(reinterpret_cast<const float4*>(heap.node(it.x)) + 1);
         u.h[i] = it.x;
         u.m[i] = it.y;
         u.lo[0 * u.cap + i] = a.x;
@@ -1649,15 +1732,15 @@ __device__ void merge_group(const Units& u, const uint2* in_items, const uint32_
         u.hi[0 * u.cap + i] = a.w;
         u.hi[1 * u.cap + i] = b.x;
         u.hi[2 * u.cap + i] = b.y;
-        u.pos[i] = __float_as_int(b.w);
-        if (i == U - 1) u.pos[U] = __float_as_int(b.w) + (__float_as_int(b.z) >> 3);
+        u.pos[i] = __float_as_int(b.w) + heap.first(it.x);
+        if (i == U - 1) u.pos[U] = u.pos[i] + (__float_as_int(b.z) >> 3);
     }
     __syncthreads();
-    unit_bottom_up<THREADS>(u, U, nodes, s_items, err, inner);
+    unit_bottom_up<THREADS, BATCH>(u, U, heap, s_items, err, inner);
     __syncthreads();
     // the items, sorted by first element (their records are stored)
     const uint32_t ni = min(*u.n_items, (uint32_t)kItemCap);
-    for (uint32_t i = t; i < ni; i += THREADS) s_ipos[i] = __ldcg(&nodes[s_items[i].x].prim_pos);
+    for (uint32_t i = t; i < ni; i += THREADS) s_ipos[i] = __ldcg(&heap.node(s_items[i].x)->prim_pos) + heap.first(s_items[i].x);
     __syncthreads();
     for (uint32_t i = t; i < ni; i += THREADS) {
         uint32_t rank = 0;
@@ -1672,13 +1755,14 @@ __device__ void merge_group(const Units& u, const uint2* in_items, const uint32_
 // per tile, most of them empty for tiles with big leaves), so that the
 // shared-memory units of eight CTAs fit an SM.  Chunk slot c's items go to
 // items + c * kItemCap, their number to counts[c].
-template <int THREADS>
+template <int THREADS, bool BATCH>
 __global__ void __launch_bounds__(THREADS) k_emit_chunks(const uint2* __restrict__ tile_units,
                                                          const uint32_t* __restrict__ tile_counts, uint32_t depth,
                                                          rt_node* nodes, uint2* items, uint32_t* counts, uint32_t* err,
-                                                         uint32_t* inner) {
+                                                         uint32_t* inner, const uint32_t* __restrict__ scene_off) {
     extern __shared__ __align__(16) uint32_t smem[];
     const Units u = units_of(smem, kChunkUnits);
+    const Heap<BATCH> heap{nodes, scene_off, depth};
     __shared__ uint32_t s_off[kMergeGroup + 1];
     __shared__ uint2 s_items[kItemCap];
     __shared__ int32_t s_ipos[kItemCap];
@@ -1691,8 +1775,8 @@ __global__ void __launch_bounds__(THREADS) k_emit_chunks(const uint2* __restrict
         if (threadIdx.x == 0) counts[c] = 0u;
         return;
     }
-    merge_group<THREADS>(u, tile_units + (size_t)tile * kUnitCap + (size_t)chunk * kChunkUnits, nullptr, cnt,
-                         (uint32_t)kChunkUnits, 1u, depth, nodes, items + (size_t)c * kItemCap, counts + c, err, inner,
+    merge_group<THREADS, BATCH>(u, tile_units + (size_t)tile * kUnitCap + (size_t)chunk * kChunkUnits, nullptr, cnt,
+                         (uint32_t)kChunkUnits, 1u, heap, items + (size_t)c * kItemCap, counts + c, err, inner,
                          s_off, s_items, s_ipos);
 }
 
@@ -1704,14 +1788,15 @@ __global__ void __launch_bounds__(THREADS) k_emit_chunks(const uint2* __restrict
 // group covers the whole tree and forms the root.  No CTA waits on another.
 // The first level's items are at out_items + g * kItemCap (counts at
 // out_counts + g), each next level's after the previous one's.
-template <int THREADS>
+template <int THREADS, bool BATCH>
 __global__ void __launch_bounds__(THREADS) k_emit_merge(const uint2* __restrict__ in_items,
                                                         const uint32_t* __restrict__ in_counts, uint32_t n_in,
                                                         uint32_t depth, rt_node* nodes, uint2* out_items,
                                                         uint32_t* out_counts, uint32_t* tickets, uint32_t* err,
-                                                        uint32_t* inner) {
+                                                        uint32_t* inner, const uint32_t* __restrict__ scene_off) {
     extern __shared__ __align__(16) uint32_t smem[];
     const Units u = units_of(smem, kUnitCap);
+    const Heap<BATCH> heap{nodes, scene_off, depth};
     __shared__ uint32_t s_off[kMergeGroup + 1];
     __shared__ uint2 s_items[kItemCap];
     __shared__ int32_t s_ipos[kItemCap];
@@ -1720,8 +1805,8 @@ __global__ void __launch_bounds__(THREADS) k_emit_merge(const uint2* __restrict_
     const int t = threadIdx.x;
     uint32_t g = blockIdx.x;
     uint32_t n_lev = (n_in + kMergeGroup - 1) / kMergeGroup;
-    merge_group<THREADS>(u, in_items + (size_t)g * kMergeGroup * kItemCap, in_counts + (size_t)g * kMergeGroup, -1,
-                         (uint32_t)kItemCap, min((uint32_t)kMergeGroup, n_in - g * kMergeGroup), depth, nodes,
+    merge_group<THREADS, BATCH>(u, in_items + (size_t)g * kMergeGroup * kItemCap, in_counts + (size_t)g * kMergeGroup, -1,
+                         (uint32_t)kItemCap, min((uint32_t)kMergeGroup, n_in - g * kMergeGroup), heap,
                          out_items + (size_t)g * kItemCap, out_counts + g, err, inner, s_off, s_items, s_ipos);
     size_t ioff = 0, coff = 0, toff = 0;
     while (n_lev > 1) {
@@ -1742,7 +1827,7 @@ __global__ void __launch_bounds__(THREADS) k_emit_merge(const uint2* __restrict_
         const size_t pcoff = coff + (size_t)parent * kMergeGroup;
         ioff += (size_t)n_lev * kItemCap;
         coff += n_lev;
-        merge_group<THREADS>(u, out_items + pioff, out_counts + pcoff, -1, (uint32_t)kItemCap, gs, depth, nodes,
+        merge_group<THREADS, BATCH>(u, out_items + pioff, out_counts + pcoff, -1, (uint32_t)kItemCap, gs, heap,
                              out_items + ioff + (size_t)parent * kItemCap, out_counts + coff + parent, err, inner,
                              s_off, s_items, s_ipos);
         toff += n_next;
@@ -1982,27 +2067,28 @@ static rt_status launch_build(rt_ctx* ctx, rt_lbvh* l, const float* d_tris, uint
     if (compact) RT_CHECK_CUDA(ctx, cudaMemsetAsync(l->inner, 0, sizeof(uint32_t) * words, st));
     // emission, pre-gather, leaf boxes and every node inside a tile in one
     // pass; the nodes above the tiles by k_emit_merge, level after level
-    RT_CHECK_CUDA(ctx, cudaFuncSetAttribute(k_emit_merge<kEmitThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    RT_CHECK_CUDA(ctx, cudaFuncSetAttribute(k_emit_merge<kEmitThreads, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             (int)kUnitSmem));
-    RT_CHECK_CUDA(ctx, cudaFuncSetAttribute(k_emit_units<kEmitThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    RT_CHECK_CUDA(ctx, cudaFuncSetAttribute(k_emit_units<kEmitThreads, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             (int)kEmitUnitsSmem));
     uint32_t* inner = compact ? l->inner : nullptr;
     // the sort's ping-pong buffers are free again: they hold the tiles' unit lists
     uint2* tile_units = reinterpret_cast<uint2*>(l->keys_alt);
     const size_t cap = l->emit_tiles_cap;
     uint32_t* tile_counts = l->item_counts + 6 * cap;
-    launch_pdl(k_emit_units<kEmitThreads>, emit_tiles, kEmitThreads, kEmitUnitsSmem, st, (const uint32_t*)l->keys,
+    launch_pdl(k_emit_units<kEmitThreads, false>, emit_tiles, kEmitThreads, kEmitUnitsSmem, st, (const uint32_t*)l->keys,
                (const uint32_t*)l->ids, d_tris, n, l->depth, (const uint32_t*)l->scan, l->nodes, l->sorted_tris,
-               tile_units, tile_counts, ctx->d_err, l->leaf_of);
+               tile_units, tile_counts, ctx->d_err, l->leaf_of, (const uint32_t*)nullptr, 0u, (uint32_t*)nullptr);
     RT_CHECK_LAUNCH(ctx, "k_emit_units");
     const uint32_t chunks = emit_tiles * kTileChunks;
-    launch_pdl(k_emit_chunks<kEmitThreads>, chunks, kEmitThreads, kChunkSmem, st, (const uint2*)tile_units,
-               (const uint32_t*)tile_counts, l->depth, l->nodes, l->items, l->item_counts, ctx->d_err, inner);
+    launch_pdl(k_emit_chunks<kEmitThreads, false>, chunks, kEmitThreads, kChunkSmem, st, (const uint2*)tile_units,
+               (const uint32_t*)tile_counts, l->depth, l->nodes, l->items, l->item_counts, ctx->d_err, inner,
+               (const uint32_t*)nullptr);
     RT_CHECK_LAUNCH(ctx, "k_emit_chunks");
-    launch_pdl(k_emit_merge<kEmitThreads>, ceil_div(chunks, kMergeGroup), kEmitThreads, kUnitSmem, st,
+    launch_pdl(k_emit_merge<kEmitThreads, false>, ceil_div(chunks, kMergeGroup), kEmitThreads, kUnitSmem, st,
                (const uint2*)l->items, (const uint32_t*)l->item_counts, chunks, l->depth, l->nodes,
                l->items + (size_t)chunks * kItemCap, l->item_counts + chunks, l->item_counts + 7 * cap, ctx->d_err,
-               inner);
+               inner, (const uint32_t*)nullptr);
     RT_CHECK_LAUNCH(ctx, "k_emit_merge");
     if (compact) {
         k_inner_rank<<<1, kRankThreads, 0, st>>>(l->inner, words, l->inner_rank);
@@ -2386,7 +2472,6 @@ extern "C" rt_status rt_radix_sort_stall_test(rt_ctx* ctx, const uint32_t* d_key
 namespace {
 
 constexpr uint32_t kChunkTris = 4096;
-constexpr int kSepBit = 31;
 
 __device__ __forceinline__ void atomic_min_f(float* a, float v) {
     v = fadd(v, 0.0f);  // -0 -> +0
@@ -2412,7 +2497,7 @@ __global__ void kb_init(float* sbounds, uint32_t S, const uint32_t* __restrict__
         hist[i] = (i >= 4 * 256 && s < S) ? tri_off[s + 1] - tri_off[s] : 0u;  // pass 4: scene sizes
     }
     for (uint32_t i = gtid; i < lb_words; i += gs) lookback[i] = 0u;
-    if (gtid < 6) counters[gtid] = 0u;
+    if (gtid < 6 || gtid == 7) counters[gtid] = 0u;  // [7]: whether the trace records are those of these trees
     if (gtid == 6) {
         const uint32_t e = counters[6] + 1u;
         counters[6] = e ? e : 1u;
@@ -2510,44 +2595,12 @@ __global__ void __launch_bounds__(256) kb_morton_hist(const float* __restrict__ 
     }
 }
 
-// Boundary deltas of a thread's chunk with a separator record at each
-// scene boundary (off: S + 1 scene offsets in shared memory).
-__device__ __forceinline__ void load_chunk_b(const uint32_t* __restrict__ keys, uint32_t n, uint32_t s,
-                                             const uint32_t* off, uint32_t S, EmitChunk& e) {
-    const uint32_t prev = (s >= 1 && s - 1 < n) ? __ldg(keys + s - 1) : 0u;
-#pragma unroll
-    for (int q = 0; q <= kEmitItems; ++q) e.c[q] = (s + q < n) ? __ldg(keys + s + q) : 0u;
-    uint32_t sc = scene_of(off, S, s < n ? s : n - 1);
-    e.dl[0] = (s >= 1 && s < n) ? (s == off[sc] ? kSepBit : delta_of(prev, e.c[0])) : -1;
-    uint32_t nb = off[sc + 1];
-#pragma unroll
-    for (int q = 0; q < kEmitItems; ++q) {
-        const uint32_t i = s + q;
-        int d = -1;
-        if (i + 1 < n) {
-            if (i + 1 == nb) {
-                d = kSepBit;
-                ++sc;
-                nb = off[sc + 1];
-            } else {
-                d = delta_of(e.c[q], e.c[q + 1]);
-            }
-        }
-        e.dl[q + 1] = d;
-        e.r[q] = (d >= 0) ? (1u << d) : 0u;
-    }
-}
-
 __global__ void __launch_bounds__(kEmitThreads) kb_emit_tiles(const uint32_t* __restrict__ keys, uint32_t n,
                                                               const uint32_t* __restrict__ tri_off, uint32_t S,
-                                                              uint32_t* scan, uint32_t* arrive, uint32_t arrive_words,
-                                                              const uint32_t* epoch_word) {
+                                                              uint32_t* scan) {
     __shared__ uint32_t s_f[8], s_b[8];
     __shared__ uint32_t s_off[kMaxBatchScenes + 1];
     for (uint32_t q = threadIdx.x; q <= S; q += blockDim.x) s_off[q] = tri_off[q];
-    if (*epoch_word == 1u)
-        for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < arrive_words; i += gridDim.x * blockDim.x)
-            arrive[i] = 0u;
     __syncthreads();
     const uint32_t s = blockIdx.x * kEmitTile + threadIdx.x * kEmitItems;
     EmitChunk e;
@@ -2571,125 +2624,6 @@ __global__ void __launch_bounds__(kEmitThreads) kb_emit_tiles(const uint32_t* __
     }
 }
 
-__global__ void __launch_bounds__(kEmitThreads) kb_emit_leaves(
-    const uint32_t* __restrict__ keys, const uint32_t* __restrict__ ids, const float* __restrict__ tris, uint32_t n,
-    const uint32_t* __restrict__ tri_off, uint32_t S, uint32_t depth, const uint32_t* __restrict__ scan,
-    rt_node* nodes, float4* __restrict__ sorted_tris, uint32_t* __restrict__ ids_local, uint32_t* leaf_list,
-    uint32_t* leaf_count, uint32_t* err) {
-    __shared__ uint32_t s_f[8], s_b[8];
-    __shared__ uint32_t s_off[kMaxBatchScenes + 1];
-    for (uint32_t q = threadIdx.x; q <= S; q += blockDim.x) s_off[q] = tri_off[q];
-    __syncthreads();
-    const uint32_t s = blockIdx.x * kEmitTile + threadIdx.x * kEmitItems;
-    EmitChunk e;
-    load_chunk_b(keys, n, s, s_off, S, e);
-    uint32_t af = 0, ab = 0;
-#pragma unroll
-    for (int q = 0; q < kEmitItems; ++q) af = rec_fwd(af, e.r[q]);
-#pragma unroll
-    for (int q = kEmitItems - 1; q >= 0; --q) ab = rec_bwd(e.r[q], ab);
-    uint32_t pre, suf;
-    block_scan_records(af, ab, &pre, &suf, s_f, s_b);
-    uint32_t L[kEmitItems + 1], R[kEmitItems + 1];
-    L[0] = rec_fwd(scan[4 * blockIdx.x + 2], pre);
-    R[kEmitItems] = rec_bwd(suf, scan[4 * blockIdx.x + 3]);
-#pragma unroll
-    for (int q = 0; q < kEmitItems; ++q) L[q + 1] = rec_fwd(L[q], e.r[q]);
-#pragma unroll
-    for (int q = kEmitItems - 1; q >= 0; --q) R[q] = rec_bwd(e.r[q], R[q + 1]);
-
-    const int leaf_depth = (int)depth - 1;
-    const int lane = threadIdx.x & 31;
-    uint32_t sc = scene_of(s_off, S, s < n ? s : n - 1);
-#pragma unroll
-    for (int q = 0; q < kEmitItems; ++q) {
-        const uint32_t k = s + q;
-        const bool valid = k < n;
-        bool head = false;
-        uint32_t h = 0;
-        if (valid) {
-            while (k >= s_off[sc + 1]) ++sc;
-            const uint32_t first = s_off[sc], last = s_off[sc + 1] - 1;
-            const uint32_t anc = (L[q] | R[q]) & 0x3fffffffu;  // drop the separator record
-            const uint32_t code = e.c[q];
-            int dep = __popc(anc);
-            uint32_t m = anc;
-            while (dep > leaf_depth) { m &= m - 1u; --dep; }
-            h = 1u;
-            while (m) {
-                const int b = hb(m);
-                h = (h << 1) | ((code >> b) & 1u);
-                m ^= 1u << b;
-            }
-            const int dprev = e.dl[q], dcur = e.dl[q + 1];
-            head = (k == first) || (dprev >= 0 && __popc(keep_above(anc, dprev)) < leaf_depth);
-            const bool tail = (k == last) || (dcur >= 0 && __popc(keep_above(anc, dcur)) < leaf_depth);
-            rt_node* tree = nodes + ((size_t)sc << depth);
-            if (head) tree[h].prim_pos = (int32_t)(k - first);
-            if (tail) tree[h].prim_count = (int32_t)(k - first);
-            h |= sc << 23;  // leaf entry: scene and heap slot
-        }
-        const uint32_t hm = __ballot_sync(kFull, head);
-        uint32_t basei = 0;
-        if (lane == 0 && hm) basei = atomicAdd(leaf_count, (uint32_t)__popc(hm));
-        basei = __shfl_sync(kFull, basei, 0);
-        if (head) leaf_list[basei + __popc(hm & lanemask_lt())] = h;
-    }
-    const uint32_t tbase = blockIdx.x * kEmitTile;
-#pragma unroll 2
-    for (int q = 0; q < kEmitItems; ++q) {
-        const uint32_t k = tbase + q * kEmitThreads + threadIdx.x;
-        if (k < n) {
-            uint32_t id = __ldg(ids + k);
-            const uint32_t sk = scene_of(s_off, S, k);
-            if (id < s_off[sk] || id >= s_off[sk + 1]) {  // only after a failed sort (look-back timeout)
-                atomicOr(err, RT_DEVERR_BOUNDS);
-                id = s_off[sk];
-            }
-            const uint32_t local = id - s_off[sk];
-            const float* tp = tris + 9 * (size_t)id;
-            float v[9];
-#pragma unroll
-            for (int c = 0; c < 9; ++c) v[c] = __ldg(tp + c);
-            sorted_tris[3 * (size_t)k + 0] = make_float4(v[0], v[1], v[2], __int_as_float((int)local));
-            sorted_tris[3 * (size_t)k + 1] = make_float4(v[3], v[4], v[5], 0.0f);
-            sorted_tris[3 * (size_t)k + 2] = make_float4(v[6], v[7], v[8], 0.0f);
-            ids_local[k] = local;
-        }
-    }
-}
-
-__global__ void __launch_bounds__(256) kb_emit_refit(const uint32_t* __restrict__ keys, const float4* sorted_tris,
-                                                     const uint32_t* __restrict__ tri_off, uint32_t depth,
-                                                     rt_node* nodes, const uint32_t* __restrict__ leaf_list,
-                                                     const uint32_t* leaf_count, uint32_t n, uint32_t* arrive,
-                                                     const uint32_t* epoch_word, uint32_t* err) {
-    const uint32_t nleaves = min(*leaf_count, n);
-    const uint32_t epoch = *epoch_word;
-    const uint32_t lane = threadIdx.x & 31;
-    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t base = warp * 32; base < nleaves; base += nwarps * 32) {
-        const uint32_t li = base + lane;
-        uint32_t sc = 0, h = 0, toff = 0, ns = 0;
-        int32_t pos = 0, end = -1;
-        bool ok = false;
-        if (li < nleaves) {
-            const uint32_t e = leaf_list[li];
-            sc = e >> 23;
-            h = e & ((1u << 23) - 1u);
-            toff = __ldg(tri_off + sc);
-            ns = __ldg(tri_off + sc + 1) - toff;
-            ok = leaf_range(h, nodes + ((size_t)sc << depth), ns, depth, &pos, &end);
-            if (!ok) atomicOr(err, RT_DEVERR_BOUNDS);
-        }
-        float mn[3], mx[3];
-        leaf_boxes((int64_t)toff + pos, ok ? end - pos + 1 : 0, sorted_tris, mn, mx);
-        if (ok)
-            refit_walk(h, pos, end, mn, mx, keys + toff, ns, depth, nodes + ((size_t)sc << depth),
-                       arrive + ((size_t)sc << (depth - 1)), epoch, err);
-    }
-}
-
 }  // namespace
 
 extern "C" rt_status rt_batch_destroy(rt_batch* b) {
@@ -2703,9 +2637,9 @@ extern "C" rt_status rt_batch_destroy(rt_batch* b) {
 }
 
 void free_batch(rt_batch* b) {
-    void* ptrs[] = {b->tri_off, b->node_off, b->chunks, b->nodes, b->keys, b->ids, b->keys_alt, b->ids_alt,
+    void* ptrs[] = {b->tri_off, b->node_off, b->chunks, b->nodes, b->keys, nullptr, b->keys_alt, b->ids_alt,
                     b->ids_local, b->sorted_tris, b->sbounds, b->counters, b->hist, b->lookback, b->scan,
-                    b->leaf_list, b->arrive, b->cams, b->lights, b->s_lists, b->s_rays};
+                    b->leaf_of, b->tnodes, b->items, b->item_counts, b->cams, b->lights, b->s_lists, b->s_rays};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     delete b;
@@ -2755,8 +2689,10 @@ extern "C" rt_status rt_batch_create(rt_ctx* ctx, uint32_t n_scenes, const uint3
     alloc((void**)&b->node_off, 4 * (n_scenes + 1));
     alloc((void**)&b->chunks, 4 * chunks.size());
     alloc((void**)&b->nodes, sizeof(rt_node) * num_nodes);
-    alloc((void**)&b->keys, 4 * n);
-    alloc((void**)&b->ids, 4 * n);
+    // one block: after the sort (whose result is in the alternate buffers) it
+    // holds the emission's per-tile unit lists (8 bytes per element)
+    alloc((void**)&b->keys, 8 * n);
+    if (e == cudaSuccess) b->ids = b->keys + n;
     alloc((void**)&b->keys_alt, 4 * n);
     alloc((void**)&b->ids_alt, 4 * n);
     alloc((void**)&b->ids_local, 4 * n);
@@ -2766,16 +2702,27 @@ extern "C" rt_status rt_batch_create(rt_ctx* ctx, uint32_t n_scenes, const uint3
     alloc((void**)&b->hist, sizeof(uint32_t) * 5 * 256);
     alloc((void**)&b->lookback, sizeof(uint32_t) * 5 * 256 * (size_t)sort_tiles);
     alloc((void**)&b->scan, sizeof(uint32_t) * 4 * (size_t)emit_tiles);
-    alloc((void**)&b->leaf_list, 4 * n);
-    alloc((void**)&b->arrive, sizeof(uint32_t) * (num_nodes >> 1));
+    alloc((void**)&b->leaf_of, 4 * n);
+    // items and counts of the merge levels, as a single tree's (rt_lbvh_create)
+    alloc((void**)&b->items, sizeof(uint2) * 6 * (size_t)kItemCap * emit_tiles);
+    alloc((void**)&b->item_counts, sizeof(uint32_t) * 8 * (size_t)emit_tiles);
     alloc((void**)&b->cams, sizeof(rt_camera) * n_scenes);
     alloc((void**)&b->lights, sizeof(float) * 3 * n_scenes);
     if (e == cudaSuccess) e = cudaMemcpy(b->tri_off, b->h_tri_off.data(), 4 * (n_scenes + 1), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(b->node_off, node_off.data(), 4 * (n_scenes + 1), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(b->chunks, chunks.data(), 4 * chunks.size(), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemset(b->counters, 0, sizeof(uint32_t) * 8);
-    if (e == cudaSuccess) e = cudaMemset(b->arrive, 0, sizeof(uint32_t) * (num_nodes >> 1));
+    if (e == cudaSuccess) e = cudaMemset(b->item_counts, 0, sizeof(uint32_t) * 8 * (size_t)emit_tiles);
     if (e == cudaSuccess) e = cudaMemset(b->nodes, 0, sizeof(rt_node) * num_nodes);
+    // the trace records, where there is room beside what such a batch needs
+    // to be traced (half of what is free)
+    size_t free_bytes = 0, all_bytes = 0;
+    const size_t rec_bytes = sizeof(TraceNode) * std::max<size_t>(n_scenes, num_nodes >> 1);
+    if (e == cudaSuccess && cudaMemGetInfo(&free_bytes, &all_bytes) == cudaSuccess && rec_bytes <= free_bytes / 2 &&
+        cudaMalloc((void**)&b->tnodes, rec_bytes) != cudaSuccess) {
+        cudaGetLastError();
+        b->tnodes = nullptr;
+    }
     if (e != cudaSuccess) {
         rt_batch_destroy(b);
         return rt_fail(ctx, RT_ERR_CUDA, "rt_batch_create: allocation failed: %s", cudaGetErrorString(e));
@@ -2815,24 +2762,33 @@ extern "C" rt_status rt_batch_build(rt_ctx* ctx, rt_batch* b, const float* d_tri
     }
     b->res_keys = kin;  // five passes: the sorted pairs are in the alternate buffers
     b->res_ids = iin;
-    kb_emit_tiles<<<emit_tiles, kEmitThreads, 0, st>>>(kin, n, b->tri_off, S, b->scan, b->arrive, num_nodes >> 1,
-                                                       b->counters + 6);
+    kb_emit_tiles<<<emit_tiles, kEmitThreads, 0, st>>>(kin, n, b->tri_off, S, b->scan);
     RT_CHECK_LAUNCH(ctx, "kb_emit_tiles");
-    k_emit_prefix<<<1, kPrefixThreads, 0, st>>>(b->scan, emit_tiles);
+    launch_pdl(k_emit_prefix, 1, kPrefixThreads, 0, st, b->scan, emit_tiles);
     RT_CHECK_LAUNCH(ctx, "k_emit_prefix");
-    kb_emit_leaves<<<emit_tiles, kEmitThreads, 0, st>>>(kin, iin, d_tris, n, b->tri_off, S, b->depth, b->scan, b->nodes,
-                                                        b->sorted_tris, b->ids_local, b->leaf_list, b->counters + 5,
-                                                        ctx->d_err);
-    RT_CHECK_LAUNCH(ctx, "kb_emit_leaves");
-    // one thread per leaf at most (no persistent cap), in blocks of two warps:
-    // a warp's time is its longest climb, and fresh warps then take the SM
-    // slots of finished ones instead of each thread walking ~40 leaves in
-    // turn (256 random-soup scenes, 11.5 M triangles: 3.89 -> 3.31 ms a
-    // batched build with 256-thread blocks, 3.15 ms with 64)
-    const uint32_t rblocks = std::max(1u, ceil_div(n, 64));
-    kb_emit_refit<<<rblocks, 64, 0, st>>>(kin, b->sorted_tris, b->tri_off, b->depth, b->nodes, b->leaf_list,
-                                           b->counters + 5, n, b->arrive, b->counters + 6, ctx->d_err);
-    RT_CHECK_LAUNCH(ctx, "kb_emit_refit");
+    // the emission of a single tree over the concatenated scenes (256 random-soup
+    // scenes, 11.5 M triangles: 1.4 ms; leaf boxes and an atomic walk with one
+    // dependent global exchange per node and level took 2.3 ms)
+    RT_CHECK_CUDA(ctx, cudaFuncSetAttribute(k_emit_merge<kEmitThreads, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            (int)kUnitSmem));
+    RT_CHECK_CUDA(ctx, cudaFuncSetAttribute(k_emit_units<kEmitThreads, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            (int)kEmitUnitsSmem));
+    uint2* tile_units = reinterpret_cast<uint2*>(b->keys);
+    uint32_t* tile_counts = b->item_counts + 6 * (size_t)emit_tiles;
+    launch_pdl(k_emit_units<kEmitThreads, true>, emit_tiles, kEmitThreads, kEmitUnitsSmem, st, (const uint32_t*)kin,
+               (const uint32_t*)iin, d_tris, n, b->depth, (const uint32_t*)b->scan, b->nodes, b->sorted_tris, tile_units,
+               tile_counts, ctx->d_err, b->leaf_of, (const uint32_t*)b->tri_off, S, b->ids_local);
+    RT_CHECK_LAUNCH(ctx, "k_emit_units");
+    const uint32_t chunks = emit_tiles * kTileChunks;
+    launch_pdl(k_emit_chunks<kEmitThreads, true>, chunks, kEmitThreads, kChunkSmem, st, (const uint2*)tile_units,
+               (const uint32_t*)tile_counts, b->depth, b->nodes, b->items, b->item_counts, ctx->d_err, (uint32_t*)nullptr,
+               (const uint32_t*)b->tri_off);
+    RT_CHECK_LAUNCH(ctx, "k_emit_chunks");
+    launch_pdl(k_emit_merge<kEmitThreads, true>, ceil_div(chunks, kMergeGroup), kEmitThreads, kUnitSmem, st,
+               (const uint2*)b->items, (const uint32_t*)b->item_counts, chunks, b->depth, b->nodes,
+               b->items + (size_t)chunks * kItemCap, b->item_counts + chunks, b->item_counts + 7 * (size_t)emit_tiles,
+               ctx->d_err, (uint32_t*)nullptr, (const uint32_t*)b->tri_off);
+    RT_CHECK_LAUNCH(ctx, "k_emit_merge");
     b->src_tris = d_tris;
     b->built = true;
     return RT_OK;

@@ -120,6 +120,7 @@ constexpr uint32_t kMaxTris = (1u << 29);
 // default budget of box + triangle tests a lane spends on one ray before it
 // hands the ray to the warp-per-ray kernel.
 constexpr uint32_t kSpillCap = 1u << 20;
+constexpr int kDoubtCount = 36;  // ctx->d_words: length of the any-hit rays' second list, its claim counter
 constexpr uint32_t kDefaultHeavyTeam = 2u;
 constexpr uint32_t kDefaultTraceBudget = 384;
 constexpr uint32_t kDefaultShadeBudget = 768;
@@ -137,7 +138,7 @@ struct rt_ctx {
     uint32_t* d_work = nullptr;  // work counters of the persistent kernels (d_words[16..])
     uint32_t* d_spill_count = nullptr;  // heavy-ray list length (d_words[32]; shading rays: [33], claims [34])
     uint32_t* d_words = nullptr; // 64 device words
-    uint32_t* d_spill = nullptr; // heavy-ray list, kSpillCap entries
+    uint32_t* d_spill = nullptr; // heavy-ray list, kSpillCap entries; then the any-hit rays' second list, as many
     float* d_terms = nullptr;    // radiance terms of a path-traced image (rt_pathtrace.cu), grown on demand
     size_t terms_bytes = 0;
     uint32_t* d_order = nullptr; // heavy-first tile order, kOrderKinds x kOrderWords (parity / counts: d_words[40..])
@@ -229,8 +230,10 @@ struct rt_batch {
     uint32_t* hist = nullptr;       // 5 x 256
     uint32_t* lookback = nullptr;   // 5 x 256 x sort tiles
     uint32_t* scan = nullptr;       // 4 per emission tile
-    uint32_t* leaf_list = nullptr;  // total
-    uint32_t* arrive = nullptr;     // S << (depth - 1)
+    TraceNode* tnodes = nullptr;    // S << (depth - 1) trace records (nullptr: no memory for them, the walks read the heaps)
+    uint32_t* leaf_of = nullptr;    // total: heap slot of the leaf whose first triangle is at a sorted position
+    uint2* items = nullptr;         // emission items and counts (rt_lbvh)
+    uint32_t* item_counts = nullptr;
     const float* src_tris = nullptr;
     bool built = false;
     // views of the batched trace (rt_batch_set_views)

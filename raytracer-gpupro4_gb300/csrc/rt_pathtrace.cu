@@ -111,10 +111,10 @@ struct PathCounts {
 // tiles, lanes of one grab taking consecutive pixels.
 constexpr int kPtShadeLanes = 10;
 constexpr int kPtSteps = 8;  // expansions between two leaf phases (5: 26.1 ms, 7: 23.5, 8: 23.5, 10: 24.1)
-// Blocks per SM: 64 registers and eight blocks where the paths fill the GPU
-// (23.5 ms; seven: 25.5), 128 and four where they don't (0.72 ms a 256 x 256
-// image; eight: 0.76).
-constexpr int kPtBlocks = 8, kPtSmallBlocks = 4;
+// Blocks per SM: 56 registers and nine blocks where the paths fill the GPU
+// (23.9 ms; eight: 24.5, seven: 26.1), 128 and four where they don't (0.70 ms a
+// 256 x 256 image; eight: 0.76).
+constexpr int kPtBlocks = 9, kPtSmallBlocks = 4;
 
 struct PathLane {
     bool live = false;           // holds a path

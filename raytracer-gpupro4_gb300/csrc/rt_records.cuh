@@ -76,44 +76,59 @@ struct Records {
     const rt_node* nodes;
     uint32_t num_nodes;
     TraceNode* tnodes;
+    uint32_t scene_depth;    // a batch's heap depth (a leaf is named by scene << 23 | heap slot); 0: one tree
 };
 
 inline Records records_of(const rt_lbvh* l) {
     return Records{l->counters + 7, reinterpret_cast<const uint2*>(l->keys_alt),
-                   l->item_counts + 6 * (size_t)l->emit_tiles_cap, l->rec_tiles, l->nodes, l->num_nodes, l->tnodes};
+                   l->item_counts + 6 * (size_t)l->emit_tiles_cap, l->rec_tiles, l->nodes, l->num_nodes, l->tnodes, 0u};
+}
+inline Records records_of(const rt_batch* b) {
+    const uint32_t tiles = (b->total + kEmitTile - 1) / kEmitTile;
+    return Records{b->counters + 7, reinterpret_cast<const uint2*>(b->keys), b->item_counts + 6 * (size_t)tiles,
+                   b->tnodes ? tiles : 0u, b->nodes, 1u << b->depth, b->tnodes, b->depth};
 }
 
 // The records of one tile's leaves (a block).  There is one internal node per
-// two neighbouring leaves, their lowest common ancestor: a thread takes a
-// leaf and the one before it.
+// two neighbouring leaves of a tree, their lowest common ancestor: a thread
+// takes a leaf and the one before it.
 __device__ __forceinline__ void make_records(const Records& R, uint32_t tile) {
-    __shared__ uint32_t s_prev;  // the last leaf of the tiles before
-    if (*R.valid) return;        // uniform
+    if (*R.valid) return;  // uniform
     const uint32_t cnt = min(__ldg(R.counts + tile), (uint32_t)kEmitTile);
-    if (cnt == 0u) return;
-    const rt_node root = R.nodes[1];
-    const float4 g = trace_grid(root.min, root.max);
-    if (threadIdx.x == 0) {
-        uint32_t h = 0u;
-        for (uint32_t q = tile; q-- > 0u && h == 0u;) {
-            const uint32_t c = min(__ldg(R.counts + q), (uint32_t)kEmitTile);
-            if (c) h = __ldg(&R.units[(size_t)q * kEmitTile + c - 1].x);
-        }
-        s_prev = h;
-        if (h == 0u)  // the tree's first leaf
-            store_trace_grid(R.tnodes, g, (root.prim_count & 4) ? leaf_word(1u, (uint32_t)root.prim_pos,
-                                                                            (uint32_t)(root.prim_count >> 3)) : 0u);
-    }
-    __syncthreads();
+    const bool batch = R.scene_depth != 0u;
     for (uint32_t i = threadIdx.x; i < cnt; i += blockDim.x) {
-        const uint32_t b = __ldg(&R.units[(size_t)tile * kEmitTile + i].x);
-        const uint32_t a = i ? __ldg(&R.units[(size_t)tile * kEmitTile + i - 1].x) : s_prev;
-        if (a == 0u || b == 0u) continue;
+        uint32_t b = __ldg(&R.units[(size_t)tile * kEmitTile + i].x), a = 0u;
+        if (i) {
+            a = __ldg(&R.units[(size_t)tile * kEmitTile + i - 1].x);
+        } else {  // the last leaf of the tiles before
+            for (uint32_t q = tile; q-- > 0u && a == 0u;) {
+                const uint32_t c = min(__ldg(R.counts + q), (uint32_t)kEmitTile);
+                if (c) a = __ldg(&R.units[(size_t)q * kEmitTile + c - 1].x);
+            }
+        }
+        const rt_node* nodes = R.nodes;
+        TraceNode* tnodes = R.tnodes;
+        if (batch) {
+            const uint32_t sc = b >> 23;
+            nodes += (size_t)sc << R.scene_depth;
+            tnodes += (size_t)sc << (R.scene_depth - 1u);
+            a = (a >> 23) == sc ? a & 0x7fffffu : 0u;
+            b &= 0x7fffffu;
+        }
+        const float4* p = reinterpret_cast<const float4*>(nodes + 1);
+        const float4 r0 = __ldg(p), r1 = __ldg(p + 1);
+        const float mn[3] = {r0.x, r0.y, r0.z}, mx[3] = {r0.w, r1.x, r1.y};
+        const float4 g = trace_grid(mn, mx);
+        if (a == 0u) {  // the tree's first leaf
+            const int pc = __float_as_int(r1.z);
+            store_trace_grid(tnodes, g, (pc & 4) ? leaf_word(1u, (uint32_t)__float_as_int(r1.w), (uint32_t)(pc >> 3)) : 0u);
+            continue;
+        }
         const int da = 31 - __clz(a), db = 31 - __clz(b), dm = min(da, db);
         const uint32_t x = (a >> (da - dm)) ^ (b >> (db - dm));
-        if (x == 0u) continue;  // only after a failed sort
+        if (b == 0u || x == 0u) continue;  // only after a failed sort
         const uint32_t h = (a >> (da - dm)) >> (32 - __clz(x));
-        if (h != 0u && 2u * h + 1u < R.num_nodes) trace_node_of(h, R.nodes, R.num_nodes, R.tnodes, g);
+        if (h != 0u && 2u * h + 1u < R.num_nodes) trace_node_of(h, nodes, R.num_nodes, tnodes, g);
     }
 }
 

@@ -150,6 +150,60 @@ __global__ void __launch_bounds__(kTraceThreads, 7) k_trace_primary(TreeRef tr, 
 }
 
 
+// Primary rays over the trace records (Walk), an 8 x 4 tile per warp at a time:
+// neighbouring rays visit the same leaves, so handing out pixels one by one to the
+// lanes that are done (as the shading rays are) was slower.
+constexpr int kPrimSteps = 3;  // 3: 1,415 us a frame of 2.1 M triangles, 4: 1,423, 8: 1,413 (65 k triangles, 512 x 512: 312, 309, 330)
+
+__global__ void __launch_bounds__(kTraceThreads, 8) k_walk_primary(TreeRef tr, rt_camera cam, rt_hit* __restrict__ hits,
+                                                                        uint32_t* __restrict__ leaves, uint32_t* work,
+                                                                        uint32_t num_tiles, Spill spill,
+                                                                        uint32_t* __restrict__ list, TileOrder ord,
+                                                                        ShadeLists sl) {
+    constexpr uint32_t kFull = 0xffffffffu;
+    grid_dep_wait();
+    mark_records(tr);
+    const uint32_t wbuf = *ord.parity, rbuf = wbuf ^ 1u, heavy = min(ord.counts[rbuf], ord.cap);
+    Walk w;
+    w.clear();
+    uint2 stack[kStackSize];
+    bool budgeted = spill.count != nullptr;
+    for (uint32_t tile = next_ordered_tile(work, ord, rbuf, heavy, num_tiles); tile < num_tiles;
+         tile = next_ordered_tile(work, ord, rbuf, heavy, num_tiles)) {
+        uint32_t i, j;
+        const bool valid = tile_pixel(tile, threadIdx.x & 31, cam.width, cam.height, &i, &j);
+        if (!valid) i = j = 0;  // lanes past the image edge only help the warp
+        int slot = -1;
+        w.tests = 0u;
+        w.start(valid, make_ray(mk3(cam.eye[0], cam.eye[1], cam.eye[2]), primary_dir(cam, i, j), 1e16f, -1), tr, 1u, stack);
+        while (__any_sync(kFull, w.have)) {
+            w.round(tr, kPrimSteps, stack);
+            if (w.have && budgeted && w.tests > spill.budget) {
+                const uint32_t e = atomicAdd(spill.count, 1u);
+                if (e < spill.cap) {
+                    slot = (int)e;
+                    w.stop();
+                } else {
+                    budgeted = false;  // list full: finish here
+                }
+            }
+        }
+        const size_t p = (size_t)j * cam.width + i;
+        const uint32_t leaf = tr.compact ? 1u : w.b.leaf;
+        const Hit h = w.hit();
+        if (valid) {
+            store_hit(hits + p, h);  // of a handed-over ray: the closest hit so far
+            if (slot >= 0) spill_record(list, slot, kHeavyPrimary, p);
+            else if (leaves) leaves[p] = leaf;
+        }
+        if (sl.lists) {  // uniform; a handed-over pixel is set up by the warp-per-ray pass
+            const int4 ph = make_int4(h.id, __float_as_int(h.u), __float_as_int(h.v), __float_as_int(h.t));
+            shade_setup_pixel(sl, cam, ph, valid && slot < 0, i, j, p, leaf);
+        }
+        record_tile_cost(ord, wbuf, tile, w.tests);
+    }
+}
+
 // Shadow (any hit) and mirror (closest hit) rays of one pixel whose primary
 // hit is ph.  Called by all lanes of the warp together (valid == false for
 // lanes past the image edge); rays of pixels whose primary ray missed, or
@@ -256,154 +310,6 @@ __global__ void __launch_bounds__(256) k_shade_setup(const float* __restrict__ s
     }
 }
 
-// k_trace_shade keeps every lane busy: a lane whose ray has finished takes
-// the next list entry as soon as kRefillLanes lanes of its warp are idle
-// (the newcomers take consecutive entries, so they stay neighbours), instead
-// of idling until the warp's slowest ray is done (dynamic ray fetch, Aila
-// and Laine 2009).  Each ray's walk and result are those of a whole-warp
-// trace_ray: the same start, the same descent, the same leaf phase.
-//
-// A lane expands at most kShadeSteps internal nodes per round before the
-// warp's leaf phase, so that lanes holding a leaf do not wait out one lane's
-// long descent (shading rays start on the surface, where descents vary
-// most).  At 2.1 M triangles / 1080p, with at most 72 registers (7 blocks per
-// SM), 4 steps and a refill at 24 idle lanes were the fastest pair of those
-// tried (steps 1-16, refill at 8-32 idle lanes): 9 % faster than an unbounded
-// descent with a refill at 16.  The primary walk is fastest unbounded.
-constexpr int kRefillLanes = 24;
-constexpr int kShadeSteps = 4;
-
-// The scenes of a batch as seen by k_trace_shade (nodes == nullptr: one tree):
-// a listed pixel g belongs to scene g / px, whose heap is at nodes + (s <<
-// depth) and whose triangles are [tri_off[s], tri_off[s + 1]) of the batch's
-// sorted-triangle array.
-struct BatchTrees {
-    const rt_node* nodes;
-    const uint32_t* tri_off;
-    uint32_t depth, px;
-};
-
-template <bool BATCH>
-__global__ void __launch_bounds__(kTraceThreads, 7) k_trace_shade(
-    TreeRef tr0, const float* __restrict__ soup, rt_camera cam, float lx, float ly, float lz,
-    const rt_hit* __restrict__ prim, const uint32_t* __restrict__ prim_leaves, uint8_t* __restrict__ vis,
-    rt_hit* __restrict__ mirror, uint32_t* __restrict__ mirror_leaves, const uint32_t* __restrict__ lists,
-    uint32_t cap, const uint32_t* counts, const float4* __restrict__ rays, const uint32_t* __restrict__ starts,
-    uint32_t* work, Spill spill, uint32_t* __restrict__ list, BatchTrees bt) {
-    grid_dep_wait();
-    TreeRef tr = tr0;  // per lane: a batch's lanes may walk different scenes
-    constexpr uint32_t kFull = 0xffffffffu;
-    const uint32_t ns = min(counts[0], cap), nm = min(counts[1], cap), total = ns + nm;
-    const int lane = threadIdx.x & 31;
-    const uint32_t lt = (1u << lane) - 1u;
-    uint32_t stack_node[kStackSize];
-    float stack_t0[kStackSize];
-    RayState r = make_ray(mk3(0.f, 0.f, 0.f), mk3(0.f, 0.f, 1.f), 1.0f, -1);
-    Best b;
-    b.key = 0;
-    b.t = 0.f;
-    b.u = b.v = -1.f;
-    b.id = -1;
-    b.leaf = 1u;
-    uint64_t bound = 0;
-    NodeBox cur;
-    cur.a = make_float4(0.f, 0.f, 0.f, 0.f);
-    cur.b = cur.a;
-    uint32_t sp = 0, node = 1, nbox = 0, ntri = 0, p = 0;
-    int slot = -1;
-    bool live = false, have = false, shadow = false, budgeted = false, drained = false;
-    for (;;) {
-        const uint32_t idle = __ballot_sync(kFull, !live);
-        if (!drained && (idle == kFull || __popc(idle) >= kRefillLanes)) {
-            uint32_t base = 0;
-            if (lane == 0) base = atomicAdd(work, (uint32_t)__popc(idle));
-            base = __shfl_sync(kFull, base, 0);
-            if (base + (uint32_t)__popc(idle) >= total) drained = true;
-            const uint32_t k = base + __popc(idle & lt);
-            const bool take = !live && k < total;
-            uint32_t start = 1u;
-            if (take) {
-                shadow = k < ns;
-                const uint32_t q = shadow ? k : cap + (k - ns);  // list slot: pixel, ray, start node
-                p = __ldg(lists + q);
-                if (BATCH) {
-                    const uint32_t sc = p / bt.px;
-                    tr.nodes = bt.nodes + ((size_t)sc << bt.depth);
-                    tr.tri_base = __ldg(bt.tri_off + sc);
-                    tr.n = __ldg(bt.tri_off + sc + 1);
-                }
-                const float4 ra = __ldg(rays + 2 * (size_t)q), rb = __ldg(rays + 2 * (size_t)q + 1);
-                r = make_ray(mk3(ra.x, ra.y, ra.z), mk3(rb.x, rb.y, rb.z), ra.w, __float_as_int(rb.w));
-                start = __ldg(starts + q);
-                b.key = hit_key(r.tmax, 0);
-                b.id = -1;
-                b.u = b.v = -1.0f;
-                b.t = r.tmax;
-                b.leaf = 1u;
-                bound = b.key;
-                sp = 0;
-                nbox = ntri = 0;
-                slot = -1;
-                budgeted = spill.count != nullptr;
-                live = true;
-            }
-            const bool ex = __any_sync(kFull, take && r.exact);  // warp-uniform choice of the box test
-            if (take) {
-                have = ex ? start_walk<true>(r, tr, start, b.t, stack_node, stack_t0, sp, node, cur, nbox)
-                          : start_walk<false>(r, tr, start, b.t, stack_node, stack_t0, sp, node, cur, nbox);
-            }
-        }
-        if (!__any_sync(kFull, live)) {
-            if (drained) break;
-            continue;
-        }
-        // one round of the walk: descend (at most kShadeSteps nodes) towards a
-        // leaf, test the held leaves together, pop
-        const bool ex = __any_sync(kFull, have && r.exact);
-        bool leaf = false;
-        if (have) {
-            have = ex ? descend<true, false, true>(tr, r, b.t, node, cur, stack_node, stack_t0, sp, 0u, nbox,
-                                                   kShadeSteps, &leaf)
-                      : descend<false, false, true>(tr, r, b.t, node, cur, stack_node, stack_t0, sp, 0u, nbox,
-                                                    kShadeSteps, &leaf);
-        }
-        __syncwarp();
-        if (__any_sync(kFull, have && leaf)) leaf_phase<false>(tr, r, have && leaf, cur, node, bound, b, ntri);
-        if (have && leaf) {
-            if (shadow && b.id >= 0) {
-                have = false;  // any hit
-            } else {
-                have = pop_node(tr, b.t, node, cur, stack_node, stack_t0, sp, 0u);
-                if (budgeted && have && nbox + ntri > spill.budget) {
-                    const uint32_t s = atomicAdd(spill.count, 1u);
-                    if (s < spill.cap) {
-                        slot = (int)s;
-                        have = false;
-                    } else {
-                        budgeted = false;  // list full: finish here
-                    }
-                }
-            }
-        }
-        if (live && !have) {  // the walk is over: the ray's result
-            if (slot >= 0) {
-                spill_record(list, slot, shadow ? kHeavyShadow : kHeavyMirror, p);
-            } else if (shadow) {
-                vis[p] = vis_code(true, true, b.id >= 0);
-            } else {
-                Hit h;
-                h.id = b.id;
-                h.u = b.u;
-                h.v = b.v;
-                h.t = b.t;
-                store_hit(mirror + p, h);
-                if (mirror_leaves) mirror_leaves[p] = tr.compact ? 1u : b.leaf;
-            }
-            live = false;
-        }
-    }
-}
-
 __device__ __forceinline__ RayState load_ray(const rt_ray* __restrict__ rays, uint32_t k, bool valid) {
     float4 a = make_float4(0.f, 0.f, 0.f, __int_as_float(-1)), b = make_float4(0.f, 0.f, 1.f, 1.f);
     if (valid) {
@@ -411,6 +317,238 @@ __device__ __forceinline__ RayState load_ray(const rt_ray* __restrict__ rays, ui
         b = __ldg(reinterpret_cast<const float4*>(rays + k) + 1);
     }
     return make_ray(mk3(a.x, a.y, a.z), mk3(b.x, b.y, b.z), b.w, __float_as_int(a.w));
+}
+
+// The shading pass keeps every lane busy: a lane whose ray has finished takes the
+// next list entry once kWalkRefill lanes of its warp are idle (the newcomers
+// take consecutive entries, so they stay neighbours), instead of idling until
+// the warp's slowest ray is done (dynamic ray fetch, Aila and Laine 2009).
+//
+// It walks the trace records (Walk).  BATCH: a listed pixel g belongs to
+// scene g / px, and a warp's lanes may walk different scenes.
+// 16 idle lanes and 4 expansions a round at 64 registers (eight blocks an SM) were
+// the fastest of 12 to 24, 3 to 10 and six to eight: 650 -> 545 us a frame of
+// 2.1 M triangles at 1080p.
+constexpr int kWalkRefill = 16;
+constexpr int kWalkSteps = 4;
+constexpr int kRayRefill = 8;  // a soup's rays: of 8 to 16, and 4 to 12 expansions
+constexpr int kRaySteps = 8;
+
+// The scenes of a batch.
+struct BatchTrees {
+    const rt_node* nodes;
+    const TraceNode* tnodes;
+    const uint32_t* tri_off;
+    uint32_t depth, px;
+};
+
+__device__ __forceinline__ void scene_tree(TreeRef& tr, const BatchTrees& bt, uint32_t sc) {
+    tr.heap = bt.nodes + ((size_t)sc << bt.depth);
+    if (bt.tnodes) tr.tnodes = bt.tnodes + ((size_t)sc << (bt.depth - 1u));
+    tr.tri_base = __ldg(bt.tri_off + sc);
+    tr.n = __ldg(bt.tri_off + sc + 1);
+}
+
+template <bool BATCH>
+__global__ void __launch_bounds__(kTraceThreads, 8) k_walk_shade(
+    TreeRef tr0, uint8_t* __restrict__ vis, rt_hit* __restrict__ mirror, uint32_t* __restrict__ mirror_leaves,
+    const uint32_t* __restrict__ lists, uint32_t cap, const uint32_t* counts, const float4* __restrict__ rays,
+    const uint32_t* __restrict__ starts, uint32_t* work, Spill spill, uint32_t* __restrict__ list,
+    BatchTrees bt) {
+    constexpr uint32_t kFull = 0xffffffffu;
+    grid_dep_wait();
+    mark_records(tr0);
+    TreeRef tr = tr0;
+    const uint32_t ns = min(counts[0], cap), nm = min(counts[1], cap), total = ns + nm;
+    const int lane = threadIdx.x & 31;
+    Walk w;
+    w.clear();
+    uint2 stack[kStackSize];
+    uint32_t p = 0;
+    bool live = false, shadow = false, budgeted = spill.count != nullptr, drained = false;
+    for (;;) {
+        const uint32_t idle = __ballot_sync(kFull, !live);
+        if (!drained && (idle == kFull || __popc(idle) >= kWalkRefill)) {
+            uint32_t base = 0;
+            if (lane == 0) base = atomicAdd(work, (uint32_t)__popc(idle));
+            base = __shfl_sync(kFull, base, 0);
+            if (base + (uint32_t)__popc(idle) >= total) drained = true;
+            const uint32_t k = base + __popc(idle & ((1u << lane) - 1u));
+            const bool take = !live && k < total;
+            RayState r = make_ray(mk3(0.f, 0.f, 0.f), mk3(0.f, 0.f, 1.f), 1.0f, -1);
+            uint32_t start = 1u;
+            if (take) {
+                shadow = k < ns;
+                const uint32_t q = shadow ? k : cap + (k - ns);  // list slot: pixel, ray, start node
+                p = __ldg(lists + q);
+                if (BATCH) scene_tree(tr, bt, p / bt.px);
+                const float4 ra = __ldg(rays + 2 * (size_t)q), rb = __ldg(rays + 2 * (size_t)q + 1);
+                r = make_ray(mk3(ra.x, ra.y, ra.z), mk3(rb.x, rb.y, rb.z), ra.w, __float_as_int(rb.w));
+                start = __ldg(starts + q);
+                live = true;
+            }
+            w.start(take, r, tr, start, stack);
+        }
+        if (!__any_sync(kFull, live)) {
+            if (drained) break;
+            continue;
+        }
+        w.round(tr, kWalkSteps, stack, shadow);
+        int slot = -1;
+        if (live && w.have && budgeted && w.tests > spill.budget) {
+            const uint32_t e = atomicAdd(spill.count, 1u);
+            if (e < spill.cap) {
+                slot = (int)e;
+                w.stop();
+            } else {
+                budgeted = false;  // list full: finish here
+            }
+        }
+        if (live && !w.have) {  // the walk is over: the ray's result
+            if (slot >= 0) spill_record(list, slot, shadow ? kHeavyShadow : kHeavyMirror, p);
+            if (!shadow) {
+                store_hit(mirror + p, w.hit());  // of a handed-over ray: the closest hit so far
+                if (mirror_leaves && slot < 0) mirror_leaves[p] = tr.compact ? 1u : w.b.leaf;
+            } else if (slot < 0) {
+                vis[p] = vis_code(true, true, w.b.id >= 0);
+            }
+            live = false;
+        }
+    }
+}
+
+// Any-hit calls of fewer rays stay with traverse(): the second walk of the rays in
+// doubt lasts as long as its longest ones, 200 us on a mesh's grazing rays (65 k
+// triangle torus, 0.5 M rays 0.36 -> 0.42 ms, 2 M rays 1.02 -> 0.78 ms; a soup gains
+// from 0.2 M rays on, 1 M rays 1.63 -> 0.79 ms).
+constexpr uint32_t kWalkAnyRays = 1u << 20;
+
+struct Doubt {
+    uint32_t* list;
+    uint32_t* count;
+    uint32_t* work;
+};
+
+// A caller's rays over the trace records.  A closest hit does not depend on the
+// walk, so a ray over the budget goes to the warp-per-ray pass.  The first
+// hit does: this walk meets the leaves in traverse()'s order, but which rays
+// traverse() hands over depends on its exact counts, which are at most the
+// counts here.  So an any-hit ray over the budget is walked again by
+// k_trace_doubt, as traverse() does, with its budget.
+__global__ void __launch_bounds__(kTraceThreads, 8) k_walk_rays(TreeRef tr, const rt_ray* __restrict__ rays, uint32_t n,
+                                                                     int any_hit, const uint32_t* __restrict__ starts,
+                                                                     rt_hit* __restrict__ hits,
+                                                                     uint32_t* __restrict__ leaves, uint32_t* work,
+                                                                     Spill spill, uint32_t* __restrict__ list, Doubt doubt) {
+    constexpr uint32_t kFull = 0xffffffffu;
+    grid_dep_wait();
+    mark_records(tr);
+    const int lane = threadIdx.x & 31;
+    Walk w;
+    w.clear();
+    uint2 stack[kStackSize];
+    uint32_t k = 0;
+    bool live = false, budgeted = spill.count != nullptr, drained = false;
+    for (;;) {
+        const uint32_t idle = __ballot_sync(kFull, !live);
+        if (!drained && (idle == kFull || __popc(idle) >= kRayRefill)) {
+            uint32_t base = 0;
+            if (lane == 0) base = atomicAdd(work, (uint32_t)__popc(idle));
+            base = __shfl_sync(kFull, base, 0);
+            if (base >= n || n - base <= (uint32_t)__popc(idle)) drained = true;
+            const uint32_t q = base + __popc(idle & ((1u << lane) - 1u));
+            const bool take = !live && base < n && q < n;
+            if (take) {
+                k = q;
+                live = true;
+            }
+            w.start(take, load_ray(rays, k, take), tr, (starts && take) ? __ldg(starts + k) : 1u, stack);
+        }
+        if (!__any_sync(kFull, live)) {
+            if (drained) break;
+            continue;
+        }
+        w.round(tr, kRaySteps, stack, any_hit != 0);
+        int slot = -1;
+        if (live && w.have && budgeted && w.tests > spill.budget) {
+            const uint32_t e = atomicAdd(any_hit ? doubt.count : spill.count, 1u);
+            if (e < spill.cap) {
+                slot = (int)e;
+                w.stop();
+            } else {
+                budgeted = false;
+            }
+        }
+        if (live && !w.have) {
+            if (slot >= 0 && any_hit) {
+                doubt.list[slot] = k;
+            } else {
+                store_hit(hits + k, w.hit());
+                if (slot >= 0) spill_record(list, slot, kHeavyRay, k);
+                else if (leaves) leaves[k] = tr.compact ? 1u : w.b.leaf;
+            }
+            live = false;
+        }
+    }
+}
+
+// The any-hit rays in doubt.
+__global__ void __launch_bounds__(kTraceThreads) k_trace_doubt(TreeRef tr, const rt_ray* __restrict__ rays,
+                                                               const uint32_t* __restrict__ starts,
+                                                               rt_hit* __restrict__ hits, uint32_t* __restrict__ leaves,
+                                                               Doubt doubt, Spill spill, uint32_t* __restrict__ list) {
+    constexpr uint32_t kFull = 0xffffffffu;
+    grid_dep_wait();
+    const uint32_t n = min(*doubt.count, spill.cap);
+    const int lane = threadIdx.x & 31;
+    Walk w;
+    w.clear();
+    uint2 stack[kStackSize];
+    uint32_t k = 0;
+    bool live = false, budgeted = spill.count != nullptr, drained = false;
+    // few rays are spread over all warps, some lanes of each
+    const uint32_t warps = gridDim.x * (kTraceThreads / 32), per = max(1u, (n + warps - 1) / warps);
+    const uint32_t lanes = per < 32u ? (1u << per) - 1u : kFull;
+    for (;;) {
+        const uint32_t idle = __ballot_sync(kFull, !live) & lanes;
+        if (!drained && (idle == lanes || __popc(idle) >= kRayRefill)) {
+            uint32_t base = 0;
+            if (lane == 0) base = atomicAdd(doubt.work, (uint32_t)__popc(idle));
+            base = __shfl_sync(kFull, base, 0);
+            if (base + (uint32_t)__popc(idle) >= n) drained = true;
+            const uint32_t q = base + __popc(idle & ((1u << lane) - 1u));
+            const bool take = ((idle >> lane) & 1u) && q < n;
+            if (take) {
+                k = doubt.list[q];
+                live = true;
+            }
+            w.start(take, load_ray(rays, k, take), tr, (starts && take) ? __ldg(starts + k) : 1u, stack, true);
+        }
+        if (!__any_sync(kFull, live)) {
+            if (drained) break;
+            continue;
+        }
+        const bool tested = w.round(tr, kRaySteps, stack, true);
+        int slot = -1;
+        if (live && tested && w.b.id < 0 && w.more && budgeted && w.at_leaf > spill.budget) {
+            const uint32_t e = atomicAdd(spill.count, 1u);
+            if (e < spill.cap) {
+                slot = (int)e;
+                w.stop();
+            } else {
+                budgeted = false;
+            }
+        }
+        if (live && !w.have) {
+            if (slot >= 0) {
+                spill_record(list, slot, kHeavyRay, k);
+            } else {
+                store_hit(hits + k, w.hit());
+                if (leaves) leaves[k] = tr.compact ? 1u : w.b.leaf;
+            }
+            live = false;
+        }
+    }
 }
 
 template <bool STATS>
@@ -432,12 +570,9 @@ __global__ void __launch_bounds__(kTraceThreads) k_trace_rays(TreeRef tr, const 
         int slot = -1;
         const Hit h = trace_ray<STATS>(r, valid, tr, any_hit != 0, &nb, &nt, &spill, &slot, start, &leaf);
         if (valid) {
-            if (slot >= 0) {
-                spill_record(list, slot, kHeavyRay, k);
-            } else {
-                store_hit(hits + k, h);
-                if (leaves) leaves[k] = leaf;
-            }
+            store_hit(hits + k, h);  // of a handed-over ray: the closest hit so far
+            if (slot >= 0) spill_record(list, slot, kHeavyRay, k);
+            else if (leaves) leaves[k] = leaf;
             if (STATS) {
                 stats[2 * k] = nb;
                 stats[2 * k + 1] = nt;
@@ -472,7 +607,25 @@ struct HeavyArgs {
     uint32_t* work;
 };
 
-__global__ void __launch_bounds__(kTraceThreads) k_trace_heavy(HeavyArgs a) {
+// The closest hit the first pass had found when it handed the ray over.
+__device__ __forceinline__ Hit hit_so_far(const rt_hit* p) {
+    const int4 v = __ldcg(reinterpret_cast<const int4*>(p));
+    Hit h;
+    h.id = v.x;
+    h.u = __int_as_float(v.y);
+    h.v = __int_as_float(v.z);
+    h.t = __int_as_float(v.w);
+    return h;
+}
+__device__ __forceinline__ Hit no_hit() {
+    Hit h;
+    h.id = -1;
+    h.u = h.v = -1.0f;
+    h.t = 0.0f;
+    return h;
+}
+
+__global__ void __launch_bounds__(kTraceThreads, 7) k_trace_heavy(HeavyArgs a) {
     grid_dep_wait();
     const uint32_t n = min(*a.count, a.cap);
     const int lane = threadIdx.x & 31;
@@ -483,7 +636,7 @@ __global__ void __launch_bounds__(kTraceThreads) k_trace_heavy(HeavyArgs a) {
             const uint32_t i = idx % a.cam.width, j = idx / a.cam.width;
             const RayState r = make_ray(mk3(a.cam.eye[0], a.cam.eye[1], a.cam.eye[2]), primary_dir(a.cam, i, j),
                                         1e16f, -1);
-            const Hit h = trace_wide(r, a.tr, false, a.wide_cap);
+            const Hit h = trace_wide(r, a.tr, false, a.wide_cap, hit_so_far(a.hits + idx));
             if (lane == 0) {
                 store_hit(a.hits + idx, h);
                 if (a.leaves) a.leaves[idx] = 1u;  // the root: a valid restart node
@@ -494,7 +647,7 @@ __global__ void __launch_bounds__(kTraceThreads) k_trace_heavy(HeavyArgs a) {
             }
         } else if (kind == kHeavyRay) {
             const RayState r = load_ray(a.rays, idx, true);
-            const Hit h = trace_wide(r, a.tr, a.any_hit != 0, a.wide_cap);
+            const Hit h = trace_wide(r, a.tr, a.any_hit != 0, a.wide_cap, a.any_hit ? no_hit() : hit_so_far(a.hits + idx));
             if (lane == 0) {
                 store_hit(a.hits + idx, h);
                 if (a.leaves) a.leaves[idx] = 1u;
@@ -504,10 +657,10 @@ __global__ void __launch_bounds__(kTraceThreads) k_trace_heavy(HeavyArgs a) {
             const int4 ph = __ldg(reinterpret_cast<const int4*>(a.prim + idx));
             const ShadeRays s = shade_rays(a.soup, a.cam, a.lx, a.ly, a.lz, ph, true, i, j, kind == kHeavyMirror);
             if (kind == kHeavyShadow) {
-                const Hit h = trace_wide(s.shadow, a.tr, true, a.wide_cap);
+                const Hit h = trace_wide(s.shadow, a.tr, true, a.wide_cap, no_hit());
                 if (lane == 0) a.vis[idx] = vis_code(s.has, s.cast, h.id >= 0);
             } else {
-                const Hit h = trace_wide(s.mirror, a.tr, false, a.wide_cap);
+                const Hit h = trace_wide(s.mirror, a.tr, false, a.wide_cap, hit_so_far(a.mirror + idx));
                 if (lane == 0) {
                     store_hit(a.mirror + idx, h);
                     if (a.mirror_leaves) a.mirror_leaves[idx] = 1u;
@@ -515,6 +668,21 @@ __global__ void __launch_bounds__(kTraceThreads) k_trace_heavy(HeavyArgs a) {
             }
         }
     }
+}
+
+// A few closest-hit rays, a warp each from the start: with a lane each they fill
+// a handful of warps, and the call lasts as long as the longest chain of dependent
+// loads: 256 rays over 65 k triangles 70 -> 14 us, 16,384 rays 132 -> 72 us; at
+// 32,768 both take 135 us.
+constexpr uint32_t kFewRays = 16384;
+
+__global__ void __launch_bounds__(kTraceThreads) k_rays_wide(TreeRef tr, const rt_ray* __restrict__ rays, uint32_t n,
+                                                             rt_hit* __restrict__ hits, uint32_t cap) {
+    grid_dep_wait();
+    const uint32_t k = blockIdx.x * kWideWarps + (threadIdx.x >> 5);
+    if (k >= n) return;
+    const Hit h = trace_wide(load_ray(rays, k, true), tr, false, cap, no_hit());
+    if ((threadIdx.x & 31) == 0) store_hit(hits + k, h);
 }
 
 // k_trace_heavy with a block per ray (traverse_team): for the handed-over
@@ -538,7 +706,7 @@ __global__ void __launch_bounds__(kTeamThreads) k_trace_heavy_team(HeavyArgs a) 
             const uint32_t i = idx % a.cam.width, j = idx / a.cam.width;
             const RayState r = make_ray(mk3(a.cam.eye[0], a.cam.eye[1], a.cam.eye[2]), primary_dir(a.cam, i, j),
                                         1e16f, -1);
-            const Hit h = trace_team(r, a.tr, false, a.team_cap, ts);
+            const Hit h = trace_team(r, a.tr, false, a.team_cap, ts, hit_so_far(a.hits + idx));
             if (tid == 0) {
                 store_hit(a.hits + idx, h);
                 if (a.leaves) a.leaves[idx] = 1u;  // the root: a valid restart node
@@ -549,7 +717,7 @@ __global__ void __launch_bounds__(kTeamThreads) k_trace_heavy_team(HeavyArgs a) 
             }
         } else if (kind == kHeavyRay) {
             const RayState r = load_ray(a.rays, idx, true);
-            const Hit h = trace_team(r, a.tr, a.any_hit != 0, a.team_cap, ts);
+            const Hit h = trace_team(r, a.tr, a.any_hit != 0, a.team_cap, ts, a.any_hit ? no_hit() : hit_so_far(a.hits + idx));
             if (tid == 0) {
                 store_hit(a.hits + idx, h);
                 if (a.leaves) a.leaves[idx] = 1u;
@@ -559,10 +727,10 @@ __global__ void __launch_bounds__(kTeamThreads) k_trace_heavy_team(HeavyArgs a) 
             const int4 ph = __ldg(reinterpret_cast<const int4*>(a.prim + idx));
             const ShadeRays sr = shade_rays(a.soup, a.cam, a.lx, a.ly, a.lz, ph, true, i, j, kind == kHeavyMirror);
             if (kind == kHeavyShadow) {
-                const Hit h = trace_team(sr.shadow, a.tr, true, a.team_cap, ts);
+                const Hit h = trace_team(sr.shadow, a.tr, true, a.team_cap, ts, no_hit());
                 if (tid == 0) a.vis[idx] = vis_code(sr.has, sr.cast, h.id >= 0);
             } else {
-                const Hit h = trace_team(sr.mirror, a.tr, false, a.team_cap, ts);
+                const Hit h = trace_team(sr.mirror, a.tr, false, a.team_cap, ts, hit_so_far(a.mirror + idx));
                 if (tid == 0) {
                     store_hit(a.mirror + idx, h);
                     if (a.mirror_leaves) a.mirror_leaves[idx] = 1u;
@@ -664,6 +832,12 @@ __device__ __forceinline__ void zero_words(uint32_t* words, unsigned long long m
     if (threadIdx.x < 64 && ((mask >> threadIdx.x) & 1ull)) words[threadIdx.x] = 0u;
 }
 
+Records no_records() {
+    Records rec;
+    memset(&rec, 0, sizeof(rec));
+    return rec;
+}
+
 // Blocks past the first make the trace records of a tile each.
 __global__ void __launch_bounds__(256) k_reset_words(uint32_t* words, unsigned long long mask, Records rec) {
     grid_dep_wait();
@@ -674,12 +848,10 @@ __global__ void __launch_bounds__(256) k_reset_words(uint32_t* words, unsigned l
     zero_words(words, mask);
 }
 
-rt_status reset_words(rt_ctx* ctx, uint64_t mask, const rt_lbvh* l = nullptr) {
-    if (!mask && !l) return RT_OK;
-    Records rec;
-    memset(&rec, 0, sizeof(rec));
-    if (l) rec = records_of(l);
-    launch_pdl(k_reset_words, 1u + rec.tiles, l ? 256 : 64, 0, ctx->stream, ctx->d_words, (unsigned long long)mask, rec);
+rt_status reset_words(rt_ctx* ctx, uint64_t mask, const Records& rec) {
+    if (!mask && !rec.tiles) return RT_OK;
+    launch_pdl(k_reset_words, 1u + rec.tiles, rec.tiles ? 256 : 64, 0, ctx->stream, ctx->d_words, (unsigned long long)mask,
+               rec);
     RT_CHECK_LAUNCH(ctx, "k_reset_words");
     return RT_OK;
 }
@@ -753,13 +925,11 @@ rt_status order_begin(rt_ctx* ctx, int kind, bool enabled, TileOrder* out, uint6
     o.lists = ctx->d_order + (size_t)kind * kOrderWords;
     o.bits = o.lists + 2 * (size_t)kOrderCap;
     if (enabled) {
-        Records rec;
-        memset(&rec, 0, sizeof(rec));
-        if (l) rec = records_of(l);
+        const Records rec = l ? records_of(l) : no_records();
         launch_pdl(k_order_begin, 1u + rec.tiles, 256, 0, ctx->stream, o, ctx->d_words, (unsigned long long)reset, rec);
         RT_CHECK_LAUNCH(ctx, "k_order_begin");
     } else {
-        rt_status s = reset_words(ctx, reset, l);
+        rt_status s = reset_words(ctx, reset, l ? records_of(l) : no_records());
         if (s != RT_OK) return s;
     }
     *out = o;
@@ -792,7 +962,7 @@ rt_status trace_primary(rt_ctx* ctx, const rt_lbvh* l, const rt_camera* cam, rt_
     uint64_t reset = word_bit(ctx, ctx->d_work + kWorkPrimary) | spill_reset_bits(ctx, sp) | extra_reset;
     if (sl && !d_stats) reset |= word_bit(ctx, sl->counts) | word_bit(ctx, sl->counts + 1);
     TileOrder ord;
-    if ((s = order_begin(ctx, 0, ctx->tile_order & 1u, &ord, reset)) != RT_OK) return s;
+    if ((s = order_begin(ctx, 0, ctx->tile_order & 1u, &ord, reset, d_stats ? nullptr : l)) != RT_OK) return s;
     const uint32_t tiles = pixel_tiles(cam);
     uint32_t* work = ctx->d_work + kWorkPrimary;
     ShadeLists none;
@@ -803,10 +973,8 @@ rt_status trace_primary(rt_ctx* ctx, const rt_lbvh* l, const rt_camera* cam, rt_
         k<<<persistent_blocks(ctx, k, kTraceThreads, tiles), kTraceThreads, 0, ctx->stream>>>(
             tree_ref(ctx, l), *cam, d_hits, d_leaves, d_stats, work, tiles, sp, ctx->d_spill, ord, none);
     } else {
-        auto k = k_trace_primary<false>;
-        launch_pdl(k, persistent_blocks(ctx, k, kTraceThreads, tiles), kTraceThreads, 0, ctx->stream,
-                   tree_ref(ctx, l), *cam, d_hits, d_leaves, (uint32_t*)nullptr, work, tiles, sp, ctx->d_spill, ord,
-                   lists);
+        launch_pdl(k_walk_primary, persistent_blocks(ctx, k_walk_primary, kTraceThreads, tiles), kTraceThreads, 0, ctx->stream,
+                   tree_ref(ctx, l), *cam, d_hits, d_leaves, work, tiles, sp, ctx->d_spill, ord, lists);
     }
     RT_CHECK_LAUNCH(ctx, "k_trace_primary");
     HeavyArgs a = heavy_args(ctx, l);
@@ -847,7 +1015,7 @@ rt_status trace_shadow_mirror(rt_ctx* ctx, const rt_lbvh* l, const rt_camera* ca
         uint32_t* counts = ctx->d_work + kShadeCounts;
         if (!prebuilt) {
             reset = shade_reset_bits(ctx, sp) | word_bit(ctx, counts) | word_bit(ctx, counts + 1);
-            if ((s = reset_words(ctx, reset)) != RT_OK) return s;
+            if ((s = reset_words(ctx, reset, records_of(l))) != RT_OK) return s;
         }
         const uint32_t cap = (uint32_t)l->s_pixels;
         if (!prebuilt) {
@@ -860,16 +1028,14 @@ rt_status trace_shadow_mirror(rt_ctx* ctx, const rt_lbvh* l, const rt_camera* ca
             RT_CHECK_LAUNCH(ctx, "k_shade_setup");
         }
         int per_sm = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_trace_shade<false>, kTraceThreads, 0) !=
-                cudaSuccess ||
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_walk_shade<false>, kTraceThreads, 0) != cudaSuccess ||
             per_sm < 1)
             per_sm = 1;
-        launch_pdl(k_trace_shade<false>, (uint32_t)per_sm * ctx->num_sms, kTraceThreads, 0, ctx->stream, tree_ref(ctx, l),
-                   l->src_tris, *cam, light[0], light[1], light[2], d_primary, d_prim_leaves, d_vis, d_mirror,
-                   d_mirror_leaves, (const uint32_t*)l->s_lists, cap, (const uint32_t*)counts,
+        launch_pdl(k_walk_shade<false>, (uint32_t)per_sm * ctx->num_sms, kTraceThreads, 0, ctx->stream, tree_ref(ctx, l), d_vis,
+                   d_mirror, d_mirror_leaves, (const uint32_t*)l->s_lists, cap, (const uint32_t*)counts,
                    (const float4*)l->s_rays, (const uint32_t*)(l->s_lists + 3 * l->s_pixels), ctx->d_work + kWorkShade,
-                   sp, ctx->d_spill, BatchTrees{nullptr, nullptr, 0u, 0u});
-        RT_CHECK_LAUNCH(ctx, "k_trace_shade");
+                   sp, ctx->d_spill, BatchTrees{nullptr, nullptr, nullptr, 0u, 0u});
+        RT_CHECK_LAUNCH(ctx, "k_walk_shade");
     }
     HeavyArgs a = heavy_args(ctx, l);
     a.soup = l->src_tris;
@@ -892,9 +1058,18 @@ rt_status trace_rays(rt_ctx* ctx, const rt_lbvh* l, const rt_ray* d_rays, uint32
     if (l->n == 0) return rt_fail(ctx, RT_ERR_INVALID, "%s: the LBVH has not been built", who);
     if (n == 0) return RT_OK;
     const Spill sp = spill_of(ctx, !d_stats && n <= kHeavyIndexMask, 2);
-    const uint64_t reset = word_bit(ctx, ctx->d_work + kWorkRays) | spill_reset_bits(ctx, sp);
+    const uint64_t reset = word_bit(ctx, ctx->d_work + kWorkRays) | spill_reset_bits(ctx, sp) |
+                           word_bit(ctx, ctx->d_words + kDoubtCount) | word_bit(ctx, ctx->d_words + kDoubtCount + 1);
     TileOrder ord;
-    rt_status s = order_begin(ctx, 2, ctx->tile_order & 4u, &ord, reset);
+    if (!d_stats && !any_hit && !d_leaves && n <= kFewRays) {
+        const uint32_t cap = wide_stack_entries(l->depth);
+        launch_pdl(k_rays_wide, (n + kWideWarps - 1) / kWideWarps, kTraceThreads, wide_smem_bytes(cap), ctx->stream,
+                   tree_ref(ctx, l), d_rays, n, d_hits, cap);
+        RT_CHECK_LAUNCH(ctx, "k_rays_wide");
+        return RT_OK;
+    }
+    const bool walk = !d_stats && !(ctx->tile_order & 4u) && !(any_hit && n < kWalkAnyRays);
+    rt_status s = order_begin(ctx, 2, ctx->tile_order & 4u, &ord, reset, walk ? l : nullptr);
     if (s != RT_OK) return s;
     const uint32_t tiles = (n + 31) / 32;
     uint32_t* work = ctx->d_work + kWorkRays;
@@ -902,6 +1077,15 @@ rt_status trace_rays(rt_ctx* ctx, const rt_lbvh* l, const rt_ray* d_rays, uint32
         auto k = k_trace_rays<true>;
         k<<<persistent_blocks(ctx, k, kTraceThreads, tiles), kTraceThreads, 0, ctx->stream>>>(
             tree_ref(ctx, l), d_rays, n, any_hit, d_starts, d_hits, d_leaves, d_stats, work, sp, ctx->d_spill, ord);
+    } else if (walk) {
+        const Doubt doubt{ctx->d_spill + kSpillCap, ctx->d_words + kDoubtCount, ctx->d_words + kDoubtCount + 1};
+        launch_pdl(k_walk_rays, persistent_blocks(ctx, k_walk_rays, kTraceThreads, tiles), kTraceThreads, 0, ctx->stream,
+                   tree_ref(ctx, l), d_rays, n, any_hit, d_starts, d_hits, d_leaves, work, sp, ctx->d_spill, doubt);
+        if (any_hit && sp.count) {
+            RT_CHECK_LAUNCH(ctx, "k_walk_rays");
+            launch_pdl(k_trace_doubt, persistent_blocks(ctx, k_trace_doubt, kTraceThreads, tiles), kTraceThreads, 0,
+                       ctx->stream, tree_ref(ctx, l), d_rays, d_starts, d_hits, d_leaves, doubt, sp, ctx->d_spill);
+        }
     } else {
         auto k = k_trace_rays<false>;
         k<<<persistent_blocks(ctx, k, kTraceThreads, tiles), kTraceThreads, 0, ctx->stream>>>(
@@ -919,7 +1103,7 @@ rt_status trace_rays(rt_ctx* ctx, const rt_lbvh* l, const rt_ray* d_rays, uint32
 }  // namespace
 
 rt_status reset_work_and_records(rt_ctx* ctx, int slot, const rt_lbvh* l) {
-    return reset_words(ctx, word_bit(ctx, ctx->d_work + slot), l);
+    return reset_words(ctx, word_bit(ctx, ctx->d_work + slot), records_of(l));
 }
 
 extern "C" rt_status rt_trace_primary(rt_ctx* ctx, const rt_lbvh* l, const rt_camera* cam, rt_hit* d_hits,
@@ -1248,10 +1432,18 @@ struct BatchListArgs {
     uint32_t* starts;
 };
 
-// LIST: the shadow rays are listed (a.lists set), else traced here (a.vis
-// set) or not cast (a.vis null).
+// Primary rays of a batch, an 8 x 4 tile of one scene per warp at a time.  LIST:
+// the shadow rays are listed; else they are traced here (a.vis set) or not
+// cast (a.vis null).
+constexpr int kBatchSteps = 6;  // 256 random soups: 4: 9.42 ms a frame, 6: 9.36, 8: 9.38, 12: 9.61
+
 template <bool LIST>
-__device__ __forceinline__ void batch_trace_body(const BatchTraceArgs& a, const BatchListArgs& la, uint32_t* work) {
+__device__ __forceinline__ void batch_trace_body(const BatchTraceArgs& a, const BatchListArgs& la, const TreeRef& tr0,
+                                                 const BatchTrees& bt, uint32_t* work) {
+    mark_records(tr0);
+    Walk w;
+    w.clear();
+    uint2 stack[kStackSize];
     const uint32_t total = a.S * a.tiles_per_scene;
     const uint32_t lane = threadIdx.x & 31;
     const size_t px = (size_t)a.width * a.height;
@@ -1264,23 +1456,18 @@ __device__ __forceinline__ void batch_trace_body(const BatchTraceArgs& a, const 
         for (uint32_t g = g0; g < g1; ++g) {
             const uint32_t s = a.order ? g % a.S : g / a.tiles_per_scene;
             const uint32_t tile = a.order ? g / a.S : g % a.tiles_per_scene;
-            const uint32_t toff = __ldg(a.tri_off + s);
-            TreeRef tr;
-            tr.compact = false;
-            tr.tri_base = 0;
-            tr.nodes = a.nodes + ((size_t)s << a.depth);
-            tr.tris = a.sorted_tris + 3 * (size_t)toff;
-            tr.num_nodes = 1u << a.depth;
-            tr.n = __ldg(a.tri_off + s + 1) - toff;
-            tr.err = a.err;
+            TreeRef tr = tr0;
+            scene_tree(tr, bt, s);
+            const uint32_t toff = tr.tri_base;
             const rt_camera cam = a.cams[s];
             uint32_t i, j;
             const bool valid = tile_pixel(tile, lane, a.width, a.height, &i, &j);
             if (!valid) i = j = 0;
             const f3 d = primary_dir(cam, i, j);
-            const RayState r = make_ray(mk3(cam.eye[0], cam.eye[1], cam.eye[2]), d, 1e16f, -1);
-            uint32_t nb = 0, nt = 0, leaf = 1;
-            const Hit h = trace_ray<false>(r, valid, tr, false, &nb, &nt, nullptr, nullptr, 1u, &leaf);
+            w.start(valid, make_ray(mk3(cam.eye[0], cam.eye[1], cam.eye[2]), d, 1e16f, -1), tr, 1u, stack);
+            while (__any_sync(0xffffffffu, w.have)) w.round(tr, kBatchSteps, stack);
+            const Hit h = w.hit();
+            const uint32_t leaf = w.b.leaf;
             const size_t p = (size_t)j * a.width + i;
             if (valid) store_hit(a.hits + s * px + p, h);
             if (LIST) {  // the shadow ray (restarting at the primary leaf) goes to the list
@@ -1291,24 +1478,26 @@ __device__ __forceinline__ void batch_trace_body(const BatchTraceArgs& a, const 
                 shade_setup_pixel(sl, cam, ph, valid, i, j, s * px + p, h.id >= 0 ? leaf : 1u);
             } else if (a.vis) {  // uniform across the grid; the shadow ray restarts at the primary leaf
                 const int4 ph = make_int4(h.id, __float_as_int(h.u), __float_as_int(h.v), __float_as_int(h.t));
-                secondary_pixel<false>(tr, a.soup + 9 * (size_t)toff, cam, __ldg(a.lights + 3 * s),
-                                       __ldg(a.lights + 3 * s + 1), __ldg(a.lights + 3 * s + 2), ph,
-                                       a.vis + s * px, nullptr, nullptr, nullptr, valid, i, j, nullptr, nullptr,
-                                       nullptr, h.id >= 0 ? leaf : 1u, nullptr);
+                const ShadeRays sr = shade_rays(a.soup + 9 * (size_t)toff, cam, __ldg(a.lights + 3 * s),
+                                                __ldg(a.lights + 3 * s + 1), __ldg(a.lights + 3 * s + 2), ph, valid, i, j,
+                                                false);
+                w.start(valid && sr.cast, sr.shadow, tr, h.id >= 0 ? leaf : 1u, stack);
+                while (__any_sync(0xffffffffu, w.have)) w.round(tr, kBatchSteps, stack, true);
+                if (valid) a.vis[s * px + p] = vis_code(sr.has, sr.cast, sr.cast && w.b.id >= 0);
             }
         }
     }
 }
 
-__global__ void __launch_bounds__(256) k_batch_trace(BatchTraceArgs a, uint32_t* work) {
+__global__ void __launch_bounds__(256) k_batch_trace(BatchTraceArgs a, TreeRef tr, BatchTrees bt, uint32_t* work) {
     grid_dep_wait();
     const BatchListArgs none = {nullptr, 0u, nullptr, nullptr, nullptr};
-    batch_trace_body<false>(a, none, work);
+    batch_trace_body<false>(a, none, tr, bt, work);
 }
 
-__global__ void __launch_bounds__(256) k_batch_list(BatchTraceArgs a, BatchListArgs la, uint32_t* work) {
+__global__ void __launch_bounds__(256) k_batch_list(BatchTraceArgs a, BatchListArgs la, TreeRef tr, BatchTrees bt, uint32_t* work) {
     grid_dep_wait();
-    batch_trace_body<true>(a, la, work);
+    batch_trace_body<true>(a, la, tr, bt, work);
 }
 
 }  // namespace
@@ -1376,8 +1565,17 @@ extern "C" rt_status rt_batch_trace(rt_ctx* ctx, const rt_batch* b, rt_hit* d_hi
     uint64_t reset = word_bit(ctx, ctx->d_work + kWorkBatch);
     if (listed)
         reset |= word_bit(ctx, ctx->d_work + kWorkShade) | word_bit(ctx, counts) | word_bit(ctx, counts + 1);
-    rt_status s = reset_words(ctx, reset);
+    rt_status s = reset_words(ctx, reset, records_of(b));
     if (s != RT_OK) return s;
+    TreeRef tr;  // the batch's arrays; heap, tnodes, tri_base and n are set per scene
+    memset(&tr, 0, sizeof(tr));
+    tr.tris = b->sorted_tris;
+    tr.leaf_of = b->leaf_of;
+    tr.num_heap = 1u << b->depth;
+    tr.num_tnodes = tr.num_heap / 2;
+    tr.records_valid = b->counters + 7;
+    tr.err = ctx->d_err;
+    const BatchTrees bt{b->nodes, b->tnodes, b->tri_off, b->depth, b->width * b->height};
     BatchTraceArgs a;
     a.nodes = b->nodes;
     a.sorted_tris = b->sorted_tris;
@@ -1406,34 +1604,21 @@ extern "C" rt_status rt_batch_trace(rt_ctx* ctx, const rt_batch* b, rt_hit* d_hi
     const uint64_t need = (items * 32 + threads - 1) / threads;
     const uint32_t blocks = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)per_sm * ctx->num_sms, need));
     if (listed)
-        launch_pdl(k_batch_list, blocks, threads, 0, ctx->stream, a, la, ctx->d_work + kWorkBatch);
+        launch_pdl(k_batch_list, blocks, threads, 0, ctx->stream, a, la, tr, bt, ctx->d_work + kWorkBatch);
     else
-        launch_pdl(k_batch_trace, blocks, threads, 0, ctx->stream, a, ctx->d_work + kWorkBatch);
+        launch_pdl(k_batch_trace, blocks, threads, 0, ctx->stream, a, tr, bt, ctx->d_work + kWorkBatch);
     RT_CHECK_LAUNCH(ctx, "k_batch_trace");
     if (!listed) return RT_OK;
-    TreeRef tr;  // the batch's whole sorted-triangle array; nodes, tri_base and n set per lane
-    tr.compact = false;
-    tr.tri_base = 0;
-    tr.nodes = b->nodes;
-    tr.tris = b->sorted_tris;
-    tr.num_nodes = 1u << b->depth;
-    tr.n = 0;
-    tr.err = ctx->d_err;
     Spill none;
     memset(&none, 0, sizeof(none));
     int shade_per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&shade_per_sm, k_trace_shade<true>, kTraceThreads, 0) !=
-            cudaSuccess ||
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&shade_per_sm, k_walk_shade<true>, kTraceThreads, 0) != cudaSuccess ||
         shade_per_sm < 1)
         shade_per_sm = 1;
-    rt_camera cam0;
-    memset(&cam0, 0, sizeof(cam0));
-    launch_pdl(k_trace_shade<true>, (uint32_t)shade_per_sm * ctx->num_sms, kTraceThreads, 0, ctx->stream, tr,
-               (const float*)nullptr, cam0, 0.0f, 0.0f, 0.0f, (const rt_hit*)nullptr, (const uint32_t*)nullptr, d_vis,
-               (rt_hit*)nullptr, (uint32_t*)nullptr, (const uint32_t*)b->s_lists, (uint32_t)cap,
-               (const uint32_t*)counts, (const float4*)b->s_rays, (const uint32_t*)(b->s_lists + cap),
-               ctx->d_work + kWorkShade, none, (uint32_t*)nullptr,
-               BatchTrees{b->nodes, b->tri_off, b->depth, b->width * b->height});
-    RT_CHECK_LAUNCH(ctx, "k_trace_shade");
+    launch_pdl(k_walk_shade<true>, (uint32_t)shade_per_sm * ctx->num_sms, kTraceThreads, 0, ctx->stream, tr, d_vis,
+               (rt_hit*)nullptr, (uint32_t*)nullptr, (const uint32_t*)b->s_lists, (uint32_t)cap, (const uint32_t*)counts,
+               (const float4*)b->s_rays, (const uint32_t*)(b->s_lists + cap), ctx->d_work + kWorkShade, none,
+               (uint32_t*)nullptr, bt);
+    RT_CHECK_LAUNCH(ctx, "k_walk_shade");
     return RT_OK;
 }

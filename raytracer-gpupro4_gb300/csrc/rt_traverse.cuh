@@ -600,18 +600,23 @@ __device__ __forceinline__ void mark_records(const TreeRef& tr) {
     if (blockIdx.x == 0 && threadIdx.x == 0) *tr.records_valid = 1u;
 }
 
-constexpr uint32_t kGeneral = 8u;
+constexpr uint32_t kGeneral = 8u;    // Walk::sgn: the records do not serve this ray
+constexpr uint32_t kInfinite = 16u;  // some 1 / d is infinite: the reference's NaN-sensitive min / max
+constexpr uint32_t kPoolMin = 3u;   // a leaf of more triangles makes the warp pool its leaves
+constexpr uint32_t kCheckMin = 4u;  // leaves above this many triangles are tested only after their exact box
 
 struct Walk {
     f3 o, d, k, n;  // k = E / d, n = (G - o) / d
-    uint32_t sgn;   // RayState::sgn; kGeneral: the records do not serve this ray
+    uint32_t sgn;   // RayState::sgn, kGeneral, kInfinite
     int exclude;
     Best b;         // key: the acceptance bound
     uint32_t cur;   // internal heap slot or leaf word; 0: pop the next one
     uint32_t pend;  // the leaf put aside (0: none)
     uint32_t sp;
-    uint32_t tests;
-    bool have;      // the walk goes on
+    uint32_t tests; // box and triangle tests, at least as many as traverse() has made at this point of the walk
+    uint32_t at_leaf;  // tests up to and with the last leaf put aside
+    bool more;         // whether the stack held anything then
+    bool have;         // the walk goes on
 
     __device__ __forceinline__ void clear() {
         o = d = k = n = mk3(0.f, 0.f, 0.f);
@@ -623,6 +628,8 @@ struct Walk {
         b.id = -1;
         b.leaf = 1u;
         cur = pend = sp = tests = 0u;
+        at_leaf = 0u;
+        more = false;
         have = false;
     }
 
@@ -638,14 +645,17 @@ struct Walk {
         cur = __uint_as_float(e.y) > b.t ? 0u : e.x;
     }
 
-    static __device__ __forceinline__ bool enter(const RayState& r, const NodeBox& nb, float bt, float* t0, bool gen) {
-        return gen ? box_enter<true>(r, nb.a.x, nb.a.y, nb.a.z, nb.a.w, nb.b.x, nb.b.y, bt, t0)
+    static __device__ __forceinline__ bool enter(const RayState& r, const NodeBox& nb, float bt, float* t0, bool inf) {
+        return inf ? box_enter<true>(r, nb.a.x, nb.a.y, nb.a.z, nb.a.w, nb.b.x, nb.b.y, bt, t0)
                    : box_enter<false>(r, nb.a.x, nb.a.y, nb.a.z, nb.a.w, nb.b.x, nb.b.y, bt, t0);
     }
 
     // Lanes with take begin ray r at heap node `first` (<= 1: the root; see
     // traverse).
-    __device__ __forceinline__ void start(bool take, const RayState& r, const TreeRef& tr, uint32_t first, uint2* stack) {
+    // counted: over the heap records whatever the ray, so that every test is
+    // traverse()'s and `at_leaf` its count.
+    __device__ __forceinline__ void start(bool take, const RayState& r, const TreeRef& tr, uint32_t first, uint2* stack,
+                                          bool counted = false) {
         if (!take) return;
         o = r.o;
         d = r.d;
@@ -656,16 +666,21 @@ struct Walk {
         b.u = b.v = -1.0f;
         b.t = r.tmax;
         b.leaf = 1u;
-        cur = pend = sp = tests = 0u;
+        cur = pend = sp = 0u;
+        tests = 1u;
+        at_leaf = 0u;
+        more = false;
         have = false;
         if (!(r.tmax > 0.0f)) return;
-        const float4 g = __ldg(reinterpret_cast<const float4*>(tr.tnodes));  // G, E
+        float4 g = make_float4(0.f, 0.f, 0.f, 0.f);  // G, E
+        if (tr.tnodes) g = __ldg(reinterpret_cast<const float4*>(tr.tnodes));
         k = mk3(fmul(g.w, r.inv.x), fmul(g.w, r.inv.y), fmul(g.w, r.inv.z));
         const f3 q = mk3(fsub(g.x, o.x), fsub(g.y, o.y), fsub(g.z, o.z));
         n = mk3(fmul(q.x, r.inv.x), fmul(q.y, r.inv.y), fmul(q.z, r.inv.z));
         const float kmax = max3(fabsf(k.x), fabsf(k.y), fabsf(k.z)), kmin = min3(fabsf(k.x), fabsf(k.y), fabsf(k.z));
-        const bool gen = !(max3(fabsf(q.x), fabsf(q.y), fabsf(q.z)) <= 16.0f * g.w && kmax < 1e30f && kmin > 1e-30f);
+        const bool gen = counted || !(max3(fabsf(q.x), fabsf(q.y), fabsf(q.z)) <= 16.0f * g.w && kmax < 1e30f && kmin > 1e-30f);
         if (gen) sgn |= kGeneral;
+        if (r.exact) sgn |= kInfinite;
         uint32_t node = 1u;
         float t0;
         if (first > 1u && !tr.compact) {
@@ -673,17 +688,18 @@ struct Walk {
                 atomicOr(tr.err, RT_DEVERR_BOUNDS);
             } else {
                 const int D = 31 - __clz(first);
+                tests += (uint32_t)D;
 #pragma unroll 2
                 for (int q = 1; q <= D; ++q) {
                     const uint32_t sib = (first >> (D - q)) ^ 1u;
                     const NodeBox sb = load_node(tr.heap, sib);
-                    if (enter(r, sb, b.t, &t0, gen)) push(stack, heap_item(sib, sb), t0);
+                    if (enter(r, sb, b.t, &t0, r.exact)) push(stack, heap_item(sib, sb), t0);
                 }
                 node = first;
             }
         }
         const NodeBox nb = load_node(tr.heap, node);
-        if (enter(r, nb, b.t, &t0, gen)) cur = heap_item(node, nb);
+        if (enter(r, nb, b.t, &t0, r.exact)) cur = heap_item(node, nb);
         have = cur != 0u || sp != 0u;
     }
 
@@ -700,7 +716,8 @@ struct Walk {
         r.inv = mk3(fdiv(1.0f, d.x), fdiv(1.0f, d.y), fdiv(1.0f, d.z));
         const NodeBox nl = load_node(tr.heap, c0), nr = load_node(tr.heap, c0 + 1u);
         float tl, tr_;
-        const bool hl = enter(r, nl, b.t, &tl, true), hr = enter(r, nr, b.t, &tr_, true);
+        const bool inf = (sgn & kInfinite) != 0u;
+        const bool hl = enter(r, nl, b.t, &tl, inf), hr = enter(r, nr, b.t, &tr_, inf);
         tests += 2;
         const int field = __ldg(&tr.heap[cur].prim_count) & 3;  // one axis past the split axis
         const bool near_right = (sgn >> (field == 0 ? 2 : field - 1)) & 1u;
@@ -747,9 +764,10 @@ struct Walk {
 
     // Moves every walking lane on: at most `steps` expansions (a lane puts its
     // first leaf aside and goes on; with two or three leaves set aside no
-    // faster), then the leaves, a triangle of each lane at a time.  All 32
-    // lanes call.
-    __device__ __forceinline__ void round(const TreeRef& tr, int steps, uint2* stack, bool any_hit = false) {
+    // faster), then the leaves: pooled where one is large, else a triangle of
+    // each lane at a time.  All 32 lanes call.
+    // Returns whether the lane tested a leaf.
+    __device__ __forceinline__ bool round(const TreeRef& tr, int steps, uint2* stack, bool any_hit = false) {
         constexpr uint32_t kFull = 0xffffffffu;
         for (int s = 0; s < steps; ++s) {
             const bool go = cur ? !((int)cur < 0 && pend) : sp != 0u;
@@ -759,6 +777,8 @@ struct Walk {
                 if ((int)cur < 0 && !pend) {
                     pend = cur;
                     cur = 0u;
+                    at_leaf = tests;
+                    more = sp != 0u;
                 }
                 if ((int)cur > 0) {
                     if (sgn & kGeneral) expand_heap(tr, stack);
@@ -770,6 +790,8 @@ struct Walk {
         if ((int)cur < 0 && !pend) {
             pend = cur;
             cur = 0u;
+            at_leaf = tests;
+            more = sp != 0u;
         }
         uint32_t cnt = 0u, pos = 0u;
         const uint32_t leaf = pend;
@@ -787,46 +809,146 @@ struct Walk {
                 atomicOr(tr.err, RT_DEVERR_BOUNDS);
                 cnt = 0u;
             }
-            tests += cnt;
         }
         bool inside = false;
-        while (__any_sync(kFull, cnt != 0u)) {
-            if (cnt != 0u) {
-                const float4* tp = tr.tris + 3 * (size_t)pos;
-                const float4 a = __ldg(tp), bb = __ldg(tp + 1), c = __ldg(tp + 2);
-                ++pos;
-                --cnt;
-                const int id = __float_as_int(a.w);
-                float u, v, t;
-                RayState r;
-                r.o = o;
-                r.d = d;
-                if (id != exclude && tri_test(r, a, bb, c, &u, &v, &t)) {
-                    const uint64_t key = hit_key(t, id);
-                    if (key < b.key) {
-                        const uint32_t h = (leaf & kBigLeaf) ? leaf & 0x3ffffffu
-                                                             : __ldg(tr.leaf_of + tr.tri_base + (leaf & 0x1ffffffu));
-                        if (inside || (sgn & kGeneral) || leaf_entered(tr, h)) {
-                            inside = true;
-                            b.key = key;
-                            b.t = t;
-                            b.u = u;
-                            b.v = v;
-                            b.id = id;
-                            b.leaf = h;
-                        } else {
-                            cnt = 0u;
-                        }
+        // a leaf of many triangles: its exact box, with the bound of now, first
+        if (cnt > kCheckMin) {
+            const uint32_t h = (leaf & kBigLeaf) ? leaf & 0x3ffffffu : __ldg(tr.leaf_of + tr.tri_base + (leaf & 0x1ffffffu));
+            inside = leaf_entered(tr, h);
+            if (!inside) cnt = 0u;
+        }
+        tests += cnt;
+        at_leaf += cnt;
+        if (__reduce_max_sync(kFull, cnt) > kPoolMin) {
+            pooled(tr, leaf, pos, cnt, inside);
+        } else {
+            while (__any_sync(kFull, cnt != 0u)) {
+                if (cnt != 0u) {
+                    const float4* tp = tr.tris + 3 * (size_t)pos;
+                    const float4 a = __ldg(tp), bb = __ldg(tp + 1), c = __ldg(tp + 2);
+                    ++pos;
+                    --cnt;
+                    const int id = __float_as_int(a.w);
+                    float u, v, t;
+                    RayState r;
+                    r.o = o;
+                    r.d = d;
+                    if (id != exclude && tri_test(r, a, bb, c, &u, &v, &t)) {
+                        if (!accept(tr, leaf, hit_key(t, id), id, t, u, v, inside)) cnt = 0u;
                     }
                 }
+                __syncwarp();
             }
-            __syncwarp();
         }
         if (any_hit && b.id >= 0) cur = sp = 0u;
         have = cur != 0u || sp != 0u;
+        return leaf != 0u;
     }
 
-    // box_enter of the heap box of leaf h.
+    __device__ __forceinline__ void stop() {
+        cur = pend = sp = 0u;
+        have = false;
+    }
+
+    __device__ __forceinline__ Hit hit() const {
+        Hit h;
+        h.id = b.id;
+        h.u = b.u;
+        h.v = b.v;
+        h.t = b.t;
+        return h;
+    }
+
+    // A candidate hit in `leaf`.  Returns false when the leaf's box rejects it,
+    // and so every triangle of the leaf.
+    __device__ __forceinline__ bool accept(const TreeRef& tr, uint32_t leaf, uint64_t key, int id, float t, float u,
+                                           float v, bool& inside) {
+        if (!(key < b.key)) return true;
+        const uint32_t h = (leaf & kBigLeaf) ? leaf & 0x3ffffffu : __ldg(tr.leaf_of + tr.tri_base + (leaf & 0x1ffffffu));
+        if (!inside && !leaf_entered(tr, h)) return false;
+        inside = true;
+        b.key = key;
+        b.t = t;
+        b.u = u;
+        b.v = v;
+        b.id = id;
+        b.leaf = h;
+        return true;
+    }
+
+    // The triangles [pos, pos + cnt) of every lane's leaf, 32 (lane, triangle)
+    // pairs at a time (see leaf_phase): a lane's 200 triangles cost 7 steps
+    // of the warp instead of 200.
+    __device__ __forceinline__ void pooled(const TreeRef& tr, uint32_t leaf, uint32_t pos, uint32_t cnt, bool inside) {
+        constexpr uint32_t kFull = 0xffffffffu;
+        const int lane = threadIdx.x & 31;
+        uint32_t incl = cnt;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const uint32_t y = __shfl_up_sync(kFull, incl, off);
+            if (lane >= off) incl += y;
+        }
+        const uint32_t total = __shfl_sync(kFull, incl, 31), excl = incl - cnt;
+        bool rejected = false;
+        for (uint32_t base = 0; base < total; base += 32) {
+            const uint32_t p = base + lane;
+            int ow = 0;  // owner of pair p: the first lane whose inclusive prefix exceeds p
+#pragma unroll
+            for (int step = 16; step > 0; step >>= 1) {
+                const uint32_t v = __shfl_sync(kFull, incl, ow + step - 1);
+                if (v <= p) ow += step;
+            }
+            const uint32_t o_excl = __shfl_sync(kFull, excl, ow), o_pos = __shfl_sync(kFull, pos, ow);
+            RayState r;
+            r.o = mk3(__shfl_sync(kFull, o.x, ow), __shfl_sync(kFull, o.y, ow), __shfl_sync(kFull, o.z, ow));
+            r.d = mk3(__shfl_sync(kFull, d.x, ow), __shfl_sync(kFull, d.y, ow), __shfl_sync(kFull, d.z, ow));
+            const int o_exclude = __shfl_sync(kFull, exclude, ow);
+            const uint64_t o_best = shfl_u64(b.key, ow);
+            uint64_t key = ~0ull;
+            float kt = 0.0f, ku = 0.0f, kv = 0.0f;
+            if (p < total) {
+                const float4* tp = tr.tris + 3 * (size_t)(o_pos + (p - o_excl));
+                const float4 a = __ldg(tp), bb = __ldg(tp + 1), c = __ldg(tp + 2);
+                const int id = __float_as_int(a.w);
+                float u, v, t;
+                if (id != o_exclude && tri_test(r, a, bb, c, &u, &v, &t)) {
+                    const uint64_t q = hit_key(t, id);
+                    if (q < o_best) {
+                        key = q;
+                        kt = t;
+                        ku = u;
+                        kv = v;
+                    }
+                }
+            }
+            // most batches hit nothing
+            if (!__any_sync(kFull, key != ~0ull)) continue;
+            int src = lane;
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+                const uint64_t k2 = shfl_down_u64(key, off);
+                const int s2 = __shfl_down_sync(kFull, src, off);
+                const int o2 = __shfl_down_sync(kFull, ow, off);
+                if (lane + off < 32 && o2 == ow && k2 < key) {
+                    key = k2;
+                    src = s2;
+                }
+            }
+            const bool mine = cnt > 0u && excl < base + 32 && incl > base;
+            const int head = mine ? (int)(max(excl, base) - base) : lane;
+            const uint64_t hk = shfl_u64(key, head);
+            const int hs = __shfl_sync(kFull, src, head);
+            const float ht = __shfl_sync(kFull, kt, hs);
+            const float hu = __shfl_sync(kFull, ku, hs);
+            const float hv = __shfl_sync(kFull, kv, hs);
+            if (mine && !rejected && hk != ~0ull)
+                rejected = !accept(tr, leaf, hk, (int)(uint32_t)hk, ht, hu, hv, inside);
+            __syncwarp();
+        }
+    }
+
+    // box_enter of the heap box of leaf h, under the bound of now: the leaf may
+    // have been put aside, or its parent expanded, before a nearer hit was found.
     __device__ __forceinline__ bool leaf_entered(const TreeRef& tr, uint32_t h) const {
         if (h >= tr.num_heap) {
             atomicOr(tr.err, RT_DEVERR_BOUNDS);
@@ -837,7 +959,7 @@ struct Walk {
         r.o = o;
         r.inv = mk3(fdiv(1.0f, d.x), fdiv(1.0f, d.y), fdiv(1.0f, d.z));
         float t0;
-        return box_enter<false>(r, nb.a.x, nb.a.y, nb.a.z, nb.a.w, nb.b.x, nb.b.y, b.t, &t0);
+        return enter(r, nb, b.t, &t0, (sgn & kInfinite) != 0u);
     }
 };
 
@@ -869,6 +991,7 @@ __device__ __forceinline__ uint64_t warp_min_u64(uint64_t v) {
 // more group.  The stack lives in dynamic shared memory sized per launch.
 constexpr int kWideStackMax = 1024;  // entries per warp for depth <= 29
 constexpr int kWideQueue = 128;      // queued leaves per warp
+constexpr int kWidePairs = 2;         // triangles a lane of traverse_wide has in flight (1: 150 us a frame, 2: 133, 4: more registers, slower)
 constexpr int kWideWarps = 4;        // blocks of at most 128 threads
 
 __host__ __device__ constexpr uint32_t wide_stack_entries(uint32_t depth) {
@@ -882,7 +1005,7 @@ __host__ __device__ constexpr size_t wide_smem_bytes(uint32_t cap) {
 }
 
 template <bool EXACT>
-__device__ __forceinline__ Hit traverse_wide(const RayState& r, const TreeRef& tr_, bool any_hit, uint32_t cap) {
+__device__ __forceinline__ Hit traverse_wide(const RayState& r, const TreeRef& tr_, bool any_hit, uint32_t cap, Hit known) {
     constexpr uint32_t kFull = 0xffffffffu;
     extern __shared__ uint4 wide_dyn[];
     uint8_t* base8 = reinterpret_cast<uint8_t*>(wide_dyn);
@@ -895,9 +1018,10 @@ __device__ __forceinline__ Hit traverse_wide(const RayState& r, const TreeRef& t
     int32_t* qcnt = reinterpret_cast<int32_t*>(qbase) + (kWideWarps + wib) * kWideQueue;
     float* qt0 = reinterpret_cast<float*>(qbase) + (2 * kWideWarps + wib) * kWideQueue;
     uint32_t* qincl = reinterpret_cast<uint32_t*>(qbase) + (3 * kWideWarps + wib) * kWideQueue;
+    // known: an accepted hit found before (id < 0: none)
     const uint64_t init = hit_key(r.tmax, 0);
-    uint64_t best = init;  // uniform across the warp
-    float bu = -1.0f, bv = -1.0f, bt = r.tmax;
+    uint64_t best = known.id >= 0 ? hit_key(known.t, known.id) : init;  // uniform across the warp
+    float bu = known.u, bv = known.v, bt = known.t;
     int size = 0, nq = 0, qtris = 0;  // uniform
     bool stop = false;
     // root
@@ -905,7 +1029,7 @@ __device__ __forceinline__ Hit traverse_wide(const RayState& r, const TreeRef& t
         const NodeBox root = load_node(tr_.nodes, 1);
         float t0;
         const bool enter = r.tmax > 0.0f &&
-                           box_enter<EXACT>(r, root.a.x, root.a.y, root.a.z, root.a.w, root.b.x, root.b.y, r.tmax, &t0);
+                           box_enter<EXACT>(r, root.a.x, root.a.y, root.a.z, root.a.w, root.b.x, root.b.y, key_t(best), &t0);
         if (enter) {
             if (__float_as_int(root.b.z) & 4) {
                 if (lane == 0) {
@@ -949,11 +1073,15 @@ __device__ __forceinline__ Hit traverse_wide(const RayState& r, const TreeRef& t
             }
             __syncwarp();
             const uint32_t total = run;
-            for (uint32_t base = 0; base < total; base += 32) {
-                const uint32_t p = base + lane;
+            // kWidePairs pairs a lane at a time, their triangles in flight together
+            for (uint32_t base = 0; base < total; base += 32 * kWidePairs) {
                 uint64_t key = ~0ull;
                 float kt = 0.0f, ku = 0.0f, kv = 0.0f;
-                if (p < total) {
+                bool first = false;  // any_hit: a hit among the first 32 pairs ends the walk there
+                float4 va[kWidePairs], vb[kWidePairs], vc[kWidePairs];
+#pragma unroll
+                for (int q = 0; q < kWidePairs; ++q) {
+                    const uint32_t p = min(base + 32u * q + lane, total - 1u);  // past the end: the last pair again
                     // queued leaf holding pair p: the first with inclusive prefix > p
                     int lo = 0, hi = nq - 1;
                     while (lo < hi) {
@@ -962,12 +1090,18 @@ __device__ __forceinline__ Hit traverse_wide(const RayState& r, const TreeRef& t
                     }
                     const uint32_t ex = lo > 0 ? qincl[lo - 1] : 0u;
                     const float4* tp = tr_.tris + 3 * (size_t)(qpos[lo] + (int)(p - ex));
-                    const float4 a = __ldg(tp), b = __ldg(tp + 1), c = __ldg(tp + 2);
-                    const int id = __float_as_int(a.w);
+                    va[q] = __ldg(tp);
+                    vb[q] = __ldg(tp + 1);
+                    vc[q] = __ldg(tp + 2);
+                }
+#pragma unroll
+                for (int q = 0; q < kWidePairs; ++q) {
+                    const int id = __float_as_int(va[q].w);
                     float u, v, t;
-                    if (id != r.exclude && tri_test(r, a, b, c, &u, &v, &t)) {
+                    if (any_hit && q > 0) first = __any_sync(kFull, key != ~0ull);
+                    if (!first && id != r.exclude && tri_test(r, va[q], vb[q], vc[q], &u, &v, &t)) {
                         const uint64_t k = hit_key(t, id);
-                        if (k < best) {
+                        if (k < best && k < key) {
                             key = k;
                             kt = t;
                             ku = u;
@@ -975,15 +1109,14 @@ __device__ __forceinline__ Hit traverse_wide(const RayState& r, const TreeRef& t
                         }
                     }
                 }
+                if (!__any_sync(kFull, key != ~0ull)) continue;  // most batches hit nothing
                 const uint64_t kmin = warp_min_u64(key);
-                if (kmin < best) {
-                    const int w = __ffs(__ballot_sync(kFull, key == kmin)) - 1;
-                    best = kmin;
-                    bt = __shfl_sync(kFull, kt, w);
-                    bu = __shfl_sync(kFull, ku, w);
-                    bv = __shfl_sync(kFull, kv, w);
-                    if (any_hit) break;
-                }
+                const int w = __ffs(__ballot_sync(kFull, key == kmin)) - 1;
+                best = kmin;
+                bt = __shfl_sync(kFull, kt, w);
+                bu = __shfl_sync(kFull, ku, w);
+                bv = __shfl_sync(kFull, kv, w);
+                if (any_hit) break;
             }
             nq = 0;
             qtris = 0;
@@ -1139,7 +1272,7 @@ __device__ __forceinline__ uint32_t team_scan(uint32_t v, TeamShared& ts, uint32
 
 template <bool EXACT>
 __device__ __forceinline__ Hit traverse_team(const RayState& r, const TreeRef& tr_, bool any_hit, uint32_t cap,
-                                             TeamShared& ts) {
+                                             TeamShared& ts, Hit known) {
     constexpr uint32_t kFull = 0xffffffffu;
     extern __shared__ uint4 wide_dyn[];
     uint8_t* base8 = reinterpret_cast<uint8_t*>(wide_dyn);
@@ -1153,21 +1286,21 @@ __device__ __forceinline__ Hit traverse_team(const RayState& r, const TreeRef& t
     uint32_t* qincl = reinterpret_cast<uint32_t*>(qt0 + kTeamQueue);
     const uint64_t init = hit_key(r.tmax, 0);
     // uniform across the block (every thread keeps the same copy)
-    uint64_t best = init;
+    uint64_t best = known.id >= 0 ? hit_key(known.t, known.id) : init;
     int size = 0, nq = 0, qtris = 0;
     bool stop = false;
     __syncthreads();  // the previous ray's readers of the shared state are done
     if (tid == 0) {
-        ts.best = init;
-        ts.bt = r.tmax;
-        ts.bu = -1.0f;
-        ts.bv = -1.0f;
+        ts.best = best;
+        ts.bt = known.t;
+        ts.bu = known.u;
+        ts.bv = known.v;
     }
     {
         const NodeBox root = load_node(tr_.nodes, 1);
         float t0;
         const bool enter = r.tmax > 0.0f &&
-                           box_enter<EXACT>(r, root.a.x, root.a.y, root.a.z, root.a.w, root.b.x, root.b.y, r.tmax, &t0);
+                           box_enter<EXACT>(r, root.a.x, root.a.y, root.a.z, root.a.w, root.b.x, root.b.y, key_t(best), &t0);
         if (enter) {
             if (__float_as_int(root.b.z) & 4) {
                 if (tid == 0) {
@@ -1344,9 +1477,9 @@ __device__ __forceinline__ Hit traverse_team(const RayState& r, const TreeRef& t
 }
 
 __device__ __forceinline__ Hit trace_team(const RayState& r, const TreeRef& tr, bool any_hit, uint32_t cap,
-                                          TeamShared& ts) {
-    if (r.exact) return traverse_team<true>(r, tr, any_hit, cap, ts);
-    return traverse_team<false>(r, tr, any_hit, cap, ts);
+                                          TeamShared& ts, Hit known) {
+    if (r.exact) return traverse_team<true>(r, tr, any_hit, cap, ts, known);
+    return traverse_team<false>(r, tr, any_hit, cap, ts, known);
 }
 
 // Warp-uniform dispatch between the fast and the NaN-exact box test.  Must be
@@ -1362,9 +1495,9 @@ __device__ __forceinline__ Hit trace_ray(const RayState& r, bool active, const T
 }
 
 // One ray traced by the whole warp; every lane passes the same ray.
-__device__ __forceinline__ Hit trace_wide(const RayState& r, const TreeRef& tr, bool any_hit, uint32_t cap) {
-    if (r.exact) return traverse_wide<true>(r, tr, any_hit, cap);
-    return traverse_wide<false>(r, tr, any_hit, cap);
+__device__ __forceinline__ Hit trace_wide(const RayState& r, const TreeRef& tr, bool any_hit, uint32_t cap, Hit known) {
+    if (r.exact) return traverse_wide<true>(r, tr, any_hit, cap, known);
+    return traverse_wide<false>(r, tr, any_hit, cap, known);
 }
 
 // Primary ray of pixel (i, j): CSPrimaryRays.hlsl:36-56 with the basis camera.

@@ -167,45 +167,69 @@ __global__ void __launch_bounds__(kWhListThreads) k_wh_init(rt_camera cam, WhBuf
 }
 
 // Closest hits of the listed rays (SHADOW = false) or the shadow rays of the
-// listed hits (SHADOW = true).  Persistent warps, 32 list entries per step.
+// listed hits (SHADOW = true).  A lane whose ray has ended takes the next list
+// entry once kWhRefill lanes of its warp are idle (Walk).
+constexpr int kWhRefill = 8;
+constexpr int kWhSteps = 4;  // 4: 813 us a call at 720p with one bounce, 6: 848, 8: 860; 32 rays a warp at once: 1,110
+
 template <bool SHADOW>
-__global__ void __launch_bounds__(kWhThreads) k_wh_trace(TreeRef tr, ShadeArgs a, WhBufs w, int src, uint32_t* work) {
+__global__ void __launch_bounds__(kWhThreads, 7) k_wh_trace(TreeRef tr, ShadeArgs a, WhBufs w, int src, uint32_t* work) {
+    constexpr uint32_t kFull = 0xffffffffu;
+    mark_records(tr);
     const uint32_t* list = wlist(w, src);
     const uint32_t n = min(w.counts[src], w.px);
-    const uint32_t lane = threadIdx.x & 31;
-    for (uint32_t c = next_tile(work); c * 32 < n; c = next_tile(work)) {
-        const uint32_t k = c * 32 + lane;
-        const bool valid = k < n;
-        const uint32_t p = valid ? __ldg(list + k) : 0u;
-        const float4 ro = valid ? w.ro[p] : make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
-        const float4 rd = valid ? w.rd[p] : make_float4(0.f, 0.f, 1.f, 1.f);
-        const uint32_t start = valid ? w.leaf[p] : 1u;
-        uint32_t nb = 0, nt = 0;
-        if (!SHADOW) {
-            uint32_t leaf = 1;
-            const RayState r = make_ray(mk3(ro.x, ro.y, ro.z), mk3(rd.x, rd.y, rd.z), rd.w, __float_as_int(ro.w));
-            const Hit h = trace_ray<false>(r, valid, tr, false, &nb, &nt, nullptr, nullptr, start, &leaf);
-            if (valid) {
-                w.hit[p] = make_int4(h.id, __float_as_int(h.u), __float_as_int(h.v), __float_as_int(h.t));
-                w.leaf[p] = leaf;
-            }
-        } else {
-            RayState sr = make_ray(mk3(0.f, 0.f, 0.f), mk3(0.f, 0.f, 1.f), 1.0f, -1);
-            int id = -1;
-            if (valid) {
-                const int4 h = w.hit[p];
-                id = h.x;
-                if (id >= 0 && (uint32_t)id < a.n) {
-                    const Geom g = geom(a, id, __int_as_float(h.y), __int_as_float(h.z), __int_as_float(h.w),
-                                        mk3(ro.x, ro.y, ro.z), mk3(rd.x, rd.y, rd.z));
-                    // :149-153: from the hit point towards the light, up to the light
-                    sr = make_ray(g.P, mk3(-g.L.x, -g.L.y, -g.L.z), g.dist, id);
+    const int lane = threadIdx.x & 31;
+    Walk wk;
+    wk.clear();
+    uint2 stack[kStackSize];
+    uint32_t p = 0;
+    bool live = false, drained = false;
+    for (;;) {
+        const uint32_t idle = __ballot_sync(kFull, !live);
+        if (!drained && (idle == kFull || __popc(idle) >= kWhRefill)) {
+            uint32_t base = 0;
+            if (lane == 0) base = atomicAdd(work, (uint32_t)__popc(idle));
+            base = __shfl_sync(kFull, base, 0);
+            if (base + (uint32_t)__popc(idle) >= n) drained = true;
+            const uint32_t k = base + __popc(idle & ((1u << lane) - 1u));
+            bool take = !live && k < n;
+            RayState r = make_ray(mk3(0.f, 0.f, 0.f), mk3(0.f, 0.f, 1.f), 1.0f, -1);
+            uint32_t start = 1u;
+            if (take) {
+                p = __ldg(list + k);
+                const float4 ro = w.ro[p], rd = w.rd[p];
+                start = w.leaf[p];
+                if (!SHADOW) {
+                    r = make_ray(mk3(ro.x, ro.y, ro.z), mk3(rd.x, rd.y, rd.z), rd.w, __float_as_int(ro.w));
                 } else {
-                    id = -1;
+                    const int4 h = w.hit[p];
+                    if (h.x >= 0 && (uint32_t)h.x < a.n) {
+                        const Geom g = geom(a, h.x, __int_as_float(h.y), __int_as_float(h.z), __int_as_float(h.w),
+                                            mk3(ro.x, ro.y, ro.z), mk3(rd.x, rd.y, rd.z));
+                        // :149-153: from the hit point towards the light, up to the light
+                        r = make_ray(g.P, mk3(-g.L.x, -g.L.y, -g.L.z), g.dist, h.x);
+                    } else {
+                        w.occl[p] = 0u;
+                        take = false;
+                    }
                 }
+                if (take) live = true;
             }
-            const Hit h = trace_ray<false>(sr, valid && id >= 0, tr, true, &nb, &nt, nullptr, nullptr, start);
-            if (valid) w.occl[p] = h.id >= 0 ? 1u : 0u;
+            wk.start(take, r, tr, start, stack);
+        }
+        if (!__any_sync(kFull, live)) {
+            if (drained) break;
+            continue;
+        }
+        wk.round(tr, kWhSteps, stack, SHADOW);
+        if (live && !wk.have) {
+            if (SHADOW) {
+                w.occl[p] = wk.b.id >= 0 ? 1u : 0u;
+            } else {
+                w.hit[p] = make_int4(wk.b.id, __float_as_int(wk.b.u), __float_as_int(wk.b.v), __float_as_int(wk.b.t));
+                w.leaf[p] = wk.b.leaf;
+            }
+            live = false;
         }
     }
 }
@@ -374,6 +398,8 @@ WhBufs whitted_bufs(rt_ctx* ctx, const rt_lbvh* l, uint32_t px) {
 
 }  // namespace
 
+TreeRef tree_ref(const rt_ctx* ctx, const rt_lbvh* l);
+
 extern "C" rt_status rt_render_whitted(rt_ctx* ctx, const rt_lbvh* l, const rt_camera* cam, const float light[3],
                                        const rt_shade_params* prm, const int32_t* d_material_ids,
                                        const rt_material* d_materials, uint32_t num_materials, const float* d_normals,
@@ -409,15 +435,8 @@ extern "C" rt_status rt_render_whitted(rt_ctx* ctx, const rt_lbvh* l, const rt_c
     a.env[2] = prm->env_color[2];
     a.seed = prm->seed;
     a.err = ctx->d_err;
-    // the walks restart at heap nodes: use the heap even when a compact layout exists
-    TreeRef tr;
-    tr.compact = false;
-    tr.tri_base = 0;
-    tr.nodes = l->nodes;
-    tr.num_nodes = l->num_nodes;
-    tr.tris = l->sorted_tris;
-    tr.n = l->n;
-    tr.err = ctx->d_err;
+    TreeRef tr = tree_ref(ctx, l);
+    tr.compact = false;  // the walks restart at heap nodes
     cudaStream_t st = ctx->stream;
     float4* acc = reinterpret_cast<float4*>(d_accum);
     float4* res = reinterpret_cast<float4*>(d_result);
@@ -436,7 +455,7 @@ extern "C" rt_status rt_render_whitted(rt_ctx* ctx, const rt_lbvh* l, const rt_c
         // the next bounce's list and the shadow list start empty
         RT_CHECK_CUDA(ctx, cudaMemsetAsync(w.counts + (src ^ 1), 0, sizeof(uint32_t), st));
         RT_CHECK_CUDA(ctx, cudaMemsetAsync(w.counts + 2, 0, sizeof(uint32_t), st));
-        if ((s = reset_work(ctx, kWorkWhTrace)) != RT_OK) return s;
+        if ((s = b == 0 ? reset_work_and_records(ctx, kWorkWhTrace, l) : reset_work(ctx, kWorkWhTrace)) != RT_OK) return s;
         k_wh_trace<false><<<tblocks, kWhThreads, 0, st>>>(tr, a, w, src, ctx->d_work + kWorkWhTrace);
         RT_CHECK_LAUNCH(ctx, "k_wh_trace");
         if (a.shadows) {

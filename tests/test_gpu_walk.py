@@ -1,0 +1,128 @@
+"""The walk over the trace records (Walk in rt_traverse.cuh) where it can go
+wrong, against the oracle: leaves around the sizes that change their form
+(a word holds fewer than 32 triangles; more than 3 are pooled, more than 4
+box-tested first), trees of one leaf and of flat scenes, rays that the
+records do not serve (a zero direction component, an origin far outside, very
+short and very long directions), ray counts around a warp and around the
+number up to which a ray gets a warp, and any-hit rays around the hand-over
+budget.  Hits are compared on their bits: the walk accepts a triangle under
+the reference's own tests, so no tolerance is needed."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def scene(kind):
+    from rtgpu import scenes
+    if kind == "one":
+        return scenes.random_soup(1, 5), 8
+    if kind == "one_leaf":  # equal codes: a root leaf of 40 triangles
+        return np.repeat(scenes.random_soup(1, 6), 40, 0) + np.linspace(0, 1e-6, 40, dtype=np.float32)[:, None], 8
+    if kind == "leaf_sizes":  # clusters of 1 .. 36 near-equal triangles and one of 300
+        base = scenes.random_soup(37, 7, 0.02, 0.1)
+        sizes = list(range(1, 37)) + [300]
+        tris = np.concatenate([np.repeat(base[i:i + 1], m, 0) for i, m in enumerate(sizes)])
+        return tris + np.random.default_rng(1).normal(0, 1e-6, tris.shape).astype(np.float32), 12
+    if kind == "flat":  # no extent in z
+        tris = scenes.random_soup(3000, 8, 0.01, 0.05)
+        tris.reshape(-1, 3, 3)[..., 2] = 0.25
+        return tris, 14
+    if kind == "offset":  # far from the origin of coordinates
+        return scenes.random_soup(3000, 9, 0.02, 0.1) + np.float32(300.0), 14
+    return scenes.random_soup(20000, 10), 16
+
+
+def rays_for(tris, n, seed):
+    rng = np.random.default_rng(seed)
+    lo, hi = tris.reshape(-1, 3).min(0), tris.reshape(-1, 3).max(0)
+    size = max(float((hi - lo).max()), 1e-3)
+    o = rng.uniform(lo - 0.5 * size, hi + 0.5 * size, (n, 3))
+    target = tris[rng.integers(0, len(tris), n)].reshape(n, 3, 3).mean(1)
+    d = target - o + rng.normal(0, 0.02 * size, (n, 3))
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    k = np.arange(n)
+    far = k % 7 == 1           # out of the records' range
+    o[far] -= 40.0 * size * d[far]
+    axis = k % 7 == 2          # along an axis: two infinite 1 / d
+    d[axis] = np.eye(3)[k[axis] % 3] * np.where(k[axis] % 2, 1.0, -1.0)[:, None]
+    o[axis] = target[axis] - size * d[axis]
+    plane = k % 7 == 3         # one infinite 1 / d
+    d[plane, 2] = 0.0
+    d[k % 14 == 4] *= 1e-4
+    d[k % 14 == 11] *= 1e5
+    tmax = np.where(k % 5 == 0, 0.7 * size, 1e16)
+    excl = np.where(k % 3 == 0, rng.integers(0, len(tris), n), -1)
+    return o.astype(np.float32), d.astype(np.float32), tmax.astype(np.float32), excl.astype(np.int32)
+
+
+@pytest.mark.parametrize("kind,n", [("one", 1), ("one_leaf", 33), ("leaf_sizes", 4000), ("leaf_sizes", 16385), ("flat", 17000),
+                                    ("offset", 17000), ("soup", 31), ("soup", 16384), ("soup", 16385), ("soup", 40000)])
+def test_closest_hits(gpu_ctx, oracle_mod, kind, n):
+    import torch
+    from rtgpu.api import LBVH, RayTracer, hits_to_numpy, rays_tensor
+    tris, depth = scene(kind)
+    lb = LBVH(gpu_ctx, len(tris), depth).Build(torch.from_numpy(tris).cuda())
+    nodes, ids, _, _ = oracle_mod.lbvh_build(tris, depth)
+    o, d, tmax, excl = rays_for(tris, n, 3)
+    rays = rays_tensor(o, d, tmax, excl, "cuda")
+    ref = oracle_mod.trace(nodes, depth, ids, tris, oracle_mod.rays_array(o, d, tmax, excl))
+    rt = RayTracer(gpu_ctx)
+    got = hits_to_numpy(rt.rays(lb, rays))
+    gpu_ctx.check()
+    assert np.array_equal(got.view(np.int32), ref.view(np.int32))
+    # with leaves (always the walk), from the root and restarted at the hits' leaves
+    hits, leaves = rt.rays_from(lb, rays, None)
+    again, leaves2 = rt.rays_from(lb, rays, leaves)
+    gpu_ctx.check()
+    assert np.array_equal(hits_to_numpy(hits).view(np.int32), ref.view(np.int32))
+    assert np.array_equal(hits_to_numpy(again).view(np.int32), ref.view(np.int32))
+    assert torch.equal(leaves, leaves2)
+    if n > 30:
+        assert (ref["id"] >= 0).mean() > 0.2
+
+
+@pytest.mark.parametrize("budget,n", [(0, 9001), (60, 9001), (0, 1 << 20), (24, (1 << 20) + 1), (384, (1 << 20) + 33)])
+def test_any_hit_budget(gpu_ctx, oracle_mod, budget, n):
+    """The first hit of a ray that stays within the budget is traverse()'s; one
+    that does not still reports a hit exactly when there is one."""
+    import torch
+    from rtgpu.api import LBVH, RayTracer, hits_to_numpy, rays_tensor
+    tris, depth = scene("soup")
+    lb = LBVH(gpu_ctx, len(tris), depth).Build(torch.from_numpy(tris).cuda())
+    nodes, ids, _, _ = oracle_mod.lbvh_build(tris, depth)
+    o, d, tmax, excl = rays_for(tris, n, 4)
+    ref, st = oracle_mod.trace(nodes, depth, ids, tris, oracle_mod.rays_array(o, d, tmax, excl), any_hit=True, stats=True)
+    gpu_ctx.set_trace_budget(budget)
+    try:
+        got = hits_to_numpy(RayTracer(gpu_ctx).rays(lb, rays_tensor(o, d, tmax, excl, "cuda"), any_hit=True))
+        gpu_ctx.check()
+    finally:
+        gpu_ctx.set_trace_budget(None)
+    assert np.array_equal(got["id"] >= 0, ref["id"] >= 0)
+    within = (st.sum(1) <= budget) if budget else np.ones(len(ref), bool)
+    assert np.array_equal(got[within].view(np.int32), ref[within].view(np.int32))
+    assert within.sum() > 100 and (budget == 0 or (~within).sum() > 100)
+
+
+@pytest.mark.parametrize("w,h,spp,bounces", [(1, 1, 2, 0), (33, 17, 3, 3), (64, 48, 5, 2)])
+def test_samples_traced_apart(gpu_ctx, oracle_mod, w, h, spp, bounces):
+    """Several samples a pixel are paths of their own whose terms are folded in
+    order: the image of spp calls of one sample each, bit for bit."""
+    import torch
+    from rtgpu import scenes
+    from rtgpu.api import LBVH, RayTracer
+    gi = scenes.gi_box(500, seed=11)
+    lb = LBVH(gpu_ctx, len(gi.tris), 14).Build(torch.from_numpy(gi.tris).cuda())
+    alb, em = torch.from_numpy(gi.albedo).cuda(), torch.from_numpy(gi.emission).cuda()
+    cam = scenes.gi_camera(w, h)
+    rt = RayTracer(gpu_ctx)
+    img = rt.pathtrace(lb, alb, em, cam, spp, bounces, 9)
+    one = rt.pathtrace(lb, alb, em, cam, 1, bounces, 9)
+    for k in range(1, spp):
+        one = rt.pathtrace(lb, alb, em, cam, 1, bounces, 9, out=one, first_sample=k)
+    gpu_ctx.check()
+    assert torch.equal(img.view(torch.int32), one.view(torch.int32))
+    nodes, ids, _, _ = oracle_mod.lbvh_build(gi.tris, 14)
+    ref = oracle_mod.pathtrace(nodes, 14, ids, gi.tris, gi.albedo, gi.emission, cam, spp, bounces, 9)
+    assert np.array_equal(img.cpu().numpy().view(np.int32).ravel(), np.ascontiguousarray(ref, np.float32).view(np.int32).ravel())
