@@ -1836,6 +1836,292 @@ __global__ void __launch_bounds__(THREADS) k_emit_merge(const uint2* __restrict_
     }
 }
 
+// k_build_small: the whole build of up to kSmallTris triangles in one block.  The
+// launches of the general build are a chain of a dozen kernels of one to a few
+// blocks each, whose latencies add up to 68 us however small the soup is; here a
+// phase costs a barrier.  Keys and ids are sorted in shared memory (the ranking
+// of k_onesweep), the record scans run over the block, and the bottom-up
+// (unit_bottom_up) takes all leaves at once, so nothing is left to merge.
+constexpr int kSmallThreads = 1024;
+constexpr int kSmallWarps = kSmallThreads / 32;
+constexpr uint32_t kSmallTris = 4 * kSmallThreads;
+constexpr uint32_t kSmallLeaf = 16;  // leaves above this many triangles are folded by a warp
+
+constexpr size_t small_smem(int items) {
+    const size_t n = (size_t)kSmallThreads * items;
+    const size_t sort = 4 * n + kSmallWarps * 256, units = (size_t)kUnitWords * n + 16;
+    return 4 * (sort > units ? sort : units);
+}
+
+template <int ITEMS>
+__global__ void __launch_bounds__(kSmallThreads, 1) k_build_small(const float* __restrict__ tris, uint32_t n, uint32_t depth,
+                                                                  uint32_t* __restrict__ keys, uint32_t* __restrict__ ids,
+                                                                  float4* sorted_tris, rt_node* nodes,
+                                                                  uint32_t* __restrict__ leaf_of, uint2* __restrict__ units,
+                                                                  uint32_t* __restrict__ counts, uint32_t tiles,
+                                                                  SceneInfo* scene, uint32_t* counters, uint32_t* err) {
+    constexpr uint32_t N = kSmallThreads * ITEMS;
+    extern __shared__ __align__(16) uint32_t smem[];
+    __shared__ uint32_t s_f[kSmallWarps], s_b[kSmallWarps], s_total, s_big, s_biglist[N / kSmallLeaf];
+    __shared__ float s_red[kSmallWarps][7];
+    __shared__ float s_par[6];
+    __shared__ uint2 s_items[kItemCap];
+    grid_dep_wait();
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+
+    // bounds (k_bounds)
+    {
+        float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
+        uint32_t bad = 0;
+        for (uint32_t v = t; v < 3 * n; v += kSmallThreads) {
+            const float p[3] = {__ldg(tris + 3 * v), __ldg(tris + 3 * v + 1), __ldg(tris + 3 * v + 2)};
+            for (int c = 0; c < 3; ++c) {
+                bad |= !isfinite(p[c]);
+                mn[c] = fminf(mn[c], p[c]);
+                mx[c] = fmaxf(mx[c], p[c]);
+            }
+        }
+        for (int off = 16; off > 0; off >>= 1)
+            for (int c = 0; c < 3; ++c) {
+                mn[c] = fminf(mn[c], __shfl_xor_sync(kFull, mn[c], off));
+                mx[c] = fmaxf(mx[c], __shfl_xor_sync(kFull, mx[c], off));
+            }
+        bad = __any_sync(kFull, bad);
+        if (lane == 0) {
+            for (int c = 0; c < 3; ++c) { s_red[w][c] = mn[c]; s_red[w][3 + c] = mx[c]; }
+            s_red[w][6] = bad ? 1.0f : 0.0f;
+        }
+        __syncthreads();
+        if (w == 0) {
+            float r[7];
+            for (int q = 0; q < 7; ++q) r[q] = s_red[lane][q];
+            for (int off = 16; off > 0; off >>= 1) {
+                for (int c = 0; c < 3; ++c) {
+                    r[c] = fminf(r[c], __shfl_xor_sync(kFull, r[c], off));
+                    r[3 + c] = fmaxf(r[3 + c], __shfl_xor_sync(kFull, r[3 + c], off));
+                }
+                r[6] = fmaxf(r[6], __shfl_xor_sync(kFull, r[6], off));
+            }
+            if (lane == 0) {
+                SceneInfo sc;
+                for (int c = 0; c < 3; ++c) {
+                    sc.bmin[c] = r[c];
+                    sc.bmax[c] = r[3 + c];
+                    const float mx3 = fmul(3.0f, r[3 + c]);           // LBVH.cpp:521-526
+                    s_par[c] = sc.lo3[c] = fmul(3.0f, r[c]);
+                    s_par[3 + c] = sc.f[c] = fdiv(1024.0f, fsub(mx3, sc.lo3[c]));
+                }
+                sc.nonfinite = r[6] != 0.0f;
+                sc.pad[0] = sc.pad[1] = sc.pad[2] = 0u;
+                *scene = sc;
+                if (sc.nonfinite) atomicOr(err, RT_DEVERR_NONFINITE);
+                counters[7] = 0u;  // the trace records are an earlier tree's
+                s_big = 0u;
+            }
+        }
+        __syncthreads();
+    }
+
+    // codes (k_morton_hist), element = warp * 32 * ITEMS + i * 32 + lane
+    uint32_t *ka = smem, *ia = ka + N, *kb = ia + N, *ib = kb + N, *hist = ib + N;
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+        const uint32_t k = w * (32 * ITEMS) + i * 32 + lane;
+        if (k < n) {
+            const float* p = tris + 9 * (size_t)k;
+            uint32_t q[3];
+            for (int c = 0; c < 3; ++c)
+                q[c] = quantize(fadd(fadd(__ldg(p + c), __ldg(p + 3 + c)), __ldg(p + 6 + c)), s_par[c], s_par[3 + c]);
+            ka[k] = (spread10(q[0]) << 2) | (spread10(q[1]) << 1) | spread10(q[2]);
+            ia[k] = k;
+        }
+    }
+    // stable LSD passes (k_onesweep with one tile)
+    const uint32_t lt = lanemask_lt();
+    for (int pass = 0; pass < kSortPasses; ++pass) {
+        for (int i = t; i < kSmallWarps * 256; i += kSmallThreads) hist[i] = 0u;
+        __syncthreads();
+        uint32_t key[ITEMS], idv[ITEMS], rank[ITEMS];
+        uint32_t* my = hist + w * 256;
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i) {
+            const uint32_t k = w * (32 * ITEMS) + i * 32 + lane;
+            const bool valid = k < n;
+            key[i] = valid ? ka[k] : 0xffffffffu;
+            idv[i] = valid ? ia[k] : 0u;
+            const uint32_t d = (key[i] >> (8 * pass)) & 0xffu;
+            uint32_t peers = __ballot_sync(kFull, valid);
+#pragma unroll
+            for (int b = 0; b < 8; ++b) {
+                const bool bit = (d >> b) & 1u;
+                const uint32_t m = __ballot_sync(kFull, bit);
+                peers &= bit ? m : ~m;
+            }
+            const uint32_t cnt = my[d];
+            __syncwarp();
+            if (valid && lane == __ffs(peers) - 1) my[d] = cnt + __popc(peers);
+            rank[i] = cnt + __popc(peers & lt);
+            __syncwarp();
+        }
+        __syncthreads();
+        // digit t / 4: four threads share its 32 warps' counts
+        const uint32_t dig = t >> 2, part = t & 3;
+        uint32_t sum = 0u;
+        for (int q = 0; q < kSmallWarps / 4; ++q) sum += hist[(part * (kSmallWarps / 4) + q) * 256 + dig];
+        uint32_t incl = sum;  // inclusive over all (digit, part) in order
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const uint32_t y = __shfl_up_sync(kFull, incl, off);
+            if (lane >= off) incl += y;
+        }
+        if (lane == 31) s_f[w] = incl;
+        __syncthreads();
+        uint32_t base = 0u;
+        for (int q = 0; q < w; ++q) base += s_f[q];
+        uint32_t run = base + incl - sum;
+        for (int q = 0; q < kSmallWarps / 4; ++q) {
+            uint32_t* c = hist + (part * (kSmallWarps / 4) + q) * 256 + dig;
+            const uint32_t v = *c;
+            *c = run;
+            run += v;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i) {
+            const uint32_t k = w * (32 * ITEMS) + i * 32 + lane;
+            if (k < n) {
+                const uint32_t g = my[(key[i] >> (8 * pass)) & 0xffu] + rank[i];
+                kb[g] = key[i];
+                ib[g] = idv[i];
+            }
+        }
+        __syncthreads();
+        uint32_t* x = ka; ka = kb; kb = x;
+        x = ia; ia = ib; ib = x;
+    }
+
+    // the sorted arrays and triangles
+    const bool soup_aligned = (reinterpret_cast<uintptr_t>(tris) & 15u) == 0;
+    for (uint32_t k = t; k < n; k += kSmallThreads) {
+        const uint32_t id = ia[k];
+        keys[k] = ka[k];
+        ids[k] = id;
+        float v[9];
+        load_tri(tris, id, n, soup_aligned, v);
+        sorted_tris[3 * k + 0] = make_float4(v[0], v[1], v[2], __int_as_float((int)id));
+        sorted_tris[3 * k + 1] = make_float4(v[3], v[4], v[5], 0.0f);
+        sorted_tris[3 * k + 2] = make_float4(v[6], v[7], v[8], 0.0f);
+    }
+
+    // ancestor masks (k_emit_units), elements t * ITEMS ..
+    const uint32_t s = t * ITEMS;
+    uint32_t c[ITEMS + 1], r[ITEMS], L[ITEMS + 1], R[ITEMS + 1];
+    int dl[ITEMS + 1];
+    const uint32_t prev = (s >= 1 && s - 1 < n) ? ka[s - 1] : 0u;
+#pragma unroll
+    for (int q = 0; q <= ITEMS; ++q) c[q] = s + q < n ? ka[s + q] : 0u;
+    dl[0] = (s >= 1 && s < n) ? delta_of(prev, c[0]) : -1;
+    uint32_t af = 0u, ab = 0u;
+#pragma unroll
+    for (int q = 0; q < ITEMS; ++q) {
+        dl[q + 1] = s + q + 1 < n ? delta_of(c[q], c[q + 1]) : -1;
+        r[q] = dl[q + 1] >= 0 ? 1u << dl[q + 1] : 0u;
+        af = rec_fwd(af, r[q]);
+    }
+#pragma unroll
+    for (int q = ITEMS - 1; q >= 0; --q) ab = rec_bwd(r[q], ab);
+    block_scan_records<kSmallThreads>(af, ab, &L[0], &R[ITEMS], s_f, s_b);  // and every read of ka is done
+#pragma unroll
+    for (int q = 0; q < ITEMS; ++q) L[q + 1] = rec_fwd(L[q], r[q]);
+#pragma unroll
+    for (int q = ITEMS - 1; q >= 0; --q) R[q] = rec_bwd(r[q], R[q + 1]);
+    const int leaf_depth = (int)depth - 1;
+    uint32_t heads = 0u;
+#pragma unroll
+    for (int q = 0; q < ITEMS; ++q)
+        if (s + q < n && (s + q == 0 || (dl[q] >= 0 && __popc(keep_above(L[q] | R[q], dl[q])) < leaf_depth))) heads |= 1u << q;
+    uint32_t ord = __popc(heads);
+    {
+        uint32_t incl = ord;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const uint32_t y = __shfl_up_sync(kFull, incl, off);
+            if (lane >= off) incl += y;
+        }
+        __syncthreads();
+        if (lane == 31) s_f[w] = incl;
+        __syncthreads();
+        uint32_t base = 0u;
+        for (int q = 0; q < w; ++q) base += s_f[q];
+        if (t == kSmallThreads - 1) s_total = base + incl;
+        ord = base + incl - ord;
+    }
+    const Units u = units_of(smem, N);  // over the sort's arrays
+#pragma unroll
+    for (int q = 0; q < ITEMS; ++q)
+        if ((heads >> q) & 1u) {
+            uint32_t m;
+            const uint32_t h = heap_index_capped(c[q], L[q] | R[q], leaf_depth, &m);
+            u.h[ord] = h;
+            u.m[ord] = m;
+            u.pos[ord] = (int32_t)(s + q);
+            ++ord;
+        }
+    __syncthreads();
+    const uint32_t U = s_total;
+    if (t == 0) {
+        u.pos[U] = (int32_t)n;
+        *u.n_items = 0u;
+    }
+    if ((uint32_t)t < tiles) {  // the leaves as k_emit_units lists them, for the trace records
+        const uint32_t before = (uint32_t)t * kEmitTile;
+        counts[t] = U > before ? min(U - before, (uint32_t)kEmitTile) : 0u;
+    }
+    __syncthreads();
+
+    // leaf records
+    auto tri_at = [&](uint32_t k) {
+        const float4 a = __ldcg(sorted_tris + 3 * k), b = __ldcg(sorted_tris + 3 * k + 1), d = __ldcg(sorted_tris + 3 * k + 2);
+        const float v[9] = {a.x, a.y, a.z, b.x, b.y, b.z, d.x, d.y, d.z};
+        return tri_box(v);
+    };
+    auto store_leaf = [&](uint32_t i, const Box& b) {
+        const uint32_t h = u.h[i], m = u.m[i];
+        const int32_t pos = u.pos[i], cnt = u.pos[i + 1] - pos;
+        store_node(nodes + h, b.lo, b.hi, (cnt << 3) | 4 | leaf_axis_of(m, cnt, depth), pos);
+        leaf_of[pos] = h;
+        units[i] = make_uint2(h, m);
+        set_box(u, (int)i, b);
+        u.arr[i] = 0u;
+    };
+    for (uint32_t i = t; i < U; i += kSmallThreads) {
+        const uint32_t pos = (uint32_t)u.pos[i], cnt = (uint32_t)u.pos[i + 1] - pos;
+        if (cnt > kSmallLeaf) {
+            s_biglist[atomicAdd(&s_big, 1u)] = i;
+            continue;
+        }
+        Box b = tri_at(pos);
+        for (uint32_t k = 1; k < cnt; ++k) b = box_union(b, tri_at(pos + k));
+        store_leaf(i, b);
+    }
+    __syncthreads();
+    for (uint32_t q = w; q < s_big; q += kSmallWarps) {
+        const uint32_t i = s_biglist[q], pos = (uint32_t)u.pos[i], cnt = (uint32_t)u.pos[i + 1] - pos;
+        Box b = empty_box();
+        for (uint32_t k0 = 0; k0 < cnt; k0 += 32) {  // in order: lanes, then batches
+            Box x = k0 + lane < cnt ? tri_at(pos + k0 + lane) : empty_box();
+            for (int off = 1; off < 32; off <<= 1) {
+                const Box y = shfl_up_box(x, off);
+                if (lane >= off) x = box_union(y, x);
+            }
+            if (lane == 31) b = box_union(b, x);
+        }
+        if (lane == 31) store_leaf(i, b);
+    }
+    __syncthreads();
+    unit_bottom_up<kSmallThreads, false>(u, (int)U, Heap<false>{nodes, nullptr, depth}, s_items, err, nullptr);
+}
+
 // Compact layout (rt_lbvh.cnodes) from the heap: inner_rank = exclusive
 // popcount prefix of the internal-node bitmap (one block), then every
 // reachable internal node x writes its two children at slots 2 rank(x) + 2
@@ -2036,8 +2322,26 @@ static rt_status launch_build(rt_ctx* ctx, rt_lbvh* l, const float* d_tris, uint
     cudaStream_t st = ctx->stream;
     l->n = n;
     l->src_tris = d_tris;
-    const uint32_t sort_tiles = ceil_div(n, kSortTile);
     const uint32_t emit_tiles = ceil_div(n, kEmitTile);
+    if (n <= kSmallTris && flags == 0u) {  // 1,000 triangles 69 -> 29 us, 2,048: 78 -> 44, 4,096: 80 -> 75
+        auto small = [&](auto kernel, int items) -> rt_status {
+            RT_CHECK_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small_smem(items)));
+            launch_pdl(kernel, 1, kSmallThreads, small_smem(items), st, d_tris, n, l->depth, l->keys, l->ids, l->sorted_tris,
+                       l->nodes, l->leaf_of, reinterpret_cast<uint2*>(l->keys_alt), l->item_counts + 6 * (size_t)l->emit_tiles_cap,
+                       emit_tiles, l->scene, l->counters, ctx->d_err);
+            RT_CHECK_LAUNCH(ctx, "k_build_small");
+            return RT_OK;
+        };
+        const rt_status s = n <= kSmallThreads       ? small(k_build_small<1>, 1)
+                            : n <= 2 * kSmallThreads ? small(k_build_small<2>, 2)
+                                                     : small(k_build_small<4>, 4);
+        if (s != RT_OK) return s;
+        l->built_keys = true;
+        l->compact_valid = false;
+        l->rec_tiles = emit_tiles;
+        return RT_OK;
+    }
+    const uint32_t sort_tiles = ceil_div(n, kSortTile);
     const uint32_t lb_pass = 256 * (sort_tiles + look_groups(sort_tiles));  // tile words, group words
     const uint32_t lb_words = kSortPasses * lb_pass;
     const uint32_t bblocks = std::max(1u, std::min(ceil_div(3ull * n, 256), l->bounds_blocks));

@@ -76,27 +76,35 @@ struct Records {
     const rt_node* nodes;
     uint32_t num_nodes;
     TraceNode* tnodes;
+    uint32_t slices;         // blocks that share a tile
     uint32_t scene_depth;    // a batch's heap depth (a leaf is named by scene << 23 | heap slot); 0: one tree
 };
 
-inline Records records_of(const rt_lbvh* l) {
-    return Records{l->counters + 7, reinterpret_cast<const uint2*>(l->keys_alt),
-                   l->item_counts + 6 * (size_t)l->emit_tiles_cap, l->rec_tiles, l->nodes, l->num_nodes, l->tnodes, 0u};
+// Few tiles are shared by up to eight blocks each, about two blocks per SM.
+inline uint32_t record_slices(uint32_t tiles, int num_sms) {
+    return std::max(1u, std::min(8u, 2u * (uint32_t)num_sms / std::max(1u, tiles)));
 }
-inline Records records_of(const rt_batch* b) {
+inline Records records_of(const rt_ctx* ctx, const rt_lbvh* l) {
+    return Records{l->counters + 7, reinterpret_cast<const uint2*>(l->keys_alt),
+                   l->item_counts + 6 * (size_t)l->emit_tiles_cap, l->rec_tiles, l->nodes, l->num_nodes, l->tnodes,
+                   record_slices(l->rec_tiles, ctx->num_sms), 0u};
+}
+inline Records records_of(const rt_ctx* ctx, const rt_batch* b) {
     const uint32_t tiles = (b->total + kEmitTile - 1) / kEmitTile;
     return Records{b->counters + 7, reinterpret_cast<const uint2*>(b->keys), b->item_counts + 6 * (size_t)tiles,
-                   b->tnodes ? tiles : 0u, b->nodes, 1u << b->depth, b->tnodes, b->depth};
+                   b->tnodes ? tiles : 0u, b->nodes, 1u << b->depth, b->tnodes,
+                   record_slices(tiles, ctx->num_sms), b->depth};
 }
 
-// The records of one tile's leaves (a block).  There is one internal node per
+// The records of a slice of one tile's leaves (block q of tiles * slices).  There is one internal node per
 // two neighbouring leaves of a tree, their lowest common ancestor: a thread
 // takes a leaf and the one before it.
-__device__ __forceinline__ void make_records(const Records& R, uint32_t tile) {
+__device__ __forceinline__ void make_records(const Records& R, uint32_t block) {
     if (*R.valid) return;  // uniform
+    const uint32_t tile = block / R.slices;
     const uint32_t cnt = min(__ldg(R.counts + tile), (uint32_t)kEmitTile);
     const bool batch = R.scene_depth != 0u;
-    for (uint32_t i = threadIdx.x; i < cnt; i += blockDim.x) {
+    for (uint32_t i = (block % R.slices) * blockDim.x + threadIdx.x; i < cnt; i += R.slices * blockDim.x) {
         uint32_t b = __ldg(&R.units[(size_t)tile * kEmitTile + i].x), a = 0u;
         if (i) {
             a = __ldg(&R.units[(size_t)tile * kEmitTile + i - 1].x);

@@ -153,7 +153,10 @@ __global__ void __launch_bounds__(kTraceThreads, 7) k_trace_primary(TreeRef tr, 
 // Primary rays over the trace records (Walk), an 8 x 4 tile per warp at a time:
 // neighbouring rays visit the same leaves, so handing out pixels one by one to the
 // lanes that are done (as the shading rays are) was slower.
-constexpr int kPrimSteps = 3;  // 3: 1,415 us a frame of 2.1 M triangles, 4: 1,423, 8: 1,413 (65 k triangles, 512 x 512: 312, 309, 330)
+#ifndef RT_PRS
+#define RT_PRS 3
+#endif
+constexpr int kPrimSteps = RT_PRS;  // 3: 1,415 us a frame of 2.1 M triangles, 4: 1,423, 8: 1,413 (65 k triangles, 512 x 512: 312, 309, 330)
 
 __global__ void __launch_bounds__(kTraceThreads, 8) k_walk_primary(TreeRef tr, rt_camera cam, rt_hit* __restrict__ hits,
                                                                         uint32_t* __restrict__ leaves, uint32_t* work,
@@ -850,7 +853,7 @@ __global__ void __launch_bounds__(256) k_reset_words(uint32_t* words, unsigned l
 
 rt_status reset_words(rt_ctx* ctx, uint64_t mask, const Records& rec) {
     if (!mask && !rec.tiles) return RT_OK;
-    launch_pdl(k_reset_words, 1u + rec.tiles, rec.tiles ? 256 : 64, 0, ctx->stream, ctx->d_words, (unsigned long long)mask,
+    launch_pdl(k_reset_words, 1u + rec.tiles * rec.slices, rec.tiles ? 256 : 64, 0, ctx->stream, ctx->d_words, (unsigned long long)mask,
                rec);
     RT_CHECK_LAUNCH(ctx, "k_reset_words");
     return RT_OK;
@@ -925,11 +928,11 @@ rt_status order_begin(rt_ctx* ctx, int kind, bool enabled, TileOrder* out, uint6
     o.lists = ctx->d_order + (size_t)kind * kOrderWords;
     o.bits = o.lists + 2 * (size_t)kOrderCap;
     if (enabled) {
-        const Records rec = l ? records_of(l) : no_records();
-        launch_pdl(k_order_begin, 1u + rec.tiles, 256, 0, ctx->stream, o, ctx->d_words, (unsigned long long)reset, rec);
+        const Records rec = l ? records_of(ctx, l) : no_records();
+        launch_pdl(k_order_begin, 1u + rec.tiles * rec.slices, 256, 0, ctx->stream, o, ctx->d_words, (unsigned long long)reset, rec);
         RT_CHECK_LAUNCH(ctx, "k_order_begin");
     } else {
-        rt_status s = reset_words(ctx, reset, l ? records_of(l) : no_records());
+        rt_status s = reset_words(ctx, reset, l ? records_of(ctx, l) : no_records());
         if (s != RT_OK) return s;
     }
     *out = o;
@@ -1015,7 +1018,7 @@ rt_status trace_shadow_mirror(rt_ctx* ctx, const rt_lbvh* l, const rt_camera* ca
         uint32_t* counts = ctx->d_work + kShadeCounts;
         if (!prebuilt) {
             reset = shade_reset_bits(ctx, sp) | word_bit(ctx, counts) | word_bit(ctx, counts + 1);
-            if ((s = reset_words(ctx, reset, records_of(l))) != RT_OK) return s;
+            if ((s = reset_words(ctx, reset, records_of(ctx, l))) != RT_OK) return s;
         }
         const uint32_t cap = (uint32_t)l->s_pixels;
         if (!prebuilt) {
@@ -1103,7 +1106,7 @@ rt_status trace_rays(rt_ctx* ctx, const rt_lbvh* l, const rt_ray* d_rays, uint32
 }  // namespace
 
 rt_status reset_work_and_records(rt_ctx* ctx, int slot, const rt_lbvh* l) {
-    return reset_words(ctx, word_bit(ctx, ctx->d_work + slot), records_of(l));
+    return reset_words(ctx, word_bit(ctx, ctx->d_work + slot), records_of(ctx, l));
 }
 
 extern "C" rt_status rt_trace_primary(rt_ctx* ctx, const rt_lbvh* l, const rt_camera* cam, rt_hit* d_hits,
@@ -1565,7 +1568,7 @@ extern "C" rt_status rt_batch_trace(rt_ctx* ctx, const rt_batch* b, rt_hit* d_hi
     uint64_t reset = word_bit(ctx, ctx->d_work + kWorkBatch);
     if (listed)
         reset |= word_bit(ctx, ctx->d_work + kWorkShade) | word_bit(ctx, counts) | word_bit(ctx, counts + 1);
-    rt_status s = reset_words(ctx, reset, records_of(b));
+    rt_status s = reset_words(ctx, reset, records_of(ctx, b));
     if (s != RT_OK) return s;
     TreeRef tr;  // the batch's arrays; heap, tnodes, tri_base and n are set per scene
     memset(&tr, 0, sizeof(tr));
