@@ -22,11 +22,12 @@
 //   k_emit_chunks   shared-memory bottom-up over each tile's units
 //   k_emit_merge    the same over groups of 32 chunks / groups, level after
 //                   level to the root, in one launch
-// The allocation-free build (rt_lbvh_build_noalloc) and the batched build
-// keep the one-level look-back and the first emission form, k_emit_leaves +
-// k_emit_refit (kb_emit_leaves + kb_emit_refit for a batch): leaf boxes,
-// then an atomic bottom-up walk with epoch-tagged arrival words that writes
-// every internal node (parent = h/2, sibling = h^1).
+// A soup of at most kSmallTris triangles takes one launch, k_build_small.  The
+// batched build runs the same emission over the concatenated scenes.  The
+// allocation-free build (rt_lbvh_build_noalloc) keeps the one-level look-back
+// and the first emission form, k_emit_leaves + k_emit_refit: leaf boxes, then an
+// atomic bottom-up walk with epoch-tagged arrival words that writes every
+// internal node (parent = h/2, sibling = h^1).
 //
 // Tree = the reference's: LBVH::build_recursive (LBVH.cpp:190-314) splits a
 // sorted range at its highest differing Morton bit, keeps equal-code runs as
@@ -120,8 +121,9 @@ __global__ void __launch_bounds__(256) k_bounds(const float* __restrict__ tris, 
     // counters: [0] bounds ticket (reset by the last block), [1..4] sort tile
     // tickets, [5] leaf count, [6] refit epoch (advanced once per build, so a
     // replayed CUDA graph of the build still tags every arrival afresh), [7]
-    // whether the trace records are those of this tree
+    // whether the trace records are those of this tree, [8] its emission tiles
     if ((gtid >= 1 && gtid < 6) || gtid == 7) counters[gtid] = 0u;
+    if (gtid == 8) counters[8] = (n + kEmitTile - 1u) / kEmitTile;
     if (gtid == 0) {
         uint32_t e = counters[6] + 1u;
         counters[6] = e ? e : 1u;  // 0 is the value of cleared arrival words
@@ -671,9 +673,10 @@ __global__ void __launch_bounds__(kEmitThreads) k_emit_tiles(const uint32_t* __r
                                                              uint32_t* scan, uint32_t* arrive, uint32_t arrive_words,
                                                              const uint32_t* epoch_word) {
     grid_dep_wait();
-    // epoch 1 means the first build or a wrapped epoch counter: the refit's
-    // arrival words may hold any old epoch and are cleared before k_emit_refit
-    if (*epoch_word == 1u)
+    // (the allocation-free build) epoch 1 means the first build or a wrapped epoch
+    // counter: the refit's arrival words may hold any old epoch and are cleared
+    // before k_emit_refit
+    if (arrive_words && *epoch_word == 1u)
         for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < arrive_words; i += gridDim.x * blockDim.x)
             arrive[i] = 0u;
     __shared__ uint32_t s_f[8], s_b[8];
@@ -1039,7 +1042,7 @@ __global__ void __launch_bounds__(256) k_emit_refit(const uint32_t* __restrict__
 }
 
 // ---------------------------------------------------------------------------
-// Emission and refit without global atomics (the single-scene build).
+// Emission and refit without global atomics (a single tree and a batch).
 //
 // k_emit_units handles one tile of kEmitTile sorted elements:
 //   1. per element: ancestor record mask (two scans), head / tail of its
@@ -1056,10 +1059,10 @@ __global__ void __launch_bounds__(256) k_emit_refit(const uint32_t* __restrict__
 //   3. a leaf that began in an earlier tile and ends in this one is finished
 //      here: its start is found by scanning back over the codes and its
 //      earlier triangles are folded in from the soup.
-// k_emit_merge then runs a shared-memory bottom-up (unit_bottom_up) over one
-// tile's units per CTA; a node whose parent's split boundary lies outside
-// the units becomes an "item" for the next level, and k_emit_merge runs
-// again over the items of kMergeGroup consecutive tiles (groups) per CTA,
+// k_emit_chunks then runs a shared-memory bottom-up (unit_bottom_up) over a
+// chunk of one tile's units per CTA; a node whose parent's split boundary lies
+// outside the units becomes an "item" for the next level, and k_emit_merge runs
+// over the items of kMergeGroup consecutive chunks (groups) per CTA,
 // level after level, until one CTA forms the root.  No node waits on another
 // CTA, and nothing needs a global arrival word.
 //
@@ -1916,6 +1919,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_build_small(const float* _
                 *scene = sc;
                 if (sc.nonfinite) atomicOr(err, RT_DEVERR_NONFINITE);
                 counters[7] = 0u;  // the trace records are an earlier tree's
+                counters[8] = tiles;
                 s_big = 0u;
             }
         }
@@ -2210,6 +2214,7 @@ __global__ void __launch_bounds__(256) k_trace_nodes(const rt_node* __restrict__
     const float4 g = trace_grid(root.min, root.max);
     const int pc = nodes[h].prim_count, pos = nodes[h].prim_pos;
     if (h == 0) {
+        if (!tnodes) return;
         store_trace_grid(tnodes, g, (root.prim_count & 4) ? leaf_word(1u, (uint32_t)root.prim_pos,
                                                                       (uint32_t)(root.prim_count >> 3)) : 0u);
         return;
@@ -2220,7 +2225,7 @@ __global__ void __launch_bounds__(256) k_trace_nodes(const rt_node* __restrict__
         if (pos >= 0 && (uint32_t)pos < n) leaf_of[pos] = h;
         return;
     }
-    if (2 * h + 1 >= num_nodes) return;  // a corrupt tree
+    if (!tnodes || 2 * h + 1 >= num_nodes) return;  // no records, or a corrupt tree
     const rt_node l = nodes[2 * h], r = nodes[2 * h + 1];
     auto word = [](const rt_node& c, uint32_t ch) {
         return (c.prim_count & 4) ? leaf_word(ch, (uint32_t)c.prim_pos, (uint32_t)(c.prim_count >> 3)) : 0u;
@@ -2257,7 +2262,6 @@ extern "C" rt_status rt_lbvh_create(rt_ctx* ctx, uint32_t max_tris, uint32_t dep
         if (e == cudaSuccess) e = cudaMalloc(p, bytes);
     };
     alloc((void**)&l->nodes, sizeof(rt_node) * l->num_nodes);
-    alloc((void**)&l->tnodes, sizeof(TraceNode) * (size_t)std::max(1u, l->num_nodes / 2));
     alloc((void**)&l->keys, 4 * cap);
     alloc((void**)&l->ids, 4 * cap);
     // one block for both ping-pong buffers: after the sort it holds the
@@ -2272,23 +2276,27 @@ extern "C" rt_status rt_lbvh_create(rt_ctx* ctx, uint32_t max_tris, uint32_t dep
     alloc((void**)&l->tris, sizeof(float) * 9 * cap);
     alloc((void**)&l->scene, sizeof(SceneInfo));
     alloc((void**)&l->partials, sizeof(float) * 8 * l->bounds_blocks);
-    alloc((void**)&l->counters, sizeof(uint32_t) * 8);
+    alloc((void**)&l->counters, sizeof(uint32_t) * 16);
     alloc((void**)&l->hist, sizeof(uint32_t) * 4 * 256);
     // per radix pass: 256 look-back words per tile, then 256 per tile group
     alloc((void**)&l->lookback,
           sizeof(uint32_t) * kSortPasses * 256 * ((size_t)l->sort_tiles_cap + look_groups(l->sort_tiles_cap)));
     alloc((void**)&l->scan, sizeof(uint32_t) * 4 * (size_t)l->emit_tiles_cap);
     alloc((void**)&l->leaf_of, 4 * cap);
-    alloc((void**)&l->arrive, sizeof(uint32_t) * std::max(1u, l->num_nodes >> 1));
     // items and item counts of every merge level (chunk slots = 4 x tiles, then
     // the groups above: < 6 x tiles in all), the tiles' unit counts (tiles),
     // the merge tickets (tiles, zero between builds)
     alloc((void**)&l->items, sizeof(uint2) * 6 * (size_t)kItemCap * l->emit_tiles_cap);
     alloc((void**)&l->item_counts, sizeof(uint32_t) * 8 * (size_t)l->emit_tiles_cap);
-    if (e == cudaSuccess) e = cudaMemset(l->counters, 0, sizeof(uint32_t) * 8);
-    if (e == cudaSuccess) e = cudaMemset(l->arrive, 0, sizeof(uint32_t) * std::max(1u, l->num_nodes >> 1));
+    if (e == cudaSuccess) e = cudaMemset(l->counters, 0, sizeof(uint32_t) * 16);
     if (e == cudaSuccess) e = cudaMemset(l->nodes, 0, sizeof(rt_node) * l->num_nodes);
     if (e == cudaSuccess) e = cudaMemset(l->item_counts, 0, sizeof(uint32_t) * 8 * (size_t)l->emit_tiles_cap);
+    // without room for the trace records the walks read the heap
+    if (e == cudaSuccess &&
+        cudaMalloc((void**)&l->tnodes, sizeof(TraceNode) * (size_t)std::max(1u, l->num_nodes / 2)) != cudaSuccess) {
+        cudaGetLastError();
+        l->tnodes = nullptr;
+    }
     if (e != cudaSuccess) {
         rt_lbvh_destroy(l);
         return rt_fail(ctx, RT_ERR_CUDA, "rt_lbvh_create: allocation failed: %s", cudaGetErrorString(e));
@@ -2308,9 +2316,9 @@ extern "C" rt_status rt_lbvh_destroy(rt_lbvh* l) {
 }
 
 void free_lbvh(rt_lbvh* l) {
-    void* ptrs[] = {l->nodes,    l->keys,     l->ids,      l->keys_alt,  nullptr,    l->sorted_tris,
+    void* ptrs[] = {l->nodes,    l->keys,     l->ids,      l->keys_alt,  l->sorted_tris,
                     l->tris,     l->scene,    l->partials, l->counters,  l->hist,    l->lookback,
-                    l->scan,     l->leaf_of,  l->arrive,  l->f_primary, l->f_mirror, l->f_vis,
+                    l->scan,     l->leaf_of,  l->f_primary, l->f_mirror, l->f_vis,
                     l->s_lists,  l->cnodes,   l->inner,    l->inner_rank, l->w_buf, l->s_rays,
                     l->items,    l->item_counts, l->tnodes};
     for (void* p : ptrs)
@@ -2323,7 +2331,10 @@ static rt_status launch_build(rt_ctx* ctx, rt_lbvh* l, const float* d_tris, uint
     l->n = n;
     l->src_tris = d_tris;
     const uint32_t emit_tiles = ceil_div(n, kEmitTile);
-    if (n <= kSmallTris && flags == 0u) {  // 1,000 triangles 69 -> 29 us, 2,048: 78 -> 44, 4,096: 80 -> 75
+    // One block against the launches below: 300 triangles 21 and 58 us, 1,000: 29 and 69,
+    // 2,048: 44 and 78, 4,096: 75 and 80; one block would need more shared memory beyond.
+    // The flags ask for passes that only the launches below have.
+    if (n <= kSmallTris && flags == 0u) {
         auto small = [&](auto kernel, int items) -> rt_status {
             RT_CHECK_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small_smem(items)));
             launch_pdl(kernel, 1, kSmallThreads, small_smem(items), st, d_tris, n, l->depth, l->keys, l->ids, l->sorted_tris,
@@ -2361,8 +2372,8 @@ static rt_status launch_build(rt_ctx* ctx, rt_lbvh* l, const float* d_tris, uint
         std::swap(iin, iout);
     }
     // four passes: sorted pairs are back in keys / ids
-    launch_pdl(k_emit_tiles, emit_tiles, kEmitThreads, 0, st, l->keys, n, l->scan, l->arrive, std::max(1u, l->num_nodes >> 1),
-                                                      l->counters + 6);
+    launch_pdl(k_emit_tiles, emit_tiles, kEmitThreads, 0, st, l->keys, n, l->scan, (uint32_t*)nullptr, 0u,
+               (const uint32_t*)nullptr);
     RT_CHECK_LAUNCH(ctx, "k_emit_tiles");
     launch_pdl(k_emit_prefix, 1, kPrefixThreads, 0, st, l->scan, emit_tiles);
     RT_CHECK_LAUNCH(ctx, "k_emit_prefix");
@@ -2435,12 +2446,13 @@ extern "C" rt_status rt_lbvh_import_host(rt_ctx* ctx, rt_lbvh* l, const rt_node*
     const uint32_t blocks = std::max(1u, std::min(ceil_div(n, 256), (uint32_t)ctx->num_sms * 8));
     k_gather_tris<<<blocks, 256, 0, st>>>(l->ids, l->tris, n, l->sorted_tris);
     RT_CHECK_LAUNCH(ctx, "k_gather_tris");
+    RT_CHECK_CUDA(ctx, cudaMemsetAsync(l->counters + 8, 0, sizeof(uint32_t), st));  // no emission tiles: these are its records
     k_trace_nodes<<<ceil_div(l->num_nodes, 256), 256, 0, st>>>(l->nodes, l->num_nodes, l->tnodes, l->leaf_of, n);
     RT_CHECK_LAUNCH(ctx, "k_trace_nodes");
     l->n = n;
     l->src_tris = l->tris;
     l->built_keys = false;
-    l->rec_tiles = 0;          // its records are made
+    l->rec_tiles = 0;
     l->compact_valid = false;  // an imported tree is traversed in its heap layout
     return RT_OK;
 }
@@ -2763,16 +2775,18 @@ extern "C" rt_status rt_radix_sort_stall_test(rt_ctx* ctx, const uint32_t* d_key
 // Batched build: S independent scenes (S <= 256) built by one pass of the
 // build kernels over their concatenated soups.  Scene s's triangles are
 // [tri_off[s], tri_off[s+1]); its tree is the single-scene tree of those
-// triangles, stored in its own heap of 1 << depth slots at node_off[s], with
+// triangles, stored in its own heap of 1 << depth slots at s << depth, with
 // PrimPos and the ordered ids local to the scene.
 //   kb_init          per-scene bounds reset, scratch reset, epoch
 //   kb_bounds        per-scene bounds over host-made one-scene chunks
 //   kb_morton_hist   codes with each scene's own Morton parameters
 //   k_onesweep x4+1  four code passes, then a stable pass on the scene
-//   kb_emit_tiles / k_emit_prefix / kb_emit_leaves
+//   kb_emit_tiles / k_emit_prefix
 //                    the record scans with a separator record (bit 31) at
 //                    every scene boundary, so no scan crosses two scenes
-//   kb_emit_refit    the per-leaf refit walk in each scene's heap
+//   k_emit_units / k_emit_chunks / k_emit_merge
+//                    a single tree's emission, a node named by its scene and
+//                    heap slot (Heap)
 namespace {
 
 constexpr uint32_t kChunkTris = 4096;
@@ -2941,7 +2955,7 @@ extern "C" rt_status rt_batch_destroy(rt_batch* b) {
 }
 
 void free_batch(rt_batch* b) {
-    void* ptrs[] = {b->tri_off, b->node_off, b->chunks, b->nodes, b->keys, nullptr, b->keys_alt, b->ids_alt,
+    void* ptrs[] = {b->tri_off, b->chunks, b->nodes, b->keys, b->keys_alt, b->ids_alt,
                     b->ids_local, b->sorted_tris, b->sbounds, b->counters, b->hist, b->lookback, b->scan,
                     b->leaf_of, b->tnodes, b->items, b->item_counts, b->cams, b->lights, b->s_lists, b->s_rays};
     for (void* p : ptrs)
@@ -2970,7 +2984,7 @@ extern "C" rt_status rt_batch_create(rt_ctx* ctx, uint32_t n_scenes, const uint3
     b->depth = depth;
     b->total = (uint32_t)total;
     b->h_tri_off.resize(n_scenes + 1);
-    std::vector<uint32_t> node_off(n_scenes + 1), chunks;
+    std::vector<uint32_t> chunks;
     b->h_tri_off[0] = 0;
     for (uint32_t s = 0; s < n_scenes; ++s) {
         b->h_tri_off[s + 1] = b->h_tri_off[s] + h_tri_counts[s];
@@ -2980,7 +2994,6 @@ extern "C" rt_status rt_batch_create(rt_ctx* ctx, uint32_t n_scenes, const uint3
             chunks.push_back(std::min(c + kChunkTris, b->h_tri_off[s + 1]));
         }
     }
-    for (uint32_t s = 0; s <= n_scenes; ++s) node_off[s] = s << depth;
     b->nchunks = (uint32_t)(chunks.size() / 3);
     const size_t n = total;
     const size_t num_nodes = (size_t)n_scenes << depth;
@@ -2990,7 +3003,6 @@ extern "C" rt_status rt_batch_create(rt_ctx* ctx, uint32_t n_scenes, const uint3
         if (e == cudaSuccess) e = cudaMalloc(p, bytes);
     };
     alloc((void**)&b->tri_off, 4 * (n_scenes + 1));
-    alloc((void**)&b->node_off, 4 * (n_scenes + 1));
     alloc((void**)&b->chunks, 4 * chunks.size());
     alloc((void**)&b->nodes, sizeof(rt_node) * num_nodes);
     // one block: after the sort (whose result is in the alternate buffers) it
@@ -3013,7 +3025,6 @@ extern "C" rt_status rt_batch_create(rt_ctx* ctx, uint32_t n_scenes, const uint3
     alloc((void**)&b->cams, sizeof(rt_camera) * n_scenes);
     alloc((void**)&b->lights, sizeof(float) * 3 * n_scenes);
     if (e == cudaSuccess) e = cudaMemcpy(b->tri_off, b->h_tri_off.data(), 4 * (n_scenes + 1), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(b->node_off, node_off.data(), 4 * (n_scenes + 1), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(b->chunks, chunks.data(), 4 * chunks.size(), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemset(b->counters, 0, sizeof(uint32_t) * 8);
     if (e == cudaSuccess) e = cudaMemset(b->item_counts, 0, sizeof(uint32_t) * 8 * (size_t)emit_tiles);

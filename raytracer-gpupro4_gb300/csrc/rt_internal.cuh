@@ -163,8 +163,8 @@ struct rt_lbvh {
     // compact layout used by the traversal: slot 1 = root, the children of
     // internal node x at slots 2 r + 2, 2 r + 3 with r = the rank of x among
     // the reachable internal nodes in heap order (its PrimPos holds 2 r + 2)
-    TraceNode* tnodes = nullptr;    // trace records, 1 << (depth - 1)
-    uint32_t rec_tiles = 0;         // emission tiles of the last build (0: the records were made by an import)
+    TraceNode* tnodes = nullptr;    // trace records, 1 << (depth - 1) (nullptr: no memory for them, the walks read the heap)
+    uint32_t rec_tiles = 0;         // emission tiles of the last build (0: an import, which makes its records itself)
     uint32_t* leaf_of = nullptr;    // heap slot of the leaf whose first triangle is at a sorted position
     rt_node* cnodes = nullptr;
     uint32_t ccap = 0;              // slots of cnodes
@@ -176,11 +176,10 @@ struct rt_lbvh {
     // build scratch
     SceneInfo* scene = nullptr;
     float* partials = nullptr;       // bounds partial reductions, 8 floats per block
-    uint32_t* counters = nullptr;    // [0] bounds ticket, [1..4] sort tile tickets, [5] leaf count, [6] refit epoch
+    uint32_t* counters = nullptr;    // [0] bounds ticket, [1..4] sort tile tickets, [7] records valid, [8] emission tiles
     uint32_t* hist = nullptr;        // 4 x 256 digit histograms
     uint32_t* lookback = nullptr;    // 4 passes x sort tiles x 256 status words
     uint32_t* scan = nullptr;        // emission tiles x 4 (fwd agg, bwd agg, fwd prefix, bwd suffix)
-    uint32_t* arrive = nullptr;      // 1 << (depth-1) refit arrival words (epoch-tagged)
     uint2* items = nullptr;          // emission items (heap index, mask) of every merge level: 6 x emit tiles x 64
     uint32_t* item_counts = nullptr; // 8 x emit tiles: item counts of every level (6x), tile unit counts, merge tickets
     uint32_t sort_tiles_cap = 0, emit_tiles_cap = 0, bounds_blocks = 0;
@@ -210,14 +209,13 @@ void free_batch(rt_batch* b);
 
 // Many independent scenes built in one pass of the build kernels and traced
 // by one persistent kernel.  Scene s owns triangles [tri_off[s], tri_off[s+1])
-// of the concatenated soup and heap slots [node_off[s], node_off[s+1]).
+// of the concatenated soup and heap slots [s << depth, (s + 1) << depth).
 struct rt_batch {
     uint32_t S = 0, depth = 0, total = 0;
     uint32_t graph_refs = 0;       // captured frames pointing into the batch (see rt_lbvh)
     bool destroy_pending = false;
     std::vector<uint32_t> h_tri_off;
     uint32_t* tri_off = nullptr;   // S + 1
-    uint32_t* node_off = nullptr;  // S + 1
     uint32_t* chunks = nullptr;    // (scene, begin, end) triples, one scene each
     uint32_t nchunks = 0;
     rt_node* nodes = nullptr;      // S << depth
@@ -226,7 +224,7 @@ struct rt_batch {
     uint32_t* ids_local = nullptr;  // scene-local triangle id at each sorted position
     float4* sorted_tris = nullptr;  // 3 x float4 per triangle, w of the first = scene-local id
     float* sbounds = nullptr;       // 8 floats per scene (min xyz, max xyz)
-    uint32_t* counters = nullptr;   // [0..4] sort tickets, [5] leaf count, [6] refit epoch
+    uint32_t* counters = nullptr;   // [0..4] sort tickets, [7] records valid
     uint32_t* hist = nullptr;       // 5 x 256
     uint32_t* lookback = nullptr;   // 5 x 256 x sort tiles
     uint32_t* scan = nullptr;       // 4 per emission tile

@@ -67,12 +67,14 @@ __device__ __forceinline__ void trace_node_of(uint32_t h, const rt_node* nodes, 
                      field == 0 ? 2 : field - 1, g);  // the field is one past the split axis
 }
 
-// What make_records needs of a tree (tiles = 0: its records are made).
+// What make_records needs of a tree (tiles = 0: no records).
 struct Records {
     const uint32_t* valid;
     const uint2* units;      // the emission's leaves, kEmitTile slots per tile
     const uint32_t* counts;  // leaves of each tile
-    uint32_t tiles;
+    uint32_t tiles;          // tiles that have blocks of their own
+    const uint32_t* built;   // tiles of the tree when the kernel runs (nullptr: `tiles`): a captured call may be
+                             // replayed over a later build
     const rt_node* nodes;
     uint32_t num_nodes;
     TraceNode* tnodes;
@@ -85,58 +87,61 @@ inline uint32_t record_slices(uint32_t tiles, int num_sms) {
     return std::max(1u, std::min(8u, 2u * (uint32_t)num_sms / std::max(1u, tiles)));
 }
 inline Records records_of(const rt_ctx* ctx, const rt_lbvh* l) {
+    const uint32_t tiles = std::max(1u, l->rec_tiles);
     return Records{l->counters + 7, reinterpret_cast<const uint2*>(l->keys_alt),
-                   l->item_counts + 6 * (size_t)l->emit_tiles_cap, l->rec_tiles, l->nodes, l->num_nodes, l->tnodes,
-                   record_slices(l->rec_tiles, ctx->num_sms), 0u};
+                   l->item_counts + 6 * (size_t)l->emit_tiles_cap, l->tnodes ? tiles : 0u, l->counters + 8, l->nodes,
+                   l->num_nodes, l->tnodes, l->rec_tiles ? record_slices(tiles, ctx->num_sms) : 1u, 0u};
 }
 inline Records records_of(const rt_ctx* ctx, const rt_batch* b) {
     const uint32_t tiles = (b->total + kEmitTile - 1) / kEmitTile;
     return Records{b->counters + 7, reinterpret_cast<const uint2*>(b->keys), b->item_counts + 6 * (size_t)tiles,
-                   b->tnodes ? tiles : 0u, b->nodes, 1u << b->depth, b->tnodes,
+                   b->tnodes ? tiles : 0u, nullptr, b->nodes, 1u << b->depth, b->tnodes,
                    record_slices(tiles, ctx->num_sms), b->depth};
 }
 
-// The records of a slice of one tile's leaves (block q of tiles * slices).  There is one internal node per
-// two neighbouring leaves of a tree, their lowest common ancestor: a thread
-// takes a leaf and the one before it.
+// The records of a slice of a tile's leaves (block q of tiles * slices).  There is
+// one internal node per two neighbouring leaves of a tree, their lowest common
+// ancestor: a thread takes a leaf and the one before it.
 __device__ __forceinline__ void make_records(const Records& R, uint32_t block) {
     if (*R.valid) return;  // uniform
-    const uint32_t tile = block / R.slices;
-    const uint32_t cnt = min(__ldg(R.counts + tile), (uint32_t)kEmitTile);
     const bool batch = R.scene_depth != 0u;
-    for (uint32_t i = (block % R.slices) * blockDim.x + threadIdx.x; i < cnt; i += R.slices * blockDim.x) {
-        uint32_t b = __ldg(&R.units[(size_t)tile * kEmitTile + i].x), a = 0u;
-        if (i) {
-            a = __ldg(&R.units[(size_t)tile * kEmitTile + i - 1].x);
-        } else {  // the last leaf of the tiles before
-            for (uint32_t q = tile; q-- > 0u && a == 0u;) {
-                const uint32_t c = min(__ldg(R.counts + q), (uint32_t)kEmitTile);
-                if (c) a = __ldg(&R.units[(size_t)q * kEmitTile + c - 1].x);
+    const uint32_t tiles = R.built ? *R.built : R.tiles;
+    for (uint32_t tile = block / R.slices; tile < tiles; tile += R.tiles) {
+        const uint32_t cnt = min(__ldg(R.counts + tile), (uint32_t)kEmitTile);
+        for (uint32_t i = (block % R.slices) * blockDim.x + threadIdx.x; i < cnt; i += R.slices * blockDim.x) {
+            uint32_t b = __ldg(&R.units[(size_t)tile * kEmitTile + i].x), a = 0u;
+            if (i) {
+                a = __ldg(&R.units[(size_t)tile * kEmitTile + i - 1].x);
+            } else {  // the last leaf of the tiles before
+                for (uint32_t q = tile; q-- > 0u && a == 0u;) {
+                    const uint32_t c = min(__ldg(R.counts + q), (uint32_t)kEmitTile);
+                    if (c) a = __ldg(&R.units[(size_t)q * kEmitTile + c - 1].x);
+                }
             }
+            const rt_node* nodes = R.nodes;
+            TraceNode* tnodes = R.tnodes;
+            if (batch) {
+                const uint32_t sc = b >> 23;
+                nodes += (size_t)sc << R.scene_depth;
+                tnodes += (size_t)sc << (R.scene_depth - 1u);
+                a = (a >> 23) == sc ? a & 0x7fffffu : 0u;
+                b &= 0x7fffffu;
+            }
+            const float4* p = reinterpret_cast<const float4*>(nodes + 1);
+            const float4 r0 = __ldg(p), r1 = __ldg(p + 1);
+            const float mn[3] = {r0.x, r0.y, r0.z}, mx[3] = {r0.w, r1.x, r1.y};
+            const float4 g = trace_grid(mn, mx);
+            if (a == 0u) {  // the tree's first leaf
+                const int pc = __float_as_int(r1.z);
+                store_trace_grid(tnodes, g, (pc & 4) ? leaf_word(1u, (uint32_t)__float_as_int(r1.w), (uint32_t)(pc >> 3)) : 0u);
+                continue;
+            }
+            const int da = 31 - __clz(a), db = 31 - __clz(b), dm = min(da, db);
+            const uint32_t x = (a >> (da - dm)) ^ (b >> (db - dm));
+            if (b == 0u || x == 0u) continue;  // only after a failed sort
+            const uint32_t h = (a >> (da - dm)) >> (32 - __clz(x));
+            if (h != 0u && 2u * h + 1u < R.num_nodes) trace_node_of(h, nodes, R.num_nodes, tnodes, g);
         }
-        const rt_node* nodes = R.nodes;
-        TraceNode* tnodes = R.tnodes;
-        if (batch) {
-            const uint32_t sc = b >> 23;
-            nodes += (size_t)sc << R.scene_depth;
-            tnodes += (size_t)sc << (R.scene_depth - 1u);
-            a = (a >> 23) == sc ? a & 0x7fffffu : 0u;
-            b &= 0x7fffffu;
-        }
-        const float4* p = reinterpret_cast<const float4*>(nodes + 1);
-        const float4 r0 = __ldg(p), r1 = __ldg(p + 1);
-        const float mn[3] = {r0.x, r0.y, r0.z}, mx[3] = {r0.w, r1.x, r1.y};
-        const float4 g = trace_grid(mn, mx);
-        if (a == 0u) {  // the tree's first leaf
-            const int pc = __float_as_int(r1.z);
-            store_trace_grid(tnodes, g, (pc & 4) ? leaf_word(1u, (uint32_t)__float_as_int(r1.w), (uint32_t)(pc >> 3)) : 0u);
-            continue;
-        }
-        const int da = 31 - __clz(a), db = 31 - __clz(b), dm = min(da, db);
-        const uint32_t x = (a >> (da - dm)) ^ (b >> (db - dm));
-        if (b == 0u || x == 0u) continue;  // only after a failed sort
-        const uint32_t h = (a >> (da - dm)) >> (32 - __clz(x));
-        if (h != 0u && 2u * h + 1u < R.num_nodes) trace_node_of(h, nodes, R.num_nodes, tnodes, g);
     }
 }
 

@@ -3,15 +3,18 @@
 // Replaces the per-bounce dispatches of RayTracerCS::Render
 // (RayTracerCS/RayTracerCS.cpp:284-295): CSGeneratePrimaryRays
 // (Shaders/CS/CSPrimaryRays.hlsl:22-69) and CSComputeIntersections
-// (CSIntersections.hlsl:18-39) are fused into k_trace_primary (rays are made
+// (CSIntersections.hlsl:18-39) are fused into k_walk_primary (rays are made
 // in registers, no 48-byte ray buffer round trip); the shadow ray and the
 // mirror bounce of CSComputeColor (CSComputeColorRT.hlsl:57-177, 203-210,
-// flat normals, no textures) are k_trace_secondary.
+// flat normals, no textures) are k_walk_shade; a caller's own rays are
+// k_walk_rays.  All three walk the trace records (Walk in rt_traverse.cuh).
+// k_trace_primary, k_trace_secondary and k_trace_rays walk the heap and count
+// every box and triangle test.
 //
-// All three kernels are persistent: a grid sized to fill every SM once, each
-// warp pulling 32-ray tiles (8 x 4 pixels) from a work counter until the
-// image is done.  Ray cost varies by three orders of magnitude across the
-// image, so a static grid leaves SMs idle behind the last heavy tiles.
+// The kernels are persistent: a grid sized to fill every SM once, each
+// warp pulling 32-ray tiles (8 x 4 pixels) or single rays from a work counter
+// until the image is done.  Ray cost varies by three orders of magnitude across
+// the image, so a static grid leaves SMs idle behind the last heavy tiles.
 #include <algorithm>
 #include <cstring>
 
@@ -106,57 +109,38 @@ __device__ __forceinline__ void shade_setup_pixel(const ShadeLists& sl, const rt
     }
 }
 
-// At most 72 registers (seven blocks per SM, no spills): a little faster
-// than the 80 the compiler picks unbounded; 64 spills and is slower.
-template <bool STATS>
+// Primary rays with their box and triangle test counts, in the oracle's order.
 __global__ void __launch_bounds__(kTraceThreads, 7) k_trace_primary(TreeRef tr, rt_camera cam,
-                                                                 rt_hit* __restrict__ hits,
-                                                                 uint32_t* __restrict__ leaves,
-                                                                 uint32_t* __restrict__ stats, uint32_t* work,
-                                                                 uint32_t num_tiles, Spill spill,
-                                                                 uint32_t* __restrict__ list, TileOrder ord,
-                                                                 ShadeLists sl) {
-    grid_dep_wait();
+                                                                    rt_hit* __restrict__ hits,
+                                                                    uint32_t* __restrict__ leaves,
+                                                                    uint32_t* __restrict__ stats, uint32_t* work,
+                                                                    uint32_t num_tiles, TileOrder ord) {
     const uint32_t wbuf = *ord.parity, rbuf = wbuf ^ 1u, heavy = min(ord.counts[rbuf], ord.cap);
     for (uint32_t tile = next_ordered_tile(work, ord, rbuf, heavy, num_tiles); tile < num_tiles;
          tile = next_ordered_tile(work, ord, rbuf, heavy, num_tiles)) {
         uint32_t i, j;
         const bool valid = tile_pixel(tile, threadIdx.x & 31, cam.width, cam.height, &i, &j);
         if (!valid) i = j = 0;  // lanes past the image edge only help the warp
-        const f3 d = primary_dir(cam, i, j);
-        const RayState r = make_ray(mk3(cam.eye[0], cam.eye[1], cam.eye[2]), d, 1e16f, -1);
+        const RayState r = make_ray(mk3(cam.eye[0], cam.eye[1], cam.eye[2]), primary_dir(cam, i, j), 1e16f, -1);
         uint32_t nb = 0, nt = 0, leaf = 1;
-        int slot = -1;
-        const Hit h = trace_ray<STATS>(r, valid, tr, false, &nb, &nt, &spill, &slot, 1u, &leaf);
-        const size_t p = (size_t)j * cam.width + i;
+        const Hit h = trace_ray<true>(r, valid, tr, false, &nb, &nt, nullptr, nullptr, 1u, &leaf);
         if (valid) {
-            if (slot >= 0) {
-                spill_record(list, slot, kHeavyPrimary, p);
-            } else {
-                store_hit(hits + p, h);
-                if (leaves) leaves[p] = leaf;
-            }
-            if (STATS) {
-                stats[2 * p] = nb;
-                stats[2 * p + 1] = nt;
-            }
-        }
-        if (sl.lists) {  // uniform; a handed-over pixel is set up by the warp-per-ray pass
-            const int4 ph = make_int4(h.id, __float_as_int(h.u), __float_as_int(h.v), __float_as_int(h.t));
-            shade_setup_pixel(sl, cam, ph, valid && slot < 0, i, j, p, leaf);
+            const size_t p = (size_t)j * cam.width + i;
+            store_hit(hits + p, h);
+            if (leaves) leaves[p] = leaf;
+            stats[2 * p] = nb;
+            stats[2 * p + 1] = nt;
         }
         record_tile_cost(ord, wbuf, tile, nb + nt);
     }
 }
 
-
 // Primary rays over the trace records (Walk), an 8 x 4 tile per warp at a time:
 // neighbouring rays visit the same leaves, so handing out pixels one by one to the
 // lanes that are done (as the shading rays are) was slower.
-#ifndef RT_PRS
-#define RT_PRS 3
-#endif
-constexpr int kPrimSteps = RT_PRS;  // 3: 1,415 us a frame of 2.1 M triangles, 4: 1,423, 8: 1,413 (65 k triangles, 512 x 512: 312, 309, 330)
+// Of kPrimSteps 3, 4 and 8: 1,415, 1,423 and 1,413 us a frame of 2.1 M triangles at
+// 1080p, 312, 309 and 330 us of 65 k triangles at 512 x 512.
+constexpr int kPrimSteps = 3;
 
 __global__ void __launch_bounds__(kTraceThreads, 8) k_walk_primary(TreeRef tr, rt_camera cam, rt_hit* __restrict__ hits,
                                                                         uint32_t* __restrict__ leaves, uint32_t* work,
@@ -207,78 +191,52 @@ __global__ void __launch_bounds__(kTraceThreads, 8) k_walk_primary(TreeRef tr, r
     }
 }
 
-// Shadow (any hit) and mirror (closest hit) rays of one pixel whose primary
-// hit is ph.  Called by all lanes of the warp together (valid == false for
-// lanes past the image edge); rays of pixels whose primary ray missed, or
-// whose light is behind the surface, are traced with active == false.
-template <bool STATS>
-__device__ __forceinline__ void secondary_pixel(const TreeRef& tr, const float* __restrict__ soup,
-                                                const rt_camera& cam, float lx, float ly, float lz, int4 ph,
-                                                uint8_t* __restrict__ vis, rt_hit* __restrict__ mirror,
-                                                uint32_t* __restrict__ sstats, uint32_t* __restrict__ mstats,
-                                                bool valid, uint32_t i, uint32_t j, const Spill* spill,
-                                                uint32_t* __restrict__ list, uint32_t* tests, uint32_t start,
-                                                uint32_t* __restrict__ mirror_leaves) {
-    const size_t p = (size_t)j * cam.width + i;
-    const ShadeRays s = shade_rays(soup, cam, lx, ly, lz, ph, valid, i, j, mirror != nullptr);
-    uint32_t snb = 0, snt = 0, mnb = 0, mnt = 0;
-    if (vis) {  // uniform across the warp
-        int slot = -1;
-        const Hit sh = trace_ray<STATS>(s.shadow, s.cast, tr, true, &snb, &snt, spill, &slot, start);
-        if (valid) {
-            if (slot >= 0) spill_record(list, slot, kHeavyShadow, p);
-            else vis[p] = vis_code(s.has, s.cast, sh.id >= 0);
-        }
-    }
-    if (mirror) {
-        int slot = -1;
-        uint32_t leaf = 1;
-        Hit mh = trace_ray<STATS>(s.mirror, s.has, tr, false, &mnb, &mnt, spill, &slot, start, &leaf);
-        if (!s.has) {
-            mh.id = -2; mh.u = -1.0f; mh.v = -1.0f; mh.t = 0.0f;
-        }
-        if (valid) {
-            if (slot >= 0) {
-                spill_record(list, slot, kHeavyMirror, p);
-            } else {
-                store_hit(mirror + p, mh);
-                if (mirror_leaves) mirror_leaves[p] = leaf;
-            }
-        }
-    }
-    if (STATS && valid) {
-        if (sstats) { sstats[2 * p] = snb; sstats[2 * p + 1] = snt; }
-        if (mstats) { mstats[2 * p] = mnb; mstats[2 * p + 1] = mnt; }
-    }
-    if (tests) *tests = snb + snt + mnb + mnt;
-}
-
 // Restart node of a pixel's shading rays: its primary hit's leaf, or the root.
 __device__ __forceinline__ uint32_t shade_start(const uint32_t* __restrict__ prim_leaves, int4 ph, bool valid,
                                                 size_t p) {
     return (prim_leaves && valid && ph.x >= 0) ? __ldg(prim_leaves + p) : 1u;
 }
 
-template <bool STATS>
+// Shadow (any hit) and mirror (closest hit) rays with their test counts, in the
+// oracle's order.  Rays of pixels whose primary ray missed, or whose light is
+// behind the surface, are traced with active == false.
 __global__ void __launch_bounds__(kTraceThreads) k_trace_secondary(
     TreeRef tr, const float* __restrict__ soup, rt_camera cam, float lx, float ly, float lz,
     const rt_hit* __restrict__ prim, const uint32_t* __restrict__ prim_leaves, uint8_t* __restrict__ vis,
     rt_hit* __restrict__ mirror, uint32_t* __restrict__ mirror_leaves, uint32_t* __restrict__ sstats,
-    uint32_t* __restrict__ mstats, uint32_t* work, uint32_t num_tiles, Spill spill, uint32_t* __restrict__ list,
-    TileOrder ord) {
+    uint32_t* __restrict__ mstats, uint32_t* work, uint32_t num_tiles, TileOrder ord) {
     const uint32_t wbuf = *ord.parity, rbuf = wbuf ^ 1u, heavy = min(ord.counts[rbuf], ord.cap);
     for (uint32_t tile = next_ordered_tile(work, ord, rbuf, heavy, num_tiles); tile < num_tiles;
          tile = next_ordered_tile(work, ord, rbuf, heavy, num_tiles)) {
         uint32_t i, j;
         const bool valid = tile_pixel(tile, threadIdx.x & 31, cam.width, cam.height, &i, &j);
-        if (!valid) i = j = 0;
+        if (!valid) i = j = 0;  // lanes past the image edge only help the warp
+        const size_t p = (size_t)j * cam.width + i;
         int4 ph = make_int4(-1, 0, 0, 0);
-        if (valid) ph = __ldg(reinterpret_cast<const int4*>(prim + (size_t)j * cam.width + i));
-        uint32_t tests = 0;
-        secondary_pixel<STATS>(tr, soup, cam, lx, ly, lz, ph, vis, mirror, sstats, mstats, valid, i, j, &spill,
-                               list, &tests, shade_start(prim_leaves, ph, valid, (size_t)j * cam.width + i),
-                               mirror_leaves);
-        record_tile_cost(ord, wbuf, tile, tests);
+        if (valid) ph = __ldg(reinterpret_cast<const int4*>(prim + p));
+        const uint32_t start = shade_start(prim_leaves, ph, valid, p);
+        const ShadeRays s = shade_rays(soup, cam, lx, ly, lz, ph, valid, i, j, mirror != nullptr);
+        uint32_t snb = 0, snt = 0, mnb = 0, mnt = 0;
+        if (vis) {  // uniform across the warp
+            const Hit sh = trace_ray<true>(s.shadow, s.cast, tr, true, &snb, &snt, nullptr, nullptr, start);
+            if (valid) vis[p] = vis_code(s.has, s.cast, sh.id >= 0);
+        }
+        if (mirror) {
+            uint32_t leaf = 1;
+            Hit mh = trace_ray<true>(s.mirror, s.has, tr, false, &mnb, &mnt, nullptr, nullptr, start, &leaf);
+            if (!s.has) {
+                mh.id = -2; mh.u = -1.0f; mh.v = -1.0f; mh.t = 0.0f;
+            }
+            if (valid) {
+                store_hit(mirror + p, mh);
+                if (mirror_leaves) mirror_leaves[p] = leaf;
+            }
+        }
+        if (valid) {
+            if (sstats) { sstats[2 * p] = snb; sstats[2 * p + 1] = snt; }
+            if (mstats) { mstats[2 * p] = mnb; mstats[2 * p + 1] = mnt; }
+        }
+        record_tile_cost(ord, wbuf, tile, snb + snt + mnb + mnt);
     }
 }
 
@@ -287,10 +245,10 @@ __global__ void __launch_bounds__(kTraceThreads) k_trace_secondary(
 // primary hit: visibility 0 and the mirror miss record; light behind the
 // surface: visibility 1) and appends the pixels that cast a shadow ray and
 // those that cast a mirror ray to two lists, a warp's pixels in order, so
-// neighbouring rays stay neighbours, each with the ray the tile pass would
-// cast and its start node.  k_trace_shade then traces the lists 32 rays per
-// warp with every lane busy (the tile pass leaves the lanes of sky pixels and
-// of pixels without a cast ray idle).
+// neighbouring rays stay neighbours, each with the ray that k_trace_secondary
+// would cast and its start node.  k_walk_shade then traces the lists with every
+// lane busy (a pass over the pixels leaves the lanes of sky pixels and of
+// pixels without a cast ray idle).
 __global__ void __launch_bounds__(256) k_shade_setup(const float* __restrict__ soup, rt_camera cam, float lx, float ly,
                                                      float lz, const rt_hit* __restrict__ prim, uint8_t* __restrict__ vis,
                                                      rt_hit* __restrict__ mirror, uint32_t* __restrict__ mirror_leaves,
@@ -426,11 +384,15 @@ __global__ void __launch_bounds__(kTraceThreads, 8) k_walk_shade(
 // from 0.2 M rays on, 1 M rays 1.63 -> 0.79 ms).
 constexpr uint32_t kWalkAnyRays = 1u << 20;
 
+// The any-hit rays in doubt: their list, or, when more than `cap` are, the marks that
+// each of them has left in its hit.
 struct Doubt {
     uint32_t* list;
     uint32_t* count;
     uint32_t* work;
+    uint32_t cap;
 };
+constexpr int kDoubtMark = -3;
 
 // A caller's rays over the trace records.  A closest hit does not depend on the
 // walk, so a ray over the budget goes to the warp-per-ray pass.  The first
@@ -473,18 +435,23 @@ __global__ void __launch_bounds__(kTraceThreads, 8) k_walk_rays(TreeRef tr, cons
         }
         w.round(tr, kRaySteps, stack, any_hit != 0);
         int slot = -1;
+        bool doubtful = false;
         if (live && w.have && budgeted && w.tests > spill.budget) {
             const uint32_t e = atomicAdd(any_hit ? doubt.count : spill.count, 1u);
-            if (e < spill.cap) {
+            if (any_hit) {
+                doubtful = true;
+                if (e < doubt.cap) doubt.list[e] = k;
+                w.stop();
+            } else if (e < spill.cap) {
                 slot = (int)e;
                 w.stop();
             } else {
-                budgeted = false;
+                budgeted = false;  // list full: finish here
             }
         }
         if (live && !w.have) {
-            if (slot >= 0 && any_hit) {
-                doubt.list[slot] = k;
+            if (doubtful) {
+                hits[k].id = kDoubtMark;
             } else {
                 store_hit(hits + k, w.hit());
                 if (slot >= 0) spill_record(list, slot, kHeavyRay, k);
@@ -495,14 +462,14 @@ __global__ void __launch_bounds__(kTraceThreads, 8) k_walk_rays(TreeRef tr, cons
     }
 }
 
-// The any-hit rays in doubt.
 __global__ void __launch_bounds__(kTraceThreads) k_trace_doubt(TreeRef tr, const rt_ray* __restrict__ rays,
-                                                               const uint32_t* __restrict__ starts,
+                                                               uint32_t num_rays, const uint32_t* __restrict__ starts,
                                                                rt_hit* __restrict__ hits, uint32_t* __restrict__ leaves,
                                                                Doubt doubt, Spill spill, uint32_t* __restrict__ list) {
     constexpr uint32_t kFull = 0xffffffffu;
     grid_dep_wait();
-    const uint32_t n = min(*doubt.count, spill.cap);
+    const bool marked = *doubt.count > doubt.cap;
+    const uint32_t n = marked ? num_rays : *doubt.count;
     const int lane = threadIdx.x & 31;
     Walk w;
     w.clear();
@@ -518,11 +485,12 @@ __global__ void __launch_bounds__(kTraceThreads) k_trace_doubt(TreeRef tr, const
             uint32_t base = 0;
             if (lane == 0) base = atomicAdd(doubt.work, (uint32_t)__popc(idle));
             base = __shfl_sync(kFull, base, 0);
-            if (base + (uint32_t)__popc(idle) >= n) drained = true;
+            if (base >= n || n - base <= (uint32_t)__popc(idle)) drained = true;
             const uint32_t q = base + __popc(idle & ((1u << lane) - 1u));
-            const bool take = ((idle >> lane) & 1u) && q < n;
+            bool take = ((idle >> lane) & 1u) && base < n && q < n;
+            if (take && marked) take = hits[q].id == kDoubtMark;
             if (take) {
-                k = doubt.list[q];
+                k = marked ? q : doubt.list[q];
                 live = true;
             }
             w.start(take, load_ray(rays, k, take), tr, (starts && take) ? __ldg(starts + k) : 1u, stack, true);
@@ -972,14 +940,13 @@ rt_status trace_primary(rt_ctx* ctx, const rt_lbvh* l, const rt_camera* cam, rt_
     memset(&none, 0, sizeof(none));
     const ShadeLists lists = (sl && !d_stats) ? *sl : none;
     if (d_stats) {
-        auto k = k_trace_primary<true>;
-        k<<<persistent_blocks(ctx, k, kTraceThreads, tiles), kTraceThreads, 0, ctx->stream>>>(
-            tree_ref(ctx, l), *cam, d_hits, d_leaves, d_stats, work, tiles, sp, ctx->d_spill, ord, none);
+        k_trace_primary<<<persistent_blocks(ctx, k_trace_primary, kTraceThreads, tiles), kTraceThreads, 0,
+                          ctx->stream>>>(tree_ref(ctx, l), *cam, d_hits, d_leaves, d_stats, work, tiles, ord);
     } else {
         launch_pdl(k_walk_primary, persistent_blocks(ctx, k_walk_primary, kTraceThreads, tiles), kTraceThreads, 0, ctx->stream,
                    tree_ref(ctx, l), *cam, d_hits, d_leaves, work, tiles, sp, ctx->d_spill, ord, lists);
     }
-    RT_CHECK_LAUNCH(ctx, "k_trace_primary");
+    RT_CHECK_LAUNCH(ctx, d_stats ? "k_trace_primary" : "k_walk_primary");
     HeavyArgs a = heavy_args(ctx, l);
     a.cam = *cam;
     a.hits = d_hits;
@@ -1007,10 +974,10 @@ rt_status trace_shadow_mirror(rt_ctx* ctx, const rt_lbvh* l, const rt_camera* ca
         TileOrder ord;
         if ((s = order_begin(ctx, 1, ctx->tile_order & 2u, &ord, reset)) != RT_OK) return s;
         uint32_t* work = ctx->d_work + kWorkSecondary;
-        auto k = k_trace_secondary<true>;
-        k<<<persistent_blocks(ctx, k, kTraceThreads, tiles), kTraceThreads, 0, ctx->stream>>>(
-            tree_ref(ctx, l), l->src_tris, *cam, light[0], light[1], light[2], d_primary, d_prim_leaves, d_vis,
-            d_mirror, d_mirror_leaves, d_shadow_stats, d_mirror_stats, work, tiles, sp, ctx->d_spill, ord);
+        k_trace_secondary<<<persistent_blocks(ctx, k_trace_secondary, kTraceThreads, tiles), kTraceThreads, 0,
+                            ctx->stream>>>(tree_ref(ctx, l), l->src_tris, *cam, light[0], light[1], light[2], d_primary,
+                                           d_prim_leaves, d_vis, d_mirror, d_mirror_leaves, d_shadow_stats,
+                                           d_mirror_stats, work, tiles, ord);
         RT_CHECK_LAUNCH(ctx, "k_trace_secondary");
     } else {  // compacted shading-ray lists
         const size_t px = (size_t)cam->width * cam->height;
@@ -1081,20 +1048,21 @@ rt_status trace_rays(rt_ctx* ctx, const rt_lbvh* l, const rt_ray* d_rays, uint32
         k<<<persistent_blocks(ctx, k, kTraceThreads, tiles), kTraceThreads, 0, ctx->stream>>>(
             tree_ref(ctx, l), d_rays, n, any_hit, d_starts, d_hits, d_leaves, d_stats, work, sp, ctx->d_spill, ord);
     } else if (walk) {
-        const Doubt doubt{ctx->d_spill + kSpillCap, ctx->d_words + kDoubtCount, ctx->d_words + kDoubtCount + 1};
+        const Doubt doubt{ctx->d_spill + kSpillCap, ctx->d_words + kDoubtCount, ctx->d_words + kDoubtCount + 1,
+                          kSpillCap};
         launch_pdl(k_walk_rays, persistent_blocks(ctx, k_walk_rays, kTraceThreads, tiles), kTraceThreads, 0, ctx->stream,
                    tree_ref(ctx, l), d_rays, n, any_hit, d_starts, d_hits, d_leaves, work, sp, ctx->d_spill, doubt);
         if (any_hit && sp.count) {
             RT_CHECK_LAUNCH(ctx, "k_walk_rays");
             launch_pdl(k_trace_doubt, persistent_blocks(ctx, k_trace_doubt, kTraceThreads, tiles), kTraceThreads, 0,
-                       ctx->stream, tree_ref(ctx, l), d_rays, d_starts, d_hits, d_leaves, doubt, sp, ctx->d_spill);
+                       ctx->stream, tree_ref(ctx, l), d_rays, n, d_starts, d_hits, d_leaves, doubt, sp, ctx->d_spill);
         }
     } else {
         auto k = k_trace_rays<false>;
         k<<<persistent_blocks(ctx, k, kTraceThreads, tiles), kTraceThreads, 0, ctx->stream>>>(
             tree_ref(ctx, l), d_rays, n, any_hit, d_starts, d_hits, d_leaves, nullptr, work, sp, ctx->d_spill, ord);
     }
-    RT_CHECK_LAUNCH(ctx, "k_trace_rays");
+    RT_CHECK_LAUNCH(ctx, walk ? (any_hit ? "k_trace_doubt" : "k_walk_rays") : "k_trace_rays");
     HeavyArgs a = heavy_args(ctx, l);
     a.rays = d_rays;
     a.any_hit = any_hit;
@@ -1412,16 +1380,12 @@ extern "C" rt_status rt_trace_frame_shader_order(rt_ctx* ctx, const rt_lbvh* l, 
 namespace {
 
 struct BatchTraceArgs {
-    const rt_node* nodes;
-    const float4* sorted_tris;
     const float* soup;
-    const uint32_t* tri_off;
     const rt_camera* cams;
     const float* lights;
     rt_hit* hits;
     uint8_t* vis;
-    uint32_t* err;
-    uint32_t S, depth, width, height, tiles_per_scene, grab, order;
+    uint32_t S, width, height, tiles_per_scene, grab, order;
 };
 
 // The shadow-ray list of a batched trace.  (A separate kernel argument:
@@ -1580,17 +1544,12 @@ extern "C" rt_status rt_batch_trace(rt_ctx* ctx, const rt_batch* b, rt_hit* d_hi
     tr.err = ctx->d_err;
     const BatchTrees bt{b->nodes, b->tnodes, b->tri_off, b->depth, b->width * b->height};
     BatchTraceArgs a;
-    a.nodes = b->nodes;
-    a.sorted_tris = b->sorted_tris;
     a.soup = b->src_tris;
-    a.tri_off = b->tri_off;
     a.cams = b->cams;
     a.lights = b->lights;
     a.hits = d_hits;
     a.vis = d_vis;
-    a.err = ctx->d_err;
     a.S = b->S;
-    a.depth = b->depth;
     a.width = b->width;
     a.height = b->height;
     a.tiles_per_scene = ((b->width + 7) / 8) * ((b->height + 3) / 4);

@@ -181,7 +181,6 @@ __device__ __forceinline__ float key_t(uint64_t key) { return __uint_as_float((u
 // hit of its leaf; that is the result of testing the leaf's triangles in any
 // order under the tie rule.  `bound` is the lane's acceptance key on entry;
 // returns true when b (and the bound) improved.
-template <bool STATS>
 __device__ __forceinline__ bool leaf_phase(const TreeRef& tr_, const RayState& r, bool have, const NodeBox& cur,
                                            uint32_t node, uint64_t& bound, Best& b, uint32_t& ntri) {
     constexpr uint32_t kFull = 0xffffffffu;
@@ -328,19 +327,12 @@ __device__ __forceinline__ bool leaf_phase(const TreeRef& tr_, const RayState& r
 // child is re-checked, LBVH.cpp:992).  The stack is a ring of kStackSize
 // entries holding [base, sp); a depth-first walk never holds more than the
 // tree depth.  Returns false when the lane has nothing left.
-//
-// CAPPED: at most max_steps internal nodes are expanded in this call; a lane
-// that runs out keeps its place (returns true with *at_leaf false) and goes
-// on at the next call.  The walk, and so every test, is the same.
-template <bool EXACT, bool STATS, bool CAPPED = false>
+template <bool EXACT>
 __device__ __forceinline__ bool descend(const TreeRef& tr_, const RayState& r, float bt, uint32_t& node, NodeBox& cur,
                                         uint32_t* stack_node, float* stack_t0, uint32_t& sp, uint32_t base,
-                                        uint32_t& nbox, int max_steps = 0, bool* at_leaf = nullptr) {
+                                        uint32_t& nbox) {
     const rt_node* __restrict__ nodes = tr_.nodes;
-    int steps = 0;
-    if (CAPPED) *at_leaf = false;
     while (!(__float_as_int(cur.b.z) & 4)) {
-        if (CAPPED && steps++ >= max_steps) return true;
         const int pc = __float_as_int(cur.b.z);
         const uint32_t c0 = child_pair(tr_, node, cur.b.w);
         if (c0 + 1 >= tr_.num_nodes) {
@@ -391,7 +383,6 @@ __device__ __forceinline__ bool descend(const TreeRef& tr_, const RayState& r, f
             cur = load_node(nodes, node);
         }
     }
-    if (CAPPED) *at_leaf = true;
     return true;
 }
 
@@ -513,9 +504,9 @@ __device__ __forceinline__ Hit traverse(const RayState& r, bool active, const Tr
     bool budgeted = !STATS && spill != nullptr && spill->count != nullptr;
     if (active) have = start_walk<EXACT>(r, tr_, start, b.t, stack_node, stack_t0, sp, node, cur, nbox);
     while (__any_sync(kFull, have)) {
-        if (have) have = descend<EXACT, STATS>(tr_, r, b.t, node, cur, stack_node, stack_t0, sp, 0u, nbox);
+        if (have) have = descend<EXACT>(tr_, r, b.t, node, cur, stack_node, stack_t0, sp, 0u, nbox);
         __syncwarp();
-        leaf_phase<STATS>(tr_, r, have, cur, node, bound, b, ntri);
+        leaf_phase(tr_, r, have, cur, node, bound, b, ntri);
         if (have) {
             if (any_hit && b.id >= 0) {
                 have = false;
@@ -602,8 +593,8 @@ __device__ __forceinline__ void mark_records(const TreeRef& tr) {
 
 constexpr uint32_t kGeneral = 8u;    // Walk::sgn: the records do not serve this ray
 constexpr uint32_t kInfinite = 16u;  // some 1 / d is infinite: the reference's NaN-sensitive min / max
-constexpr uint32_t kPoolMin = 3u;   // a leaf of more triangles makes the warp pool its leaves
-constexpr uint32_t kCheckMin = 4u;  // leaves above this many triangles are tested only after their exact box
+constexpr uint32_t kPoolMin = 3u;    // a leaf of more triangles makes the warp pool its leaves
+constexpr uint32_t kCheckMin = 4u;   // leaves above this many triangles are tested only after their exact box
 
 struct Walk {
     f3 o, d, k, n;  // k = E / d, n = (G - o) / d
@@ -651,8 +642,7 @@ struct Walk {
     }
 
     // Lanes with take begin ray r at heap node `first` (<= 1: the root; see
-    // traverse).
-    // counted: over the heap records whatever the ray, so that every test is
+    // traverse).  counted: over the heap records whatever the ray, so that every test is
     // traverse()'s and `at_leaf` its count.
     __device__ __forceinline__ void start(bool take, const RayState& r, const TreeRef& tr, uint32_t first, uint2* stack,
                                           bool counted = false) {
@@ -991,7 +981,7 @@ __device__ __forceinline__ uint64_t warp_min_u64(uint64_t v) {
 // more group.  The stack lives in dynamic shared memory sized per launch.
 constexpr int kWideStackMax = 1024;  // entries per warp for depth <= 29
 constexpr int kWideQueue = 128;      // queued leaves per warp
-constexpr int kWidePairs = 2;         // triangles a lane of traverse_wide has in flight (1: 150 us a frame, 2: 133, 4: more registers, slower)
+constexpr int kWidePairs = 2;        // triangles a lane has in flight (1: 150 us a frame, 2: 133; 4: more registers, slower)
 constexpr int kWideWarps = 4;        // blocks of at most 128 threads
 
 __host__ __device__ constexpr uint32_t wide_stack_entries(uint32_t depth) {

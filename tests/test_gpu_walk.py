@@ -126,3 +126,44 @@ def test_samples_traced_apart(gpu_ctx, oracle_mod, w, h, spp, bounces):
     nodes, ids, _, _ = oracle_mod.lbvh_build(gi.tris, 14)
     ref = oracle_mod.pathtrace(nodes, 14, ids, gi.tris, gi.albedo, gi.emission, cam, spp, bounces, 9)
     assert np.array_equal(img.cpu().numpy().view(np.int32).ravel(), np.ascontiguousarray(ref, np.float32).view(np.int32).ravel())
+
+
+@pytest.mark.parametrize("first,then", [("build", "build"), ("import", "build"), ("build", "import")])
+def test_captured_trace_over_a_later_tree(gpu_ctx, oracle_mod, first, then):
+    """A captured trace call makes the records of the tree that is there when it
+    is replayed, whoever made that tree."""
+    import torch
+    from rtgpu import scenes
+    from rtgpu.api import Context, LBVH, RayTracer, hits_to_numpy
+    n, depth = 20000, 16
+    cam = scenes.look_at((1.7, 1.2, 1.5), (0.5, 0.5, 0.5), vfov_deg=45.0, width=150, height=90)
+    soups = [scenes.random_soup(n, 21), scenes.random_soup(n - 700, 22)]
+    dev = [torch.from_numpy(s).cuda() for s in soups]
+    stream = torch.cuda.Stream()
+    ctx = Context(0, stream)
+    lb, rt = LBVH(ctx, n, depth), RayTracer(ctx)
+
+    def put(how, i):
+        if how == "build":
+            lb.Build(dev[i])
+        else:
+            nodes, ids, _, _ = oracle_mod.lbvh_build(soups[i], depth)
+            lb.Import(nodes, ids, soups[i])
+
+    torch.cuda.synchronize()
+    out = torch.empty((cam.width * cam.height, 4), dtype=torch.int32, device="cuda")
+    put(first, 0)
+    rt.primary(lb, cam, out=out)
+    stream.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=stream):
+        rt.primary(lb, cam, out=out)
+    put(then, 1)
+    stream.synchronize()
+    g.replay()
+    torch.cuda.synchronize()
+    ctx.check()
+    nodes, ids, _, _ = oracle_mod.lbvh_build(soups[1], depth)
+    ref = oracle_mod.trace(nodes, depth, ids, soups[1], oracle_mod.primary_rays(cam))
+    assert np.array_equal(hits_to_numpy(out).view(np.int32).ravel(), np.ascontiguousarray(ref).view(np.int32).ravel())
+    assert (ref["id"] >= 0).mean() > 0.2
