@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(256) k_bounds(const float* __restrict__ tris, 
     // replayed CUDA graph of the build still tags every arrival afresh), [7]
     // whether the trace records are those of this tree, [8] its emission tiles
     if ((gtid >= 1 && gtid < 6) || gtid == 7) counters[gtid] = 0u;
-    if (gtid == 8) counters[8] = (n + kEmitTile - 1u) / kEmitTile;
+    if (gtid == 8) counters[8] = (n + kTreeTile - 1u) / kTreeTile;
     if (gtid == 0) {
         uint32_t e = counters[6] + 1u;
         counters[6] = e ? e : 1u;  // 0 is the value of cleared arrival words
@@ -359,7 +359,17 @@ constexpr uint32_t kLookGroup = 32;
 
 __host__ __device__ constexpr uint32_t look_groups(uint32_t tiles) { return (tiles + kLookGroup - 1) / kLookGroup; }
 
-template <bool SCENE, bool GROUPED = false>
+// Keys per thread of the single-scene build's sort.  A pass of few tiles lasts as
+// long as one tile: 66,000 triangles are built in 94 us with 16 keys a thread,
+// in 85 us with 8, in 80 us with 4 (2: 80, 1: 80).  Above a tile of 4 keys a thread
+// per SM the look-back costs more than that saves (260,000: 114 us with 4, 113 with
+// 8; 400,000: 140 and 139; 1.2 M: 232 and 208), and above one wave of tiles of 8 keys
+// (four blocks an SM) 16 are faster (2.1 M: 336, 310 and 298 us with 4, 8 and 16).
+constexpr uint32_t kSort4Keys = 152u * 4u * kSortThreads;
+constexpr uint32_t kSort8Keys = 4u * 152u * 8u * kSortThreads;
+int sort_items_of(uint32_t n) { return n <= kSort4Keys ? 4 : n <= kSort8Keys ? 8 : kSortItems; }
+
+template <bool SCENE, bool GROUPED = false, int ITEMS = kSortItems>
 __global__ void __launch_bounds__(kSortThreads, 4) k_onesweep(const uint32_t* __restrict__ keys_in,
                                                            const uint32_t* __restrict__ ids_in,
                                                            uint32_t* __restrict__ keys_out,
@@ -368,9 +378,10 @@ __global__ void __launch_bounds__(kSortThreads, 4) k_onesweep(const uint32_t* __
                                                            uint32_t* tile_counter, uint32_t* err,
                                                            const uint32_t* __restrict__ scene_off = nullptr,
                                                            uint32_t S = 0, uint32_t spin_limit = kSpinLimit) {
+    constexpr int kTile = kSortThreads * ITEMS;
     grid_dep_wait();
-    __shared__ uint32_t s_keys[kSortTile];
-    __shared__ uint32_t s_ids[kSortTile];
+    __shared__ uint32_t s_keys[kTile];
+    __shared__ uint32_t s_ids[kTile];
     __shared__ uint32_t s_warp[kSortThreads / 32][256];
     __shared__ uint32_t s_lstart[256];
     __shared__ uint32_t s_gofs[256];
@@ -385,21 +396,21 @@ __global__ void __launch_bounds__(kSortThreads, 4) k_onesweep(const uint32_t* __
     for (int i = lane; i < 256; i += 32) s_warp[w][i] = 0u;
     const uint32_t gbase = block_excl_sum_256(hist[pass * 256 + t], s_tmp);  // includes __syncthreads
     const uint32_t tile = s_tile;
-    const uint32_t base = tile * (uint32_t)kSortTile;
+    const uint32_t base = tile * (uint32_t)kTile;
     const int shift = 8 * pass;
 
-    uint32_t key[kSortItems], idv[kSortItems], rank[kSortItems];
+    uint32_t key[ITEMS], idv[ITEMS], rank[ITEMS];
 #pragma unroll
-    for (int i = 0; i < kSortItems; ++i) {
-        const uint32_t idx = base + w * (32 * kSortItems) + i * 32 + lane;
+    for (int i = 0; i < ITEMS; ++i) {
+        const uint32_t idx = base + w * (32 * ITEMS) + i * 32 + lane;
         const bool valid = idx < n;
         key[i] = valid ? keys_in[idx] : 0xffffffffu;
         idv[i] = valid ? ids_in[idx] : 0u;
     }
     const uint32_t lt = lanemask_lt();
 #pragma unroll
-    for (int i = 0; i < kSortItems; ++i) {
-        const uint32_t idx = base + w * (32 * kSortItems) + i * 32 + lane;
+    for (int i = 0; i < ITEMS; ++i) {
+        const uint32_t idx = base + w * (32 * ITEMS) + i * 32 + lane;
         const bool valid = idx < n;
         const uint32_t d = sort_digit<SCENE>(key[i], idv[i], shift, s_off, S);
         uint32_t peers = __ballot_sync(kFull, valid);
@@ -429,7 +440,7 @@ __global__ void __launch_bounds__(kSortThreads, 4) k_onesweep(const uint32_t* __
 
     uint32_t excl = 0;
     if (GROUPED) {
-        const uint32_t T = (n + kSortTile - 1) / kSortTile;  // the pass's tiles (the grid may start later)
+        const uint32_t T = (n + kTile - 1) / kTile;  // the pass's tiles (the grid may start later)
         uint32_t* gwords = lookback + (size_t)T * 256;
         const uint32_t G = tile / kLookGroup, g0 = G * kLookGroup;
         const bool group_last = (tile - g0 == kLookGroup - 1) || (tile + 1 == T);
@@ -538,12 +549,12 @@ __global__ void __launch_bounds__(kSortThreads, 4) k_onesweep(const uint32_t* __
     __syncthreads();
 
 #pragma unroll
-    for (int i = 0; i < kSortItems; ++i) {
-        const uint32_t idx = base + w * (32 * kSortItems) + i * 32 + lane;
+    for (int i = 0; i < ITEMS; ++i) {
+        const uint32_t idx = base + w * (32 * ITEMS) + i * 32 + lane;
         if (idx < n) {
             const uint32_t d = sort_digit<SCENE>(key[i], idv[i], shift, s_off, S);
             const uint32_t pos = s_lstart[d] + s_warp[w][d] + rank[i];
-            if (pos < (uint32_t)kSortTile) {
+            if (pos < (uint32_t)kTile) {
                 s_keys[pos] = key[i];
                 s_ids[pos] = idv[i];
             } else {
@@ -552,7 +563,7 @@ __global__ void __launch_bounds__(kSortThreads, 4) k_onesweep(const uint32_t* __
         }
     }
     __syncthreads();
-    const uint32_t tile_n = (n - base < (uint32_t)kSortTile) ? (n - base) : (uint32_t)kSortTile;
+    const uint32_t tile_n = (n - base < (uint32_t)kTile) ? (n - base) : (uint32_t)kTile;
     for (uint32_t j = t; j < tile_n; j += kSortThreads) {
         const uint32_t k = s_keys[j];
         const uint32_t gp = s_gofs[sort_digit<SCENE>(k, s_ids[j], shift, s_off, S)] + j;
@@ -618,19 +629,21 @@ __device__ __forceinline__ void block_scan_records(uint32_t vf, uint32_t vb, uin
 }
 
 // Loads the codes a thread needs and its boundary record bits.
+template <int ITEMS = kEmitItems>
 struct EmitChunk {
-    uint32_t c[kEmitItems + 1];  // codes of elements s .. s+8 (0 beyond n)
-    uint32_t r[kEmitItems];      // record bit of boundaries s .. s+7
-    int dl[kEmitItems + 1];      // delta of boundaries s-1 .. s+7 (dl[q] = delta_{s+q-1})
+    uint32_t c[ITEMS + 1];  // codes of elements s .. s+ITEMS (0 beyond n)
+    uint32_t r[ITEMS];      // record bit of boundaries s .. s+ITEMS-1
+    int dl[ITEMS + 1];      // delta of boundaries s-1 .. s+ITEMS-1 (dl[q] = delta_{s+q-1})
 };
 
-__device__ __forceinline__ void load_chunk(const uint32_t* __restrict__ keys, uint32_t n, uint32_t s, EmitChunk& e) {
+template <int ITEMS>
+__device__ __forceinline__ void load_chunk(const uint32_t* __restrict__ keys, uint32_t n, uint32_t s, EmitChunk<ITEMS>& e) {
     uint32_t prev = (s >= 1 && s - 1 < n) ? __ldg(keys + s - 1) : 0u;
 #pragma unroll
-    for (int q = 0; q <= kEmitItems; ++q) e.c[q] = (s + q < n) ? __ldg(keys + s + q) : 0u;
+    for (int q = 0; q <= ITEMS; ++q) e.c[q] = (s + q < n) ? __ldg(keys + s + q) : 0u;
     e.dl[0] = (s >= 1 && s < n) ? delta_of(prev, e.c[0]) : -1;
 #pragma unroll
-    for (int q = 0; q < kEmitItems; ++q) {
+    for (int q = 0; q < ITEMS; ++q) {
         const uint32_t i = s + q;  // boundary i between i and i+1
         const int d = (i + 1 < n) ? delta_of(e.c[q], e.c[q + 1]) : -1;
         e.dl[q + 1] = d;
@@ -642,16 +655,17 @@ constexpr int kSepBit = 31;  // a batch's separator record, above every code bit
 
 // Boundary deltas of a thread's chunk with a separator record at each
 // scene boundary (off: S + 1 scene offsets in shared memory).
+template <int ITEMS>
 __device__ __forceinline__ void load_chunk_b(const uint32_t* __restrict__ keys, uint32_t n, uint32_t s,
-                                             const uint32_t* off, uint32_t S, EmitChunk& e) {
+                                             const uint32_t* off, uint32_t S, EmitChunk<ITEMS>& e) {
     const uint32_t prev = (s >= 1 && s - 1 < n) ? __ldg(keys + s - 1) : 0u;
 #pragma unroll
-    for (int q = 0; q <= kEmitItems; ++q) e.c[q] = (s + q < n) ? __ldg(keys + s + q) : 0u;
+    for (int q = 0; q <= ITEMS; ++q) e.c[q] = (s + q < n) ? __ldg(keys + s + q) : 0u;
     uint32_t sc = scene_of(off, S, s < n ? s : n - 1);
     e.dl[0] = (s >= 1 && s < n) ? (s == off[sc] ? kSepBit : delta_of(prev, e.c[0])) : -1;
     uint32_t nb = off[sc + 1];
 #pragma unroll
-    for (int q = 0; q < kEmitItems; ++q) {
+    for (int q = 0; q < ITEMS; ++q) {
         const uint32_t i = s + q;
         int d = -1;
         if (i + 1 < n) {
@@ -669,6 +683,7 @@ __device__ __forceinline__ void load_chunk_b(const uint32_t* __restrict__ keys, 
 }
 
 // k_emit_tiles: per-tile fwd/bwd aggregates of the boundary record masks.
+template <int ITEMS>
 __global__ void __launch_bounds__(kEmitThreads) k_emit_tiles(const uint32_t* __restrict__ keys, uint32_t n,
                                                              uint32_t* scan, uint32_t* arrive, uint32_t arrive_words,
                                                              const uint32_t* epoch_word) {
@@ -680,14 +695,14 @@ __global__ void __launch_bounds__(kEmitThreads) k_emit_tiles(const uint32_t* __r
         for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < arrive_words; i += gridDim.x * blockDim.x)
             arrive[i] = 0u;
     __shared__ uint32_t s_f[8], s_b[8];
-    const uint32_t s = blockIdx.x * kEmitTile + threadIdx.x * kEmitItems;
-    EmitChunk e;
+    const uint32_t s = (blockIdx.x * kEmitThreads + threadIdx.x) * ITEMS;
+    EmitChunk<ITEMS> e;
     load_chunk(keys, n, s, e);
     uint32_t af = 0, ab = 0;
 #pragma unroll
-    for (int q = 0; q < kEmitItems; ++q) af = rec_fwd(af, e.r[q]);
+    for (int q = 0; q < ITEMS; ++q) af = rec_fwd(af, e.r[q]);
 #pragma unroll
-    for (int q = kEmitItems - 1; q >= 0; --q) ab = rec_bwd(e.r[q], ab);
+    for (int q = ITEMS - 1; q >= 0; --q) ab = rec_bwd(e.r[q], ab);
     af = warp_reduce_ordered<true>(af);
     ab = warp_reduce_ordered<false>(ab);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -760,7 +775,7 @@ __global__ void __launch_bounds__(kEmitThreads) k_emit_leaves(const uint32_t* __
     grid_dep_wait();
     __shared__ uint32_t s_f[8], s_b[8];
     const uint32_t s = blockIdx.x * kEmitTile + threadIdx.x * kEmitItems;
-    EmitChunk e;
+    EmitChunk<> e;
     load_chunk(keys, n, s, e);
     uint32_t af = 0, ab = 0;
 #pragma unroll
@@ -1060,7 +1075,7 @@ __global__ void __launch_bounds__(256) k_emit_refit(const uint32_t* __restrict__
 //      here: its start is found by scanning back over the codes and its
 //      earlier triangles are folded in from the soup.
 // k_emit_chunks then runs a shared-memory bottom-up (unit_bottom_up) over a
-// chunk of one tile's units per CTA; a node whose parent's split boundary lies
+// tile's units per CTA; a node whose parent's split boundary lies
 // outside the units becomes an "item" for the next level, and k_emit_merge runs
 // over the items of kMergeGroup consecutive chunks (groups) per CTA,
 // level after level, until one CTA forms the root.  No node waits on another
@@ -1074,23 +1089,18 @@ __global__ void __launch_bounds__(256) k_emit_refit(const uint32_t* __restrict__
 constexpr uint32_t kHeadBit = 1u << 30;
 constexpr uint32_t kTailBit = 1u << 31;
 constexpr uint32_t kMaskBits = kHeadBit - 1u;
-constexpr int kUnitCap = kEmitTile;  // units of one CTA: the leaves of a tile, the items of a group
-constexpr int kChunkUnits = 512;     // units of one CTA of the tile level (a tile's leaves in chunks)
-constexpr int kTileChunks = kUnitCap / kChunkUnits;
 constexpr int kItemCap = 64;         // items one tile or group hands on (2 x depth + 2 <= 54)
 constexpr int kMergeGroup = 32;      // tiles (groups) per CTA of the next level
 constexpr int kUnitWords = 12;       // shared words per unit
+constexpr int kUnitCap = kMergeGroup * kItemCap;  // units of one CTA of the merge: the items of a group
 constexpr size_t kUnitSmem = (size_t)kUnitWords * kUnitCap * sizeof(uint32_t) + 16;
-constexpr size_t kChunkSmem = (size_t)kUnitWords * kChunkUnits * sizeof(uint32_t) + 16;
+constexpr size_t kChunkSmem = (size_t)kUnitWords * kTreeTile * sizeof(uint32_t) + 16;
 // k_emit_units: the tile's triangle boxes, six planes of kBoxStride floats
 // (element e at e + e / 32, so that a warp reading eight consecutive
 // elements per lane hits 32 different banks), then one staging buffer of
 // 32 triangles (96 float4) per warp
-constexpr int kBoxStride = kEmitTile + kEmitTile / 32;
-constexpr int kGatherBatch = 4;  // triangles a thread has in flight in the gather
-constexpr size_t kEmitUnitsSmem = 6 * kBoxStride * sizeof(float) + (kEmitThreads / 32) * 96 * sizeof(float4);
+constexpr int kBoxStride = kTreeTile + kTreeTile / 32;
 static_assert((6 * kBoxStride) % 4 == 0, "staging buffer must start 16-byte aligned");
-static_assert(kEmitItems % kGatherBatch == 0, "gather batches must tile a thread's elements");
 
 // Triangle `id` of a soup of n triangles (9 floats each): three 16-byte
 // loads of the 12 floats starting at float 9 id - (id mod 4), which is 16-byte
@@ -1336,8 +1346,8 @@ struct Seg {
     int32_t head;
 };
 
-template <int THREADS, bool BATCH>
-__global__ void __launch_bounds__(THREADS) k_emit_units(const uint32_t* __restrict__ keys,
+template <bool BATCH>
+__global__ void __launch_bounds__(kEmitThreads) k_emit_units(const uint32_t* __restrict__ keys,
                                                         const uint32_t* __restrict__ ids,
                                                         const float* __restrict__ tris, uint32_t n, uint32_t depth,
                                                         const uint32_t* __restrict__ scan, rt_node* nodes,
@@ -1346,14 +1356,14 @@ __global__ void __launch_bounds__(THREADS) k_emit_units(const uint32_t* __restri
                                                         uint32_t* __restrict__ leaf_of,
                                                         const uint32_t* __restrict__ scene_off, uint32_t S,
                                                         uint32_t* __restrict__ ids_local) {
+    constexpr int THREADS = kEmitThreads, ITEMS = kTreeItems, TILE = kTreeTile;
     __shared__ uint32_t s_f[THREADS / 32], s_b[THREADS / 32], s_tmp[THREADS / 32];
     __shared__ uint32_t s_first_head, s_first_tail, s_last_head, s_last_tail, s_cont_tail;
     __shared__ float s_red[THREADS / 32][6];
     __shared__ int32_t s_rhead[THREADS / 32];
     __shared__ int s_found;
     __shared__ float s_cont_box[6];
-    static_assert(THREADS == kEmitThreads, "the shared-memory layout is sized for kEmitThreads");
-    extern __shared__ float4 emit_smem[];
+    __shared__ float4 emit_smem[6 * kBoxStride / 4 + (THREADS / 32) * 96];
     float* s_box = reinterpret_cast<float*>(emit_smem);  // [6][kBoxStride]: lo xyz, hi xyz
 
     __shared__ uint32_t s_off[BATCH ? kMaxBatchScenes + 1 : 1];
@@ -1365,10 +1375,10 @@ __global__ void __launch_bounds__(THREADS) k_emit_units(const uint32_t* __restri
     }
     const Heap<BATCH> heap{nodes, scene_off, depth};
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-    const uint32_t tbase = blockIdx.x * (uint32_t)kEmitTile;
-    uint2* my_units = units + (size_t)blockIdx.x * kUnitCap;
+    const uint32_t tbase = blockIdx.x * (uint32_t)TILE;
+    uint2* my_units = units + (size_t)blockIdx.x * TILE;
     if (t == 0) {
-        s_first_head = s_first_tail = kEmitTile;
+        s_first_head = s_first_tail = TILE;
         s_last_head = s_last_tail = 0u;
     }
     // 0. pre-gather in sorted order (A.xyz,id | B.xyz,0 | C.xyz,0): element
@@ -1377,84 +1387,81 @@ __global__ void __launch_bounds__(THREADS) k_emit_units(const uint32_t* __restri
     {
         float4* stage = emit_smem + (6 * kBoxStride) / 4 + w * 96;
         const bool soup_aligned = (reinterpret_cast<uintptr_t>(tris) & 15u) == 0;
-#pragma unroll 1
-        for (int g = 0; g < kEmitItems; g += kGatherBatch) {
-            uint32_t idv[kGatherBatch], loc[kGatherBatch];  // the triangle, and its id in its own tree
-            float v[kGatherBatch][9];
+        uint32_t idv[ITEMS], loc[ITEMS];  // the triangle, and its id in its own tree
+        float v[ITEMS][9];
 #pragma unroll
-            for (int b = 0; b < kGatherBatch; ++b) {
-                const uint32_t k = tbase + (uint32_t)((g + b) * THREADS + t);
-                uint32_t id = k < n ? __ldg(ids + k) : 0u;
-                if (BATCH) {
-                    const uint32_t sk = scene_of(s_off, S, min(k, n - 1u));
-                    if (k < n && (id < s_off[sk] || id >= s_off[sk + 1])) {  // only after a failed sort
-                        atomicOr(err, RT_DEVERR_BOUNDS);
-                        id = s_off[sk];
-                    }
-                    loc[b] = id - s_off[sk];
-                    if (k < n) ids_local[k] = loc[b];
-                } else if (id >= n) {  // only after a failed sort (look-back timeout)
+        for (int b = 0; b < ITEMS; ++b) {
+            const uint32_t k = tbase + (uint32_t)(b * THREADS + t);
+            uint32_t id = k < n ? __ldg(ids + k) : 0u;
+            if (BATCH) {
+                const uint32_t sk = scene_of(s_off, S, min(k, n - 1u));
+                if (k < n && (id < s_off[sk] || id >= s_off[sk + 1])) {  // only after a failed sort
                     atomicOr(err, RT_DEVERR_BOUNDS);
-                    id = 0;
+                    id = s_off[sk];
                 }
-                idv[b] = id;
-                if (!BATCH) loc[b] = id;
+                loc[b] = id - s_off[sk];
+                if (k < n) ids_local[k] = loc[b];
+            } else if (id >= n) {  // only after a failed sort (look-back timeout)
+                atomicOr(err, RT_DEVERR_BOUNDS);
+                id = 0;
             }
+            idv[b] = id;
+            if (!BATCH) loc[b] = id;
+        }
 #pragma unroll
-            for (int b = 0; b < kGatherBatch; ++b) load_tri(tris, idv[b], n, soup_aligned, v[b]);
+        for (int b = 0; b < ITEMS; ++b) load_tri(tris, idv[b], n, soup_aligned, v[b]);
 #pragma unroll
-            for (int b = 0; b < kGatherBatch; ++b) {
-                const uint32_t e0 = (uint32_t)((g + b) * THREADS + w * 32);  // the warp's first element
-                const uint32_t el = e0 + lane;
-                const Box tb = tri_box(v[b]);
-                const uint32_t pb = el + (el >> 5);
+        for (int b = 0; b < ITEMS; ++b) {
+            const uint32_t e0 = (uint32_t)(b * THREADS + w * 32);  // the warp's first element
+            const uint32_t el = e0 + lane;
+            const Box tb = tri_box(v[b]);
+            const uint32_t pb = el + (el >> 5);
 #pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    s_box[c * kBoxStride + pb] = tb.lo[c];
-                    s_box[(3 + c) * kBoxStride + pb] = tb.hi[c];
-                }
-                stage[3 * lane + 0] = make_float4(v[b][0], v[b][1], v[b][2], __int_as_float((int)loc[b]));
-                stage[3 * lane + 1] = make_float4(v[b][3], v[b][4], v[b][5], 0.0f);
-                stage[3 * lane + 2] = make_float4(v[b][6], v[b][7], v[b][8], 0.0f);
-                __syncwarp();
-                const uint32_t kw = tbase + e0;
-                const uint32_t live = kw < n ? min(32u, n - kw) : 0u;  // the run's elements inside the soup
-#pragma unroll
-                for (int j = 0; j < 3; ++j) {
-                    const uint32_t f = (uint32_t)(lane + 32 * j);
-                    if (f < 3 * live) sorted_tris[3 * (size_t)kw + f] = stage[f];
-                }
-                __syncwarp();
+            for (int c = 0; c < 3; ++c) {
+                s_box[c * kBoxStride + pb] = tb.lo[c];
+                s_box[(3 + c) * kBoxStride + pb] = tb.hi[c];
             }
+            stage[3 * lane + 0] = make_float4(v[b][0], v[b][1], v[b][2], __int_as_float((int)loc[b]));
+            stage[3 * lane + 1] = make_float4(v[b][3], v[b][4], v[b][5], 0.0f);
+            stage[3 * lane + 2] = make_float4(v[b][6], v[b][7], v[b][8], 0.0f);
+            __syncwarp();
+            const uint32_t kw = tbase + e0;
+            const uint32_t live = kw < n ? min(32u, n - kw) : 0u;  // the run's elements inside the soup
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                const uint32_t f = (uint32_t)(lane + 32 * j);
+                if (f < 3 * live) sorted_tris[3 * (size_t)kw + f] = stage[f];
+            }
+            __syncwarp();
         }
     }
 
     // 1. capped mask, head and tail of this thread's elements; heap index at
     // heads and tails (the elements between them share their leaf's)
-    const uint32_t s = tbase + (uint32_t)t * kEmitItems;
-    EmitChunk e;
+    const uint32_t s = tbase + (uint32_t)t * ITEMS;
+    EmitChunk<ITEMS> e;
     if constexpr (BATCH) load_chunk_b(keys, n, s, s_off, S, e);
     else load_chunk(keys, n, s, e);
     uint32_t af = 0, ab = 0;
 #pragma unroll
-    for (int q = 0; q < kEmitItems; ++q) af = rec_fwd(af, e.r[q]);
+    for (int q = 0; q < ITEMS; ++q) af = rec_fwd(af, e.r[q]);
 #pragma unroll
-    for (int q = kEmitItems - 1; q >= 0; --q) ab = rec_bwd(e.r[q], ab);
+    for (int q = ITEMS - 1; q >= 0; --q) ab = rec_bwd(e.r[q], ab);
     uint32_t pre, suf;
     block_scan_records<THREADS>(af, ab, &pre, &suf, s_f, s_b);  // includes __syncthreads
-    uint32_t L[kEmitItems + 1], R[kEmitItems + 1];
+    uint32_t L[ITEMS + 1], R[ITEMS + 1];
     L[0] = rec_fwd(scan[4 * blockIdx.x + 2], pre);
-    R[kEmitItems] = rec_bwd(suf, scan[4 * blockIdx.x + 3]);
+    R[ITEMS] = rec_bwd(suf, scan[4 * blockIdx.x + 3]);
 #pragma unroll
-    for (int q = 0; q < kEmitItems; ++q) L[q + 1] = rec_fwd(L[q], e.r[q]);
+    for (int q = 0; q < ITEMS; ++q) L[q + 1] = rec_fwd(L[q], e.r[q]);
 #pragma unroll
-    for (int q = kEmitItems - 1; q >= 0; --q) R[q] = rec_bwd(e.r[q], R[q + 1]);
+    for (int q = ITEMS - 1; q >= 0; --q) R[q] = rec_bwd(e.r[q], R[q + 1]);
     const int leaf_depth = (int)depth - 1;
-    uint32_t hm[kEmitItems], hh[kEmitItems];  // capped mask | head | tail; heap index (heads, tails)
+    uint32_t hm[ITEMS], hh[ITEMS];  // capped mask | head | tail; heap index (heads, tails)
     uint32_t heads = 0u, tails = 0u;
     uint32_t sc = BATCH ? scene_of(s_off, S, min(s, n - 1u)) : 0u;
 #pragma unroll
-    for (int q = 0; q < kEmitItems; ++q) {
+    for (int q = 0; q < ITEMS; ++q) {
         const uint32_t k = s + q;
         hm[q] = 0u;
         hh[q] = 0u;
@@ -1482,10 +1489,10 @@ __global__ void __launch_bounds__(THREADS) k_emit_units(const uint32_t* __restri
         }
     }
     {  // the tile's first / last head and tail: warp reductions, one shared atomic per warp
-        const uint32_t j0 = (uint32_t)t * kEmitItems;
-        const uint32_t fh = __reduce_min_sync(kFull, heads ? j0 + __ffs(heads) - 1 : (uint32_t)kEmitTile);
+        const uint32_t j0 = (uint32_t)t * ITEMS;
+        const uint32_t fh = __reduce_min_sync(kFull, heads ? j0 + __ffs(heads) - 1 : (uint32_t)TILE);
         const uint32_t lh = __reduce_max_sync(kFull, heads ? j0 + (32 - __clz(heads)) : 0u);
-        const uint32_t ft = __reduce_min_sync(kFull, tails ? j0 + __ffs(tails) - 1 : (uint32_t)kEmitTile);
+        const uint32_t ft = __reduce_min_sync(kFull, tails ? j0 + __ffs(tails) - 1 : (uint32_t)TILE);
         const uint32_t lt = __reduce_max_sync(kFull, tails ? j0 + (32 - __clz(tails)) : 0u);
         if (lane == 0) {
             atomicMin(&s_first_head, fh);
@@ -1499,7 +1506,7 @@ __global__ void __launch_bounds__(THREADS) k_emit_units(const uint32_t* __restri
     // then every leaf with its head and tail in the tile; a last leaf that
     // runs past the tile is the next tile's
     const uint32_t first_head = s_first_head, first_tail = s_first_tail;
-    const uint32_t cont = (first_tail < kEmitTile && first_tail < first_head) ? 1u : 0u;
+    const uint32_t cont = (first_tail < TILE && first_tail < first_head) ? 1u : 0u;
     const bool last_open = s_last_head > s_last_tail;  // the last head's leaf has no tail in the tile
 
     // 2. the leaf boxes: each thread folds its own elements' boxes (gathered
@@ -1514,10 +1521,10 @@ __global__ void __launch_bounds__(THREADS) k_emit_units(const uint32_t* __restri
     int32_t run_pos = -1;
     uint32_t run_h = 0u, run_m = 0u;  // heap index and mask of the current leaf
 #pragma unroll
-    for (int q = 0; q < kEmitItems; ++q) {
+    for (int q = 0; q < ITEMS; ++q) {
         const uint32_t k = s + q;
         if (k >= n) break;
-        const uint32_t el = (uint32_t)t * kEmitItems + q, pb = el + (el >> 5);
+        const uint32_t el = (uint32_t)t * ITEMS + q, pb = el + (el >> 5);
         Box tb;
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
@@ -1527,10 +1534,10 @@ __global__ void __launch_bounds__(THREADS) k_emit_units(const uint32_t* __restri
         const bool head = (hm[q] & kHeadBit) != 0, tail = (hm[q] & kTailBit) != 0;
         if (head) {
             const uint32_t idx = cont + hbase + ord++;
-            const uint32_t j = t * kEmitItems + q;
+            const uint32_t j = t * ITEMS + q;
             run_h = hh[q];
             run_m = hm[q] & kMaskBits;
-            if (idx < (uint32_t)kUnitCap && !(last_open && j + 1 == s_last_head)) my_units[idx] = make_uint2(run_h, run_m);
+            if (idx < (uint32_t)TILE && !(last_open && j + 1 == s_last_head)) my_units[idx] = make_uint2(run_h, run_m);
             run = tb;
             seen_head = true;
             run_pos = (int32_t)k;
@@ -1603,7 +1610,7 @@ __global__ void __launch_bounds__(THREADS) k_emit_units(const uint32_t* __restri
     }
     if (first_tail_q >= 0) {  // the segment entering this thread ends here
         const Box fin = box_union(x.b, part);
-        const uint32_t j = t * kEmitItems + first_tail_q;
+        const uint32_t j = t * ITEMS + first_tail_q;
         if (x.head >= 0) {  // its head is in an earlier thread of this tile
             const int32_t count = (int32_t)(tbase + j) - x.head + 1;
             store_node(heap.node(ft_h), fin.lo, fin.hi, (count << 3) | 4 | leaf_axis_of(ft_m, count, depth),
@@ -1683,7 +1690,7 @@ __global__ void __launch_bounds__(THREADS) k_emit_units(const uint32_t* __restri
     }
     if (t == THREADS - 1) {  // units: cont + heads, less an open last leaf
         const uint32_t total_heads = hbase + __popc(heads);
-        unit_counts[blockIdx.x] = min((uint32_t)kUnitCap, cont + total_heads - (last_open ? 1u : 0u));
+        unit_counts[blockIdx.x] = min((uint32_t)TILE, cont + total_heads - (last_open ? 1u : 0u));
     }
 }
 
@@ -1694,15 +1701,12 @@ __global__ void __launch_bounds__(THREADS) k_emit_units(const uint32_t* __restri
 // The nodes that cannot be formed here are written to `out` sorted by first
 // element, their number to *out_count.
 template <int THREADS, bool BATCH>
-__device__ void merge_group(const Units& u, const uint2* in_items, const uint32_t* in_counts, int fixed_count,
-                            uint32_t in_stride, uint32_t ng, const Heap<BATCH>& heap, uint2* out,
+__device__ void merge_group(const Units& u, const uint2* in_items, const uint32_t* in_counts, uint32_t in_stride, uint32_t ng, const Heap<BATCH>& heap, uint2* out,
                             uint32_t* out_count, uint32_t* err, uint32_t* inner, uint32_t* s_off, uint2* s_items,
                             int32_t* s_ipos) {
     const int t = threadIdx.x;
     if (t < 32) {  // unit offsets of the groups: one warp, a prefix sum over <= 32 counts
-        const uint32_t c = (uint32_t)t < ng ? min(fixed_count >= 0 ? (uint32_t)fixed_count : __ldcg(in_counts + t),
-                                                  in_stride)
-                                            : 0u;
+        const uint32_t c = (uint32_t)t < ng ? min(__ldcg(in_counts + t), in_stride) : 0u;
         uint32_t incl = c;
         for (int off = 1; off < 32; off <<= 1) {
             const uint32_t y = __shfl_up_sync(kFull, incl, off);
@@ -1753,34 +1757,28 @@ __device__ void merge_group(const Units& u, const uint2* in_items, const uint32_
     if (t == 0) *out_count = ni;
 }
 
-// k_emit_chunks: the tile level.  A tile's leaves are merged in chunks of
-// kChunkUnits consecutive leaves, one CTA per chunk (kTileChunks chunk slots
-// per tile, most of them empty for tiles with big leaves), so that the
-// shared-memory units of eight CTAs fit an SM.  Chunk slot c's items go to
-// items + c * kItemCap, their number to counts[c].
-template <int THREADS, bool BATCH>
-__global__ void __launch_bounds__(THREADS) k_emit_chunks(const uint2* __restrict__ tile_units,
-                                                         const uint32_t* __restrict__ tile_counts, uint32_t depth,
-                                                         rt_node* nodes, uint2* items, uint32_t* counts, uint32_t* err,
-                                                         uint32_t* inner, const uint32_t* __restrict__ scene_off) {
+// k_emit_chunks: the tile level.  One CTA merges the leaves of a tile; tile c's
+// items go to items + c * kItemCap, their number to counts[c].
+template <bool BATCH>
+__global__ void __launch_bounds__(kEmitThreads) k_emit_chunks(const uint2* __restrict__ tile_units,
+                                                              const uint32_t* __restrict__ tile_counts, uint32_t depth,
+                                                              rt_node* nodes, uint2* items, uint32_t* counts,
+                                                              uint32_t* err, uint32_t* inner,
+                                                              const uint32_t* __restrict__ scene_off) {
     extern __shared__ __align__(16) uint32_t smem[];
-    const Units u = units_of(smem, kChunkUnits);
+    const Units u = units_of(smem, kTreeTile);
     const Heap<BATCH> heap{nodes, scene_off, depth};
     __shared__ uint32_t s_off[kMergeGroup + 1];
     __shared__ uint2 s_items[kItemCap];
     __shared__ int32_t s_ipos[kItemCap];
     grid_dep_wait();
-    const uint32_t tiles = gridDim.x / kTileChunks, tile = blockIdx.x % tiles, chunk = blockIdx.x / tiles,
-                   c = tile * kTileChunks + chunk;
-    const uint32_t tc = min(__ldcg(tile_counts + tile), (uint32_t)kUnitCap);
-    const int cnt = (int)min((uint32_t)kChunkUnits, tc > chunk * kChunkUnits ? tc - chunk * kChunkUnits : 0u);
-    if (cnt == 0) {
+    const uint32_t c = blockIdx.x;
+    if (__ldcg(tile_counts + c) == 0u) {  // inside one leaf
         if (threadIdx.x == 0) counts[c] = 0u;
         return;
     }
-    merge_group<THREADS, BATCH>(u, tile_units + (size_t)tile * kUnitCap + (size_t)chunk * kChunkUnits, nullptr, cnt,
-                         (uint32_t)kChunkUnits, 1u, heap, items + (size_t)c * kItemCap, counts + c, err, inner,
-                         s_off, s_items, s_ipos);
+    merge_group<kEmitThreads, BATCH>(u, tile_units + (size_t)c * kTreeTile, tile_counts + c, (uint32_t)kTreeTile, 1u, heap,
+                                     items + (size_t)c * kItemCap, counts + c, err, inner, s_off, s_items, s_ipos);
 }
 
 // k_emit_merge: the levels above.  One CTA per kMergeGroup consecutive units
@@ -1791,8 +1789,8 @@ __global__ void __launch_bounds__(THREADS) k_emit_chunks(const uint2* __restrict
 // group covers the whole tree and forms the root.  No CTA waits on another.
 // The first level's items are at out_items + g * kItemCap (counts at
 // out_counts + g), each next level's after the previous one's.
-template <int THREADS, bool BATCH>
-__global__ void __launch_bounds__(THREADS) k_emit_merge(const uint2* __restrict__ in_items,
+template <bool BATCH>
+__global__ void __launch_bounds__(kEmitThreads) k_emit_merge(const uint2* __restrict__ in_items,
                                                         const uint32_t* __restrict__ in_counts, uint32_t n_in,
                                                         uint32_t depth, rt_node* nodes, uint2* out_items,
                                                         uint32_t* out_counts, uint32_t* tickets, uint32_t* err,
@@ -1808,7 +1806,7 @@ __global__ void __launch_bounds__(THREADS) k_emit_merge(const uint2* __restrict_
     const int t = threadIdx.x;
     uint32_t g = blockIdx.x;
     uint32_t n_lev = (n_in + kMergeGroup - 1) / kMergeGroup;
-    merge_group<THREADS, BATCH>(u, in_items + (size_t)g * kMergeGroup * kItemCap, in_counts + (size_t)g * kMergeGroup, -1,
+    merge_group<kEmitThreads, BATCH>(u, in_items + (size_t)g * kMergeGroup * kItemCap, in_counts + (size_t)g * kMergeGroup,
                          (uint32_t)kItemCap, min((uint32_t)kMergeGroup, n_in - g * kMergeGroup), heap,
                          out_items + (size_t)g * kItemCap, out_counts + g, err, inner, s_off, s_items, s_ipos);
     size_t ioff = 0, coff = 0, toff = 0;
@@ -1830,7 +1828,7 @@ __global__ void __launch_bounds__(THREADS) k_emit_merge(const uint2* __restrict_
         const size_t pcoff = coff + (size_t)parent * kMergeGroup;
         ioff += (size_t)n_lev * kItemCap;
         coff += n_lev;
-        merge_group<THREADS, BATCH>(u, out_items + pioff, out_counts + pcoff, -1, (uint32_t)kItemCap, gs, heap,
+        merge_group<kEmitThreads, BATCH>(u, out_items + pioff, out_counts + pcoff, (uint32_t)kItemCap, gs, heap,
                              out_items + ioff + (size_t)parent * kItemCap, out_counts + coff + parent, err, inner,
                              s_off, s_items, s_ipos);
         toff += n_next;
@@ -2078,8 +2076,8 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_build_small(const float* _
         *u.n_items = 0u;
     }
     if ((uint32_t)t < tiles) {  // the leaves as k_emit_units lists them, for the trace records
-        const uint32_t before = (uint32_t)t * kEmitTile;
-        counts[t] = U > before ? min(U - before, (uint32_t)kEmitTile) : 0u;
+        const uint32_t before = (uint32_t)t * kTreeTile;
+        counts[t] = U > before ? min(U - before, (uint32_t)kTreeTile) : 0u;
     }
     __syncthreads();
 
@@ -2253,8 +2251,9 @@ extern "C" rt_status rt_lbvh_create(rt_ctx* ctx, uint32_t max_tris, uint32_t dep
     l->cap = max_tris;
     l->depth = depth;
     l->num_nodes = 1u << depth;
-    l->sort_tiles_cap = ceil_div(max_tris, kSortTile);
-    l->emit_tiles_cap = ceil_div(max_tris, kEmitTile);
+    l->sort_tiles_cap = std::max({ceil_div(max_tris, kSortTile), ceil_div(std::min(max_tris, kSort4Keys), 4 * kSortThreads),
+                                  ceil_div(std::min(max_tris, kSort8Keys), 8 * kSortThreads)});
+    l->emit_tiles_cap = ceil_div(max_tris, kTreeTile);
     l->bounds_blocks = std::max(1u, std::min(ceil_div(3ull * max_tris, 256), (uint32_t)ctx->num_sms * 4));
     const size_t cap = max_tris;
     cudaError_t e = cudaSuccess;
@@ -2330,11 +2329,11 @@ static rt_status launch_build(rt_ctx* ctx, rt_lbvh* l, const float* d_tris, uint
     cudaStream_t st = ctx->stream;
     l->n = n;
     l->src_tris = d_tris;
-    const uint32_t emit_tiles = ceil_div(n, kEmitTile);
     // One block against the launches below: 300 triangles 21 and 58 us, 1,000: 29 and 69,
     // 2,048: 44 and 78, 4,096: 75 and 80; one block would need more shared memory beyond.
     // The flags ask for passes that only the launches below have.
     if (n <= kSmallTris && flags == 0u) {
+        const uint32_t emit_tiles = ceil_div(n, kTreeTile);
         auto small = [&](auto kernel, int items) -> rt_status {
             RT_CHECK_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small_smem(items)));
             launch_pdl(kernel, 1, kSmallThreads, small_smem(items), st, d_tris, n, l->depth, l->keys, l->ids, l->sorted_tris,
@@ -2352,7 +2351,9 @@ static rt_status launch_build(rt_ctx* ctx, rt_lbvh* l, const float* d_tris, uint
         l->rec_tiles = emit_tiles;
         return RT_OK;
     }
-    const uint32_t sort_tiles = ceil_div(n, kSortTile);
+    const uint32_t emit_tiles = ceil_div(n, kTreeTile);
+    const int sort_items = sort_items_of(n);
+    const uint32_t sort_tiles = ceil_div(n, kSortThreads * sort_items);
     const uint32_t lb_pass = 256 * (sort_tiles + look_groups(sort_tiles));  // tile words, group words
     const uint32_t lb_words = kSortPasses * lb_pass;
     const uint32_t bblocks = std::max(1u, std::min(ceil_div(3ull * n, 256), l->bounds_blocks));
@@ -2364,7 +2365,7 @@ static rt_status launch_build(rt_ctx* ctx, rt_lbvh* l, const float* d_tris, uint
     RT_CHECK_LAUNCH(ctx, "k_morton_hist");
     uint32_t *kin = l->keys, *iin = l->ids, *kout = l->keys_alt, *iout = l->ids_alt;
     for (int p = 0; p < kSortPasses; ++p) {
-        launch_pdl(k_onesweep<false, true>, sort_tiles, kSortThreads, 0, st, (const uint32_t*)kin, (const uint32_t*)iin,
+        launch_pdl(sort_items == 4 ? k_onesweep<false, true, 4> : sort_items == 8 ? k_onesweep<false, true, 8> : k_onesweep<false, true>, sort_tiles, kSortThreads, 0, st, (const uint32_t*)kin, (const uint32_t*)iin,
                    kout, iout, n, p, (const uint32_t*)l->hist, l->lookback + (size_t)p * lb_pass,
                    l->counters + 1 + p, ctx->d_err, (const uint32_t*)nullptr, 0u, kSpinLimit);
         RT_CHECK_LAUNCH(ctx, "k_onesweep");
@@ -2372,7 +2373,7 @@ static rt_status launch_build(rt_ctx* ctx, rt_lbvh* l, const float* d_tris, uint
         std::swap(iin, iout);
     }
     // four passes: sorted pairs are back in keys / ids
-    launch_pdl(k_emit_tiles, emit_tiles, kEmitThreads, 0, st, l->keys, n, l->scan, (uint32_t*)nullptr, 0u,
+    launch_pdl(k_emit_tiles<kTreeItems>, emit_tiles, kEmitThreads, 0, st, l->keys, n, l->scan, (uint32_t*)nullptr, 0u,
                (const uint32_t*)nullptr);
     RT_CHECK_LAUNCH(ctx, "k_emit_tiles");
     launch_pdl(k_emit_prefix, 1, kPrefixThreads, 0, st, l->scan, emit_tiles);
@@ -2382,27 +2383,24 @@ static rt_status launch_build(rt_ctx* ctx, rt_lbvh* l, const float* d_tris, uint
     if (compact) RT_CHECK_CUDA(ctx, cudaMemsetAsync(l->inner, 0, sizeof(uint32_t) * words, st));
     // emission, pre-gather, leaf boxes and every node inside a tile in one
     // pass; the nodes above the tiles by k_emit_merge, level after level
-    RT_CHECK_CUDA(ctx, cudaFuncSetAttribute(k_emit_merge<kEmitThreads, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    RT_CHECK_CUDA(ctx, cudaFuncSetAttribute(k_emit_merge<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             (int)kUnitSmem));
-    RT_CHECK_CUDA(ctx, cudaFuncSetAttribute(k_emit_units<kEmitThreads, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            (int)kEmitUnitsSmem));
     uint32_t* inner = compact ? l->inner : nullptr;
     // the sort's ping-pong buffers are free again: they hold the tiles' unit lists
     uint2* tile_units = reinterpret_cast<uint2*>(l->keys_alt);
     const size_t cap = l->emit_tiles_cap;
     uint32_t* tile_counts = l->item_counts + 6 * cap;
-    launch_pdl(k_emit_units<kEmitThreads, false>, emit_tiles, kEmitThreads, kEmitUnitsSmem, st, (const uint32_t*)l->keys,
+    launch_pdl(k_emit_units<false>, emit_tiles, kEmitThreads, 0, st, (const uint32_t*)l->keys,
                (const uint32_t*)l->ids, d_tris, n, l->depth, (const uint32_t*)l->scan, l->nodes, l->sorted_tris,
                tile_units, tile_counts, ctx->d_err, l->leaf_of, (const uint32_t*)nullptr, 0u, (uint32_t*)nullptr);
     RT_CHECK_LAUNCH(ctx, "k_emit_units");
-    const uint32_t chunks = emit_tiles * kTileChunks;
-    launch_pdl(k_emit_chunks<kEmitThreads, false>, chunks, kEmitThreads, kChunkSmem, st, (const uint2*)tile_units,
+    launch_pdl(k_emit_chunks<false>, emit_tiles, kEmitThreads, kChunkSmem, st, (const uint2*)tile_units,
                (const uint32_t*)tile_counts, l->depth, l->nodes, l->items, l->item_counts, ctx->d_err, inner,
                (const uint32_t*)nullptr);
     RT_CHECK_LAUNCH(ctx, "k_emit_chunks");
-    launch_pdl(k_emit_merge<kEmitThreads, false>, ceil_div(chunks, kMergeGroup), kEmitThreads, kUnitSmem, st,
-               (const uint2*)l->items, (const uint32_t*)l->item_counts, chunks, l->depth, l->nodes,
-               l->items + (size_t)chunks * kItemCap, l->item_counts + chunks, l->item_counts + 7 * cap, ctx->d_err,
+    launch_pdl(k_emit_merge<false>, ceil_div(emit_tiles, kMergeGroup), kEmitThreads, kUnitSmem, st,
+               (const uint2*)l->items, (const uint32_t*)l->item_counts, emit_tiles, l->depth, l->nodes,
+               l->items + (size_t)emit_tiles * kItemCap, l->item_counts + emit_tiles, l->item_counts + 7 * cap, ctx->d_err,
                inner, (const uint32_t*)nullptr);
     RT_CHECK_LAUNCH(ctx, "k_emit_merge");
     if (compact) {
@@ -2651,7 +2649,7 @@ extern "C" rt_status rt_lbvh_build_noalloc(rt_ctx* ctx, void* stream, const floa
         std::swap(kin, kout);
         std::swap(iin, iout);
     }
-    k_emit_tiles<<<emit_tiles, kEmitThreads, 0, st>>>(d_keys, n, scan, arrive, std::max(1u, num_nodes >> 1), counters + 6);
+    k_emit_tiles<kEmitItems><<<emit_tiles, kEmitThreads, 0, st>>>(d_keys, n, scan, arrive, std::max(1u, num_nodes >> 1), counters + 6);
     k_emit_prefix<<<1, kPrefixThreads, 0, st>>>(scan, emit_tiles);
     k_emit_leaves<<<emit_tiles, kEmitThreads, 0, st>>>(d_keys, d_ids, d_tris, n, depth, scan, d_nodes,
                                                        reinterpret_cast<float4*>(d_sorted_tris), leaves, counters + 5, err);
@@ -2920,14 +2918,14 @@ __global__ void __launch_bounds__(kEmitThreads) kb_emit_tiles(const uint32_t* __
     __shared__ uint32_t s_off[kMaxBatchScenes + 1];
     for (uint32_t q = threadIdx.x; q <= S; q += blockDim.x) s_off[q] = tri_off[q];
     __syncthreads();
-    const uint32_t s = blockIdx.x * kEmitTile + threadIdx.x * kEmitItems;
-    EmitChunk e;
+    const uint32_t s = (blockIdx.x * kEmitThreads + threadIdx.x) * kTreeItems;
+    EmitChunk<kTreeItems> e;
     load_chunk_b(keys, n, s, s_off, S, e);
     uint32_t af = 0, ab = 0;
 #pragma unroll
-    for (int q = 0; q < kEmitItems; ++q) af = rec_fwd(af, e.r[q]);
+    for (int q = 0; q < kTreeItems; ++q) af = rec_fwd(af, e.r[q]);
 #pragma unroll
-    for (int q = kEmitItems - 1; q >= 0; --q) ab = rec_bwd(e.r[q], ab);
+    for (int q = kTreeItems - 1; q >= 0; --q) ab = rec_bwd(e.r[q], ab);
     af = warp_reduce_ordered<true>(af);
     ab = warp_reduce_ordered<false>(ab);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -2997,7 +2995,7 @@ extern "C" rt_status rt_batch_create(rt_ctx* ctx, uint32_t n_scenes, const uint3
     b->nchunks = (uint32_t)(chunks.size() / 3);
     const size_t n = total;
     const size_t num_nodes = (size_t)n_scenes << depth;
-    const uint32_t sort_tiles = ceil_div(n, kSortTile), emit_tiles = ceil_div(n, kEmitTile);
+    const uint32_t sort_tiles = ceil_div(n, kSortTile), emit_tiles = ceil_div(n, kTreeTile);
     cudaError_t e = cudaSuccess;
     auto alloc = [&](void** p, size_t bytes) {
         if (e == cudaSuccess) e = cudaMalloc(p, bytes);
@@ -3051,7 +3049,7 @@ extern "C" rt_status rt_batch_build(rt_ctx* ctx, rt_batch* b, const float* d_tri
     if (!b || !d_tris) return rt_fail(ctx, RT_ERR_INVALID, "rt_batch_build: null argument");
     cudaStream_t st = ctx->stream;
     const uint32_t n = b->total, S = b->S;
-    const uint32_t sort_tiles = ceil_div(n, kSortTile), emit_tiles = ceil_div(n, kEmitTile);
+    const uint32_t sort_tiles = ceil_div(n, kSortTile), emit_tiles = ceil_div(n, kTreeTile);
     const uint32_t lb_words = 5 * 256 * sort_tiles;
     const uint32_t num_nodes = S << b->depth;
     kb_init<<<std::max(1u, std::min(ceil_div(std::max(lb_words, num_nodes), 256), (uint32_t)ctx->num_sms * 8)), 256, 0,
@@ -3084,24 +3082,21 @@ extern "C" rt_status rt_batch_build(rt_ctx* ctx, rt_batch* b, const float* d_tri
     // the emission of a single tree over the concatenated scenes (256 random-soup
     // scenes, 11.5 M triangles: 1.4 ms; leaf boxes and an atomic walk with one
     // dependent global exchange per node and level took 2.3 ms)
-    RT_CHECK_CUDA(ctx, cudaFuncSetAttribute(k_emit_merge<kEmitThreads, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    RT_CHECK_CUDA(ctx, cudaFuncSetAttribute(k_emit_merge<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             (int)kUnitSmem));
-    RT_CHECK_CUDA(ctx, cudaFuncSetAttribute(k_emit_units<kEmitThreads, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            (int)kEmitUnitsSmem));
     uint2* tile_units = reinterpret_cast<uint2*>(b->keys);
     uint32_t* tile_counts = b->item_counts + 6 * (size_t)emit_tiles;
-    launch_pdl(k_emit_units<kEmitThreads, true>, emit_tiles, kEmitThreads, kEmitUnitsSmem, st, (const uint32_t*)kin,
+    launch_pdl(k_emit_units<true>, emit_tiles, kEmitThreads, 0, st, (const uint32_t*)kin,
                (const uint32_t*)iin, d_tris, n, b->depth, (const uint32_t*)b->scan, b->nodes, b->sorted_tris, tile_units,
                tile_counts, ctx->d_err, b->leaf_of, (const uint32_t*)b->tri_off, S, b->ids_local);
     RT_CHECK_LAUNCH(ctx, "k_emit_units");
-    const uint32_t chunks = emit_tiles * kTileChunks;
-    launch_pdl(k_emit_chunks<kEmitThreads, true>, chunks, kEmitThreads, kChunkSmem, st, (const uint2*)tile_units,
+    launch_pdl(k_emit_chunks<true>, emit_tiles, kEmitThreads, kChunkSmem, st, (const uint2*)tile_units,
                (const uint32_t*)tile_counts, b->depth, b->nodes, b->items, b->item_counts, ctx->d_err, (uint32_t*)nullptr,
                (const uint32_t*)b->tri_off);
     RT_CHECK_LAUNCH(ctx, "k_emit_chunks");
-    launch_pdl(k_emit_merge<kEmitThreads, true>, ceil_div(chunks, kMergeGroup), kEmitThreads, kUnitSmem, st,
-               (const uint2*)b->items, (const uint32_t*)b->item_counts, chunks, b->depth, b->nodes,
-               b->items + (size_t)chunks * kItemCap, b->item_counts + chunks, b->item_counts + 7 * (size_t)emit_tiles,
+    launch_pdl(k_emit_merge<true>, ceil_div(emit_tiles, kMergeGroup), kEmitThreads, kUnitSmem, st,
+               (const uint2*)b->items, (const uint32_t*)b->item_counts, emit_tiles, b->depth, b->nodes,
+               b->items + (size_t)emit_tiles * kItemCap, b->item_counts + emit_tiles, b->item_counts + 7 * (size_t)emit_tiles,
                ctx->d_err, (uint32_t*)nullptr, (const uint32_t*)b->tri_off);
     RT_CHECK_LAUNCH(ctx, "k_emit_merge");
     b->src_tris = d_tris;

@@ -111,7 +111,9 @@ constexpr int kSortTile = kSortThreads * kSortItems;  // 4096 keys per onesweep 
 constexpr int kSortPasses = 4;                        // 8-bit digits over 30-bit codes
 constexpr int kEmitThreads = 256;
 constexpr int kEmitItems = 8;
-constexpr int kEmitTile = kEmitThreads * kEmitItems;  // 2048 elements per emission tile
+constexpr int kEmitTile = kEmitThreads * kEmitItems;  // 2048 elements per tile of the allocation-free emission
+constexpr int kTreeItems = 2;
+constexpr int kTreeTile = kEmitThreads * kTreeItems;  // 512 elements per emission tile
 constexpr int kMaxDepth = 26;
 constexpr uint32_t kMaxTris = (1u << 29);
 

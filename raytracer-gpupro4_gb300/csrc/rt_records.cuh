@@ -70,7 +70,7 @@ __device__ __forceinline__ void trace_node_of(uint32_t h, const rt_node* nodes, 
 // What make_records needs of a tree (tiles = 0: no records).
 struct Records {
     const uint32_t* valid;
-    const uint2* units;      // the emission's leaves, kEmitTile slots per tile
+    const uint2* units;      // the emission's leaves, kTreeTile slots per tile
     const uint32_t* counts;  // leaves of each tile
     uint32_t tiles;          // tiles that have blocks of their own
     const uint32_t* built;   // tiles of the tree when the kernel runs (nullptr: `tiles`): a captured call may be
@@ -82,9 +82,9 @@ struct Records {
     uint32_t scene_depth;    // a batch's heap depth (a leaf is named by scene << 23 | heap slot); 0: one tree
 };
 
-// Few tiles are shared by up to eight blocks each, about two blocks per SM.
+// Few tiles are shared by two blocks each, about two blocks per SM.
 inline uint32_t record_slices(uint32_t tiles, int num_sms) {
-    return std::max(1u, std::min(8u, 2u * (uint32_t)num_sms / std::max(1u, tiles)));
+    return std::max(1u, std::min(2u, 2u * (uint32_t)num_sms / std::max(1u, tiles)));
 }
 inline Records records_of(const rt_ctx* ctx, const rt_lbvh* l) {
     const uint32_t tiles = std::max(1u, l->rec_tiles);
@@ -93,7 +93,7 @@ inline Records records_of(const rt_ctx* ctx, const rt_lbvh* l) {
                    l->num_nodes, l->tnodes, l->rec_tiles ? record_slices(tiles, ctx->num_sms) : 1u, 0u};
 }
 inline Records records_of(const rt_ctx* ctx, const rt_batch* b) {
-    const uint32_t tiles = (b->total + kEmitTile - 1) / kEmitTile;
+    const uint32_t tiles = (b->total + kTreeTile - 1) / kTreeTile;
     return Records{b->counters + 7, reinterpret_cast<const uint2*>(b->keys), b->item_counts + 6 * (size_t)tiles,
                    b->tnodes ? tiles : 0u, nullptr, b->nodes, 1u << b->depth, b->tnodes,
                    record_slices(tiles, ctx->num_sms), b->depth};
@@ -107,15 +107,15 @@ __device__ __forceinline__ void make_records(const Records& R, uint32_t block) {
     const bool batch = R.scene_depth != 0u;
     const uint32_t tiles = R.built ? *R.built : R.tiles;
     for (uint32_t tile = block / R.slices; tile < tiles; tile += R.tiles) {
-        const uint32_t cnt = min(__ldg(R.counts + tile), (uint32_t)kEmitTile);
+        const uint32_t cnt = min(__ldg(R.counts + tile), (uint32_t)kTreeTile);
         for (uint32_t i = (block % R.slices) * blockDim.x + threadIdx.x; i < cnt; i += R.slices * blockDim.x) {
-            uint32_t b = __ldg(&R.units[(size_t)tile * kEmitTile + i].x), a = 0u;
+            uint32_t b = __ldg(&R.units[(size_t)tile * kTreeTile + i].x), a = 0u;
             if (i) {
-                a = __ldg(&R.units[(size_t)tile * kEmitTile + i - 1].x);
+                a = __ldg(&R.units[(size_t)tile * kTreeTile + i - 1].x);
             } else {  // the last leaf of the tiles before
                 for (uint32_t q = tile; q-- > 0u && a == 0u;) {
-                    const uint32_t c = min(__ldg(R.counts + q), (uint32_t)kEmitTile);
-                    if (c) a = __ldg(&R.units[(size_t)q * kEmitTile + c - 1].x);
+                    const uint32_t c = min(__ldg(R.counts + q), (uint32_t)kTreeTile);
+                    if (c) a = __ldg(&R.units[(size_t)q * kTreeTile + c - 1].x);
                 }
             }
             const rt_node* nodes = R.nodes;

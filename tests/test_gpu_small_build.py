@@ -52,3 +52,22 @@ def test_handle_shared_with_the_general_build(gpu_ctx, oracle_mod):
     lb = LBVH(gpu_ctx, 9000, 15)
     for n in (9000, 700, 5000, 4096, 3):
         check(gpu_ctx, oracle_mod, lb, scenes.random_soup(n, n + 1), 15)
+
+
+@pytest.mark.parametrize("n,depth", [(4608, 20), (4609, 4), (155648, 20), (155649, 12), (1245184, 22), (1245185, 22)])
+def test_tiles_of_the_general_build(gpu_ctx, oracle_mod, n, depth):
+    """Around a whole emission tile and around the sizes where the sort changes
+    its tile; the handle is larger than the soup."""
+    from rtgpu import scenes
+    from rtgpu.api import LBVH
+    check(gpu_ctx, oracle_mod, LBVH(gpu_ctx, n + 300000, depth), scenes.random_soup(n, n, 0.001, 0.02), depth)
+
+
+def test_long_leaves_across_tiles(gpu_ctx, oracle_mod):
+    """Equal codes over several emission tiles, a leaf that ends at a tile's end and
+    tiles inside one leaf."""
+    from rtgpu import scenes
+    from rtgpu.api import LBVH
+    runs = (300, 212, 2048, 1, 3000, 511, 1, 600)
+    tris = np.repeat(scenes.random_soup(len(runs), 4, 0.05, 0.2), runs, 0)
+    check(gpu_ctx, oracle_mod, LBVH(gpu_ctx, len(tris), 14), np.ascontiguousarray(tris), 14)
