@@ -15,7 +15,7 @@
 //                   shared-memory staged scatter.  Result = qsort(cmpMorton)
 //                   order (LBVH.cpp:21-38).
 //   k_emit_tiles    per-tile aggregates of the boundary "record masks"
-//   k_emit_prefix   tile prefixes (one block)
+//   k_emit_prefix   tile prefixes, 1,024 tiles a block
 //   k_emit_units    per tile: each leaf's heap index and range, the triangle
 //                   pre-gather in sorted order, the leaf records (boxes by a
 //                   segmented scan) and the tile's leaves as ordered units
@@ -344,7 +344,7 @@ __device__ __forceinline__ uint32_t sort_digit(uint32_t key, uint32_t id, int sh
     return SCENE ? scene_of(s_off, S, id) : ((key >> shift) & 0xffu);
 }
 
-// Grouped look-back (GROUPED = true, the single-scene build): the tiles form
+// Grouped look-back (GROUPED = true, a tree and a batch): the tiles form
 // groups of kLookGroup consecutive tickets.  A tile publishes its digit
 // counts, sums those of the earlier tiles of its group (one round of
 // parallel loads), and the group's last tile publishes the group's
@@ -682,8 +682,36 @@ __device__ __forceinline__ void load_chunk_b(const uint32_t* __restrict__ keys, 
     }
 }
 
-// k_emit_tiles: per-tile fwd/bwd aggregates of the boundary record masks.
-template <int ITEMS>
+// Aggregates of the tiles of a block's kEmitTile elements from the threads' own.
+template <int TILE>
+__device__ __forceinline__ void store_tile_records(const EmitChunk<>& e, uint32_t tiles, uint32_t* scan) {
+    constexpr int kWarps = TILE / (32 * kEmitItems);  // warps of a tile
+    __shared__ uint32_t s_f[kEmitThreads / 32], s_b[kEmitThreads / 32];
+    uint32_t af = 0, ab = 0;
+#pragma unroll
+    for (int q = 0; q < kEmitItems; ++q) af = rec_fwd(af, e.r[q]);
+#pragma unroll
+    for (int q = kEmitItems - 1; q >= 0; --q) ab = rec_bwd(e.r[q], ab);
+    af = warp_reduce_ordered<true>(af);
+    ab = warp_reduce_ordered<false>(ab);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (lane == 0) { s_f[w] = af; s_b[w] = ab; }
+    __syncthreads();
+    const uint32_t tile = blockIdx.x * (kEmitTile / TILE) + threadIdx.x;
+    if (threadIdx.x < kEmitTile / TILE && tile < tiles) {
+        const int w0 = threadIdx.x * kWarps;
+        uint32_t tf = 0, tb = 0;
+        for (int q = 0; q < kWarps; ++q) tf = rec_fwd(tf, s_f[w0 + q]);
+        for (int q = kWarps - 1; q >= 0; --q) tb = rec_bwd(s_b[w0 + q], tb);
+        scan[4 * tile + 0] = tf;
+        scan[4 * tile + 1] = tb;
+    }
+}
+
+// k_emit_tiles: per-tile fwd/bwd aggregates of the boundary record masks,
+// kEmitTile elements a block whatever the tile (a block per tile of 512 took 60 us
+// for a batch of 11.5 M triangles).
+template <int TILE>
 __global__ void __launch_bounds__(kEmitThreads) k_emit_tiles(const uint32_t* __restrict__ keys, uint32_t n,
                                                              uint32_t* scan, uint32_t* arrive, uint32_t arrive_words,
                                                              const uint32_t* epoch_word) {
@@ -694,71 +722,34 @@ __global__ void __launch_bounds__(kEmitThreads) k_emit_tiles(const uint32_t* __r
     if (arrive_words && *epoch_word == 1u)
         for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < arrive_words; i += gridDim.x * blockDim.x)
             arrive[i] = 0u;
-    __shared__ uint32_t s_f[8], s_b[8];
-    const uint32_t s = (blockIdx.x * kEmitThreads + threadIdx.x) * ITEMS;
-    EmitChunk<ITEMS> e;
-    load_chunk(keys, n, s, e);
-    uint32_t af = 0, ab = 0;
-#pragma unroll
-    for (int q = 0; q < ITEMS; ++q) af = rec_fwd(af, e.r[q]);
-#pragma unroll
-    for (int q = ITEMS - 1; q >= 0; --q) ab = rec_bwd(e.r[q], ab);
-    af = warp_reduce_ordered<true>(af);
-    ab = warp_reduce_ordered<false>(ab);
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if (lane == 0) { s_f[w] = af; s_b[w] = ab; }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t tf = 0, tb = 0;
-        for (int q = 0; q < kEmitThreads / 32; ++q) tf = rec_fwd(tf, s_f[q]);
-        for (int q = kEmitThreads / 32 - 1; q >= 0; --q) tb = rec_bwd(s_b[q], tb);
-        scan[4 * blockIdx.x + 0] = tf;
-        scan[4 * blockIdx.x + 1] = tb;
-    }
+    EmitChunk<> e;
+    load_chunk(keys, n, blockIdx.x * kEmitTile + threadIdx.x * kEmitItems, e);
+    store_tile_records<TILE>(e, (n + TILE - 1) / TILE, scan);
 }
 
-// k_emit_prefix: exclusive fwd prefix / bwd suffix over the tiles (one block
-// of 1024 threads, each over a contiguous run of tiles).
-constexpr int kPrefixThreads = 1024;
+// k_emit_prefix: exclusive fwd prefix / bwd suffix over the tiles of each group of
+// kPrefixTiles, a block a group, a thread a tile; with several groups their totals
+// follow the tiles' words and k_emit_units combines them (one block over all tiles
+// took 10 us for 2.1 M triangles and 52 us for a batch of 11.5 M).
+constexpr int kPrefixTiles = 1024;
+__host__ __device__ constexpr uint32_t prefix_groups(uint32_t tiles) { return (tiles + kPrefixTiles - 1) / kPrefixTiles; }
+__host__ __device__ constexpr size_t scan_words(uint32_t tiles) { return 4 * (size_t)tiles + 2 * (size_t)prefix_groups(tiles); }
 
-__global__ void __launch_bounds__(kPrefixThreads) k_emit_prefix(uint32_t* scan, uint32_t tiles) {
+__global__ void __launch_bounds__(kPrefixTiles) k_emit_prefix(uint32_t* scan, uint32_t tiles) {
     grid_dep_wait();
-    __shared__ uint32_t s_f[kPrefixThreads / 32], s_b[kPrefixThreads / 32];
-    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-    const uint32_t per = (tiles + kPrefixThreads - 1) / kPrefixThreads;
-    const uint32_t lo = min(tiles, (uint32_t)t * per), hi = min(tiles, lo + per);
-    uint32_t af = 0, ab = 0;
-    for (uint32_t q = lo; q < hi; ++q) af = rec_fwd(af, scan[4 * q + 0]);
-    for (uint32_t q = hi; q > lo; --q) ab = rec_bwd(scan[4 * (q - 1) + 1], ab);
-    uint32_t xf = af, xb = ab;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        const uint32_t y = __shfl_up_sync(kFull, xf, off);
-        if (lane >= off) xf = rec_fwd(y, xf);
-        const uint32_t z = __shfl_down_sync(kFull, xb, off);
-        if (lane + off < 32) xb = rec_bwd(xb, z);
+    __shared__ uint32_t s_f[kPrefixTiles / 32], s_b[kPrefixTiles / 32];
+    const uint32_t tile = blockIdx.x * kPrefixTiles + threadIdx.x;
+    const uint32_t af = tile < tiles ? scan[4 * (size_t)tile + 0] : 0u, ab = tile < tiles ? scan[4 * (size_t)tile + 1] : 0u;
+    uint32_t pre, suf;
+    block_scan_records<kPrefixTiles>(af, ab, &pre, &suf, s_f, s_b);
+    if (tile < tiles) {
+        scan[4 * (size_t)tile + 2] = pre;
+        scan[4 * (size_t)tile + 3] = suf;
     }
-    if (lane == 31) s_f[w] = xf;  // inclusive fwd total of the warp
-    if (lane == 0) s_b[w] = xb;   // inclusive bwd total of the warp
-    __syncthreads();
-    uint32_t wf = 0, wb = 0;
-    for (int q = 0; q < w; ++q) wf = rec_fwd(wf, s_f[q]);
-    for (int q = kPrefixThreads / 32 - 1; q > w; --q) wb = rec_bwd(s_b[q], wb);
-    uint32_t ef = __shfl_up_sync(kFull, xf, 1);
-    if (lane == 0) ef = 0;
-    uint32_t eb = __shfl_down_sync(kFull, xb, 1);
-    if (lane == 31) eb = 0;
-    uint32_t run = rec_fwd(wf, ef);
-    for (uint32_t q = lo; q < hi; ++q) {
-        const uint32_t a = scan[4 * q + 0];
-        scan[4 * q + 2] = run;
-        run = rec_fwd(run, a);
-    }
-    run = rec_bwd(eb, wb);
-    for (uint32_t q = hi; q > lo; --q) {
-        const uint32_t a = scan[4 * (q - 1) + 1];
-        scan[4 * (q - 1) + 3] = run;
-        run = rec_bwd(a, run);
+    if (gridDim.x > 1) {
+        uint32_t* total = scan + 4 * (size_t)tiles + 2 * blockIdx.x;
+        if (threadIdx.x == kPrefixTiles - 1) total[0] = rec_fwd(pre, af);
+        if (threadIdx.x == 0) total[1] = rec_bwd(ab, suf);
     }
 }
 
@@ -1450,8 +1441,18 @@ __global__ void __launch_bounds__(kEmitThreads) k_emit_units(const uint32_t* __r
     uint32_t pre, suf;
     block_scan_records<THREADS>(af, ab, &pre, &suf, s_f, s_b);  // includes __syncthreads
     uint32_t L[ITEMS + 1], R[ITEMS + 1];
-    L[0] = rec_fwd(scan[4 * blockIdx.x + 2], pre);
-    R[ITEMS] = rec_bwd(suf, scan[4 * blockIdx.x + 3]);
+    uint32_t tpre = scan[4 * (size_t)blockIdx.x + 2], tsuf = scan[4 * (size_t)blockIdx.x + 3];
+    {  // the other groups of tiles
+        const uint32_t* total = scan + 4 * (size_t)gridDim.x;
+        const uint32_t G = prefix_groups(gridDim.x), my = blockIdx.x / kPrefixTiles;
+        uint32_t gf = 0u, gb = 0u;
+        for (uint32_t g = 0; g < my; ++g) gf = rec_fwd(gf, __ldg(total + 2 * g));
+        for (uint32_t g = G - 1; g > my; --g) gb = rec_bwd(__ldg(total + 2 * g + 1), gb);
+        tpre = rec_fwd(gf, tpre);
+        tsuf = rec_bwd(tsuf, gb);
+    }
+    L[0] = rec_fwd(tpre, pre);
+    R[ITEMS] = rec_bwd(suf, tsuf);
 #pragma unroll
     for (int q = 0; q < ITEMS; ++q) L[q + 1] = rec_fwd(L[q], e.r[q]);
 #pragma unroll
@@ -2280,7 +2281,7 @@ extern "C" rt_status rt_lbvh_create(rt_ctx* ctx, uint32_t max_tris, uint32_t dep
     // per radix pass: 256 look-back words per tile, then 256 per tile group
     alloc((void**)&l->lookback,
           sizeof(uint32_t) * kSortPasses * 256 * ((size_t)l->sort_tiles_cap + look_groups(l->sort_tiles_cap)));
-    alloc((void**)&l->scan, sizeof(uint32_t) * 4 * (size_t)l->emit_tiles_cap);
+    alloc((void**)&l->scan, sizeof(uint32_t) * scan_words(l->emit_tiles_cap));
     alloc((void**)&l->leaf_of, 4 * cap);
     // items and item counts of every merge level (chunk slots = 4 x tiles, then
     // the groups above: < 6 x tiles in all), the tiles' unit counts (tiles),
@@ -2373,10 +2374,10 @@ static rt_status launch_build(rt_ctx* ctx, rt_lbvh* l, const float* d_tris, uint
         std::swap(iin, iout);
     }
     // four passes: sorted pairs are back in keys / ids
-    launch_pdl(k_emit_tiles<kTreeItems>, emit_tiles, kEmitThreads, 0, st, l->keys, n, l->scan, (uint32_t*)nullptr, 0u,
+    launch_pdl(k_emit_tiles<kTreeTile>, ceil_div(n, kEmitTile), kEmitThreads, 0, st, l->keys, n, l->scan, (uint32_t*)nullptr, 0u,
                (const uint32_t*)nullptr);
     RT_CHECK_LAUNCH(ctx, "k_emit_tiles");
-    launch_pdl(k_emit_prefix, 1, kPrefixThreads, 0, st, l->scan, emit_tiles);
+    launch_pdl(k_emit_prefix, prefix_groups(emit_tiles), kPrefixTiles, 0, st, l->scan, emit_tiles);
     RT_CHECK_LAUNCH(ctx, "k_emit_prefix");
     const bool compact = (flags & RT_BUILD_COMPACT) != 0;
     const uint32_t words = std::max(1u, l->num_nodes / 32);
@@ -2539,6 +2540,7 @@ constexpr size_t kNaIdsAlt = kNaKeysAlt + RT_NOALLOC_MAX_TRIS;
 constexpr size_t kNaArrive = kNaIdsAlt + RT_NOALLOC_MAX_TRIS;                       // 1 << (depth - 1)
 constexpr size_t kNaErr = kNaArrive + ((size_t)1 << (RT_NOALLOC_MAX_DEPTH - 1));   // error word (ctx == NULL)
 constexpr size_t kNaWords = kNaErr + 64;
+static_assert(prefix_groups(kNoAllocEmitTiles) == 1, "k_emit_leaves reads one group's prefixes");
 static_assert(kNaWords * sizeof(uint32_t) == 5577088, "the documented size of the fixed scratch");
 
 static __device__ __align__(256) uint32_t g_noalloc_scratch[kNaWords];
@@ -2649,8 +2651,8 @@ extern "C" rt_status rt_lbvh_build_noalloc(rt_ctx* ctx, void* stream, const floa
         std::swap(kin, kout);
         std::swap(iin, iout);
     }
-    k_emit_tiles<kEmitItems><<<emit_tiles, kEmitThreads, 0, st>>>(d_keys, n, scan, arrive, std::max(1u, num_nodes >> 1), counters + 6);
-    k_emit_prefix<<<1, kPrefixThreads, 0, st>>>(scan, emit_tiles);
+    k_emit_tiles<kEmitTile><<<emit_tiles, kEmitThreads, 0, st>>>(d_keys, n, scan, arrive, std::max(1u, num_nodes >> 1), counters + 6);
+    k_emit_prefix<<<prefix_groups(emit_tiles), kPrefixTiles, 0, st>>>(scan, emit_tiles);
     k_emit_leaves<<<emit_tiles, kEmitThreads, 0, st>>>(d_keys, d_ids, d_tris, n, depth, scan, d_nodes,
                                                        reinterpret_cast<float4*>(d_sorted_tris), leaves, counters + 5, err);
     const uint32_t rblocks = std::max(1u, std::min(ceil_div(n, 256), (uint32_t)D.num_sms * 8));
@@ -2775,7 +2777,7 @@ extern "C" rt_status rt_radix_sort_stall_test(rt_ctx* ctx, const uint32_t* d_key
 // [tri_off[s], tri_off[s+1]); its tree is the single-scene tree of those
 // triangles, stored in its own heap of 1 << depth slots at s << depth, with
 // PrimPos and the ordered ids local to the scene.
-//   kb_init          per-scene bounds reset, scratch reset, epoch
+//   kb_init          per-scene bounds reset, scratch reset
 //   kb_bounds        per-scene bounds over host-made one-scene chunks
 //   kb_morton_hist   codes with each scene's own Morton parameters
 //   k_onesweep x4+1  four code passes, then a stable pass on the scene
@@ -2803,6 +2805,7 @@ __device__ __forceinline__ void atomic_max_f(float* a, float v) {
 __global__ void kb_init(float* sbounds, uint32_t S, const uint32_t* __restrict__ tri_off, uint32_t* counters,
                         uint32_t* hist, uint32_t* lookback, uint32_t lb_words, rt_node* nodes, uint32_t num_nodes,
                         int clear_nodes) {
+    grid_dep_wait();
     const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x, gs = gridDim.x * blockDim.x;
     for (uint32_t i = gtid; i < 8 * S; i += gs) {
         const uint32_t c = i & 7u;
@@ -2814,10 +2817,6 @@ __global__ void kb_init(float* sbounds, uint32_t S, const uint32_t* __restrict__
     }
     for (uint32_t i = gtid; i < lb_words; i += gs) lookback[i] = 0u;
     if (gtid < 6 || gtid == 7) counters[gtid] = 0u;  // [7]: whether the trace records are those of these trees
-    if (gtid == 6) {
-        const uint32_t e = counters[6] + 1u;
-        counters[6] = e ? e : 1u;
-    }
     if (clear_nodes)
         for (uint32_t i = gtid; i < num_nodes; i += gs) {
             rt_node s;
@@ -2831,6 +2830,7 @@ __global__ void kb_init(float* sbounds, uint32_t S, const uint32_t* __restrict__
 
 __global__ void __launch_bounds__(256) kb_bounds(const float* __restrict__ tris, const uint32_t* __restrict__ chunks,
                                                  float* sbounds, uint32_t* err) {
+    grid_dep_wait();
     const uint32_t s = chunks[3 * blockIdx.x], beg = chunks[3 * blockIdx.x + 1], end = chunks[3 * blockIdx.x + 2];
     float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
     uint32_t bad = 0;
@@ -2872,6 +2872,7 @@ __global__ void __launch_bounds__(256) kb_bounds(const float* __restrict__ tris,
 __global__ void __launch_bounds__(256) kb_morton_hist(const float* __restrict__ tris, const uint32_t* __restrict__ chunks,
                                                       const float* __restrict__ sbounds, uint32_t* __restrict__ keys,
                                                       uint32_t* __restrict__ ids, uint32_t* hist) {
+    grid_dep_wait();
     __shared__ uint32_t s_hist[4][256];
     __shared__ float s_par[6];
     for (int i = threadIdx.x; i < 4 * 256; i += blockDim.x) (&s_hist[0][0])[i] = 0u;
@@ -2914,30 +2915,13 @@ __global__ void __launch_bounds__(256) kb_morton_hist(const float* __restrict__ 
 __global__ void __launch_bounds__(kEmitThreads) kb_emit_tiles(const uint32_t* __restrict__ keys, uint32_t n,
                                                               const uint32_t* __restrict__ tri_off, uint32_t S,
                                                               uint32_t* scan) {
-    __shared__ uint32_t s_f[8], s_b[8];
+    grid_dep_wait();
     __shared__ uint32_t s_off[kMaxBatchScenes + 1];
     for (uint32_t q = threadIdx.x; q <= S; q += blockDim.x) s_off[q] = tri_off[q];
     __syncthreads();
-    const uint32_t s = (blockIdx.x * kEmitThreads + threadIdx.x) * kTreeItems;
-    EmitChunk<kTreeItems> e;
-    load_chunk_b(keys, n, s, s_off, S, e);
-    uint32_t af = 0, ab = 0;
-#pragma unroll
-    for (int q = 0; q < kTreeItems; ++q) af = rec_fwd(af, e.r[q]);
-#pragma unroll
-    for (int q = kTreeItems - 1; q >= 0; --q) ab = rec_bwd(e.r[q], ab);
-    af = warp_reduce_ordered<true>(af);
-    ab = warp_reduce_ordered<false>(ab);
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if (lane == 0) { s_f[w] = af; s_b[w] = ab; }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t tf = 0, tb = 0;
-        for (int q = 0; q < kEmitThreads / 32; ++q) tf = rec_fwd(tf, s_f[q]);
-        for (int q = kEmitThreads / 32 - 1; q >= 0; --q) tb = rec_bwd(s_b[q], tb);
-        scan[4 * blockIdx.x + 0] = tf;
-        scan[4 * blockIdx.x + 1] = tb;
-    }
+    EmitChunk<> e;
+    load_chunk_b(keys, n, blockIdx.x * kEmitTile + threadIdx.x * kEmitItems, s_off, S, e);
+    store_tile_records<kTreeTile>(e, (n + kTreeTile - 1) / kTreeTile, scan);
 }
 
 }  // namespace
@@ -2995,7 +2979,7 @@ extern "C" rt_status rt_batch_create(rt_ctx* ctx, uint32_t n_scenes, const uint3
     b->nchunks = (uint32_t)(chunks.size() / 3);
     const size_t n = total;
     const size_t num_nodes = (size_t)n_scenes << depth;
-    const uint32_t sort_tiles = ceil_div(n, kSortTile), emit_tiles = ceil_div(n, kTreeTile);
+    const uint32_t sort_tiles = ceil_div(n, kSortThreads * sort_items_of((uint32_t)n)), emit_tiles = ceil_div(n, kTreeTile);
     cudaError_t e = cudaSuccess;
     auto alloc = [&](void** p, size_t bytes) {
         if (e == cudaSuccess) e = cudaMalloc(p, bytes);
@@ -3014,8 +2998,8 @@ extern "C" rt_status rt_batch_create(rt_ctx* ctx, uint32_t n_scenes, const uint3
     alloc((void**)&b->sbounds, sizeof(float) * 8 * n_scenes);
     alloc((void**)&b->counters, sizeof(uint32_t) * 8);
     alloc((void**)&b->hist, sizeof(uint32_t) * 5 * 256);
-    alloc((void**)&b->lookback, sizeof(uint32_t) * 5 * 256 * (size_t)sort_tiles);
-    alloc((void**)&b->scan, sizeof(uint32_t) * 4 * (size_t)emit_tiles);
+    alloc((void**)&b->lookback, sizeof(uint32_t) * 5 * 256 * ((size_t)sort_tiles + look_groups(sort_tiles)));
+    alloc((void**)&b->scan, sizeof(uint32_t) * scan_words(emit_tiles));
     alloc((void**)&b->leaf_of, 4 * n);
     // items and counts of the merge levels, as a single tree's (rt_lbvh_create)
     alloc((void**)&b->items, sizeof(uint2) * 6 * (size_t)kItemCap * emit_tiles);
@@ -3049,35 +3033,38 @@ extern "C" rt_status rt_batch_build(rt_ctx* ctx, rt_batch* b, const float* d_tri
     if (!b || !d_tris) return rt_fail(ctx, RT_ERR_INVALID, "rt_batch_build: null argument");
     cudaStream_t st = ctx->stream;
     const uint32_t n = b->total, S = b->S;
-    const uint32_t sort_tiles = ceil_div(n, kSortTile), emit_tiles = ceil_div(n, kTreeTile);
-    const uint32_t lb_words = 5 * 256 * sort_tiles;
+    const int sort_items = sort_items_of(n);
+    const uint32_t sort_tiles = ceil_div(n, kSortThreads * sort_items), emit_tiles = ceil_div(n, kTreeTile);
+    const uint32_t lb_pass = 256 * (sort_tiles + look_groups(sort_tiles)), lb_words = 5 * lb_pass;
     const uint32_t num_nodes = S << b->depth;
-    kb_init<<<std::max(1u, std::min(ceil_div(std::max(lb_words, num_nodes), 256), (uint32_t)ctx->num_sms * 8)), 256, 0,
-              st>>>(b->sbounds, S, b->tri_off, b->counters, b->hist, b->lookback, lb_words, b->nodes, num_nodes,
-                    (flags & RT_BUILD_CLEAR_UNREACHED) ? 1 : 0);
+    const int clear = (flags & RT_BUILD_CLEAR_UNREACHED) ? 1 : 0;
+    launch_pdl(kb_init, std::max(1u, std::min(ceil_div(std::max(lb_words, clear ? num_nodes : 0u), 256), (uint32_t)ctx->num_sms * 8)),
+               256, 0, st, b->sbounds, S, b->tri_off, b->counters, b->hist, b->lookback, lb_words, b->nodes, num_nodes, clear);
     RT_CHECK_LAUNCH(ctx, "kb_init");
-    kb_bounds<<<b->nchunks, 256, 0, st>>>(d_tris, b->chunks, b->sbounds, ctx->d_err);
+    launch_pdl(kb_bounds, b->nchunks, 256, 0, st, d_tris, b->chunks, b->sbounds, ctx->d_err);
     RT_CHECK_LAUNCH(ctx, "kb_bounds");
-    kb_morton_hist<<<b->nchunks, 256, 0, st>>>(d_tris, b->chunks, b->sbounds, b->keys, b->ids, b->hist);
+    launch_pdl(kb_morton_hist, b->nchunks, 256, 0, st, d_tris, b->chunks, b->sbounds, b->keys, b->ids, b->hist);
     RT_CHECK_LAUNCH(ctx, "kb_morton_hist");
     uint32_t *kin = b->keys, *iin = b->ids, *kout = b->keys_alt, *iout = b->ids_alt;
     for (int p = 0; p < 5; ++p) {
-        uint32_t* lbp = b->lookback + (size_t)p * 256 * sort_tiles;
-        if (p < 4)
-            k_onesweep<false><<<sort_tiles, kSortThreads, 0, st>>>(kin, iin, kout, iout, n, p, b->hist, lbp,
-                                                                   b->counters + p, ctx->d_err);
-        else
-            k_onesweep<true><<<sort_tiles, kSortThreads, 0, st>>>(kin, iin, kout, iout, n, p, b->hist, lbp,
-                                                                  b->counters + p, ctx->d_err, b->tri_off, S);
+        const auto code = sort_items == 4   ? k_onesweep<false, true, 4>
+                          : sort_items == 8 ? k_onesweep<false, true, 8>
+                                            : k_onesweep<false, true>;
+        const auto scene = sort_items == 4   ? k_onesweep<true, true, 4>
+                           : sort_items == 8 ? k_onesweep<true, true, 8>
+                                             : k_onesweep<true, true>;
+        launch_pdl(p < 4 ? code : scene, sort_tiles, kSortThreads, 0, st, (const uint32_t*)kin, (const uint32_t*)iin, kout,
+                   iout, n, p, (const uint32_t*)b->hist, b->lookback + (size_t)p * lb_pass, b->counters + p, ctx->d_err,
+                   (const uint32_t*)(p < 4 ? nullptr : b->tri_off), p < 4 ? 0u : S, kSpinLimit);
         RT_CHECK_LAUNCH(ctx, "k_onesweep");
         std::swap(kin, kout);
         std::swap(iin, iout);
     }
     b->res_keys = kin;  // five passes: the sorted pairs are in the alternate buffers
     b->res_ids = iin;
-    kb_emit_tiles<<<emit_tiles, kEmitThreads, 0, st>>>(kin, n, b->tri_off, S, b->scan);
+    launch_pdl(kb_emit_tiles, ceil_div(n, kEmitTile), kEmitThreads, 0, st, kin, n, b->tri_off, S, b->scan);
     RT_CHECK_LAUNCH(ctx, "kb_emit_tiles");
-    launch_pdl(k_emit_prefix, 1, kPrefixThreads, 0, st, b->scan, emit_tiles);
+    launch_pdl(k_emit_prefix, prefix_groups(emit_tiles), kPrefixTiles, 0, st, b->scan, emit_tiles);
     RT_CHECK_LAUNCH(ctx, "k_emit_prefix");
     // the emission of a single tree over the concatenated scenes (256 random-soup
     // scenes, 11.5 M triangles: 1.4 ms; leaf boxes and an atomic walk with one

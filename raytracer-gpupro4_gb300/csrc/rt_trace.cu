@@ -142,7 +142,19 @@ __global__ void __launch_bounds__(kTraceThreads, 7) k_trace_primary(TreeRef tr, 
 // 1080p, 312, 309 and 330 us of 65 k triangles at 512 x 512.
 constexpr int kPrimSteps = 3;
 
-__global__ void __launch_bounds__(kTraceThreads, 8) k_walk_primary(TreeRef tr, rt_camera cam, rt_hit* __restrict__ hits,
+// Blocks per SM: with few tiles a warp the image lasts as long as its slowest tiles,
+// and 72 registers (no spills) move a lane faster; with many, 64 registers and
+// another block per SM hide more latency (65 k triangles at 512 x 512 275 us a frame with
+// eight blocks and 272 with seven, 330 k at 720p 583 and 576, 2.1 M at 1080p
+// 1,404 and 1,412).
+constexpr uint32_t kPrimWarps = 8u * kTraceThreads / 32u;  // warps an SM
+uint32_t prim_blocks(const rt_ctx* ctx, uint32_t tiles) {
+    return tiles > 8u * kPrimWarps * (uint32_t)ctx->num_sms ? 8u : 7u;
+}
+
+template <int BLOCKS>
+__global__ void __launch_bounds__(kTraceThreads, BLOCKS) k_walk_primary(TreeRef tr, rt_camera cam,
+                                                                        rt_hit* __restrict__ hits,
                                                                         uint32_t* __restrict__ leaves, uint32_t* work,
                                                                         uint32_t num_tiles, Spill spill,
                                                                         uint32_t* __restrict__ list, TileOrder ord,
@@ -287,9 +299,10 @@ __device__ __forceinline__ RayState load_ray(const rt_ray* __restrict__ rays, ui
 //
 // It walks the trace records (Walk).  BATCH: a listed pixel g belongs to
 // scene g / px, and a warp's lanes may walk different scenes.
-// 16 idle lanes and 4 expansions a round at 64 registers (eight blocks an SM) were
-// the fastest of 12 to 24, 3 to 10 and six to eight: 650 -> 545 us a frame of
-// 2.1 M triangles at 1080p.
+// 16 idle lanes and 4 expansions a round were the fastest of 12 to 24 and 3 to 10:
+// 650 -> 545 us a frame of 2.1 M triangles at 1080p.  A frame's rays take 72 registers
+// (seven blocks an SM; five to eight at 330 k triangles and 720p: 570, 561, 555 and 565 us,
+// at 2.1 M and 1080p 1,509, 1,446, 1,410 and 1,404), a batch's many scenes 64.
 constexpr int kWalkRefill = 16;
 constexpr int kWalkSteps = 4;
 constexpr int kRayRefill = 8;  // a soup's rays: of 8 to 16, and 4 to 12 expansions
@@ -311,7 +324,7 @@ __device__ __forceinline__ void scene_tree(TreeRef& tr, const BatchTrees& bt, ui
 }
 
 template <bool BATCH>
-__global__ void __launch_bounds__(kTraceThreads, 8) k_walk_shade(
+__global__ void __launch_bounds__(kTraceThreads, BATCH ? 8 : 7) k_walk_shade(
     TreeRef tr0, uint8_t* __restrict__ vis, rt_hit* __restrict__ mirror, uint32_t* __restrict__ mirror_leaves,
     const uint32_t* __restrict__ lists, uint32_t cap, const uint32_t* counts, const float4* __restrict__ rays,
     const uint32_t* __restrict__ starts, uint32_t* work, Spill spill, uint32_t* __restrict__ list,
@@ -943,8 +956,8 @@ rt_status trace_primary(rt_ctx* ctx, const rt_lbvh* l, const rt_camera* cam, rt_
         k_trace_primary<<<persistent_blocks(ctx, k_trace_primary, kTraceThreads, tiles), kTraceThreads, 0,
                           ctx->stream>>>(tree_ref(ctx, l), *cam, d_hits, d_leaves, d_stats, work, tiles, ord);
     } else {
-        launch_pdl(k_walk_primary, persistent_blocks(ctx, k_walk_primary, kTraceThreads, tiles), kTraceThreads, 0, ctx->stream,
-                   tree_ref(ctx, l), *cam, d_hits, d_leaves, work, tiles, sp, ctx->d_spill, ord, lists);
+        auto k = prim_blocks(ctx, tiles) == 8u ? k_walk_primary<8> : k_walk_primary<7>;
+        launch_pdl(k, persistent_blocks(ctx, k, kTraceThreads, tiles), kTraceThreads, 0, ctx->stream, tree_ref(ctx, l), *cam, d_hits, d_leaves, work, tiles, sp, ctx->d_spill, ord, lists);
     }
     RT_CHECK_LAUNCH(ctx, d_stats ? "k_trace_primary" : "k_walk_primary");
     HeavyArgs a = heavy_args(ctx, l);
@@ -1456,13 +1469,23 @@ __device__ __forceinline__ void batch_trace_body(const BatchTraceArgs& a, const 
     }
 }
 
-__global__ void __launch_bounds__(256) k_batch_trace(BatchTraceArgs a, TreeRef tr, BatchTrees bt, uint32_t* work) {
+// Blocks of 256 threads per SM (48 and 64 registers; unbounded 80): the scenes of a large
+// batch do not fit the caches, and more warps hide that (256 scenes at 256 x 256
+// 9.88 ms a frame unbounded, 8.59 with four, 8.38 with five, 8.34 with six; primary
+// rays only, 64 scenes, 1,453, 1,178, 1,112 and 1,135 us); with few tiles a warp the spills
+// cost more (16 scenes at 128 x 128 601, 602, 620 and 639 us).
+bool many_tiles(const rt_ctx* ctx, uint64_t tiles) { return tiles > 8ull * 32u * (uint32_t)ctx->num_sms; }
+
+template <int BLOCKS>
+__global__ void __launch_bounds__(256, BLOCKS) k_batch_trace(BatchTraceArgs a, TreeRef tr, BatchTrees bt, uint32_t* work) {
     grid_dep_wait();
     const BatchListArgs none = {nullptr, 0u, nullptr, nullptr, nullptr};
     batch_trace_body<false>(a, none, tr, bt, work);
 }
 
-__global__ void __launch_bounds__(256) k_batch_list(BatchTraceArgs a, BatchListArgs la, TreeRef tr, BatchTrees bt, uint32_t* work) {
+template <int BLOCKS>
+__global__ void __launch_bounds__(256, BLOCKS) k_batch_list(BatchTraceArgs a, BatchListArgs la, TreeRef tr, BatchTrees bt,
+                                                            uint32_t* work) {
     grid_dep_wait();
     batch_trace_body<true>(a, la, tr, bt, work);
 }
@@ -1557,19 +1580,21 @@ extern "C" rt_status rt_batch_trace(rt_ctx* ctx, const rt_batch* b, rt_hit* d_hi
     a.order = b->tuning.order;
     const BatchListArgs la = {b->s_lists, (uint32_t)cap, counts, b->s_rays, b->s_lists + cap};
     const int threads = (int)b->tuning.threads;
+    const uint64_t items = (uint64_t)a.S * a.tiles_per_scene;
+    const auto list = many_tiles(ctx, items) ? k_batch_list<5> : k_batch_list<4>;
+    const auto trace = many_tiles(ctx, items) ? k_batch_trace<5> : k_batch_trace<4>;
     int per_sm = 0;
-    const cudaError_t oe = listed ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_list, threads, 0)
-                                  : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_trace, threads, 0);
+    const cudaError_t oe = listed ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, list, threads, 0)
+                                  : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace, threads, 0);
     if (oe != cudaSuccess || per_sm < 1) per_sm = 1;
     if (b->tuning.blocks_per_sm) per_sm = std::min(per_sm, (int)b->tuning.blocks_per_sm);
-    const uint64_t items = (uint64_t)a.S * a.tiles_per_scene;
     const uint64_t need = (items * 32 + threads - 1) / threads;
     const uint32_t blocks = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)per_sm * ctx->num_sms, need));
     if (listed)
-        launch_pdl(k_batch_list, blocks, threads, 0, ctx->stream, a, la, tr, bt, ctx->d_work + kWorkBatch);
+        launch_pdl(list, blocks, threads, 0, ctx->stream, a, la, tr, bt, ctx->d_work + kWorkBatch);
     else
-        launch_pdl(k_batch_trace, blocks, threads, 0, ctx->stream, a, tr, bt, ctx->d_work + kWorkBatch);
-    RT_CHECK_LAUNCH(ctx, "k_batch_trace");
+        launch_pdl(trace, blocks, threads, 0, ctx->stream, a, tr, bt, ctx->d_work + kWorkBatch);
+    RT_CHECK_LAUNCH(ctx, listed ? "k_batch_list" : "k_batch_trace");
     if (!listed) return RT_OK;
     Spill none;
     memset(&none, 0, sizeof(none));

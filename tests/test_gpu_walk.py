@@ -167,3 +167,44 @@ def test_captured_trace_over_a_later_tree(gpu_ctx, oracle_mod, first, then):
     ref = oracle_mod.trace(nodes, depth, ids, soups[1], oracle_mod.primary_rays(cam))
     assert np.array_equal(hits_to_numpy(out).view(np.int32).ravel(), np.ascontiguousarray(ref).view(np.int32).ravel())
     assert (ref["id"] >= 0).mean() > 0.2
+
+
+def test_images_of_many_tiles(gpu_ctx, oracle_mod):
+    """The variants for more than eight tiles a warp: an image against the oracle, a
+    batch against two halves of it that take the other variant."""
+    import torch
+    from rtgpu import scenes
+    from rtgpu.api import Batch, LBVH, RayTracer, hits_to_numpy
+    tris, depth = scene("soup")
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    tiles = 8 * 32 * sms + 1
+    cam = scenes.look_at((1.7, 1.2, 1.5), (0.5, 0.5, 0.5), vfov_deg=45.0, width=1600, height=4 * -(-tiles // 200))
+    lb = LBVH(gpu_ctx, len(tris), depth).Build(torch.from_numpy(tris).cuda())
+    nodes, ids, _, _ = oracle_mod.lbvh_build(tris, depth)
+    got = hits_to_numpy(RayTracer(gpu_ctx).primary(lb, cam))
+    ref = oracle_mod.trace(nodes, depth, ids, tris, oracle_mod.primary_rays(cam))
+    gpu_ctx.check()
+    assert np.array_equal(got.view(np.int32), ref.view(np.int32))
+
+    counts = scenes.batch_sizes(2 * (-(-tiles // 1024)), 300, 3000, 5)  # 1,024 tiles a scene
+    soup = torch.from_numpy(scenes.random_soup(int(counts.sum()), 6, 0.02, 0.1)).cuda()
+    cams, lights = scenes.batch_views(len(counts), 256, 128)
+    half = len(counts) // 2
+    cut = int(counts[:half].sum())
+
+    def traced(c, t, k, li, shadow):
+        b = Batch(gpu_ctx, c, 14)
+        b.set_views(k, li)
+        hits, vis = b.alloc_outputs(shadow)
+        b.build(t.contiguous())
+        b.trace(hits, vis)
+        gpu_ctx.check()
+        return hits.reshape(-1), vis
+
+    for shadow in (True, False):
+        whole, vis = traced(counts, soup, cams, lights, shadow)
+        parts = [traced(counts[:half], soup[:cut], cams[:half], lights[:half], shadow),
+                 traced(counts[half:], soup[cut:], cams[half:], lights[half:], shadow)]
+        assert torch.equal(whole.view(torch.int32), torch.cat([p[0] for p in parts]).view(torch.int32))
+        if shadow:
+            assert torch.equal(vis.reshape(-1), torch.cat([p[1].reshape(-1) for p in parts]))
