@@ -1083,6 +1083,14 @@ constexpr uint32_t kMaskBits = kHeadBit - 1u;
 constexpr int kItemCap = 64;         // items one tile or group hands on (2 x depth + 2 <= 54)
 constexpr int kMergeGroup = 32;      // tiles (groups) per CTA of the next level
 constexpr int kUnitWords = 12;       // shared words per unit
+// Threads of a merge CTA: four units each instead of eight (66,000 triangles 82 -> 79 us
+// a build, 400,000: 139 -> 131, 2.1 M: 292 -> 288; 1,024 threads the same).
+constexpr int kMergeThreads = 512;
+// A chunk takes a thread per leaf while its tiles are few (66,000 triangles 79 -> 75 us,
+// 400,000: 131 -> 125, 700,000: 165 -> 162), and in a batch (256 scenes 8,370 -> 8,248 us);
+// with more tiles of one tree two leaves a thread are faster (1.2 M: 205 and 200 us,
+// 2.1 M: 297 and 288).
+constexpr uint32_t kChunkWideTris = 1u << 20;
 constexpr int kUnitCap = kMergeGroup * kItemCap;  // units of one CTA of the merge: the items of a group
 constexpr size_t kUnitSmem = (size_t)kUnitWords * kUnitCap * sizeof(uint32_t) + 16;
 constexpr size_t kChunkSmem = (size_t)kUnitWords * kTreeTile * sizeof(uint32_t) + 16;
@@ -1760,8 +1768,8 @@ __device__ void merge_group(const Units& u, const uint2* in_items, const uint32_
 
 // k_emit_chunks: the tile level.  One CTA merges the leaves of a tile; tile c's
 // items go to items + c * kItemCap, their number to counts[c].
-template <bool BATCH>
-__global__ void __launch_bounds__(kEmitThreads) k_emit_chunks(const uint2* __restrict__ tile_units,
+template <int THREADS, bool BATCH>
+__global__ void __launch_bounds__(THREADS) k_emit_chunks(const uint2* __restrict__ tile_units,
                                                               const uint32_t* __restrict__ tile_counts, uint32_t depth,
                                                               rt_node* nodes, uint2* items, uint32_t* counts,
                                                               uint32_t* err, uint32_t* inner,
@@ -1778,7 +1786,7 @@ __global__ void __launch_bounds__(kEmitThreads) k_emit_chunks(const uint2* __res
         if (threadIdx.x == 0) counts[c] = 0u;
         return;
     }
-    merge_group<kEmitThreads, BATCH>(u, tile_units + (size_t)c * kTreeTile, tile_counts + c, (uint32_t)kTreeTile, 1u, heap,
+    merge_group<THREADS, BATCH>(u, tile_units + (size_t)c * kTreeTile, tile_counts + c, (uint32_t)kTreeTile, 1u, heap,
                                      items + (size_t)c * kItemCap, counts + c, err, inner, s_off, s_items, s_ipos);
 }
 
@@ -1791,7 +1799,7 @@ __global__ void __launch_bounds__(kEmitThreads) k_emit_chunks(const uint2* __res
 // The first level's items are at out_items + g * kItemCap (counts at
 // out_counts + g), each next level's after the previous one's.
 template <bool BATCH>
-__global__ void __launch_bounds__(kEmitThreads) k_emit_merge(const uint2* __restrict__ in_items,
+__global__ void __launch_bounds__(kMergeThreads) k_emit_merge(const uint2* __restrict__ in_items,
                                                         const uint32_t* __restrict__ in_counts, uint32_t n_in,
                                                         uint32_t depth, rt_node* nodes, uint2* out_items,
                                                         uint32_t* out_counts, uint32_t* tickets, uint32_t* err,
@@ -1807,7 +1815,7 @@ __global__ void __launch_bounds__(kEmitThreads) k_emit_merge(const uint2* __rest
     const int t = threadIdx.x;
     uint32_t g = blockIdx.x;
     uint32_t n_lev = (n_in + kMergeGroup - 1) / kMergeGroup;
-    merge_group<kEmitThreads, BATCH>(u, in_items + (size_t)g * kMergeGroup * kItemCap, in_counts + (size_t)g * kMergeGroup,
+    merge_group<kMergeThreads, BATCH>(u, in_items + (size_t)g * kMergeGroup * kItemCap, in_counts + (size_t)g * kMergeGroup,
                          (uint32_t)kItemCap, min((uint32_t)kMergeGroup, n_in - g * kMergeGroup), heap,
                          out_items + (size_t)g * kItemCap, out_counts + g, err, inner, s_off, s_items, s_ipos);
     size_t ioff = 0, coff = 0, toff = 0;
@@ -1829,7 +1837,7 @@ __global__ void __launch_bounds__(kEmitThreads) k_emit_merge(const uint2* __rest
         const size_t pcoff = coff + (size_t)parent * kMergeGroup;
         ioff += (size_t)n_lev * kItemCap;
         coff += n_lev;
-        merge_group<kEmitThreads, BATCH>(u, out_items + pioff, out_counts + pcoff, (uint32_t)kItemCap, gs, heap,
+        merge_group<kMergeThreads, BATCH>(u, out_items + pioff, out_counts + pcoff, (uint32_t)kItemCap, gs, heap,
                              out_items + ioff + (size_t)parent * kItemCap, out_counts + coff + parent, err, inner,
                              s_off, s_items, s_ipos);
         toff += n_next;
@@ -2395,11 +2403,12 @@ static rt_status launch_build(rt_ctx* ctx, rt_lbvh* l, const float* d_tris, uint
                (const uint32_t*)l->ids, d_tris, n, l->depth, (const uint32_t*)l->scan, l->nodes, l->sorted_tris,
                tile_units, tile_counts, ctx->d_err, l->leaf_of, (const uint32_t*)nullptr, 0u, (uint32_t*)nullptr);
     RT_CHECK_LAUNCH(ctx, "k_emit_units");
-    launch_pdl(k_emit_chunks<false>, emit_tiles, kEmitThreads, kChunkSmem, st, (const uint2*)tile_units,
+    const int chunk_threads = n <= kChunkWideTris ? kTreeTile : kEmitThreads;
+    launch_pdl(n <= kChunkWideTris ? k_emit_chunks<kTreeTile, false> : k_emit_chunks<kEmitThreads, false>, emit_tiles, chunk_threads, kChunkSmem, st, (const uint2*)tile_units,
                (const uint32_t*)tile_counts, l->depth, l->nodes, l->items, l->item_counts, ctx->d_err, inner,
                (const uint32_t*)nullptr);
     RT_CHECK_LAUNCH(ctx, "k_emit_chunks");
-    launch_pdl(k_emit_merge<false>, ceil_div(emit_tiles, kMergeGroup), kEmitThreads, kUnitSmem, st,
+    launch_pdl(k_emit_merge<false>, ceil_div(emit_tiles, kMergeGroup), kMergeThreads, kUnitSmem, st,
                (const uint2*)l->items, (const uint32_t*)l->item_counts, emit_tiles, l->depth, l->nodes,
                l->items + (size_t)emit_tiles * kItemCap, l->item_counts + emit_tiles, l->item_counts + 7 * cap, ctx->d_err,
                inner, (const uint32_t*)nullptr);
@@ -3077,11 +3086,11 @@ extern "C" rt_status rt_batch_build(rt_ctx* ctx, rt_batch* b, const float* d_tri
                (const uint32_t*)iin, d_tris, n, b->depth, (const uint32_t*)b->scan, b->nodes, b->sorted_tris, tile_units,
                tile_counts, ctx->d_err, b->leaf_of, (const uint32_t*)b->tri_off, S, b->ids_local);
     RT_CHECK_LAUNCH(ctx, "k_emit_units");
-    launch_pdl(k_emit_chunks<true>, emit_tiles, kEmitThreads, kChunkSmem, st, (const uint2*)tile_units,
+    launch_pdl(k_emit_chunks<kTreeTile, true>, emit_tiles, kTreeTile, kChunkSmem, st, (const uint2*)tile_units,
                (const uint32_t*)tile_counts, b->depth, b->nodes, b->items, b->item_counts, ctx->d_err, (uint32_t*)nullptr,
                (const uint32_t*)b->tri_off);
     RT_CHECK_LAUNCH(ctx, "k_emit_chunks");
-    launch_pdl(k_emit_merge<true>, ceil_div(emit_tiles, kMergeGroup), kEmitThreads, kUnitSmem, st,
+    launch_pdl(k_emit_merge<true>, ceil_div(emit_tiles, kMergeGroup), kMergeThreads, kUnitSmem, st,
                (const uint2*)b->items, (const uint32_t*)b->item_counts, emit_tiles, b->depth, b->nodes,
                b->items + (size_t)emit_tiles * kItemCap, b->item_counts + emit_tiles, b->item_counts + 7 * (size_t)emit_tiles,
                ctx->d_err, (uint32_t*)nullptr, (const uint32_t*)b->tri_off);

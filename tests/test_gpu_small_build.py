@@ -54,10 +54,11 @@ def test_handle_shared_with_the_general_build(gpu_ctx, oracle_mod):
         check(gpu_ctx, oracle_mod, lb, scenes.random_soup(n, n + 1), 15)
 
 
-@pytest.mark.parametrize("n,depth", [(4608, 20), (4609, 4), (155648, 20), (155649, 12), (1245184, 22), (1245185, 22)])
+@pytest.mark.parametrize("n,depth", [(4608, 20), (4609, 4), (155648, 20), (155649, 12), (1048576, 20), (1048577, 21),
+                                     (1245184, 22), (1245185, 22)])
 def test_tiles_of_the_general_build(gpu_ctx, oracle_mod, n, depth):
     """Around a whole emission tile and around the sizes where the sort changes
-    its tile; the handle is larger than the soup."""
+    its tile and the chunks their threads; the handle is larger than the soup."""
     from rtgpu import scenes
     from rtgpu.api import LBVH
     check(gpu_ctx, oracle_mod, LBVH(gpu_ctx, n + 300000, depth), scenes.random_soup(n, n, 0.001, 0.02), depth)
