@@ -17,6 +17,7 @@
 // the image, so a static grid leaves SMs idle behind the last heavy tiles.
 #include <algorithm>
 #include <cstring>
+#include <initializer_list>
 
 #include "rt_records.cuh"
 #include "rt_traverse.cuh"
@@ -1085,6 +1086,16 @@ rt_status trace_rays(rt_ctx* ctx, const rt_lbvh* l, const rt_ray* d_rays, uint32
 }
 
 }  // namespace
+
+Spill shadow_spill(rt_ctx* ctx) { return spill_of(ctx, true, 1); }
+
+// Zeroes the counters of a bounce of the colour stage (words of ctx->d_words and the
+// shadow rays' hand-over) and makes the trace records if the tree has none.
+rt_status begin_bounce(rt_ctx* ctx, const rt_lbvh* l, const Spill& shadow, std::initializer_list<uint32_t*> words) {
+    uint64_t mask = spill_reset_bits(ctx, shadow);
+    for (uint32_t* w : words) mask |= word_bit(ctx, w);
+    return reset_words(ctx, mask, records_of(ctx, l));
+}
 
 rt_status reset_work_and_records(rt_ctx* ctx, int slot, const rt_lbvh* l) {
     return reset_words(ctx, word_bit(ctx, ctx->d_work + slot), records_of(ctx, l));

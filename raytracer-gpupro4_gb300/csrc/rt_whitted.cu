@@ -13,6 +13,7 @@
 //   k_wh_setup         the shading geometry of each hit; pixels that cast a
 //                      shadow ray are appended to the shadow list
 //   k_wh_trace<true>   the shadow rays (first hit), restarted at the hit's leaf
+//   k_wh_heavy         the shadow rays that it handed over, a warp each
 //   k_wh_finish        colour, accumulation and result; the next ray (mirror
 //                      or refracted) and the next bounce's list
 //
@@ -23,6 +24,7 @@
 // divides by the length and pow(x, 49) is x^32 x^16 x, so the oracle's
 // restatement (or_render_whitted) gives the same bits.
 #include <algorithm>
+#include <initializer_list>
 
 #include "rt_traverse.cuh"
 
@@ -147,6 +149,7 @@ __device__ __forceinline__ void append(bool take, uint32_t p, uint32_t* list, ui
 // in 8 x 4 tile order; accumulation and result cleared.
 __global__ void __launch_bounds__(kWhListThreads) k_wh_init(rt_camera cam, WhBufs w, float4* __restrict__ accum,
                                                             float4* __restrict__ result, uint32_t num_tiles) {
+    grid_dep_wait();
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
     for (uint32_t t = warp; t < num_tiles; t += nwarps) {
@@ -166,15 +169,41 @@ __global__ void __launch_bounds__(kWhListThreads) k_wh_init(rt_camera cam, WhBuf
     }
 }
 
+// Pixel p's ray: the live ray, or the shadow ray of its hit (false: none).
+template <bool SHADOW>
+__device__ __forceinline__ bool wh_ray(const ShadeArgs& a, const WhBufs& w, uint32_t p, RayState* r) {
+    const float4 ro = w.ro[p], rd = w.rd[p];
+    if (!SHADOW) {
+        *r = make_ray(mk3(ro.x, ro.y, ro.z), mk3(rd.x, rd.y, rd.z), rd.w, __float_as_int(ro.w));
+        return true;
+    }
+    const int4 h = w.hit[p];
+    if (h.x < 0 || (uint32_t)h.x >= a.n) return false;
+    const Geom g = geom(a, h.x, __int_as_float(h.y), __int_as_float(h.z), __int_as_float(h.w), mk3(ro.x, ro.y, ro.z),
+                        mk3(rd.x, rd.y, rd.z));
+    // :149-153: from the hit point towards the light, up to the light
+    *r = make_ray(g.P, mk3(-g.L.x, -g.L.y, -g.L.z), g.dist, h.x);
+    return true;
+}
+
 // Closest hits of the listed rays (SHADOW = false) or the shadow rays of the
 // listed hits (SHADOW = true).  A lane whose ray has ended takes the next list
-// entry once kWhRefill lanes of its warp are idle (Walk).
+// entry once kWhRefill lanes of its warp are idle (Walk).  Shadow rays over the
+// hand-over budget go to k_wh_heavy, and once the list is empty those over kWhTail
+// tests too: the pass waited for its longest rays with 13 % of the warp slots in use.
+// The call at 720p with one bounce 811 -> 722 us with 160 tests, 728 and 739 with 128
+// and 192; a soup with three bounces 2,013 -> 1,597 us, a torus' few long rays 650 -> 643.
+// The closest hits' hand-over gained on the soup (1,375 us) and lost on the others
+// (720p 771, torus 673).
+constexpr uint32_t kWhTail = 160;
 constexpr int kWhRefill = 8;
 constexpr int kWhSteps = 4;  // 4: 813 us a call at 720p with one bounce, 6: 848, 8: 860; 32 rays a warp at once: 1,110
 
 template <bool SHADOW>
-__global__ void __launch_bounds__(kWhThreads, 7) k_wh_trace(TreeRef tr, ShadeArgs a, WhBufs w, int src, uint32_t* work) {
+__global__ void __launch_bounds__(kWhThreads, 7) k_wh_trace(TreeRef tr, ShadeArgs a, WhBufs w, int src, uint32_t* work,
+                                                           Spill spill, uint32_t* __restrict__ heavy) {
     constexpr uint32_t kFull = 0xffffffffu;
+    grid_dep_wait();
     mark_records(tr);
     const uint32_t* list = wlist(w, src);
     const uint32_t n = min(w.counts[src], w.px);
@@ -183,7 +212,7 @@ __global__ void __launch_bounds__(kWhThreads, 7) k_wh_trace(TreeRef tr, ShadeArg
     wk.clear();
     uint2 stack[kStackSize];
     uint32_t p = 0;
-    bool live = false, drained = false;
+    bool live = false, drained = false, budgeted = SHADOW && spill.count != nullptr;
     for (;;) {
         const uint32_t idle = __ballot_sync(kFull, !live);
         if (!drained && (idle == kFull || __popc(idle) >= kWhRefill)) {
@@ -197,22 +226,9 @@ __global__ void __launch_bounds__(kWhThreads, 7) k_wh_trace(TreeRef tr, ShadeArg
             uint32_t start = 1u;
             if (take) {
                 p = __ldg(list + k);
-                const float4 ro = w.ro[p], rd = w.rd[p];
                 start = w.leaf[p];
-                if (!SHADOW) {
-                    r = make_ray(mk3(ro.x, ro.y, ro.z), mk3(rd.x, rd.y, rd.z), rd.w, __float_as_int(ro.w));
-                } else {
-                    const int4 h = w.hit[p];
-                    if (h.x >= 0 && (uint32_t)h.x < a.n) {
-                        const Geom g = geom(a, h.x, __int_as_float(h.y), __int_as_float(h.z), __int_as_float(h.w),
-                                            mk3(ro.x, ro.y, ro.z), mk3(rd.x, rd.y, rd.z));
-                        // :149-153: from the hit point towards the light, up to the light
-                        r = make_ray(g.P, mk3(-g.L.x, -g.L.y, -g.L.z), g.dist, h.x);
-                    } else {
-                        w.occl[p] = 0u;
-                        take = false;
-                    }
-                }
+                take = wh_ray<SHADOW>(a, w, p, &r);
+                if (SHADOW && !take) w.occl[p] = 0u;
                 if (take) live = true;
             }
             wk.start(take, r, tr, start, stack);
@@ -222,7 +238,16 @@ __global__ void __launch_bounds__(kWhThreads, 7) k_wh_trace(TreeRef tr, ShadeArg
             continue;
         }
         wk.round(tr, kWhSteps, stack, SHADOW);
-        if (live && !wk.have) {
+        if (live && wk.have && budgeted && wk.tests > (drained ? min(spill.budget, kWhTail) : spill.budget)) {
+            const uint32_t e = atomicAdd(spill.count, 1u);
+            if (e < spill.cap) {
+                heavy[e] = p;
+                wk.stop();
+            } else {
+                budgeted = false;  // list full: finish here
+            }
+        }
+        if (live && !wk.have) {  // of a handed-over ray: not blocked so far
             if (SHADOW) {
                 w.occl[p] = wk.b.id >= 0 ? 1u : 0u;
             } else {
@@ -234,8 +259,27 @@ __global__ void __launch_bounds__(kWhThreads, 7) k_wh_trace(TreeRef tr, ShadeArg
     }
 }
 
+// The shadow rays handed over, a warp each (traverse_wide).
+__global__ void __launch_bounds__(kWhThreads, 7) k_wh_heavy(TreeRef tr, ShadeArgs a, WhBufs w, Spill spill,
+                                                            const uint32_t* __restrict__ heavy, uint32_t cap) {
+    grid_dep_wait();
+    const uint32_t n = min(*spill.count, spill.cap);
+    for (uint32_t e = next_tile(spill.work); e < n; e = next_tile(spill.work)) {
+        const uint32_t p = heavy[e];
+        RayState r;
+        if (!wh_ray<true>(a, w, p, &r)) continue;  // not listed
+        Hit none;
+        none.id = -1;
+        none.u = none.v = -1.0f;
+        none.t = 0.0f;
+        const Hit h = trace_wide(r, tr, true, cap, none);
+        if ((threadIdx.x & 31) == 0) w.occl[p] = h.id >= 0 ? 1u : 0u;
+    }
+}
+
 // Pixels of the live list whose hit casts a shadow ray join the shadow list.
 __global__ void __launch_bounds__(kWhListThreads) k_wh_setup(ShadeArgs a, WhBufs w, int src) {
+    grid_dep_wait();
     const uint32_t n = min(w.counts[src], w.px);
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += stride) {  // uniform per warp
@@ -260,6 +304,7 @@ __global__ void __launch_bounds__(kWhListThreads) k_wh_setup(ShadeArgs a, WhBufs
 __global__ void __launch_bounds__(kWhListThreads) k_wh_finish(ShadeArgs a, WhBufs w, int src, uint32_t bounce,
                                                               bool last, float4* __restrict__ accum,
                                                               float4* __restrict__ result) {
+    grid_dep_wait();
     const uint32_t n = min(w.counts[src], w.px);
     const int dst = src ^ 1;
     const uint32_t stride = gridDim.x * blockDim.x;
@@ -399,6 +444,8 @@ WhBufs whitted_bufs(rt_ctx* ctx, const rt_lbvh* l, uint32_t px) {
 }  // namespace
 
 TreeRef tree_ref(const rt_ctx* ctx, const rt_lbvh* l);
+Spill shadow_spill(rt_ctx* ctx);
+rt_status begin_bounce(rt_ctx* ctx, const rt_lbvh* l, const Spill& shadow, std::initializer_list<uint32_t*> words);
 
 extern "C" rt_status rt_render_whitted(rt_ctx* ctx, const rt_lbvh* l, const rt_camera* cam, const float light[3],
                                        const rt_shade_params* prm, const int32_t* d_material_ids,
@@ -437,35 +484,47 @@ extern "C" rt_status rt_render_whitted(rt_ctx* ctx, const rt_lbvh* l, const rt_c
     a.err = ctx->d_err;
     TreeRef tr = tree_ref(ctx, l);
     tr.compact = false;  // the walks restart at heap nodes
+    tr.nodes = l->nodes;
+    tr.num_nodes = l->num_nodes;
     cudaStream_t st = ctx->stream;
     float4* acc = reinterpret_cast<float4*>(d_accum);
     float4* res = reinterpret_cast<float4*>(d_result);
     const uint32_t tiles = (uint32_t)(((cam->width + 7) / 8) * ((cam->height + 3) / 4));
     RT_CHECK_CUDA(ctx, cudaMemsetAsync(w.counts, 0, 3 * sizeof(uint32_t), st));
     const uint32_t lblocks = (uint32_t)std::max(1, ctx->num_sms * 8);
-    k_wh_init<<<std::min<uint32_t>(lblocks, (tiles + 7) / 8), kWhListThreads, 0, st>>>(*cam, w, acc, res, tiles);
+    launch_pdl(k_wh_init, std::min<uint32_t>(lblocks, (tiles + 7) / 8), kWhListThreads, 0, st, *cam, w, acc, res, tiles);
     RT_CHECK_LAUNCH(ctx, "k_wh_init");
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_wh_trace<false>, kWhThreads, 0) != cudaSuccess ||
         per_sm < 1)
         per_sm = 1;
     const uint32_t tblocks = (uint32_t)per_sm * ctx->num_sms;
+    const Spill shadow = shadow_spill(ctx);
+    const uint32_t cap = wide_stack_entries(l->depth);
+    const size_t hsmem = wide_smem_bytes(cap);
+    int heavy_per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&heavy_per_sm, k_wh_heavy, kWhThreads, hsmem) != cudaSuccess ||
+        heavy_per_sm < 1)
+        heavy_per_sm = 1;
+    const uint32_t hblocks = (uint32_t)heavy_per_sm * ctx->num_sms;
+    uint32_t *work = ctx->d_work + kWorkWhTrace, *shadow_work = ctx->d_work + kWorkWhShadow;
     for (uint32_t b = 0; b <= prm->bounces; ++b) {
         const int src = (int)(b & 1u);
         // the next bounce's list and the shadow list start empty
-        RT_CHECK_CUDA(ctx, cudaMemsetAsync(w.counts + (src ^ 1), 0, sizeof(uint32_t), st));
-        RT_CHECK_CUDA(ctx, cudaMemsetAsync(w.counts + 2, 0, sizeof(uint32_t), st));
-        if ((s = b == 0 ? reset_work_and_records(ctx, kWorkWhTrace, l) : reset_work(ctx, kWorkWhTrace)) != RT_OK) return s;
-        k_wh_trace<false><<<tblocks, kWhThreads, 0, st>>>(tr, a, w, src, ctx->d_work + kWorkWhTrace);
+        if ((s = begin_bounce(ctx, l, shadow, {work, shadow_work, w.counts + (src ^ 1), w.counts + 2})) != RT_OK) return s;
+        launch_pdl(k_wh_trace<false>, tblocks, kWhThreads, 0, st, tr, a, w, src, work, shadow, ctx->d_spill);
         RT_CHECK_LAUNCH(ctx, "k_wh_trace");
         if (a.shadows) {
-            k_wh_setup<<<lblocks, kWhListThreads, 0, st>>>(a, w, src);
+            launch_pdl(k_wh_setup, lblocks, kWhListThreads, 0, st, a, w, src);
             RT_CHECK_LAUNCH(ctx, "k_wh_setup");
-            if ((s = reset_work(ctx, kWorkWhShadow)) != RT_OK) return s;
-            k_wh_trace<true><<<tblocks, kWhThreads, 0, st>>>(tr, a, w, 2, ctx->d_work + kWorkWhShadow);
+            launch_pdl(k_wh_trace<true>, tblocks, kWhThreads, 0, st, tr, a, w, 2, shadow_work, shadow, ctx->d_spill);
             RT_CHECK_LAUNCH(ctx, "k_wh_trace_shadow");
+            if (shadow.count) {
+                launch_pdl(k_wh_heavy, hblocks, kWhThreads, hsmem, st, tr, a, w, shadow, (const uint32_t*)ctx->d_spill, cap);
+                RT_CHECK_LAUNCH(ctx, "k_wh_heavy_shadow");
+            }
         }
-        k_wh_finish<<<lblocks, kWhListThreads, 0, st>>>(a, w, src, b, b == prm->bounces, acc, res);
+        launch_pdl(k_wh_finish, lblocks, kWhListThreads, 0, st, a, w, src, b, b == prm->bounces, acc, res);
         RT_CHECK_LAUNCH(ctx, "k_wh_finish");
     }
     return RT_OK;

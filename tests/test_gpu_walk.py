@@ -208,3 +208,30 @@ def test_images_of_many_tiles(gpu_ctx, oracle_mod):
         assert torch.equal(whole.view(torch.int32), torch.cat([p[0] for p in parts]).view(torch.int32))
         if shadow:
             assert torch.equal(vis.reshape(-1), torch.cat([p[1].reshape(-1) for p in parts]))
+
+
+@pytest.mark.parametrize("budget", [0, 1, 200, None])
+def test_colour_stage_hands_over_shadow_rays(gpu_ctx, oracle_mod, budget):
+    """Shadow rays traced by their lane, by a warp, or handed over once the list is
+    empty: the oracle's image."""
+    import torch
+    from rtgpu import scenes
+    from rtgpu.api import LBVH, RayTracer
+    from test_gpu_whitted import materials
+    tris, depth = scene("soup")
+    mats = materials()
+    mids = np.random.default_rng(2).integers(0, len(mats), len(tris)).astype(np.int32)
+    lb = LBVH(gpu_ctx, len(tris), depth).Build(torch.from_numpy(tris).cuda())
+    nodes, ids, _, _ = oracle_mod.lbvh_build(tris, depth)
+    cam = scenes.look_at((1.7, 1.2, 1.5), (0.5, 0.5, 0.5), vfov_deg=45.0, width=183, height=97)
+    light = (0.5, 3.0, 0.4)
+    gpu_ctx.set_trace_budget(budget)
+    try:
+        acc, _ = RayTracer(gpu_ctx).whitted(lb, cam, light, mats, torch.from_numpy(mids).cuda(), bounces=2, shadows=True)
+        gpu_ctx.check()
+    finally:
+        gpu_ctx.set_trace_budget(None)
+    ref, _ = oracle_mod.render_whitted(nodes, depth, ids, tris, cam, light, mats, mids, None, bounces=2, shadows=True)
+    got = acc.cpu().numpy()
+    assert np.array_equal(got.view(np.int32).ravel(), np.ascontiguousarray(ref, np.float32).view(np.int32).ravel())
+    assert ref[:, :3].max() > 0.1
