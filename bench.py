@@ -377,9 +377,9 @@ def run_ours(args, dist: Dist):
     # stage: (ms, algorithmic bytes, kernels of the stage's ncu traffic)
     nb = build_launches(n)
     build_label = f"build ({nb} kernels)"
-    groups = {"k_trace_primary (+ k_trace_heavy)": (prim_ms, bytes_primary, ("k_trace_primary", "k_trace_heavy")),
-              "k_trace_shade (+ k_trace_heavy_team)": (sec_ms, bytes_secondary,
-                                                      ("k_trace_shade", "k_trace_heavy_team")),
+    groups = {"k_walk_primary (+ k_trace_heavy)": (prim_ms, bytes_primary, ("k_walk_primary", "k_trace_heavy")),
+              "k_walk_shade (+ k_trace_heavy_team)": (sec_ms, bytes_secondary,
+                                                     ("k_walk_shade", "k_trace_heavy_team")),
               build_label: (build_ms, BUILD_BYTES_PER_TRI * n,
                             ("k_bounds", "k_morton_hist") + ("k_onesweep",) * 4 +
                             ("k_emit_tiles", "k_emit_prefix", "k_emit_units", "k_emit_chunks", "k_emit_merge"))}
@@ -408,9 +408,9 @@ def run_ours(args, dist: Dist):
                 "stages": {"build": {"ms": round(float(build_ms), 4), "frac": frac(BUILD_BYTES_PER_TRI * n, build_ms),
                                      "traffic": ncu_traffic(*groups[build_label][2])},
                            "primary": {"ms": round(float(prim_ms), 4), "frac": frac(bytes_primary, prim_ms),
-                                       "cache": ncu_cache_fractions("k_trace_primary")},
+                                       "cache": ncu_cache_fractions("k_walk_primary")},
                            "shading": {"ms": round(float(sec_ms), 4), "frac": frac(bytes_secondary, sec_ms),
-                                       "cache": ncu_cache_fractions("k_trace_shade")}}}
+                                       "cache": ncu_cache_fractions("k_walk_shade")}}}
     out = {
         "metric": METRIC, "value": round(value, 3), "unit": "Mtri/s", "n_gpus": dist.world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": round(float(step_ms.mean()), 4), "higher_is_better": True,
@@ -427,8 +427,8 @@ def run_ours(args, dist: Dist):
         "roofline": roofline,
         "e2e": e2e,
         # per graph: the build's kernels; k_order_begin (which also zeroes the
-        # frame's counters), k_trace_primary (which also lists the shading
-        # rays), k_trace_heavy; k_trace_shade, k_trace_heavy_team
+        # frame's counters and makes the trace records), k_walk_primary (which
+        # also lists the shading rays), k_trace_heavy; k_walk_shade, k_trace_heavy_team
         "gpu_launches": (nb + 5) * args.steps,
     }
     out["clocks"] = clk.summary()
@@ -450,10 +450,11 @@ def run_ours(args, dist: Dist):
 
 
 def build_launches(n: int) -> int:
-    """Kernels of one rt_lbvh_build: k_bounds, k_morton_hist, four radix
+    """Kernels of one rt_lbvh_build of more than 2,048 triangles (k_build_small
+    alone below): k_bounds, k_morton_hist, four radix
     passes, k_emit_tiles, k_emit_prefix, k_emit_units, k_emit_chunks (the
     tile level of the merge), k_emit_merge (every level above it)."""
-    return 11
+    return 11 if n > 2048 else 1
 
 
 def frame_config(name, n, npx, depth):
@@ -648,7 +649,7 @@ def run_batch(args, dist: Dist):
         frame.close()
 
     peak, peak_kind = measured_peaks()
-    groups = {"k_batch_trace": (trace_ms, trace_bytes), "batched build (12 kernels)": (build_ms, BUILD_BYTES_PER_TRI * total)}
+    groups = {"k_batch_list + k_walk_shade": (trace_ms, trace_bytes), "batched build (13 kernels)": (build_ms, BUILD_BYTES_PER_TRI * total)}
     dom = max(groups, key=lambda g: groups[g][0])
     ms, byts = groups[dom]
     achieved = byts / (ms / 1e3) / 1e9
@@ -670,9 +671,11 @@ def run_batch(args, dist: Dist):
                      "frac": round(achieved / peak, 4), "peak_kind": peak_kind, "traffic": ncu_traffic(dom),
                      "algorithmic_bytes_per_launch": int(byts), "avg_launch_ms": round(float(ms), 4)},
         "e2e": e2e,
-        # per graph: 12 build kernels, k_reset_words, k_batch_trace (primary rays, listing the
-        # shadow rays), k_trace_shade (the shadow rays)
-        "gpu_launches": 15 * args.steps,
+        # per graph: 13 build kernels (three kb_*, five radix passes, kb_emit_tiles,
+        # k_emit_prefix, k_emit_units, k_emit_chunks, k_emit_merge), k_reset_words (which
+        # also makes the trace records), k_batch_list (primary rays, listing the
+        # shadow rays), k_walk_shade (the shadow rays)
+        "gpu_launches": 16 * args.steps,
     }
     out["clocks"] = clk.summary()
     if dist.rank == 0 and dist.world == 1 and not args.no_cpu_baseline:
@@ -958,8 +961,10 @@ def run_pt(args, dist: Dist, adjoint: bool = False):
                           "forward_msegments_s": round(segs_per_s, 1)},
            "roofline": roofline,
            "clocks": clk.summary(),
-           # per step: 10 build kernels + the render (+ the adjoint kernel)
-           "gpu_launches": (build_launches(n) + 1 + (1 if adjoint else 0)) * args.steps}
+           # per step: the build's kernels; k_reset_words (which also makes the trace records),
+           # k_pathtrace and, with several samples, k_fold_terms; k_reset_words and
+           # k_pathtrace_adjoint
+           "gpu_launches": (build_launches(n) + (3 if spp > 1 else 2) + (2 if adjoint else 0)) * args.steps}
     if adjoint:
         out["components"]["backward_ms"] = round(bwd_ms, 4)
         out["components"]["backward_over_forward"] = round(bwd_ms / fwd_ms, 3)

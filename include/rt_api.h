@@ -500,7 +500,10 @@ typedef struct rt_pt_params {
  * (RayTracerCS.cpp:306), and n0 = 0 its reset on camera motion
  * (RayTracerCS.cpp:246-250); d_image is not read when n0 = 0.  Sample n of
  * a pixel has its own PCG32 stream, so two calls of k samples with n0 = 0
- * and n0 = k give the image of one call of 2k samples, bit for bit. */
+ * and n0 = k give the image of one call of 2k samples, bit for bit.
+ * A call of several samples keeps their terms in scratch of the context (at most
+ * 512 MB, allocated by the first call that needs more; not inside a stream
+ * capture, where a pixel's samples follow one another instead). */
 rt_status rt_pathtrace(rt_ctx* ctx, const rt_lbvh* lbvh, const float* d_albedo, const float* d_emission,
                        const rt_camera* cam, const rt_pt_params* p, float* d_image);
 /* rt_pathtrace that also adds its walk counts to d_counts (device, 4 x

@@ -1848,13 +1848,13 @@ __global__ void __launch_bounds__(kMergeThreads) k_emit_merge(const uint2* __res
 
 // k_build_small: the whole build of up to kSmallTris triangles in one block.  The
 // launches of the general build are a chain of a dozen kernels of one to a few
-// blocks each, whose latencies add up to 68 us however small the soup is; here a
+// blocks each, whose latencies add up to 40 us however small the soup is; here a
 // phase costs a barrier.  Keys and ids are sorted in shared memory (the ranking
 // of k_onesweep), the record scans run over the block, and the bottom-up
 // (unit_bottom_up) takes all leaves at once, so nothing is left to merge.
 constexpr int kSmallThreads = 1024;
 constexpr int kSmallWarps = kSmallThreads / 32;
-constexpr uint32_t kSmallTris = 4 * kSmallThreads;
+constexpr uint32_t kSmallTris = 2 * kSmallThreads;
 constexpr uint32_t kSmallLeaf = 16;  // leaves above this many triangles are folded by a warp
 
 constexpr size_t small_smem(int items) {
@@ -2338,8 +2338,8 @@ static rt_status launch_build(rt_ctx* ctx, rt_lbvh* l, const float* d_tris, uint
     cudaStream_t st = ctx->stream;
     l->n = n;
     l->src_tris = d_tris;
-    // One block against the launches below: 300 triangles 21 and 58 us, 1,000: 29 and 69,
-    // 2,048: 44 and 78, 4,096: 75 and 80; one block would need more shared memory beyond.
+    // One block against the launches below: 300 triangles 21 and 40 us, 1,000: 29 and 46,
+    // 2,048: 44 and 49, 3,000: 62 and 49.
     // The flags ask for passes that only the launches below have.
     if (n <= kSmallTris && flags == 0u) {
         const uint32_t emit_tiles = ceil_div(n, kTreeTile);
@@ -2351,9 +2351,7 @@ static rt_status launch_build(rt_ctx* ctx, rt_lbvh* l, const float* d_tris, uint
             RT_CHECK_LAUNCH(ctx, "k_build_small");
             return RT_OK;
         };
-        const rt_status s = n <= kSmallThreads       ? small(k_build_small<1>, 1)
-                            : n <= 2 * kSmallThreads ? small(k_build_small<2>, 2)
-                                                     : small(k_build_small<4>, 4);
+        const rt_status s = n <= kSmallThreads ? small(k_build_small<1>, 1) : small(k_build_small<2>, 2);
         if (s != RT_OK) return s;
         l->built_keys = true;
         l->compact_valid = false;

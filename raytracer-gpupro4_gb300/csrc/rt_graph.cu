@@ -2,8 +2,8 @@
 //
 // RayTracerCS::Render with dynamic = 1 (RayTracerCS.cpp:258-295) issues the
 // rebuild (2*depth + 46 dispatches in the reference) and the trace stages
-// every frame.  Here the 10 build kernels, the two work-counter resets and
-// the two trace kernels of one frame are captured once and replayed with a
+// every frame.  Here the build kernels (eleven, or one for a small soup) and
+// the trace kernels of one frame are captured once and replayed with a
 // single cudaGraphLaunch, so the frame carries no per-kernel launch cost.
 // Every kernel parameter (soup pointer, camera, output buffers) is fixed at
 // capture time; a caller that streams new vertex data writes it into the

@@ -1412,9 +1412,7 @@ struct BatchTraceArgs {
     uint32_t S, width, height, tiles_per_scene, grab, order;
 };
 
-// The shadow-ray list of a batched trace.  (A separate kernel argument:
-// with these fields inside BatchTraceArgs the compiler gives k_batch_trace
-// 78 registers instead of 64, and its primary rays run 20 % slower.)
+// The shadow-ray list of a batched trace.
 struct BatchListArgs {
     uint32_t* lists;
     uint32_t cap;

@@ -1,4 +1,4 @@
-"""The one-block build (k_build_small) at the edges of its warps, of its three
+"""The one-block build (k_build_small) at the edges of its warps, of its two
 sizes and of its range, against the oracle: codes, permutation, reachable nodes
 and sorted triangles bit for bit, and a trace through the records made from
 it.  Beside soups: runs of equal codes (leaves above and below the size that a
