@@ -278,7 +278,7 @@ __global__ void __launch_bounds__(kPtThreads, BLOCKS) k_pathtrace(
                 continue;
             }
         }
-        w.round(tr, kPtSteps, stack);
+        w.round<kPathPoolMin>(tr, kPtSteps, stack);
     }
 }
 
@@ -446,7 +446,7 @@ __global__ void __launch_bounds__(kPtThreads, kPtBlocks) k_pathtrace_adjoint(
                 continue;
             }
         }
-        w.round(tr, kPtSteps, stack);
+        w.round<kPathPoolMin>(tr, kPtSteps, stack);
     }
     // emitter gradient: warp reduction, one atomic per warp and channel
     for (int c = 0; c < 3; ++c) {

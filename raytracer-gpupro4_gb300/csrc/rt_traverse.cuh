@@ -593,8 +593,11 @@ __device__ __forceinline__ void mark_records(const TreeRef& tr) {
 
 constexpr uint32_t kGeneral = 8u;    // Walk::sgn: the records do not serve this ray
 constexpr uint32_t kInfinite = 16u;  // some 1 / d is infinite: the reference's NaN-sensitive min / max
-constexpr uint32_t kPoolMin = 3u;    // a leaf of more triangles makes the warp pool its leaves
-constexpr uint32_t kCheckMin = 4u;   // leaves above this many triangles are tested only after their exact box
+// A leaf of more triangles makes the warp pool its leaves: 2 for rays that stay
+// neighbours (330 k triangles at 720p 561 us a frame with 3, 538 with 2; 1: the same), 3
+// for paths (24.2 ms with 3, 24.5 with 2, 25.9 with 1).
+constexpr uint32_t kPoolMin = 2u;
+constexpr uint32_t kPathPoolMin = 3u;
 
 struct Walk {
     f3 o, d, k, n;  // k = E / d, n = (G - o) / d
@@ -757,6 +760,7 @@ struct Walk {
     // faster), then the leaves: pooled where one is large, else a triangle of
     // each lane at a time.  All 32 lanes call.
     // Returns whether the lane tested a leaf.
+    template <uint32_t POOL_MIN = kPoolMin>
     __device__ __forceinline__ bool round(const TreeRef& tr, int steps, uint2* stack, bool any_hit = false) {
         constexpr uint32_t kFull = 0xffffffffu;
         for (int s = 0; s < steps; ++s) {
@@ -801,15 +805,15 @@ struct Walk {
             }
         }
         bool inside = false;
-        // a leaf of many triangles: its exact box, with the bound of now, first
-        if (cnt > kCheckMin) {
-            const uint32_t h = (leaf & kBigLeaf) ? leaf & 0x3ffffffu : __ldg(tr.leaf_of + tr.tri_base + (leaf & 0x1ffffffu));
-            inside = leaf_entered(tr, h);
+        // a leaf of 32 or more triangles: its exact box, with the bound of now, first (of
+        // 5 or more, 330 k triangles at 720p took 9 us a frame longer)
+        if (leaf & kBigLeaf) {
+            inside = leaf_entered(tr, leaf & 0x3ffffffu);
             if (!inside) cnt = 0u;
         }
         tests += cnt;
         at_leaf += cnt;
-        if (__reduce_max_sync(kFull, cnt) > kPoolMin) {
+        if (__reduce_max_sync(kFull, cnt) > POOL_MIN) {
             pooled(tr, leaf, pos, cnt, inside);
         } else {
             while (__any_sync(kFull, cnt != 0u)) {

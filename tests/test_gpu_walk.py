@@ -1,7 +1,7 @@
 """The walk over the trace records (Walk in rt_traverse.cuh) where it can go
 wrong, against the oracle: leaves around the sizes that change their form
-(a word holds fewer than 32 triangles; more than 3 are pooled, more than 4
-box-tested first), trees of one leaf and of flat scenes, rays that the
+(a word holds fewer than 32 triangles, larger leaves are box-tested first; more
+than 2 or 3 are pooled), trees of one leaf and of flat scenes, rays that the
 records do not serve (a zero direction component, an origin far outside, very
 short and very long directions), ray counts around a warp and around the
 number up to which a ray gets a warp, and any-hit rays around the hand-over
