@@ -397,43 +397,71 @@ __global__ void __launch_bounds__(kPtThreads, kPtBlocks) k_pathtrace_adjoint(
     bool drained = false;
     for (;;) {
         if (shade_now(w.have, L.live, drained)) {
-            bool fresh = false;
+            bool fresh = false, ending = false;
+            const bool missed = w.b.id < 0;
             if (L.live && !w.have) {
-                const bool missed = w.b.id < 0;
                 if (!missed) seg[ns++] = w.b.id;
                 if (!missed && L.s != P.bounces) {
                     bounce(L, soup, w.b.id, w.b.t, tr.compact ? 1u : w.b.leaf);
                     fresh = true;
                 } else {
-                    const float4 g4 = __ldg(dimage + (size_t)L.j * P.cam.width + L.i);
-                    const float gimg[3] = {g4.x, g4.y, g4.z};
-                    // weight of sample n in the progressive mean after the call
-                    float wn = 1.0f / (float)(L.n + 1);
-                    for (uint32_t m = L.n + 1; m < P.n0 + P.spp; ++m) wn *= (float)m / (float)(m + 1);
-                    float beta[kMaxSeg][3];
-                    beta[0][0] = beta[0][1] = beta[0][2] = 1.0f;
-                    for (int q = 0; q + 1 < ns; ++q)
-                        for (int c = 0; c < 3; ++c) beta[q + 1][c] = beta[q][c] * __ldg(albedo + 3 * (size_t)seg[q] + c);
-                    float G[3] = {0.0f, 0.0f, 0.0f};
-                    if (missed)
-                        for (int c = 0; c < 3; ++c) G[c] = P.sky[c];
-                    for (int q = ns - 1; q >= 0; --q) {
-                        const float* al = albedo + 3 * (size_t)seg[q];
-                        const float* le = emission + 3 * (size_t)seg[q];
-                        const float l0 = __ldg(le), l1 = __ldg(le + 1), l2 = __ldg(le + 2);
-                        const bool emitter = (l0 != 0.0f) || (l1 != 0.0f) || (l2 != 0.0f);
-                        const float lev[3] = {l0, l1, l2};
-                        for (int c = 0; c < 3; ++c) {
-                            const float gw = gimg[c] * wn;
-                            const float da = gw * beta[q][c] * G[c];
-                            if (da != 0.0f) atomicAdd(dalbedo + 3 * (size_t)seg[q] + c, da);
-                            if (emitter) dle[c] += gw * beta[q][c];
-                            G[c] = lev[c] + __ldg(al + c) * G[c];
-                        }
-                    }
-                    ns = 0;
-                    L.live = false;
+                    ending = true;
                 }
+            }
+            const int rounds = __reduce_max_sync(kFull, ending ? ns : 0);
+            float gw[3] = {0.0f, 0.0f, 0.0f}, beta[kMaxSeg][3], G[3] = {0.0f, 0.0f, 0.0f};
+            if (ending) {
+                const float4 g4 = __ldg(dimage + (size_t)L.j * P.cam.width + L.i);
+                // weight of sample n in the progressive mean after the call
+                float wn = 1.0f / (float)(L.n + 1);
+                for (uint32_t m = L.n + 1; m < P.n0 + P.spp; ++m) wn *= (float)m / (float)(m + 1);
+                gw[0] = g4.x * wn;
+                gw[1] = g4.y * wn;
+                gw[2] = g4.z * wn;
+                beta[0][0] = beta[0][1] = beta[0][2] = 1.0f;
+                for (int q = 0; q + 1 < ns; ++q)
+                    for (int c = 0; c < 3; ++c) beta[q + 1][c] = beta[q][c] * __ldg(albedo + 3 * (size_t)seg[q] + c);
+                if (missed)
+                    for (int c = 0; c < 3; ++c) G[c] = P.sky[c];
+            }
+            for (int q = rounds - 1; q >= 0; --q) {
+                const bool on = ending && q < ns;
+                float da[3] = {0.0f, 0.0f, 0.0f};
+                if (on) {
+                    const float* al = albedo + 3 * (size_t)seg[q];
+                    const float* le = emission + 3 * (size_t)seg[q];
+                    const float l0 = __ldg(le), l1 = __ldg(le + 1), l2 = __ldg(le + 2);
+                    const bool emitter = (l0 != 0.0f) || (l1 != 0.0f) || (l2 != 0.0f);
+                    const float lev[3] = {l0, l1, l2};
+                    for (int c = 0; c < 3; ++c) {
+                        da[c] = gw[c] * beta[q][c] * G[c];
+                        if (emitter) dle[c] += gw[c] * beta[q][c];
+                        G[c] = lev[c] + __ldg(al + c) * G[c];
+                    }
+                }
+                // the lanes that hit one triangle are summed first: fewer roundings than an
+                // atomic each
+                uint32_t peers = __match_any_sync(kFull, on ? seg[q] : -1 - (int)(threadIdx.x & 31));
+                const uint32_t lane = threadIdx.x & 31;
+                const bool leader = (peers & ((1u << lane) - 1u)) == 0u;
+                uint32_t rank = __popc(peers & ((1u << lane) - 1u));
+                peers &= 0xfffffffeu << lane;
+                while (__any_sync(kFull, peers != 0u)) {
+                    const int next = __ffs(peers);  // the next lane of the triangle that still holds a sum
+                    for (int c = 0; c < 3; ++c) {
+                        const float t = __shfl_sync(kFull, da[c], next ? next - 1 : (int)lane);
+                        if (next) da[c] += t;
+                    }
+                    peers &= __ballot_sync(kFull, (rank & 1u) == 0u);
+                    rank >>= 1;
+                }
+                if (on && leader)
+                    for (int c = 0; c < 3; ++c)
+                        if (da[c] != 0.0f) atomicAdd(dalbedo + 3 * (size_t)seg[q] + c, da[c]);
+            }
+            if (ending) {
+                ns = 0;
+                L.live = false;
             }
             if (grab_path(L, P, first, per, work, total, drained)) {
                 ns = 0;
@@ -448,11 +476,19 @@ __global__ void __launch_bounds__(kPtThreads, kPtBlocks) k_pathtrace_adjoint(
         }
         w.round<kPathPoolMin>(tr, kPtSteps, stack);
     }
-    // emitter gradient: warp reduction, one atomic per warp and channel
+    // emitter gradient: warp and block sums, one atomic per block and channel (one per
+    // warp rounds as often again as there are warps in a block)
+    __shared__ float s_dle[kPtThreads / 32][3];
     for (int c = 0; c < 3; ++c) {
         float v = dle[c];
         for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(kFull, v, off);
-        if ((threadIdx.x & 31) == 0 && v != 0.0f) atomicAdd(demission + c, v);
+        if ((threadIdx.x & 31) == 0) s_dle[threadIdx.x >> 5][c] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x < 3) {
+        float v = 0.0f;
+        for (int q = 0; q < kPtThreads / 32; ++q) v += s_dle[q][threadIdx.x];
+        if (v != 0.0f) atomicAdd(demission + threadIdx.x, v);
     }
 }
 
