@@ -103,6 +103,11 @@ constexpr uint32_t kBigLeaf = 1u << 30;
 __host__ __device__ inline uint32_t leaf_word(uint32_t h, uint32_t pos, uint32_t cnt) {
     return (cnt < 32u && pos < (1u << 25)) ? kLeafFlag | (cnt << 25) | pos : kLeafFlag | kBigLeaf | h;
 }
+// Whether [pos, pos + cnt) lies within n triangles.  An imported tree's fields are
+// the caller's: read unsigned, a negative one is too large, and no sum can wrap.
+__host__ __device__ inline bool leaf_in_range(uint32_t pos, uint32_t cnt, uint32_t n) {
+    return cnt <= n && pos <= n - cnt;
+}
 
 // Tiling constants
 constexpr int kSortThreads = 256;

@@ -798,11 +798,11 @@ struct Walk {
                 pos = (uint32_t)z.y;
                 cnt = (uint32_t)(z.x >> 3);
             }
-            pos += tr.tri_base;
-            if (pos + cnt > tr.n) {
+            if (!leaf_in_range(pos, cnt, tr.n - tr.tri_base)) {
                 atomicOr(tr.err, RT_DEVERR_BOUNDS);
-                cnt = 0u;
+                pos = cnt = 0u;
             }
+            pos += tr.tri_base;
         }
         bool inside = false;
         // a leaf of 32 or more triangles: its exact box, with the bound of now, first (of

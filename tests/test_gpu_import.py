@@ -1,0 +1,65 @@
+"""Imported trees (rt_lbvh_import_host), which the caller made: leaves whose triangle range
+is not the tree's end in the bounds error and are not read."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+N, DEPTH = 5000, 14
+
+
+def made(oracle_mod, seed=31):
+    from rtgpu import scenes
+    tris = scenes.random_soup(N, seed, 0.02, 0.1)
+    nodes, ids, _, _ = oracle_mod.lbvh_build(tris, DEPTH)
+    return tris, nodes, ids
+
+
+def reached_leaves(nodes):
+    out, todo = [], [1]
+    while todo:
+        h = todo.pop()
+        if int(nodes[h]["prim_count"]) & 4:
+            out.append(h)
+        else:
+            todo += [2 * h, 2 * h + 1]
+    return out
+
+
+def rays_at(tris, n, seed=3):
+    rng = np.random.default_rng(seed)
+    o = rng.uniform(-1, 2, (n, 3)).astype(np.float32)
+    d = tris[rng.integers(0, len(tris), n), :3] - o
+    d = (d / np.linalg.norm(d, axis=1, keepdims=True)).astype(np.float32)
+    return o, d, np.full(n, 1e16, np.float32), np.full(n, -1, np.int32)
+
+
+@pytest.mark.parametrize("pos,count", [(-1, 40), (-1, 2), (-2**31, 31), (N - 39, 40), (N, 1), (0, -1), (100, -2**20), (7, N)])
+def test_leaf_out_of_range(gpu_ctx, oracle_mod, pos, count):
+    import torch
+    from rtgpu import scenes
+    from rtgpu._lib import RtError
+    from rtgpu.api import LBVH, RayTracer, rays_tensor
+    from test_gpu_whitted import materials
+    tris, nodes, ids = made(oracle_mod)
+    for h in reached_leaves(nodes):
+        nodes[h]["prim_pos"] = pos
+        nodes[h]["prim_count"] = (count << 3) | (int(nodes[h]["prim_count"]) & 7)
+    lb = LBVH(gpu_ctx, N, DEPTH).Import(nodes, ids, tris)
+    rt = RayTracer(gpu_ctx)
+    cam = scenes.look_at((1.7, 1.2, 1.5), (0.5, 0.5, 0.5), vfov_deg=45.0, width=160, height=96)
+    rays = rays_tensor(*rays_at(tris, 20000), "cuda")
+    colour = torch.full((N, 3), 0.5, device="cuda")
+
+    def refused(call):
+        call()
+        with pytest.raises(RtError, match="bounds check"):
+            gpu_ctx.check()
+
+    refused(lambda: rt.primary(lb, cam))
+    refused(lambda: rt.rays(lb, rays))
+    refused(lambda: rt.rays_from(lb, rays, None))
+    refused(lambda: rt.rays(lb, rays, any_hit=True))
+    refused(lambda: rt.whitted(lb, cam, (0.5, 3.0, 0.4), materials(), bounces=0))
+    refused(lambda: rt.pathtrace(lb, colour, colour, cam, 2, 1, 5))
+    gpu_ctx.check()  # the error was cleared
