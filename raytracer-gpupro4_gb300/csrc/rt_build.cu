@@ -2201,9 +2201,13 @@ __global__ void __launch_bounds__(256) k_compact(const rt_node* __restrict__ nod
 
 // Pre-gather for imported trees (ids + soup uploaded from the host).
 __global__ void k_gather_tris(const uint32_t* __restrict__ ids, const float* __restrict__ tris, uint32_t n,
-                              float4* __restrict__ sorted_tris) {
+                              float4* __restrict__ sorted_tris, uint32_t* err) {
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-        const uint32_t id = ids[k];
+        uint32_t id = ids[k];
+        if (id >= n) {  // the caller's list: a hit's id indexes the soup
+            atomicOr(err, RT_DEVERR_BOUNDS);
+            id = 0;
+        }
         const float* tp = tris + 9 * (size_t)id;
         sorted_tris[3 * (size_t)k + 0] = make_float4(tp[0], tp[1], tp[2], __int_as_float((int)id));
         sorted_tris[3 * (size_t)k + 1] = make_float4(tp[3], tp[4], tp[5], 0.0f);
@@ -2450,7 +2454,7 @@ extern "C" rt_status rt_lbvh_import_host(rt_ctx* ctx, rt_lbvh* l, const rt_node*
     RT_CHECK_CUDA(ctx, cudaMemcpyAsync(l->ids, h_ids, 4 * (size_t)n, cudaMemcpyHostToDevice, st));
     RT_CHECK_CUDA(ctx, cudaMemcpyAsync(l->tris, h_tris, sizeof(float) * 9 * (size_t)n, cudaMemcpyHostToDevice, st));
     const uint32_t blocks = std::max(1u, std::min(ceil_div(n, 256), (uint32_t)ctx->num_sms * 8));
-    k_gather_tris<<<blocks, 256, 0, st>>>(l->ids, l->tris, n, l->sorted_tris);
+    k_gather_tris<<<blocks, 256, 0, st>>>(l->ids, l->tris, n, l->sorted_tris, ctx->d_err);
     RT_CHECK_LAUNCH(ctx, "k_gather_tris");
     RT_CHECK_CUDA(ctx, cudaMemsetAsync(l->counters + 8, 0, sizeof(uint32_t), st));  // no emission tiles: these are its records
     k_trace_nodes<<<ceil_div(l->num_nodes, 256), 256, 0, st>>>(l->nodes, l->num_nodes, l->tnodes, l->leaf_of, n);

@@ -1,5 +1,5 @@
 """Imported trees (rt_lbvh_import_host), which the caller made: leaves whose triangle range
-is not the tree's end in the bounds error and are not read."""
+is not the tree's and ids past the soup end in the bounds error and are not read."""
 import numpy as np
 import pytest
 
@@ -63,3 +63,20 @@ def test_leaf_out_of_range(gpu_ctx, oracle_mod, pos, count):
     refused(lambda: rt.whitted(lb, cam, (0.5, 3.0, 0.4), materials(), bounces=0))
     refused(lambda: rt.pathtrace(lb, colour, colour, cam, 2, 1, 5))
     gpu_ctx.check()  # the error was cleared
+
+
+@pytest.mark.parametrize("bad", [N, 2**31, 2**32 - 1])
+def test_id_out_of_range(gpu_ctx, oracle_mod, bad):
+    from rtgpu._lib import RtError
+    from rtgpu.api import LBVH, RayTracer, hits_to_numpy, rays_tensor
+    tris, nodes, ids = made(oracle_mod)
+    wrong = ids.copy()
+    wrong[[0, 77, N - 1]] = bad
+    lb = LBVH(gpu_ctx, N, DEPTH).Import(nodes, wrong, tris)
+    with pytest.raises(RtError, match="bounds check"):
+        gpu_ctx.check()
+    hits = hits_to_numpy(RayTracer(gpu_ctx).rays(lb, rays_tensor(*rays_at(tris, 20000), "cuda")))
+    gpu_ctx.check()
+    assert hits["id"].min() >= -1 and hits["id"].max() < N
+    lb.Import(nodes, ids, tris)  # the handle still serves
+    gpu_ctx.check()
