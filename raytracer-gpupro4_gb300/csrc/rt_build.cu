@@ -2215,31 +2215,43 @@ __global__ void k_gather_tris(const uint32_t* __restrict__ ids, const float* __r
     }
 }
 
+// Whether slot h of an imported tree lies below a leaf.
+__device__ __forceinline__ bool below_leaf(const rt_node* nodes, uint32_t h) {
+    for (int k = 31 - __clz(h); k > 0; --k)
+        if (__ldg(&nodes[h >> k].prim_count) & 4) return true;
+    return false;
+}
+
+// leaf_of of an imported tree (all zero before), and whether two of its leaves begin
+// at one triangle: a caller's tree may list a triangle in several leaves.
+__global__ void __launch_bounds__(256) k_import_leaves(const rt_node* __restrict__ nodes, uint32_t num_nodes,
+                                                       uint32_t* leaf_of, uint32_t n, uint32_t* shared) {
+    const uint32_t h = blockIdx.x * blockDim.x + threadIdx.x;
+    if (h == 0 || h >= num_nodes) return;
+    const int pc = nodes[h].prim_count, pos = nodes[h].prim_pos;
+    if (!(pc & 4) || (pc >> 3) == 0 || pos < 0 || (uint32_t)pos >= n || below_leaf(nodes, h)) return;
+    if (atomicExch(leaf_of + pos, h) != 0u) *shared = 1u;
+}
+
 // Trace records of an imported tree: every internal node that the root reaches.
 __global__ void __launch_bounds__(256) k_trace_nodes(const rt_node* __restrict__ nodes, uint32_t num_nodes,
-                                                     TraceNode* __restrict__ tnodes, uint32_t* __restrict__ leaf_of,
-                                                     uint32_t n) {
+                                                     TraceNode* __restrict__ tnodes, const uint32_t* shared) {
     const uint32_t h = blockIdx.x * blockDim.x + threadIdx.x;
     if (h >= num_nodes) return;
+    const bool by_slot = *shared != 0u;
     const rt_node root = nodes[1];
-    const float4 g = trace_grid(root.min, root.max);
-    const int pc = nodes[h].prim_count, pos = nodes[h].prim_pos;
+    float4 g = trace_grid(root.min, root.max);
+    const int pc = nodes[h].prim_count;
     if (h == 0) {
-        if (!tnodes) return;
-        store_trace_grid(tnodes, g, (root.prim_count & 4) ? leaf_word(1u, (uint32_t)root.prim_pos,
-                                                                      (uint32_t)(root.prim_count >> 3)) : 0u);
+        store_trace_grid(tnodes, g, by_slot);
         return;
     }
-    for (int k = 31 - __clz(h); k > 0; --k)
-        if (__ldg(&nodes[h >> k].prim_count) & 4) return;  // below a leaf
-    if (pc & 4) {
-        if (pos >= 0 && (uint32_t)pos < n) leaf_of[pos] = h;
-        return;
-    }
-    if (!tnodes || 2 * h + 1 >= num_nodes) return;  // no records, or a corrupt tree
+    if ((pc & 4) || 2 * h + 1 >= num_nodes || below_leaf(nodes, h)) return;  // (or a corrupt tree)
     const rt_node l = nodes[2 * h], r = nodes[2 * h + 1];
-    auto word = [](const rt_node& c, uint32_t ch) {
-        return (c.prim_count & 4) ? leaf_word(ch, (uint32_t)c.prim_pos, (uint32_t)(c.prim_count >> 3)) : 0u;
+    auto word = [by_slot](const rt_node& c, uint32_t ch) {
+        return !(c.prim_count & 4) ? 0u
+               : by_slot           ? slot_word(ch)
+                                   : leaf_word(ch, (uint32_t)c.prim_pos, (uint32_t)(c.prim_count >> 3));
     };
     const int field = pc & 3;  // one axis past the split axis
     store_trace_node(tnodes, h, l.min, l.max, r.min, r.max, word(l, 2 * h), word(r, 2 * h + 1),
@@ -2456,9 +2468,15 @@ extern "C" rt_status rt_lbvh_import_host(rt_ctx* ctx, rt_lbvh* l, const rt_node*
     const uint32_t blocks = std::max(1u, std::min(ceil_div(n, 256), (uint32_t)ctx->num_sms * 8));
     k_gather_tris<<<blocks, 256, 0, st>>>(l->ids, l->tris, n, l->sorted_tris, ctx->d_err);
     RT_CHECK_LAUNCH(ctx, "k_gather_tris");
-    RT_CHECK_CUDA(ctx, cudaMemsetAsync(l->counters + 8, 0, sizeof(uint32_t), st));  // no emission tiles: these are its records
-    k_trace_nodes<<<ceil_div(l->num_nodes, 256), 256, 0, st>>>(l->nodes, l->num_nodes, l->tnodes, l->leaf_of, n);
-    RT_CHECK_LAUNCH(ctx, "k_trace_nodes");
+    // no emission tiles (these are its records); no leaves at one position so far
+    RT_CHECK_CUDA(ctx, cudaMemsetAsync(l->counters + 8, 0, 2 * sizeof(uint32_t), st));
+    RT_CHECK_CUDA(ctx, cudaMemsetAsync(l->leaf_of, 0, 4 * (size_t)n, st));
+    k_import_leaves<<<ceil_div(l->num_nodes, 256), 256, 0, st>>>(l->nodes, l->num_nodes, l->leaf_of, n, l->counters + 9);
+    RT_CHECK_LAUNCH(ctx, "k_import_leaves");
+    if (l->tnodes) {
+        k_trace_nodes<<<ceil_div(l->num_nodes, 256), 256, 0, st>>>(l->nodes, l->num_nodes, l->tnodes, l->counters + 9);
+        RT_CHECK_LAUNCH(ctx, "k_trace_nodes");
+    }
     l->n = n;
     l->src_tris = l->tris;
     l->built_keys = false;

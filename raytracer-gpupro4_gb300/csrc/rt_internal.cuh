@@ -83,25 +83,22 @@ struct SceneInfo {
 //     node's split axis.
 //   word[child]  0: an internal node; a leaf is the word that the walk keeps
 //     for it (leaf_word).
-// Slot 0 holds the tree's grid and, as word[1], a root that is a leaf.
+// Slot 0 holds the tree's grid; the sign of E says that every leaf is named by its
+// slot (slot_word), because two leaves of an imported tree begin at one triangle.
 struct __align__(32) TraceNode {
     uint32_t box[2][3];
     uint32_t word[2];
 };
-struct __align__(32) TraceGrid {
-    float G[3], E;
-    uint32_t pad[3];
-    uint32_t root_word;
-};
-static_assert(sizeof(TraceNode) == 32 && sizeof(TraceGrid) == 32 && offsetof(TraceGrid, root_word) == 28, "");
+static_assert(sizeof(TraceNode) == 32, "");
 
 // A leaf in one word: bit 31; then, for fewer than 32 triangles that begin
 // below position 2^25, the count in bits 29 .. 25 and the position (its heap
 // slot is leaf_of[position]); else bit 30 and the heap slot.
 constexpr uint32_t kLeafFlag = 1u << 31;
 constexpr uint32_t kBigLeaf = 1u << 30;
+__host__ __device__ inline uint32_t slot_word(uint32_t h) { return kLeafFlag | kBigLeaf | h; }
 __host__ __device__ inline uint32_t leaf_word(uint32_t h, uint32_t pos, uint32_t cnt) {
-    return (cnt < 32u && pos < (1u << 25)) ? kLeafFlag | (cnt << 25) | pos : kLeafFlag | kBigLeaf | h;
+    return (cnt < 32u && pos < (1u << 25)) ? kLeafFlag | (cnt << 25) | pos : slot_word(h);
 }
 // Whether [pos, pos + cnt) lies within n triangles.  An imported tree's fields are
 // the caller's: read unsigned, a negative one is too large, and no sum can wrap.
@@ -183,7 +180,7 @@ struct rt_lbvh {
     // build scratch
     SceneInfo* scene = nullptr;
     float* partials = nullptr;       // bounds partial reductions, 8 floats per block
-    uint32_t* counters = nullptr;    // [0] bounds ticket, [1..4] sort tile tickets, [7] records valid, [8] emission tiles
+    uint32_t* counters = nullptr;    // [0] bounds ticket, [1..4] sort tile tickets, [7] records valid, [8] emission tiles, [9] see k_import_leaves
     uint32_t* hist = nullptr;        // 4 x 256 digit histograms
     uint32_t* lookback = nullptr;    // 4 passes x sort tiles x 256 status words
     uint32_t* scan = nullptr;        // emission tiles x 4 (fwd agg, bwd agg, fwd prefix, bwd suffix)

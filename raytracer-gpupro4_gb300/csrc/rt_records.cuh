@@ -17,10 +17,8 @@ __device__ __forceinline__ float4 trace_grid(const float mn[3], const float mx[3
     const float E = fmaxf(fsub(mx[0], mn[0]), fmaxf(fsub(mx[1], mn[1]), fsub(mx[2], mn[2])));
     return make_float4(fsub(mn[0], E), fsub(mn[1], E), fsub(mn[2], E), E);
 }
-__device__ __forceinline__ void store_trace_grid(TraceNode* tnodes, float4 g, uint32_t root_word) {
-    float4* p = reinterpret_cast<float4*>(tnodes);
-    p[0] = g;
-    p[1] = make_float4(0.f, 0.f, 0.f, __uint_as_float(root_word));
+__device__ __forceinline__ void store_trace_grid(TraceNode* tnodes, float4 g, bool by_slot) {
+    *reinterpret_cast<float4*>(tnodes) = make_float4(g.x, g.y, g.z, by_slot ? -fabsf(g.w) : fabsf(g.w));
 }
 
 // One axis of a child's box; rE = 1 / E.  The lowest bit of the grid step is
@@ -132,8 +130,7 @@ __device__ __forceinline__ void make_records(const Records& R, uint32_t block) {
             const float mn[3] = {r0.x, r0.y, r0.z}, mx[3] = {r0.w, r1.x, r1.y};
             const float4 g = trace_grid(mn, mx);
             if (a == 0u) {  // the tree's first leaf
-                const int pc = __float_as_int(r1.z);
-                store_trace_grid(tnodes, g, (pc & 4) ? leaf_word(1u, (uint32_t)__float_as_int(r1.w), (uint32_t)(pc >> 3)) : 0u);
+                store_trace_grid(tnodes, g, false);
                 continue;
             }
             const int da = 31 - __clz(a), db = 31 - __clz(b), dm = min(da, db);

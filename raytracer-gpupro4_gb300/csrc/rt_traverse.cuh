@@ -593,6 +593,7 @@ __device__ __forceinline__ void mark_records(const TreeRef& tr) {
 
 constexpr uint32_t kGeneral = 8u;    // Walk::sgn: the records do not serve this ray
 constexpr uint32_t kInfinite = 16u;  // some 1 / d is infinite: the reference's NaN-sensitive min / max
+constexpr uint32_t kBySlot = 32u;    // the tree's leaves are named by their slots
 // A leaf of more triangles makes the warp pool its leaves: 2 for rays that stay
 // neighbours (330 k triangles at 720p 561 us a frame with 3, 538 with 2; 1: the same), 3
 // for paths (24.2 ms with 3, 24.5 with 2, 25.9 with 1).
@@ -667,6 +668,8 @@ struct Walk {
         if (!(r.tmax > 0.0f)) return;
         float4 g = make_float4(0.f, 0.f, 0.f, 0.f);  // G, E
         if (tr.tnodes) g = __ldg(reinterpret_cast<const float4*>(tr.tnodes));
+        if (!tr.tnodes || signbit(g.w)) sgn |= kBySlot;
+        g.w = fabsf(g.w);
         k = mk3(fmul(g.w, r.inv.x), fmul(g.w, r.inv.y), fmul(g.w, r.inv.z));
         const f3 q = mk3(fsub(g.x, o.x), fsub(g.y, o.y), fsub(g.z, o.z));
         n = mk3(fmul(q.x, r.inv.x), fmul(q.y, r.inv.y), fmul(q.z, r.inv.z));
@@ -720,9 +723,10 @@ struct Walk {
         cur = (hl || hr) ? (go_right ? r_ : l) : 0u;
     }
 
-    static __device__ __forceinline__ uint32_t heap_item(uint32_t h, const NodeBox& nb) {
+    __device__ __forceinline__ uint32_t heap_item(uint32_t h, const NodeBox& nb) const {
         const int pc = __float_as_int(nb.b.z);
-        return (pc & 4) ? leaf_word(h, (uint32_t)__float_as_int(nb.b.w), (uint32_t)(pc >> 3)) : h;
+        if (!(pc & 4)) return h;
+        return (sgn & kBySlot) ? slot_word(h) : leaf_word(h, (uint32_t)__float_as_int(nb.b.w), (uint32_t)(pc >> 3));
     }
 
     // One expansion of a lane that holds an internal node: cur = the near

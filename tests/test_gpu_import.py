@@ -1,5 +1,7 @@
 """Imported trees (rt_lbvh_import_host), which the caller made: leaves whose triangle range
-is not the tree's and ids past the soup end in the bounds error and are not read."""
+is not the tree's and ids past the soup end in the bounds error and are not read; trees
+that no build makes, with empty leaves and with several leaves over the same triangles,
+are traced as the oracle traces them, to the bit."""
 import numpy as np
 import pytest
 
@@ -80,3 +82,58 @@ def test_id_out_of_range(gpu_ctx, oracle_mod, bad):
     assert hits["id"].min() >= -1 and hits["id"].max() < N
     lb.Import(nodes, ids, tris)  # the handle still serves
     gpu_ctx.check()
+
+
+def split_leaves(nodes, depth, how):
+    """Every leaf becomes an internal node: of it and an empty leaf at the same position (right
+    or left), or of two leaves over the same triangles, one per half of the box."""
+    out = np.zeros(1 << depth, nodes.dtype)
+    out[:len(nodes)] = nodes
+    for h in reached_leaves(nodes):
+        leaf = nodes[h]
+        l, r = leaf.copy(), leaf.copy()
+        if how == "shared":
+            a = int(np.argmax(leaf["max"] - leaf["min"]))
+            l["max"][a] = r["min"][a] = np.float32(0.5) * (leaf["min"][a] + leaf["max"][a])
+        else:
+            e = r if how == "empty right" else l
+            e["prim_count"] = 4
+            e["max"] = e["min"]
+        out[2 * h], out[2 * h + 1] = l, r
+        out[h]["prim_count"] = (int(leaf["prim_count"]) >> 3) << 3 | 1
+    return out
+
+
+@pytest.mark.parametrize("how", ["empty right", "empty left", "shared"])
+def test_leaves_at_one_position(gpu_ctx, oracle_mod, how):
+    import torch
+    from rtgpu import scenes
+    from rtgpu.api import LBVH, RayTracer, hits_to_numpy, rays_tensor
+    tris, nodes, ids = made(oracle_mod)
+    depth = DEPTH + 1
+    nodes = split_leaves(nodes, depth, how)
+    lb = LBVH(gpu_ctx, N, depth).Import(nodes, ids, tris)
+    rt = RayTracer(gpu_ctx)
+    o, d, tmax, excl = rays_at(tris, 40000)
+    d[::5, 2] = 0.0  # rays that the trace records do not serve
+    ref = oracle_mod.trace(nodes, depth, ids, tris, oracle_mod.rays_array(o, d, tmax, excl))
+    rays = rays_tensor(o, d, tmax, excl, "cuda")
+    got, leaves = rt.rays_from(lb, rays, None)
+    again, _ = rt.rays_from(lb, rays, leaves)
+    few = rt.rays(lb, rays[:5000].contiguous())
+    cam = scenes.look_at((1.7, 1.2, 1.5), (0.5, 0.5, 0.5), vfov_deg=45.0, width=161, height=97)
+    prim = rt.primary(lb, cam)
+    gpu_ctx.check()
+    same = lambda a, b: np.array_equal(hits_to_numpy(a).view(np.int32), b.view(np.int32))  # noqa: E731
+    assert same(got, ref) and same(again, ref) and same(few, ref[:5000])
+    assert same(prim, oracle_mod.trace(nodes, depth, ids, tris, oracle_mod.primary_rays(cam)))
+    hit = ref["id"] >= 0
+    slots = leaves.cpu().numpy()
+    assert hit.mean() > 0.2 and (slots[~hit] == 1).all()
+    hit &= slots != 1  # a handed-over ray reports the root
+    assert hit.mean() > 0.2
+    pc, pos = nodes["prim_count"][slots[hit]], nodes["prim_pos"][slots[hit]]
+    where = np.empty(N, np.int64)
+    where[ids] = np.arange(N)
+    at = where[ref["id"][hit]]
+    assert (pc & 4).all() and ((pos <= at) & (at < pos + (pc >> 3))).all()
