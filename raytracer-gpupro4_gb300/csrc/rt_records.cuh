@@ -12,9 +12,11 @@
 
 namespace rt {
 
-// The grid of a tree with bounds [mn, mx]: G, E.
+// The grid of a tree with bounds [mn, mx]: G, E.  Bounds that are NaN make E NaN, and
+// every ray reads the heap.
 __device__ __forceinline__ float4 trace_grid(const float mn[3], const float mx[3]) {
-    const float E = fmaxf(fsub(mx[0], mn[0]), fmaxf(fsub(mx[1], mn[1]), fsub(mx[2], mn[2])));
+    const float d[3] = {fsub(mx[0], mn[0]), fsub(mx[1], mn[1]), fsub(mx[2], mn[2])};
+    const float E = isnan(d[0]) || isnan(d[1]) || isnan(d[2]) ? NAN : fmaxf(d[0], fmaxf(d[1], d[2]));
     return make_float4(fsub(mn[0], E), fsub(mn[1], E), fsub(mn[2], E), E);
 }
 __device__ __forceinline__ void store_trace_grid(TraceNode* tnodes, float4 g, bool by_slot) {
@@ -22,13 +24,16 @@ __device__ __forceinline__ void store_trace_grid(TraceNode* tnodes, float4 g, bo
 }
 
 // One axis of a child's box; rE = 1 / E.  The lowest bit of the grid step is
-// `bit` when bit >= 0.
+// `bit` when bit >= 0.  box_enter ignores an axis whose bounds are both NaN (a soup with
+// NaN vertices), so such an axis gets the whole line; and it takes the bounds in
+// either order (an imported tree may hold them so).
 __device__ __forceinline__ uint32_t trace_box_word(float mn, float mx, float G, float E, float rE, int bit) {
+    if (!isfinite(mn) || !isfinite(mx)) return 0x7e808000u | (uint32_t)max(bit, 0);  // half-extent 2^126
     const float q = fminf(fmaxf(rintf((0.5f * mn + 0.5f * mx - (G + E)) * rE * 32768.0f), 0.0f), 32767.0f);
     uint32_t step = (uint32_t)q;
     if (bit >= 0) step = (step & ~1u) | (uint32_t)bit;
     const float X = fmaf(E, 1.0f + (float)step * (1.0f / 32768.0f), G);  // the centre, within 2^-24 |X|
-    float e = fmaxf(__fsub_ru(mx, X), __fsub_ru(X, mn));
+    float e = fmaxf(fmaxf(__fsub_ru(mx, X), __fsub_ru(X, mn)), fmaxf(__fsub_ru(X, mx), __fsub_ru(mn, X)));
     e = __fadd_ru(e, __fmaf_ru(fabsf(X), 1.0f / 4194304.0f, E * (1.0f / 65536.0f)));  // 256 u E, and X's own error
     e = __fmul_ru(__fmul_ru(e, rE), 1.0f + 1.0f / 1048576.0f);                        // rE and k are rounded
     const uint32_t bits = __float_as_uint(fmaxf(e, 0.0f));
