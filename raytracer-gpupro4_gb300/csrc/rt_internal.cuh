@@ -124,6 +124,7 @@ constexpr uint32_t kMaxTris = (1u << 29);
 // default budget of box + triangle tests a lane spends on one ray before it
 // hands the ray to the warp-per-ray kernel.
 constexpr uint32_t kSpillCap = 1u << 20;
+constexpr int kTeamClaims = 38;  // ctx->d_words: claims of the block-per-ray passes (two)
 constexpr int kDoubtCount = 36;  // ctx->d_words: length of the any-hit rays' second list, its claim counter
 constexpr uint32_t kDefaultHeavyTeam = 2u;
 constexpr uint32_t kDefaultTraceBudget = 384;

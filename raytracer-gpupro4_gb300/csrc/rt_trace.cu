@@ -567,19 +567,23 @@ __global__ void __launch_bounds__(kTraceThreads) k_trace_rays(TreeRef tr, const 
     }
 }
 
-// Second pass over the rays the first pass handed over: one ray per warp
-// (trace_wide), rebuilt from its list entry exactly as the first pass made
-// it, and its result written where the first pass would have written it.
+// Second pass over the rays the first pass handed over: one ray per warp, rebuilt
+// from its list entry exactly as the first pass made it, and its result written where
+// the first pass would have written it.  A closest hit is the one that the first pass
+// would have found (trace_ordered), so the budget, and which tests count towards it,
+// change no hit.
 struct HeavyArgs {
     TreeRef tr;
     const float* soup;
     rt_camera cam;
     float lx, ly, lz;
     const rt_hit* prim;   // primary hits (shadow / mirror entries)
+    const uint32_t* prim_leaves;  // and their leaves, where the shading rays start (nullable: the root)
     rt_hit* hits;         // primary or generic-ray output
     uint8_t* vis;
     rt_hit* mirror;
     const rt_ray* rays;
+    const uint32_t* starts;  // start nodes of generic rays (nullable)
     int any_hit;          // generic rays
     uint32_t* leaves;     // primary / generic-ray leaf output (nullable)
     uint32_t* mirror_leaves;
@@ -590,6 +594,7 @@ struct HeavyArgs {
     const uint32_t* count;
     uint32_t cap;
     uint32_t* work;
+    uint32_t* work2;      // claims of the block-per-ray pass
 };
 
 // The closest hit the first pass had found when it handed the ray over.
@@ -610,47 +615,68 @@ __device__ __forceinline__ Hit no_hit() {
     return h;
 }
 
+__device__ __forceinline__ bool heavy_any_hit(const HeavyArgs& a, uint32_t entry) {
+    const uint32_t kind = entry >> 30;
+    return kind == kHeavyShadow || (kind == kHeavyRay && a.any_hit);
+}
+
+__device__ __forceinline__ ShadeRays heavy_shade_rays(const HeavyArgs& a, uint32_t idx, bool mirror, uint32_t* start) {
+    const uint32_t i = idx % a.cam.width, j = idx / a.cam.width;
+    const int4 ph = __ldg(reinterpret_cast<const int4*>(a.prim + idx));
+    *start = shade_start(a.prim_leaves, ph, true, idx);
+    return shade_rays(a.soup, a.cam, a.lx, a.ly, a.lz, ph, true, i, j, mirror);
+}
+
+// A closest-hit entry, by a warp.
+__device__ __forceinline__ void heavy_closest(const HeavyArgs& a, uint32_t entry) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t kind = entry >> 30, idx = entry & kHeavyIndexMask;
+    RayState r;
+    uint32_t start = 1u;
+    rt_hit* out = a.hits + idx;
+    uint32_t* leaves = a.leaves;
+    if (kind == kHeavyPrimary) {
+        r = make_ray(mk3(a.cam.eye[0], a.cam.eye[1], a.cam.eye[2]), primary_dir(a.cam, idx % a.cam.width, idx / a.cam.width),
+                     1e16f, -1);
+    } else if (kind == kHeavyRay) {
+        r = load_ray(a.rays, idx, true);
+        if (a.starts) start = __ldg(a.starts + idx);
+    } else {
+        r = heavy_shade_rays(a, idx, true, &start).mirror;
+        out = a.mirror + idx;
+        leaves = a.mirror_leaves;
+    }
+    const Hit h = trace_ordered(r, a.tr, a.wide_cap, hit_so_far(out), start);
+    if (lane == 0) {
+        store_hit(out, h);
+        if (leaves) leaves[idx] = 1u;  // the root: a valid restart node
+    }
+    if (kind == kHeavyPrimary && a.sl.lists) {
+        const int4 ph = make_int4(h.id, __float_as_int(h.u), __float_as_int(h.v), __float_as_int(h.t));
+        shade_setup_pixel(a.sl, a.cam, ph, lane == 0, idx % a.cam.width, idx / a.cam.width, idx, 1u);
+    }
+}
+
 __global__ void __launch_bounds__(kTraceThreads, 7) k_trace_heavy(HeavyArgs a) {
     grid_dep_wait();
     const uint32_t n = min(*a.count, a.cap);
     const int lane = threadIdx.x & 31;
     for (uint32_t e = next_tile(a.work); e < n; e = next_tile(a.work)) {
         const uint32_t entry = __ldg(a.list + e);
-        const uint32_t kind = entry >> 30, idx = entry & kHeavyIndexMask;
-        if (kind == kHeavyPrimary) {
-            const uint32_t i = idx % a.cam.width, j = idx / a.cam.width;
-            const RayState r = make_ray(mk3(a.cam.eye[0], a.cam.eye[1], a.cam.eye[2]), primary_dir(a.cam, i, j),
-                                        1e16f, -1);
-            const Hit h = trace_wide(r, a.tr, false, a.wide_cap, hit_so_far(a.hits + idx));
-            if (lane == 0) {
-                store_hit(a.hits + idx, h);
-                if (a.leaves) a.leaves[idx] = 1u;  // the root: a valid restart node
-            }
-            if (a.sl.lists) {
-                const int4 ph = make_int4(h.id, __float_as_int(h.u), __float_as_int(h.v), __float_as_int(h.t));
-                shade_setup_pixel(a.sl, a.cam, ph, lane == 0, i, j, idx, 1u);
-            }
-        } else if (kind == kHeavyRay) {
-            const RayState r = load_ray(a.rays, idx, true);
-            const Hit h = trace_wide(r, a.tr, a.any_hit != 0, a.wide_cap, a.any_hit ? no_hit() : hit_so_far(a.hits + idx));
+        const uint32_t idx = entry & kHeavyIndexMask;
+        if (!heavy_any_hit(a, entry)) {
+            heavy_closest(a, entry);
+        } else if ((entry >> 30) == kHeavyRay) {
+            const Hit h = trace_wide(load_ray(a.rays, idx, true), a.tr, a.wide_cap);
             if (lane == 0) {
                 store_hit(a.hits + idx, h);
                 if (a.leaves) a.leaves[idx] = 1u;
             }
         } else {
-            const uint32_t i = idx % a.cam.width, j = idx / a.cam.width;
-            const int4 ph = __ldg(reinterpret_cast<const int4*>(a.prim + idx));
-            const ShadeRays s = shade_rays(a.soup, a.cam, a.lx, a.ly, a.lz, ph, true, i, j, kind == kHeavyMirror);
-            if (kind == kHeavyShadow) {
-                const Hit h = trace_wide(s.shadow, a.tr, true, a.wide_cap, no_hit());
-                if (lane == 0) a.vis[idx] = vis_code(s.has, s.cast, h.id >= 0);
-            } else {
-                const Hit h = trace_wide(s.mirror, a.tr, false, a.wide_cap, hit_so_far(a.mirror + idx));
-                if (lane == 0) {
-                    store_hit(a.mirror + idx, h);
-                    if (a.mirror_leaves) a.mirror_leaves[idx] = 1u;
-                }
-            }
+            uint32_t start;
+            const ShadeRays s = heavy_shade_rays(a, idx, false, &start);
+            const Hit h = trace_wide(s.shadow, a.tr, a.wide_cap);
+            if (lane == 0) a.vis[idx] = vis_code(s.has, s.cast, h.id >= 0);
         }
     }
 }
@@ -666,65 +692,48 @@ __global__ void __launch_bounds__(kTraceThreads) k_rays_wide(TreeRef tr, const r
     grid_dep_wait();
     const uint32_t k = blockIdx.x * kWideWarps + (threadIdx.x >> 5);
     if (k >= n) return;
-    const Hit h = trace_wide(load_ray(rays, k, true), tr, false, cap, no_hit());
+    const Hit h = trace_ordered(load_ray(rays, k, true), tr, cap, no_hit(), 1u);
     if ((threadIdx.x & 31) == 0) store_hit(hits + k, h);
 }
 
-// k_trace_heavy with a block per ray (traverse_team): for the handed-over
+// k_trace_heavy with a block per any-hit ray (traverse_team): for the handed-over
 // shading rays, a few hundred grazing rays whose walks run for thousands of
-// tests, where a warp per ray leaves the GPU waiting on the longest few.
+// tests, where a warp per ray leaves the GPU waiting on the longest few.  The closest-hit
+// entries come first, a warp each (a block each: 3 us of 1,400 for the mirror rays of
+// 2.1 M triangles at 1080p).
 __global__ void __launch_bounds__(kTeamThreads) k_trace_heavy_team(HeavyArgs a) {
     grid_dep_wait();
     __shared__ TeamShared ts;
     __shared__ uint32_t s_e;
     const uint32_t n = min(*a.count, a.cap);
     const int tid = threadIdx.x;
+    for (uint32_t e = next_tile(a.work); e < n; e = next_tile(a.work)) {
+        const uint32_t entry = __ldg(a.list + e);
+        if (!heavy_any_hit(a, entry)) heavy_closest(a, entry);
+    }
     for (;;) {
-        if (tid == 0) s_e = atomicAdd(a.work, 1u);
+        __syncthreads();
+        if (tid == 0) s_e = atomicAdd(a.work2, 1u);
         __syncthreads();
         const uint32_t e = s_e;
-        __syncthreads();
         if (e >= n) break;
         const uint32_t entry = __ldg(a.list + e);
-        const uint32_t kind = entry >> 30, idx = entry & kHeavyIndexMask;
-        if (kind == kHeavyPrimary) {
-            const uint32_t i = idx % a.cam.width, j = idx / a.cam.width;
-            const RayState r = make_ray(mk3(a.cam.eye[0], a.cam.eye[1], a.cam.eye[2]), primary_dir(a.cam, i, j),
-                                        1e16f, -1);
-            const Hit h = trace_team(r, a.tr, false, a.team_cap, ts, hit_so_far(a.hits + idx));
-            if (tid == 0) {
-                store_hit(a.hits + idx, h);
-                if (a.leaves) a.leaves[idx] = 1u;  // the root: a valid restart node
-            }
-            if (a.sl.lists && tid < 32) {
-                const int4 ph = make_int4(h.id, __float_as_int(h.u), __float_as_int(h.v), __float_as_int(h.t));
-                shade_setup_pixel(a.sl, a.cam, ph, tid == 0, i, j, idx, 1u);
-            }
-        } else if (kind == kHeavyRay) {
-            const RayState r = load_ray(a.rays, idx, true);
-            const Hit h = trace_team(r, a.tr, a.any_hit != 0, a.team_cap, ts, a.any_hit ? no_hit() : hit_so_far(a.hits + idx));
+        const uint32_t idx = entry & kHeavyIndexMask;
+        if (!heavy_any_hit(a, entry)) continue;
+        if ((entry >> 30) == kHeavyRay) {
+            const Hit h = trace_team(load_ray(a.rays, idx, true), a.tr, a.team_cap, ts);
             if (tid == 0) {
                 store_hit(a.hits + idx, h);
                 if (a.leaves) a.leaves[idx] = 1u;
             }
         } else {
-            const uint32_t i = idx % a.cam.width, j = idx / a.cam.width;
-            const int4 ph = __ldg(reinterpret_cast<const int4*>(a.prim + idx));
-            const ShadeRays sr = shade_rays(a.soup, a.cam, a.lx, a.ly, a.lz, ph, true, i, j, kind == kHeavyMirror);
-            if (kind == kHeavyShadow) {
-                const Hit h = trace_team(sr.shadow, a.tr, true, a.team_cap, ts, no_hit());
-                if (tid == 0) a.vis[idx] = vis_code(sr.has, sr.cast, h.id >= 0);
-            } else {
-                const Hit h = trace_team(sr.mirror, a.tr, false, a.team_cap, ts, hit_so_far(a.mirror + idx));
-                if (tid == 0) {
-                    store_hit(a.mirror + idx, h);
-                    if (a.mirror_leaves) a.mirror_leaves[idx] = 1u;
-                }
-            }
+            uint32_t start;
+            const ShadeRays s = heavy_shade_rays(a, idx, false, &start);
+            const Hit h = trace_team(s.shadow, a.tr, a.team_cap, ts);
+            if (tid == 0) a.vis[idx] = vis_code(s.has, s.cast, h.id >= 0);
         }
     }
 }
-
 
 uint32_t pixel_tiles(const rt_camera* cam) {
     return (uint32_t)(((cam->width + 7) / 8) * ((cam->height + 3) / 4));
@@ -796,15 +805,20 @@ Spill spill_of(rt_ctx* ctx, bool enabled, int kind) {
     return sp;
 }
 
+// Claims of the block-per-ray pass, one word for the shading rays and one for the others.
+uint32_t* team_claims(const rt_ctx* ctx, const Spill& sp) {
+    return ctx->d_words + kTeamClaims + (sp.work == ctx->d_spill_count + 2 ? 1 : 0);
+}
+
 // A trace call zeroes its counters (words of ctx->d_words) in one small
 // kernel launched before its first pass, k_order_begin where the call has a
 // tile order to advance, k_reset_words otherwise: one graph node instead of a
 // memset per counter, and a programmatic edge to the pass.
 uint64_t word_bit(const rt_ctx* ctx, const uint32_t* p) { return 1ull << (uint32_t)(p - ctx->d_words); }
 
-// The list length and the warp-per-ray pass's claim counter.
+// The list length and the second pass's claim counters.
 uint64_t spill_reset_bits(const rt_ctx* ctx, const Spill& sp) {
-    return sp.count ? word_bit(ctx, sp.count) | word_bit(ctx, sp.work) : 0ull;
+    return sp.count ? word_bit(ctx, sp.count) | word_bit(ctx, sp.work) | word_bit(ctx, team_claims(ctx, sp)) : 0ull;
 }
 
 // The counters of the compacted shading-ray pass.
@@ -847,8 +861,9 @@ rt_status launch_heavy(rt_ctx* ctx, const Spill& sp, HeavyArgs a, int kind) {
     a.count = sp.count;
     a.cap = kSpillCap;
     a.work = sp.work;
+    a.work2 = team_claims(ctx, sp);
     if ((ctx->heavy_team >> kind) & 1u) {
-        const size_t smem = team_smem_bytes(a.team_cap);
+        const size_t smem = std::max(team_smem_bytes(a.team_cap), wide_smem_bytes(a.wide_cap));
         if (smem > 48u * 1024u)
             RT_CHECK_CUDA(ctx, cudaFuncSetAttribute(k_trace_heavy_team, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                     (int)smem));
@@ -1028,6 +1043,7 @@ rt_status trace_shadow_mirror(rt_ctx* ctx, const rt_lbvh* l, const rt_camera* ca
     a.ly = light[1];
     a.lz = light[2];
     a.prim = d_primary;
+    a.prim_leaves = d_prim_leaves;
     a.vis = d_vis;
     a.mirror = d_mirror;
     a.mirror_leaves = d_mirror_leaves;
@@ -1079,6 +1095,7 @@ rt_status trace_rays(rt_ctx* ctx, const rt_lbvh* l, const rt_ray* d_rays, uint32
     RT_CHECK_LAUNCH(ctx, walk ? (any_hit ? "k_trace_doubt" : "k_walk_rays") : "k_trace_rays");
     HeavyArgs a = heavy_args(ctx, l);
     a.rays = d_rays;
+    a.starts = d_starts;
     a.any_hit = any_hit;
     a.hits = d_hits;
     a.leaves = d_leaves;

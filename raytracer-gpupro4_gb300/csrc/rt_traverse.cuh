@@ -970,7 +970,7 @@ __device__ __forceinline__ uint64_t warp_min_u64(uint64_t v) {
     return v;
 }
 
-// One ray traced by the whole warp (every lane passes the same ray): a
+// One any-hit ray traced by the whole warp (every lane passes the same ray): a
 // frontier walk.  The warp keeps a stack of the internal nodes the ray enters
 // (as the slot of their children pair, with the entry distance) and a queue
 // of leaves in shared memory.  Each step
@@ -978,11 +978,9 @@ __device__ __forceinline__ uint64_t warp_min_u64(uint64_t v) {
 // at the scale of a warp, which bounds the stack by 32 entries per level),
 // tests both children of each, and pushes the entered internal children and
 // queues the entered leaves.  When the queue holds 64 or more triangles, or
-// the stack is empty, the queued leaves still in front of the closest hit are
-// tested 32 (leaf, triangle) pairs at a time and the warp minimum of the
-// (t, id) keys becomes the shared bound.  The closest hit under the tie rule
-// does not depend on the order of the tests, so the hit equals traverse()'s.
-// For any_hit the walk stops at the first accepted hit.
+// the stack is empty, the queued leaves are tested 32 (leaf, triangle) pairs at a
+// time, and the walk stops at the first accepted hit.  Whether there is one does
+// not depend on the order of the tests.
 // Each step pops the newest 32 entries, so every group of pushed children
 // leaves at most 32 entries behind, one group per tree level: a tree of
 // depth D needs at most 32 (D + 1) entries, and wide_stack_entries adds one
@@ -996,30 +994,44 @@ __host__ __device__ constexpr uint32_t wide_stack_entries(uint32_t depth) {
     return (depth + 2u) * 32u < (uint32_t)kWideStackMax ? (depth + 2u) * 32u : (uint32_t)kWideStackMax;
 }
 
-// Dynamic shared memory of a block running traverse_wide with `cap` stack
-// entries per warp: stack nodes and entry distances, then the leaf queue.
+// Dynamic shared memory of a block running traverse_wide or traverse_ordered with
+// `cap` stack entries per warp: stack nodes and entry distances, then the leaves
+// (and pending hits) of each warp.
+constexpr int kWideScratch = 2432;
+static_assert(kWideQueue * 16 <= kWideScratch, "");
 __host__ __device__ constexpr size_t wide_smem_bytes(uint32_t cap) {
-    return (size_t)kWideWarps * (cap * 8u + kWideQueue * 16u);
+    return (size_t)kWideWarps * (cap * 8u + kWideScratch);
+}
+struct WideSmem {
+    uint32_t* snode;   // [cap]
+    float* st0;        // [cap]
+    uint8_t* scratch;  // [kWideScratch]
+};
+__device__ __forceinline__ WideSmem wide_smem(uint32_t cap) {
+    extern __shared__ uint4 wide_dyn[];
+    uint8_t* base8 = reinterpret_cast<uint8_t*>(wide_dyn);
+    const int wib = threadIdx.x >> 5;
+    WideSmem w;
+    w.snode = reinterpret_cast<uint32_t*>(base8) + (size_t)wib * cap;
+    w.st0 = reinterpret_cast<float*>(base8 + (size_t)kWideWarps * cap * 4u) + (size_t)wib * cap;
+    w.scratch = base8 + (size_t)kWideWarps * cap * 8u + (size_t)wib * kWideScratch;
+    return w;
 }
 
 template <bool EXACT>
-__device__ __forceinline__ Hit traverse_wide(const RayState& r, const TreeRef& tr_, bool any_hit, uint32_t cap, Hit known) {
+__device__ __forceinline__ Hit traverse_wide(const RayState& r, const TreeRef& tr_, uint32_t cap) {
     constexpr uint32_t kFull = 0xffffffffu;
-    extern __shared__ uint4 wide_dyn[];
-    uint8_t* base8 = reinterpret_cast<uint8_t*>(wide_dyn);
     const int lane = threadIdx.x & 31;
-    const int wib = threadIdx.x >> 5;
-    uint32_t* snode = reinterpret_cast<uint32_t*>(base8) + (size_t)wib * cap;
-    float* st0 = reinterpret_cast<float*>(base8 + (size_t)kWideWarps * cap * 4u) + (size_t)wib * cap;
-    uint8_t* qbase = base8 + (size_t)kWideWarps * cap * 8u;
-    int32_t* qpos = reinterpret_cast<int32_t*>(qbase) + wib * kWideQueue;
-    int32_t* qcnt = reinterpret_cast<int32_t*>(qbase) + (kWideWarps + wib) * kWideQueue;
-    float* qt0 = reinterpret_cast<float*>(qbase) + (2 * kWideWarps + wib) * kWideQueue;
-    uint32_t* qincl = reinterpret_cast<uint32_t*>(qbase) + (3 * kWideWarps + wib) * kWideQueue;
-    // known: an accepted hit found before (id < 0: none)
+    const WideSmem ws = wide_smem(cap);
+    uint32_t* snode = ws.snode;
+    float* st0 = ws.st0;
+    int32_t* qpos = reinterpret_cast<int32_t*>(ws.scratch);
+    int32_t* qcnt = qpos + kWideQueue;
+    float* qt0 = reinterpret_cast<float*>(qcnt + kWideQueue);
+    uint32_t* qincl = reinterpret_cast<uint32_t*>(qt0 + kWideQueue);
     const uint64_t init = hit_key(r.tmax, 0);
-    uint64_t best = known.id >= 0 ? hit_key(known.t, known.id) : init;  // uniform across the warp
-    float bu = known.u, bv = known.v, bt = known.t;
+    uint64_t best = init;  // uniform across the warp
+    float bu = -1.0f, bv = -1.0f, bt = 0.0f;
     int size = 0, nq = 0, qtris = 0;  // uniform
     bool stop = false;
     // root
@@ -1075,7 +1087,7 @@ __device__ __forceinline__ Hit traverse_wide(const RayState& r, const TreeRef& t
             for (uint32_t base = 0; base < total; base += 32 * kWidePairs) {
                 uint64_t key = ~0ull;
                 float kt = 0.0f, ku = 0.0f, kv = 0.0f;
-                bool first = false;  // any_hit: a hit among the first 32 pairs ends the walk there
+                bool first = false;  // a hit among the first 32 pairs ends the walk there
                 float4 va[kWidePairs], vb[kWidePairs], vc[kWidePairs];
 #pragma unroll
                 for (int q = 0; q < kWidePairs; ++q) {
@@ -1096,7 +1108,7 @@ __device__ __forceinline__ Hit traverse_wide(const RayState& r, const TreeRef& t
                 for (int q = 0; q < kWidePairs; ++q) {
                     const int id = __float_as_int(va[q].w);
                     float u, v, t;
-                    if (any_hit && q > 0) first = __any_sync(kFull, key != ~0ull);
+                    if (q > 0) first = __any_sync(kFull, key != ~0ull);
                     if (!first && id != r.exclude && tri_test(r, va[q], vb[q], vc[q], &u, &v, &t)) {
                         const uint64_t k = hit_key(t, id);
                         if (k < best && k < key) {
@@ -1114,12 +1126,12 @@ __device__ __forceinline__ Hit traverse_wide(const RayState& r, const TreeRef& t
                 bt = __shfl_sync(kFull, kt, w);
                 bu = __shfl_sync(kFull, ku, w);
                 bv = __shfl_sync(kFull, kv, w);
-                if (any_hit) break;
+                break;
             }
             nq = 0;
             qtris = 0;
             __syncwarp();
-            if (any_hit && best < init) stop = true;
+            if (best < init) stop = true;
             continue;
         }
         // pop up to 32 internal nodes from the top
@@ -1214,14 +1226,323 @@ __device__ __forceinline__ Hit traverse_wide(const RayState& r, const TreeRef& t
     return h;
 }
 
-// One ray traced by a whole block of kTeamThreads threads: traverse_wide's
+// One closest-hit ray traced by the whole warp (every lane passes the same ray), with
+// traverse()'s hit whatever the scene.  Where surfaces coincide, the rounded entry
+// distance of a leaf's box can lie above the distance of a hit inside it, and whether the
+// leaf is still entered depends on the hits found before it, so on the order.  The
+// frontier therefore stays in traverse()'s order, the next node on top:
+//   - a step pops up to 32 entries, the next ones in that order, and puts back in
+//     their places the internal children that are entered and, for the leaves among
+//     the children, a hit (the leaf's entry distance and its closest triangle);
+//   - a hit that comes to the top has everything before it behind it: it is accepted
+//     exactly when traverse() would enter its leaf and accept its triangle;
+//   - an entry is dropped early only for what holds at its turn in any case: the
+//     bound so far, and, below a pending hit, the larger of that hit's two
+//     distances (its leaf is entered and the bound is the hit's distance at most, or
+//     is not and the bound is below the leaf's entry distance).
+// Entry distances grow from parent to child, so one test at a leaf's turn says what
+// the tests at its ancestors' turns would have; where a NaN breaks that (a ray along a
+// face of a box), and when the pending hits or the stack overflow, one lane walks the
+// ray alone.  `known`: the hit of a walk in the same order that was broken off (id
+// < 0: none); going over its part again with that bound changes nothing.  `start`: as in
+// traverse().
+constexpr uint32_t kEntryHit = 1u << 31, kEntryLeaf = 1u << 30, kEntryRight = 1u << 29;
+constexpr int kOrderedLeaves = 64, kOrderedHits = 32;
+static_assert(kOrderedLeaves * 28 + kOrderedHits * 20 <= kWideScratch, "");
+
+__device__ __forceinline__ uint32_t ordered_entry(const TreeRef& tr, const RayState& r, uint32_t node, float prim_count,
+                                                  float prim_pos) {
+    const int pc = __float_as_int(prim_count), field = pc & 3;
+    if (pc & 4) return kEntryLeaf | node;
+    return child_pair(tr, node, prim_pos) | (((r.sgn >> (field == 0 ? 2 : field - 1)) & 1u) ? kEntryRight : 0u);
+}
+
+// traverse() by one lane of the warp (out of line: rare).
+template <bool EXACT>
+__device__ __noinline__ Hit traverse_alone(const RayState& r, const TreeRef& tr, uint32_t start) {
+    Hit h = traverse<EXACT, false>(r, (threadIdx.x & 31) == 0, tr, false, nullptr, nullptr, nullptr, nullptr, start);
+    h.id = __shfl_sync(0xffffffffu, h.id, 0);
+    h.u = __shfl_sync(0xffffffffu, h.u, 0);
+    h.v = __shfl_sync(0xffffffffu, h.v, 0);
+    h.t = __shfl_sync(0xffffffffu, h.t, 0);
+    return h;
+}
+
+template <bool EXACT>
+__device__ __forceinline__ Hit traverse_ordered(const RayState& r, const TreeRef& tr_, uint32_t cap, const Hit& known,
+                                                uint32_t start) {
+    constexpr uint32_t kFull = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const uint32_t lt = (1u << lane) - 1u;
+    const WideSmem ws = wide_smem(cap);
+    uint32_t* snode = ws.snode;
+    float* st0 = ws.st0;
+    // the leaves of a step, in order
+    uint64_t* qbest = reinterpret_cast<uint64_t*>(ws.scratch);
+    uint64_t* pkey = qbest + kOrderedLeaves;  // the pending hits
+    float* qt = reinterpret_cast<float*>(pkey + kOrderedHits);
+    float* qu = qt + kOrderedLeaves;
+    float* qv = qu + kOrderedLeaves;
+    int32_t* qpos = reinterpret_cast<int32_t*>(qv + kOrderedLeaves);
+    uint32_t* qincl = reinterpret_cast<uint32_t*>(qpos + kOrderedLeaves);
+    float* pt = reinterpret_cast<float*>(qincl + kOrderedLeaves);
+    float* pu = pt + kOrderedHits;
+    float* pv = pu + kOrderedHits;
+    const uint64_t init = hit_key(r.tmax, 0);
+    uint64_t best = known.id >= 0 ? hit_key(known.t, known.id) : init;  // uniform across the warp
+    float bu = known.u, bv = known.v, bt = known.t;
+    uint32_t used = 0u;  // pending hits in use (uniform)
+    int size = 0;        // uniform
+    bool alone = false;
+    __syncwarp();
+    if (r.tmax > 0.0f) {  // the siblings of start's ancestors, the deepest on top, then start
+        uint32_t first = 1u;
+        if (start > 1u && !tr_.compact) {
+            if (start < tr_.num_nodes) first = start;
+            else if (lane == 0) atomicOr(tr_.err, RT_DEVERR_BOUNDS);
+        }
+        const int D = 31 - __clz(first);  // <= kMaxDepth < 32
+        uint32_t e = 0u;
+        float t0 = 0.0f;
+        if (lane <= D) {
+            const uint32_t node = lane < D ? (first >> (D - 1 - lane)) ^ 1u : first;
+            const NodeBox nb = load_node(tr_.nodes, node);
+            if (box_enter<EXACT>(r, nb.a.x, nb.a.y, nb.a.z, nb.a.w, nb.b.x, nb.b.y, key_t(best), &t0))
+                e = ordered_entry(tr_, r, node, nb.b.z, nb.b.w);
+        }
+        const uint32_t m = __ballot_sync(kFull, e != 0u);
+        if (e) {
+            snode[__popc(m & lt)] = e;
+            st0[__popc(m & lt)] = t0;
+        }
+        size = __popc(m);
+        alone = EXACT && __any_sync(kFull, e && isnan(t0));
+        __syncwarp();
+    }
+    while (size > 0 && !alone) {
+        {  // a hit on top: its turn
+            const uint32_t e = snode[size - 1];
+            if (e & kEntryHit) {
+                const uint32_t q = e & ~kEntryHit;
+                const uint64_t key = pkey[q];
+                if (key < best && !(st0[size - 1] > key_t(best))) {
+                    best = key;
+                    bt = pt[q];
+                    bu = pu[q];
+                    bv = pv[q];
+                }
+                used &= ~(1u << q);
+                --size;
+                continue;
+            }
+        }
+        // the next entries in order, lane 0 the first
+        const int k = min(32, size);
+        uint32_t e = 0u;
+        float t0 = 0.0f;
+        if (lane < k) {
+            e = snode[size - 1 - lane];
+            t0 = st0[size - 1 - lane];
+        }
+        float bound = key_t(best);  // at this entry's turn it is this at most
+        const bool is_hit = (e & kEntryHit) != 0u;
+        const uint32_t q_hit = e & ~kEntryHit;
+        float hit_t = 0.0f;
+        if (__any_sync(kFull, is_hit)) {
+            if (is_hit) hit_t = key_t(pkey[q_hit]);
+            float m = is_hit ? fmaxf(hit_t, t0) : INFINITY;
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+                const float y = __shfl_up_sync(kFull, m, off);
+                if (lane >= off) m = fminf(m, y);
+            }
+            m = __shfl_up_sync(kFull, m, 1);
+            if (lane > 0) bound = fminf(bound, m);
+        }
+        size -= k;
+        __syncwarp();
+        // what takes the entry's place: up to two entries, or leaves to test
+        uint32_t o[2] = {0u, 0u};
+        float ot[2] = {0.0f, 0.0f};
+        int pos[2] = {0, 0}, cnt[2] = {0, 0};
+        bool nan = false;
+        if (e && !(t0 > bound)) {
+            if (is_hit) {
+                if (!(hit_t > bound)) {
+                    o[0] = e;
+                    ot[0] = t0;
+                }
+            } else if (e & kEntryLeaf) {
+                const float4 b = load_node(tr_.nodes, e & ~kEntryLeaf).b;
+                pos[0] = __float_as_int(b.w);
+                cnt[0] = __float_as_int(b.z) >> 3;
+                ot[0] = t0;
+            } else {
+                const uint32_t c0 = e & ~kEntryRight;
+                if (c0 + 1 >= tr_.num_nodes) {
+                    atomicOr(tr_.err, RT_DEVERR_BOUNDS);
+                } else {
+                    const float4* p = reinterpret_cast<const float4*>(tr_.nodes + c0);
+                    const float4 l0 = __ldg(p), l1 = __ldg(p + 1), r0 = __ldg(p + 2), r1 = __ldg(p + 3);
+                    float tl, tr;
+                    const bool hl = box_enter<EXACT>(r, l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, bound, &tl);
+                    const bool hr = box_enter<EXACT>(r, r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, bound, &tr);
+                    nan = EXACT && ((hl && isnan(tl)) || (hr && isnan(tr)));
+                    const bool right = (e & kEntryRight) != 0u;
+#pragma unroll
+                    for (int c = 0; c < 2; ++c) {  // the near child, then the far one
+                        const bool rc = right == (c == 0);
+                        if (!(rc ? hr : hl)) continue;
+                        const float pc = rc ? r1.z : l1.z, pp = rc ? r1.w : l1.w;
+                        ot[c] = rc ? tr : tl;
+                        if (__float_as_int(pc) & 4) {
+                            pos[c] = __float_as_int(pp);
+                            cnt[c] = __float_as_int(pc) >> 3;
+                        } else {
+                            o[c] = ordered_entry(tr_, r, c0 + (rc ? 1u : 0u), pc, pp);
+                        }
+                    }
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < 2; ++c)
+                if (!leaf_in_range((uint32_t)pos[c], (uint32_t)cnt[c], tr_.n)) {
+                    atomicOr(tr_.err, RT_DEVERR_BOUNDS);
+                    cnt[c] = 0;
+                }
+        }
+        if (EXACT && __any_sync(kFull, nan)) {
+            alone = true;
+            break;
+        }
+        {  // the hits that were dropped
+            const uint32_t gone = __ballot_sync(kFull, is_hit && o[0] == 0u);
+            if (gone) used &= ~__reduce_or_sync(kFull, (gone >> lane) & 1u ? 1u << q_hit : 0u);
+        }
+        // the leaves, 32 (leaf, triangle) pairs at a time
+        const uint32_t la = __ballot_sync(kFull, cnt[0] > 0), lb = __ballot_sync(kFull, cnt[1] > 0);
+        if (la | lb) {
+            const int q0 = __popc(la & lt) + __popc(lb & lt), q1 = q0 + (cnt[0] > 0 ? 1 : 0);
+            const int nq = __popc(la) + __popc(lb);
+            uint32_t incl = (uint32_t)(cnt[0] + cnt[1]);
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+                const uint32_t y = __shfl_up_sync(kFull, incl, off);
+                if (lane >= off) incl += y;
+            }
+            const uint32_t total = __shfl_sync(kFull, incl, 31);
+            if (cnt[0] > 0) {
+                qpos[q0] = pos[0];
+                qincl[q0] = incl - (uint32_t)cnt[1];
+                qbest[q0] = ~0ull;
+            }
+            if (cnt[1] > 0) {
+                qpos[q1] = pos[1];
+                qincl[q1] = incl;
+                qbest[q1] = ~0ull;
+            }
+            __syncwarp();
+            for (uint32_t base = 0; base < total; base += 32 * kWidePairs) {
+                float4 va[kWidePairs], vb[kWidePairs], vc[kWidePairs];
+                int leaf[kWidePairs];
+#pragma unroll
+                for (int q = 0; q < kWidePairs; ++q) {
+                    const uint32_t p = min(base + 32u * q + lane, total - 1u);  // past the end: the last pair again
+                    int lo = 0, hi = nq - 1;  // the first leaf with inclusive prefix > p
+                    while (lo < hi) {
+                        const int mid = (lo + hi) >> 1;
+                        if (qincl[mid] > p) hi = mid; else lo = mid + 1;
+                    }
+                    leaf[q] = lo;
+                    const float4* tp = tr_.tris + 3 * (size_t)(qpos[lo] + (int)(p - (lo > 0 ? qincl[lo - 1] : 0u)));
+                    va[q] = __ldg(tp);
+                    vb[q] = __ldg(tp + 1);
+                    vc[q] = __ldg(tp + 2);
+                }
+#pragma unroll
+                for (int q = 0; q < kWidePairs; ++q) {
+                    const int id = __float_as_int(va[q].w);
+                    float u = 0.0f, v = 0.0f, t = 0.0f;
+                    uint64_t key = ~0ull;
+                    if (id != r.exclude && tri_test(r, va[q], vb[q], vc[q], &u, &v, &t)) key = hit_key(t, id);
+                    const bool in = key < best;
+                    if (!__any_sync(kFull, in)) continue;
+                    if (in) atomicMin(reinterpret_cast<unsigned long long*>(qbest + leaf[q]), (unsigned long long)key);
+                    __syncwarp();
+                    if (in && qbest[leaf[q]] == key) {
+                        qt[leaf[q]] = t;
+                        qu[leaf[q]] = u;
+                        qv[leaf[q]] = v;
+                    }
+                    __syncwarp();
+                }
+            }
+            const uint64_t k0 = cnt[0] > 0 ? qbest[q0] : ~0ull, k1 = cnt[1] > 0 ? qbest[q1] : ~0ull;
+            const bool h0 = k0 != ~0ull && !(key_t(k0) > bound), h1 = k1 != ~0ull && !(key_t(k1) > bound);
+            const uint32_t ha = __ballot_sync(kFull, h0), hb = __ballot_sync(kFull, h1);
+            if (ha | hb) {
+                if (__popc(ha) + __popc(hb) > kOrderedHits - __popc(used)) {
+                    alone = true;
+                    break;
+                }
+                const uint32_t rank = (uint32_t)(__popc(ha & lt) + __popc(hb & lt));
+                uint32_t mine = 0u;
+                auto put = [&](int q, uint64_t key, uint32_t nth) {
+                    const uint32_t slot = __fns(~used, 0, (int)nth + 1);
+                    pkey[slot] = key;
+                    pt[slot] = qt[q];
+                    pu[slot] = qu[q];
+                    pv[slot] = qv[q];
+                    mine |= 1u << slot;
+                    return kEntryHit | slot;
+                };
+                if (h0) o[0] = put(q0, k0, rank);
+                if (h1) o[1] = put(q1, k1, rank + (h0 ? 1u : 0u));
+                used |= __reduce_or_sync(kFull, mine);
+            }
+        }
+        const uint32_t oa = __ballot_sync(kFull, o[0] != 0u), ob = __ballot_sync(kFull, o[1] != 0u);
+        const int total = __popc(oa) + __popc(ob);
+        if (size + total > (int)cap) {
+            alone = true;
+            break;
+        }
+        int at = size + total - 1 - (__popc(oa & lt) + __popc(ob & lt));
+        if (o[0]) {
+            snode[at] = o[0];
+            st0[at] = ot[0];
+            --at;
+        }
+        if (o[1]) {
+            snode[at] = o[1];
+            st0[at] = ot[1];
+        }
+        size += total;
+        __syncwarp();
+    }
+    if (alone) return traverse_alone<EXACT>(r, tr_, start);
+    Hit h;
+    if (best < init) {
+        h.id = (int)(uint32_t)best;
+        h.t = bt;
+        h.u = bu;
+        h.v = bv;
+    } else {
+        h.id = -1;
+        h.u = -1.0f;
+        h.v = -1.0f;
+        h.t = r.tmax;
+    }
+    return h;
+}
+
+// One any-hit ray traced by a whole block of kTeamThreads threads: traverse_wide's
 // frontier walk with the block as the team.  Each step pops up to
 // kTeamThreads nodes (the deepest), tests their children, and pushes /
 // queues them at offsets from a block-wide prefix sum; the queued leaves are
 // tested kTeamThreads (leaf, triangle) pairs at a time, the block minimum of
 // the (t, id) keys (a shared-memory atomicMin) becoming the shared bound.
-// The hit is traverse_wide's (the tie rule makes it order-free); a ray whose
-// frontier is wide (grazing rays with thousands of tests) finishes in a
+// A ray whose frontier is wide (grazing rays with thousands of tests) finishes in a
 // quarter of the steps.  Every thread of the block calls it with the same
 // ray; it synchronises the block.  Stack bound as in traverse_wide with
 // kTeamThreads entries per level.
@@ -1269,8 +1590,7 @@ __device__ __forceinline__ uint32_t team_scan(uint32_t v, TeamShared& ts, uint32
 }
 
 template <bool EXACT>
-__device__ __forceinline__ Hit traverse_team(const RayState& r, const TreeRef& tr_, bool any_hit, uint32_t cap,
-                                             TeamShared& ts, Hit known) {
+__device__ __forceinline__ Hit traverse_team(const RayState& r, const TreeRef& tr_, uint32_t cap, TeamShared& ts) {
     constexpr uint32_t kFull = 0xffffffffu;
     extern __shared__ uint4 wide_dyn[];
     uint8_t* base8 = reinterpret_cast<uint8_t*>(wide_dyn);
@@ -1284,16 +1604,11 @@ __device__ __forceinline__ Hit traverse_team(const RayState& r, const TreeRef& t
     uint32_t* qincl = reinterpret_cast<uint32_t*>(qt0 + kTeamQueue);
     const uint64_t init = hit_key(r.tmax, 0);
     // uniform across the block (every thread keeps the same copy)
-    uint64_t best = known.id >= 0 ? hit_key(known.t, known.id) : init;
+    uint64_t best = init;
     int size = 0, nq = 0, qtris = 0;
     bool stop = false;
     __syncthreads();  // the previous ray's readers of the shared state are done
-    if (tid == 0) {
-        ts.best = best;
-        ts.bt = known.t;
-        ts.bu = known.u;
-        ts.bv = known.v;
-    }
+    if (tid == 0) ts.best = best;
     {
         const NodeBox root = load_node(tr_.nodes, 1);
         float t0;
@@ -1373,11 +1688,11 @@ __device__ __forceinline__ Hit traverse_team(const RayState& r, const TreeRef& t
                 }
                 best = bmin;
                 __syncthreads();
-                if (any_hit && best < init) break;
+                if (best < init) break;
             }
             nq = 0;
             qtris = 0;
-            if (any_hit && best < init) stop = true;
+            if (best < init) stop = true;
             continue;
         }
         // pop up to kTeamThreads internal nodes from the top
@@ -1474,10 +1789,9 @@ __device__ __forceinline__ Hit traverse_team(const RayState& r, const TreeRef& t
     return h;
 }
 
-__device__ __forceinline__ Hit trace_team(const RayState& r, const TreeRef& tr, bool any_hit, uint32_t cap,
-                                          TeamShared& ts, Hit known) {
-    if (r.exact) return traverse_team<true>(r, tr, any_hit, cap, ts, known);
-    return traverse_team<false>(r, tr, any_hit, cap, ts, known);
+__device__ __forceinline__ Hit trace_team(const RayState& r, const TreeRef& tr, uint32_t cap, TeamShared& ts) {
+    if (r.exact) return traverse_team<true>(r, tr, cap, ts);
+    return traverse_team<false>(r, tr, cap, ts);
 }
 
 // Warp-uniform dispatch between the fast and the NaN-exact box test.  Must be
@@ -1492,10 +1806,17 @@ __device__ __forceinline__ Hit trace_ray(const RayState& r, bool active, const T
     return traverse<false, STATS>(r, active, tr, any_hit, nbox, ntri, spill, slot, start, leaf);
 }
 
-// One ray traced by the whole warp; every lane passes the same ray.
-__device__ __forceinline__ Hit trace_wide(const RayState& r, const TreeRef& tr, bool any_hit, uint32_t cap, Hit known) {
-    if (r.exact) return traverse_wide<true>(r, tr, any_hit, cap, known);
-    return traverse_wide<false>(r, tr, any_hit, cap, known);
+// One any-hit ray traced by the whole warp; every lane passes the same ray.
+__device__ __forceinline__ Hit trace_wide(const RayState& r, const TreeRef& tr, uint32_t cap) {
+    if (r.exact) return traverse_wide<true>(r, tr, cap);
+    return traverse_wide<false>(r, tr, cap);
+}
+
+// One closest-hit ray traced by the whole warp; every lane passes the same ray.
+__device__ __forceinline__ Hit trace_ordered(const RayState& r, const TreeRef& tr, uint32_t cap, const Hit& known,
+                                             uint32_t start) {
+    if (r.exact) return traverse_ordered<true>(r, tr, cap, known, start);
+    return traverse_ordered<false>(r, tr, cap, known, start);
 }
 
 // Primary ray of pixel (i, j): CSPrimaryRays.hlsl:36-56 with the basis camera.

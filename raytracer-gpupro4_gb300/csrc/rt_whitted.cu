@@ -268,11 +268,7 @@ __global__ void __launch_bounds__(kWhThreads, 7) k_wh_heavy(TreeRef tr, ShadeArg
         const uint32_t p = heavy[e];
         RayState r;
         if (!wh_ray<true>(a, w, p, &r)) continue;  // not listed
-        Hit none;
-        none.id = -1;
-        none.u = none.v = -1.0f;
-        none.t = 0.0f;
-        const Hit h = trace_wide(r, tr, true, cap, none);
+        const Hit h = trace_wide(r, tr, cap);
         if ((threadIdx.x & 31) == 0) w.occl[p] = h.id >= 0 ? 1u : 0u;
     }
 }
