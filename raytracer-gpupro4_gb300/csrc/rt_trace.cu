@@ -306,8 +306,16 @@ __device__ __forceinline__ RayState load_ray(const rt_ray* __restrict__ rays, ui
 // at 2.1 M and 1080p 1,509, 1,446, 1,410 and 1,404), a batch's many scenes 64.
 constexpr int kWalkRefill = 16;
 constexpr int kWalkSteps = 4;
-constexpr int kRayRefill = 8;  // a soup's rays: of 8 to 16, and 4 to 12 expansions
-constexpr int kRaySteps = 8;
+// A caller's rays: of 8 to 16 idle lanes, and 3 to 12 expansions a round.  A call that
+// gives each lane one ray lasts as long as its longest chain of rounds, and a ray that reads the
+// heap needs more of each: 20,000 rays from 60 extents away over 65 k triangles 228 us with
+// 8 expansions, 220 with 6, 183 with 4, near ones 170, 168 and 169.  Many rays: 2^20 near ones over a
+// soup 897, 890 and 957 us, along an axis 862, 834 and 889.
+constexpr int kRayRefill = 8;
+constexpr int kRaySteps = 6;
+constexpr int kFewSteps = 4;
+constexpr uint32_t kRayBlocks = 8u;
+uint32_t ray_lanes(const rt_ctx* ctx) { return kRayBlocks * kTraceThreads * (uint32_t)ctx->num_sms; }
 
 // The scenes of a batch.
 struct BatchTrees {
@@ -414,7 +422,8 @@ constexpr int kDoubtMark = -3;
 // traverse() hands over depends on its exact counts, which are at most the
 // counts here.  So an any-hit ray over the budget is walked again by
 // k_trace_doubt, as traverse() does, with its budget.
-__global__ void __launch_bounds__(kTraceThreads, 8) k_walk_rays(TreeRef tr, const rt_ray* __restrict__ rays, uint32_t n,
+template <int STEPS>
+__global__ void __launch_bounds__(kTraceThreads, kRayBlocks) k_walk_rays(TreeRef tr, const rt_ray* __restrict__ rays, uint32_t n,
                                                                      int any_hit, const uint32_t* __restrict__ starts,
                                                                      rt_hit* __restrict__ hits,
                                                                      uint32_t* __restrict__ leaves, uint32_t* work,
@@ -447,7 +456,7 @@ __global__ void __launch_bounds__(kTraceThreads, 8) k_walk_rays(TreeRef tr, cons
             if (drained) break;
             continue;
         }
-        w.round(tr, kRaySteps, stack, any_hit != 0);
+        w.round(tr, STEPS, stack, any_hit != 0);
         int slot = -1;
         bool doubtful = false;
         if (live && w.have && budgeted && w.tests > spill.budget) {
@@ -476,7 +485,7 @@ __global__ void __launch_bounds__(kTraceThreads, 8) k_walk_rays(TreeRef tr, cons
     }
 }
 
-__global__ void __launch_bounds__(kTraceThreads) k_trace_doubt(TreeRef tr, const rt_ray* __restrict__ rays,
+__global__ void __launch_bounds__(kTraceThreads, 6) k_trace_doubt(TreeRef tr, const rt_ray* __restrict__ rays,
                                                                uint32_t num_rays, const uint32_t* __restrict__ starts,
                                                                rt_hit* __restrict__ hits, uint32_t* __restrict__ leaves,
                                                                Doubt doubt, Spill spill, uint32_t* __restrict__ list) {
@@ -1080,7 +1089,8 @@ rt_status trace_rays(rt_ctx* ctx, const rt_lbvh* l, const rt_ray* d_rays, uint32
     } else if (walk) {
         const Doubt doubt{ctx->d_spill + kSpillCap, ctx->d_words + kDoubtCount, ctx->d_words + kDoubtCount + 1,
                           kSpillCap};
-        launch_pdl(k_walk_rays, persistent_blocks(ctx, k_walk_rays, kTraceThreads, tiles), kTraceThreads, 0, ctx->stream,
+        auto k = n <= ray_lanes(ctx) ? k_walk_rays<kFewSteps> : k_walk_rays<kRaySteps>;
+        launch_pdl(k, persistent_blocks(ctx, k, kTraceThreads, tiles), kTraceThreads, 0, ctx->stream,
                    tree_ref(ctx, l), d_rays, n, any_hit, d_starts, d_hits, d_leaves, work, sp, ctx->d_spill, doubt);
         if (any_hit && sp.count) {
             RT_CHECK_LAUNCH(ctx, "k_walk_rays");

@@ -583,6 +583,12 @@ __device__ __forceinline__ void ldg32(const void* p, uint32_t w[8]) {
     w[4] = (uint32_t)c; w[5] = (uint32_t)(c >> 32);
     w[6] = (uint32_t)d; w[7] = (uint32_t)(d >> 32);
 }
+__device__ __forceinline__ NodeBox node_of(const uint32_t w[8]) {
+    NodeBox nb;
+    nb.a = make_float4(__uint_as_float(w[0]), __uint_as_float(w[1]), __uint_as_float(w[2]), __uint_as_float(w[3]));
+    nb.b = make_float4(__uint_as_float(w[4]), __uint_as_float(w[5]), __uint_as_float(w[6]), __uint_as_float(w[7]));
+    return nb;
+}
 __device__ __forceinline__ float grid_centre(uint32_t w) { return __uint_as_float(__byte_perm(w, 0x3f000000u, 0x7104)); }
 
 // First statement of a kernel that walks the records (after the wait for the
@@ -594,6 +600,9 @@ __device__ __forceinline__ void mark_records(const TreeRef& tr) {
 constexpr uint32_t kGeneral = 8u;    // Walk::sgn: the records do not serve this ray
 constexpr uint32_t kInfinite = 16u;  // some 1 / d is infinite: the reference's NaN-sensitive min / max
 constexpr uint32_t kBySlot = 32u;    // the tree's leaves are named by their slots
+// An internal node in hand of a ray that reads the heap: its slot, and its axis field above.
+constexpr uint32_t kAxisShift = 26u, kSlotMask = (1u << kAxisShift) - 1u;
+static_assert(kMaxDepth <= (int)kAxisShift, "");
 // A leaf of more triangles makes the warp pool its leaves: 2 for rays that stay
 // neighbours (330 k triangles at 720p 561 us a frame with 3, 538 with 2; 1: the same), 3
 // for paths (24.2 ms with 3, 24.5 with 2, 25.9 with 1).
@@ -601,7 +610,7 @@ constexpr uint32_t kPoolMin = 2u;
 constexpr uint32_t kPathPoolMin = 3u;
 
 struct Walk {
-    f3 o, d, k, n;  // k = E / d, n = (G - o) / d
+    f3 o, d, k, n;  // k = E / d, n = (G - o) / d; of a ray that reads the heap k = 1 / d
     uint32_t sgn;   // RayState::sgn, kGeneral, kInfinite
     int exclude;
     Best b;         // key: the acceptance bound
@@ -675,7 +684,10 @@ struct Walk {
         n = mk3(fmul(q.x, r.inv.x), fmul(q.y, r.inv.y), fmul(q.z, r.inv.z));
         const float kmax = max3(fabsf(k.x), fabsf(k.y), fabsf(k.z)), kmin = min3(fabsf(k.x), fabsf(k.y), fabsf(k.z));
         const bool gen = counted || !(max3(fabsf(q.x), fabsf(q.y), fabsf(q.z)) <= 16.0f * g.w && kmax < 1e30f && kmin > 1e-30f);
-        if (gen) sgn |= kGeneral;
+        if (gen) {
+            sgn |= kGeneral;
+            k = r.inv;
+        }
         if (r.exact) sgn |= kInfinite;
         uint32_t node = 1u;
         float t0;
@@ -699,9 +711,10 @@ struct Walk {
         have = cur != 0u || sp != 0u;
     }
 
-    // expand() of a ray that the records do not serve, over the heap.
+    // expand() of a ray that the records do not serve, over the heap: what the step
+    // needs (1 / d, the node's axis) is held, so that its only loads are the two children.
     __device__ __forceinline__ void expand_heap(const TreeRef& tr, uint2* stack) {
-        const uint32_t c0 = cur << 1;
+        const uint32_t c0 = (cur & kSlotMask) << 1;
         if (c0 + 1u >= tr.num_heap) {
             atomicOr(tr.err, RT_DEVERR_BOUNDS);
             cur = sp = 0u;
@@ -709,14 +722,23 @@ struct Walk {
         }
         RayState r;
         r.o = o;
-        r.inv = mk3(fdiv(1.0f, d.x), fdiv(1.0f, d.y), fdiv(1.0f, d.z));
-        const NodeBox nl = load_node(tr.heap, c0), nr = load_node(tr.heap, c0 + 1u);
+        r.inv = k;
+        uint32_t wl[8], wr[8];
+        ldg32(tr.heap + c0, wl);
+        ldg32(tr.heap + c0 + 1u, wr);
+        const NodeBox nl = node_of(wl), nr = node_of(wr);
         float tl, tr_;
-        const bool inf = (sgn & kInfinite) != 0u;
-        const bool hl = enter(r, nl, b.t, &tl, inf), hr = enter(r, nr, b.t, &tr_, inf);
+        bool hl, hr;
+        if (sgn & kInfinite) {
+            hl = enter(r, nl, b.t, &tl, true);
+            hr = enter(r, nr, b.t, &tr_, true);
+        } else {
+            hl = enter(r, nl, b.t, &tl, false);
+            hr = enter(r, nr, b.t, &tr_, false);
+        }
         tests += 2;
-        const int field = __ldg(&tr.heap[cur].prim_count) & 3;  // one axis past the split axis
-        const bool near_right = (sgn >> (field == 0 ? 2 : field - 1)) & 1u;
+        const uint32_t field = cur >> kAxisShift;  // one axis past the split axis
+        const bool near_right = (sgn >> (field == 0u ? 2u : field - 1u)) & 1u;
         const bool go_right = near_right ? hr : !hl;
         const uint32_t l = heap_item(c0, nl), r_ = heap_item(c0 + 1u, nr);
         if (hl && hr) push(stack, near_right ? l : r_, near_right ? tl : tr_);
@@ -725,7 +747,7 @@ struct Walk {
 
     __device__ __forceinline__ uint32_t heap_item(uint32_t h, const NodeBox& nb) const {
         const int pc = __float_as_int(nb.b.z);
-        if (!(pc & 4)) return h;
+        if (!(pc & 4)) return (sgn & kGeneral) ? h | (uint32_t)(pc & 3) << kAxisShift : h;
         return (sgn & kBySlot) ? slot_word(h) : leaf_word(h, (uint32_t)__float_as_int(nb.b.w), (uint32_t)(pc >> 3));
     }
 
@@ -798,7 +820,7 @@ struct Walk {
             pos = leaf & 0x1ffffffu;
             cnt = (leaf >> 25) & 31u;
             if (leaf & kBigLeaf) {
-                const int2 z = __ldg(reinterpret_cast<const int2*>(tr.heap + (leaf & 0x3ffffffu)) + 3);
+                const int2 z = __ldg(reinterpret_cast<const int2*>(tr.heap + (leaf & kSlotMask)) + 3);
                 pos = (uint32_t)z.y;
                 cnt = (uint32_t)(z.x >> 3);
             }
@@ -808,11 +830,12 @@ struct Walk {
             }
             pos += tr.tri_base;
         }
-        bool inside = false;
+        // the heap's boxes were tested exactly, under this bound while there is no hit
+        bool inside = POOL_MIN == kPoolMin && (sgn & kGeneral) && b.id < 0;
         // a leaf of 32 or more triangles: its exact box, with the bound of now, first (of
         // 5 or more, 330 k triangles at 720p took 9 us a frame longer)
-        if (leaf & kBigLeaf) {
-            inside = leaf_entered(tr, leaf & 0x3ffffffu);
+        if ((leaf & kBigLeaf) && !inside) {
+            inside = leaf_entered(tr, leaf & kSlotMask);
             if (!inside) cnt = 0u;
         }
         tests += cnt;
@@ -862,7 +885,7 @@ struct Walk {
     __device__ __forceinline__ bool accept(const TreeRef& tr, uint32_t leaf, uint64_t key, int id, float t, float u,
                                            float v, bool& inside) {
         if (!(key < b.key)) return true;
-        const uint32_t h = (leaf & kBigLeaf) ? leaf & 0x3ffffffu : __ldg(tr.leaf_of + tr.tri_base + (leaf & 0x1ffffffu));
+        const uint32_t h = (leaf & kBigLeaf) ? leaf & kSlotMask : __ldg(tr.leaf_of + tr.tri_base + (leaf & 0x1ffffffu));
         if (!inside && !leaf_entered(tr, h)) return false;
         inside = true;
         b.key = key;
@@ -955,7 +978,8 @@ struct Walk {
         const NodeBox nb = load_node(tr.heap, h);
         RayState r;
         r.o = o;
-        r.inv = mk3(fdiv(1.0f, d.x), fdiv(1.0f, d.y), fdiv(1.0f, d.z));
+        r.inv = k;
+        if (!(sgn & kGeneral)) r.inv = mk3(fdiv(1.0f, d.x), fdiv(1.0f, d.y), fdiv(1.0f, d.z));
         float t0;
         return enter(r, nb, b.t, &t0, (sgn & kInfinite) != 0u);
     }
