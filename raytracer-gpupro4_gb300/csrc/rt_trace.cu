@@ -401,10 +401,14 @@ __global__ void __launch_bounds__(kTraceThreads, BATCH ? 8 : 7) k_walk_shade(
 }
 
 // Any-hit calls of fewer rays stay with traverse(): the second walk of the rays in
-// doubt lasts as long as its longest ones, 200 us on a mesh's grazing rays (65 k
-// triangle torus, 0.5 M rays 0.36 -> 0.42 ms, 2 M rays 1.02 -> 0.78 ms; a soup gains
-// from 0.2 M rays on, 1 M rays 1.63 -> 0.79 ms).
-constexpr uint32_t kWalkAnyRays = 1u << 20;
+// doubt lasts as long as its longest ones, 150 us on a mesh's grazing rays, whatever
+// their number.  Where the record walk becomes the faster one (us, traverse() and records):
+// rays at a torus of 65 k triangles from around it 500,000 (448, 446), along planes through it
+// 700,000 (555, 553); at 260 k triangles 460,000, and along planes 680,000; in a soup 150,000;
+// short rays everywhere from the first thousand.  At 700,000 no kind is slower but rays along an
+// axis of the 260 k triangles (232, 249; 4 M: 848, 989).  Restarted rays often end in their first
+// leaf, and the second walk is then most of the call (2^20: 256, 470; rays that go on 782, 692).
+constexpr uint32_t kWalkAnyRays = 700000u;
 
 // The any-hit rays in doubt: their list, or, when more than `cap` are, the marks that
 // each of them has left in its hit.
@@ -1077,7 +1081,7 @@ rt_status trace_rays(rt_ctx* ctx, const rt_lbvh* l, const rt_ray* d_rays, uint32
         RT_CHECK_LAUNCH(ctx, "k_rays_wide");
         return RT_OK;
     }
-    const bool walk = !d_stats && !(ctx->tile_order & 4u) && !(any_hit && n < kWalkAnyRays);
+    const bool walk = !d_stats && !(ctx->tile_order & 4u) && !(any_hit && (n < kWalkAnyRays || d_starts));
     rt_status s = order_begin(ctx, 2, ctx->tile_order & 4u, &ord, reset, walk ? l : nullptr);
     if (s != RT_OK) return s;
     const uint32_t tiles = (n + 31) / 32;

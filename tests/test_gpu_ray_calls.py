@@ -1,5 +1,6 @@
 """The dispatch of a caller's rays at the sizes where it changes: a warp per ray or a lane, a ray
-for every lane of the GPU and one more.  Half of the rays are ones that the records do not serve (along
+for every lane of the GPU and one more, any-hit calls from which on the trace records are
+walked, and restarted any-hit rays.  Half of the rays are ones that the records do not serve (along
 an axis or a plane, from far away).  Hits are the oracle's on their bits."""
 import numpy as np
 import pytest
@@ -44,3 +45,28 @@ def test_closest(gpu_ctx, oracle_mod, scene, n):
     got = hits_to_numpy(RayTracer(gpu_ctx).rays(lb, rays_tensor(*r, "cuda")))
     gpu_ctx.check()
     assert np.array_equal(got.view(np.int32), ref.view(np.int32))
+
+
+@pytest.mark.parametrize("n", [699999, 700000])
+@pytest.mark.parametrize("restart", [False, True])
+def test_any_hit(gpu_ctx, oracle_mod, scene, n, restart):
+    import torch
+    from rtgpu.api import RayTracer, hits_to_numpy, rays_tensor
+    tris, depth, lb, nodes, ids = scene
+    r = make_rays(tris, n)
+    rays = oracle_mod.rays_array(*r)
+    starts = None
+    if restart:
+        _, starts = oracle_mod.trace_from(nodes, depth, ids, tris, rays)
+    ref, _, st = oracle_mod.trace_from(nodes, depth, ids, tris, rays, starts, any_hit=True, stats=True)
+    rt = RayTracer(gpu_ctx)
+    t = rays_tensor(*r, "cuda")
+    if restart:
+        got, _ = rt.rays_from(lb, t, torch.from_numpy(starts.view(np.int32)).cuda(), any_hit=True)
+    else:
+        got = rt.rays(lb, t, any_hit=True)
+    gpu_ctx.check()
+    got = hits_to_numpy(got)
+    assert np.array_equal(got["id"] >= 0, ref["id"] >= 0)
+    within = st.sum(1) <= 384  # a ray over the budget reports some hit
+    assert np.array_equal(got[within].view(np.int32), ref[within].view(np.int32)) and within.mean() > 0.5
