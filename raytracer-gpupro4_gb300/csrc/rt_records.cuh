@@ -111,16 +111,20 @@ __device__ __forceinline__ void make_records(const Records& R, uint32_t block) {
     const uint32_t tiles = R.built ? *R.built : R.tiles;
     for (uint32_t tile = block / R.slices; tile < tiles; tile += R.tiles) {
         const uint32_t cnt = min(__ldg(R.counts + tile), (uint32_t)kTreeTile);
-        for (uint32_t i = (block % R.slices) * blockDim.x + threadIdx.x; i < cnt; i += R.slices * blockDim.x) {
-            uint32_t b = __ldg(&R.units[(size_t)tile * kTreeTile + i].x), a = 0u;
-            if (i) {
-                a = __ldg(&R.units[(size_t)tile * kTreeTile + i - 1].x);
-            } else {  // the last leaf of the tiles before
-                for (uint32_t q = tile; q-- > 0u && a == 0u;) {
-                    const uint32_t c = min(__ldg(R.counts + q), (uint32_t)kTreeTile);
-                    if (c) a = __ldg(&R.units[(size_t)q * kTreeTile + c - 1].x);
-                }
+        uint32_t prev = 0u;  // thread 0 of slice 0: the last leaf of the tiles before, by its warp (a leaf may span many)
+        if (cnt && block % R.slices == 0u && threadIdx.x < 32u) {
+            for (uint32_t top = tile; top > 0u; top -= min(top, 32u)) {
+                const uint32_t c = threadIdx.x < top ? min(__ldg(R.counts + (top - 1u - threadIdx.x)), (uint32_t)kTreeTile) : 0u;
+                const uint32_t m = __ballot_sync(0xffffffffu, c != 0u);
+                if (!m) continue;
+                const int w = __ffs(m) - 1;
+                prev = __ldg(&R.units[(size_t)(top - 1u - w) * kTreeTile + __shfl_sync(0xffffffffu, c, w) - 1u].x);
+                break;
             }
+        }
+        for (uint32_t i = (block % R.slices) * blockDim.x + threadIdx.x; i < cnt; i += R.slices * blockDim.x) {
+            uint32_t b = __ldg(&R.units[(size_t)tile * kTreeTile + i].x);
+            uint32_t a = i ? __ldg(&R.units[(size_t)tile * kTreeTile + i - 1].x) : prev;
             const rt_node* nodes = R.nodes;
             TraceNode* tnodes = R.tnodes;
             if (batch) {
