@@ -111,6 +111,24 @@ rt_status rt_ctx_set_heavy_block(rt_ctx* ctx, uint32_t kinds);
  * same kind on this context, then the rest in image order.  Results do not
  * depend on the order.  Default: primary rays only (1). */
 rt_status rt_ctx_set_tile_order(rt_ctx* ctx, uint32_t kinds);
+/* Limits of what the context's calls hold or take at once; each call does the same work
+ * within any limit.
+ * RT_LIMIT_PATH_SCRATCH (default 512 MB): bytes of radiance terms that rt_pathtrace may
+ *   keep for a call of several samples (see there); what is held above a new limit is freed.
+ *   0: none, and no call of rt_pathtrace allocates.
+ * RT_LIMIT_TRACE_RECORDS (default no limit): bytes of trace records a tree or batch created
+ *   from now on may have (half of its nodes' memory); those of a larger one are not made, and its
+ *   walks read the nodes, more slowly.
+ * RT_LIMIT_PATHS (32 to 2^31, the default): paths that one launch of rt_pathtrace_adjoint takes.
+ * RT_LIMIT_RECHECKED_RAYS (1 to 2^20, the default): any-hit rays over the budget that
+ *   rt_trace_rays lists; more are marked in their hits. */
+enum {
+    RT_LIMIT_PATH_SCRATCH = 0,
+    RT_LIMIT_TRACE_RECORDS = 1,
+    RT_LIMIT_PATHS = 2,
+    RT_LIMIT_RECHECKED_RAYS = 3
+};
+rt_status rt_ctx_set_limit(rt_ctx* ctx, uint32_t limit, uint64_t value);
 rt_status rt_ctx_sync(rt_ctx* ctx);
 /* Synchronises, then reports a device-side error flag raised since the
  * last check (RT_ERR_TIMEOUT, RT_ERR_NONFINITE) and clears it. */
@@ -502,8 +520,8 @@ typedef struct rt_pt_params {
  * a pixel has its own PCG32 stream, so two calls of k samples with n0 = 0
  * and n0 = k give the image of one call of 2k samples, bit for bit.
  * A call of several samples keeps their terms in scratch of the context (at most
- * 512 MB, allocated by the first call that needs more; not inside a stream
- * capture, where a pixel's samples follow one another instead). */
+ * RT_LIMIT_PATH_SCRATCH, allocated by the first call that needs more; where there is
+ * none, and inside a stream capture, a pixel's samples follow one another instead). */
 rt_status rt_pathtrace(rt_ctx* ctx, const rt_lbvh* lbvh, const float* d_albedo, const float* d_emission,
                        const rt_camera* cam, const rt_pt_params* p, float* d_image);
 /* rt_pathtrace that also adds its walk counts to d_counts (device, 4 x

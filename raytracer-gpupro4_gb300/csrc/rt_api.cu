@@ -105,6 +105,36 @@ extern "C" rt_status rt_ctx_set_tile_order(rt_ctx* ctx, uint32_t kinds) {
     return RT_OK;
 }
 
+extern "C" rt_status rt_ctx_set_limit(rt_ctx* ctx, uint32_t limit, uint64_t value) {
+    if (!ctx) return RT_ERR_INVALID;
+    switch (limit) {
+        case RT_LIMIT_PATH_SCRATCH:
+            if (ctx->terms_bytes > value) {
+                RT_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+                cudaFree(ctx->d_terms);
+                ctx->d_terms = nullptr;
+                ctx->terms_bytes = 0;
+            }
+            ctx->terms_limit = (size_t)value;
+            return RT_OK;
+        case RT_LIMIT_TRACE_RECORDS:
+            ctx->records_limit = (size_t)value;
+            return RT_OK;
+        case RT_LIMIT_PATHS:
+            if (value < 32u || value > (1ull << 31))
+                return rt_fail(ctx, RT_ERR_INVALID, "rt_ctx_set_limit: RT_LIMIT_PATHS is in [32, 2^31]");
+            ctx->paths_limit = (uint32_t)value;
+            return RT_OK;
+        case RT_LIMIT_RECHECKED_RAYS:
+            if (value < 1u || value > kSpillCap)
+                return rt_fail(ctx, RT_ERR_INVALID, "rt_ctx_set_limit: RT_LIMIT_RECHECKED_RAYS is in [1, %u]", kSpillCap);
+            ctx->doubt_limit = (uint32_t)value;
+            return RT_OK;
+        default:
+            return rt_fail(ctx, RT_ERR_INVALID, "rt_ctx_set_limit: unknown limit %u", limit);
+    }
+}
+
 extern "C" rt_status rt_ctx_sync(rt_ctx* ctx) {
     if (!ctx) return RT_ERR_INVALID;
     RT_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));

@@ -2340,8 +2340,8 @@ extern "C" rt_status rt_lbvh_create(rt_ctx* ctx, uint32_t max_tris, uint32_t dep
     if (e == cudaSuccess) e = cudaMemset(l->nodes, 0, sizeof(rt_node) * l->num_nodes);
     if (e == cudaSuccess) e = cudaMemset(l->item_counts, 0, sizeof(uint32_t) * 8 * (size_t)l->emit_tiles_cap);
     // without room for the trace records the walks read the heap
-    if (e == cudaSuccess &&
-        cudaMalloc((void**)&l->tnodes, sizeof(TraceNode) * (size_t)std::max(1u, l->num_nodes / 2)) != cudaSuccess) {
+    const size_t rec_bytes = sizeof(TraceNode) * (size_t)std::max(1u, l->num_nodes / 2);
+    if (e == cudaSuccess && rec_bytes <= ctx->records_limit && cudaMalloc((void**)&l->tnodes, rec_bytes) != cudaSuccess) {
         cudaGetLastError();
         l->tnodes = nullptr;
     }
@@ -3068,7 +3068,7 @@ extern "C" rt_status rt_batch_create(rt_ctx* ctx, uint32_t n_scenes, const uint3
     // to be traced (half of what is free)
     size_t free_bytes = 0, all_bytes = 0;
     const size_t rec_bytes = sizeof(TraceNode) * std::max<size_t>(n_scenes, num_nodes >> 1);
-    if (e == cudaSuccess && cudaMemGetInfo(&free_bytes, &all_bytes) == cudaSuccess && rec_bytes <= free_bytes / 2 &&
+    if (e == cudaSuccess && rec_bytes <= ctx->records_limit && cudaMemGetInfo(&free_bytes, &all_bytes) == cudaSuccess && rec_bytes <= free_bytes / 2 &&
         cudaMalloc((void**)&b->tnodes, rec_bytes) != cudaSuccess) {
         cudaGetLastError();
         b->tnodes = nullptr;

@@ -146,6 +146,9 @@ struct rt_ctx {
     uint32_t* d_spill = nullptr; // heavy-ray list, kSpillCap entries; then the any-hit rays' second list, as many
     float* d_terms = nullptr;    // radiance terms of a path-traced image (rt_pathtrace.cu), grown on demand
     size_t terms_bytes = 0;
+    // rt_ctx_set_limit
+    size_t terms_limit = (size_t)512 << 20, records_limit = ~(size_t)0;
+    uint32_t paths_limit = 1u << 31, doubt_limit = kSpillCap;
     uint32_t* d_order = nullptr; // heavy-first tile order, kOrderKinds x kOrderWords (parity / counts: d_words[40..])
     // hand-over budget per trace kind (0 primary, 1 shading, 2 generic rays); 0: no hand-over
     uint32_t trace_budget[3] = {kDefaultTraceBudget, kDefaultShadeBudget, kDefaultTraceBudget};

@@ -519,16 +519,14 @@ uint32_t px_tiles(const rt_camera* cam) {
 
 TreeRef tree_ref(const rt_ctx* ctx, const rt_lbvh* l);
 
-// Bytes of radiance terms a context keeps at most.
-constexpr size_t kTermBytes = (size_t)512 << 20;
-
 // The term buffers for as many of the call's samples as fit (0: trace each
 // pixel's samples one after another).  Never in a stream capture: a graph must
 // not hold a buffer that a later call may replace.
-static uint32_t ensure_terms(rt_ctx* ctx, size_t px, uint32_t segs, uint32_t spp, PathTerms* T) {
+static uint32_t ensure_terms(rt_ctx* ctx, size_t px, uint32_t tiles, uint32_t segs, uint32_t spp, PathTerms* T) {
     const size_t sample = px * ((size_t)segs * 12 + 1);
-    const uint32_t m = (uint32_t)std::min<size_t>(spp, kTermBytes / sample);
-    if (m < 2) return 0;  // so px < 2^25, and a launch has at most 2^31 paths
+    // the path counter holds 2^31 of them a launch
+    const uint32_t m = (uint32_t)std::min<size_t>({spp, ctx->terms_limit / sample, ((size_t)1 << 31) / (32 * (size_t)tiles)});
+    if (m < 2) return 0;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(ctx->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
         cudaGetLastError();
@@ -536,11 +534,17 @@ static uint32_t ensure_terms(rt_ctx* ctx, size_t px, uint32_t segs, uint32_t spp
     }
     const size_t need = m * sample;
     if (need > ctx->terms_bytes) {
-        if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) return 0;
+        if (ctx->d_terms && cudaStreamSynchronize(ctx->stream) != cudaSuccess) return 0;
+        // an allocation would break another thread's stream capture in the global mode
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
         if (ctx->d_terms) cudaFree(ctx->d_terms);
         ctx->d_terms = nullptr;
         ctx->terms_bytes = 0;
-        if (cudaMalloc((void**)&ctx->d_terms, need) != cudaSuccess) {
+        const bool ok = cudaMalloc((void**)&ctx->d_terms, need) == cudaSuccess;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (!ok) {
+            ctx->d_terms = nullptr;
             cudaGetLastError();
             return 0;
         }
@@ -576,7 +580,7 @@ static rt_status launch_pathtrace(rt_ctx* ctx, const rt_lbvh* l, const float* d_
     // and a smaller image could not fill the GPU.
     const uint32_t segs = P.bounces + 1u;
     PathTerms T = {nullptr, nullptr};
-    const uint32_t chunk = P.spp > 1 ? ensure_terms(ctx, px, segs, P.spp, &T) : 0u;
+    const uint32_t chunk = P.spp > 1 ? ensure_terms(ctx, px, tiles, segs, P.spp, &T) : 0u;
     auto launch = [&](auto kernel, uint32_t per) {
         kernel<<<persistent_blocks(ctx, kernel, kPtThreads, tiles * per), kPtThreads, 0, ctx->stream>>>(
             tree_ref(ctx, l), l->src_tris, d_albedo, d_emission, P, image, work, tiles, T);
@@ -624,7 +628,7 @@ extern "C" rt_status rt_pathtrace_adjoint(rt_ctx* ctx, const rt_lbvh* l, const f
     if (!d_dimage || !d_dalbedo || !d_demission) return rt_fail(ctx, RT_ERR_INVALID, "rt_pathtrace_adjoint: null buffer");
     const uint32_t tiles = px_tiles(cam);
     // a sample of a pixel is a path; the path counter holds 2^31 of them a launch
-    const uint32_t most = std::max(1u, (1u << 31) / std::max(32u, tiles * 32u));
+    const uint32_t most = std::max(1u, ctx->paths_limit / std::max(32u, tiles * 32u));
     for (uint32_t done = 0; done < P.spp; done += most) {
         const uint32_t per = std::min(most, P.spp - done);
         if ((s = reset_work_and_records(ctx, kWorkAdjoint, l)) != RT_OK) return s;

@@ -1092,7 +1092,7 @@ rt_status trace_rays(rt_ctx* ctx, const rt_lbvh* l, const rt_ray* d_rays, uint32
             tree_ref(ctx, l), d_rays, n, any_hit, d_starts, d_hits, d_leaves, d_stats, work, sp, ctx->d_spill, ord);
     } else if (walk) {
         const Doubt doubt{ctx->d_spill + kSpillCap, ctx->d_words + kDoubtCount, ctx->d_words + kDoubtCount + 1,
-                          kSpillCap};
+                          ctx->doubt_limit};
         auto k = n <= ray_lanes(ctx) ? k_walk_rays<kFewSteps> : k_walk_rays<kRaySteps>;
         launch_pdl(k, persistent_blocks(ctx, k, kTraceThreads, tiles), kTraceThreads, 0, ctx->stream,
                    tree_ref(ctx, l), d_rays, n, any_hit, d_starts, d_hits, d_leaves, work, sp, ctx->d_spill, doubt);

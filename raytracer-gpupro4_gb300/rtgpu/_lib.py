@@ -15,6 +15,7 @@ from .build import LIB
 RT_OK, RT_ERR_INVALID, RT_ERR_CAPACITY, RT_ERR_CUDA, RT_ERR_TIMEOUT, RT_ERR_NONFINITE = range(6)
 RT_BUILD_CLEAR_UNREACHED = 1
 RT_BUILD_COMPACT = 2
+RT_LIMIT_PATH_SCRATCH, RT_LIMIT_TRACE_RECORDS, RT_LIMIT_PATHS, RT_LIMIT_RECHECKED_RAYS = range(4)
 RT_NOALLOC_MAX_TRIS = 262144
 RT_NOALLOC_MAX_DEPTH = 20
 RT_NODE_SENTINEL = -2147483647
@@ -27,7 +28,7 @@ assert NODE_DTYPE.itemsize == 32 and HIT_DTYPE.itemsize == 16 and RAY_DTYPE.item
 
 EXPORTED = [
     "rt_api_version", "rt_status_string", "rt_ctx_create", "rt_ctx_destroy", "rt_ctx_set_stream", "rt_ctx_sync",
-    "rt_ctx_set_trace_budget", "rt_ctx_set_trace_budget_kind", "rt_ctx_set_heavy_block", "rt_ctx_set_tile_order",
+    "rt_ctx_set_trace_budget", "rt_ctx_set_trace_budget_kind", "rt_ctx_set_heavy_block", "rt_ctx_set_tile_order", "rt_ctx_set_limit",
     "rt_ctx_check", "rt_last_error", "rt_lbvh_create", "rt_lbvh_destroy", "rt_lbvh_build", "rt_lbvh_build_host",
     "rt_lbvh_import_host", "rt_lbvh_view_get", "rt_lbvh_compact_get", "rt_lbvh_world_bound", "rt_lbvh_download", "rt_trace_primary",
     "rt_trace_shadow_mirror", "rt_trace_rays", "rt_trace_primary_leaves", "rt_trace_shadow_mirror_from",
@@ -99,6 +100,7 @@ def lib() -> C.CDLL:
         "rt_ctx_set_trace_budget_kind": (i32, [vp, u32, u32]),
         "rt_ctx_set_heavy_block": (i32, [vp, u32]),
         "rt_ctx_set_tile_order": (i32, [vp, u32]),
+        "rt_ctx_set_limit": (i32, [vp, u32, C.c_uint64]),
         "rt_ctx_check": (i32, [vp]),
         "rt_last_error": (C.c_char_p, [vp]),
         "rt_lbvh_create": (i32, [vp, u32, u32, C.POINTER(vp)]),

@@ -66,6 +66,14 @@ class Context:
         """Heavy-first tile order per trace kind (bit 0 primary, 1 shading, 2 generic rays)."""
         L.check(L.lib().rt_ctx_set_tile_order(self.h, int(kinds)), self.h, "rt_ctx_set_tile_order")
 
+    DEFAULT_LIMITS = (512 << 20, (1 << 64) - 1, 1 << 31, 1 << 20)
+
+    def set_limit(self, limit: int, value: int | None):
+        """What the context's calls may hold or take at once (rt_ctx_set_limit, L.RT_LIMIT_*);
+        None restores the default."""
+        v = self.DEFAULT_LIMITS[limit] if value is None else int(value)
+        L.check(L.lib().rt_ctx_set_limit(self.h, int(limit), v), self.h, "rt_ctx_set_limit")
+
     DEFAULT_BUDGETS = (384, 768, 384)  # primary, shadow / mirror, generic rays
 
     def set_trace_budget(self, budget: int | None, kind: int | None = None):
