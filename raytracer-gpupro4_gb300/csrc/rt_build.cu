@@ -1092,6 +1092,16 @@ constexpr int kMergeThreads = 512;
 // with more tiles of one tree two leaves a thread are faster (1.2 M: 205 and 200 us,
 // 2.1 M: 297 and 288).
 constexpr uint32_t kChunkWideTris = 1u << 20;
+// Chunks and groups of all merge levels over `tiles` emission tiles, one group at the top.
+constexpr uint32_t merge_slots(uint32_t tiles) {
+    uint32_t sum = tiles, n = tiles;
+    do {
+        n = (n + kMergeGroup - 1) / kMergeGroup;
+        sum += n;
+    } while (n > 1);
+    return sum;
+}
+static_assert(merge_slots(1) == 2 && merge_slots(32) == 33 && merge_slots(33) == 36 && merge_slots(1025) == 1025 + 33 + 2 + 1, "");
 constexpr int kUnitCap = kMergeGroup * kItemCap;  // units of one CTA of the merge: the items of a group
 constexpr size_t kUnitSmem = (size_t)kUnitWords * kUnitCap * sizeof(uint32_t) + 16;
 constexpr size_t kChunkSmem = (size_t)kUnitWords * kTreeTile * sizeof(uint32_t) + 16;
@@ -2331,10 +2341,9 @@ extern "C" rt_status rt_lbvh_create(rt_ctx* ctx, uint32_t max_tris, uint32_t dep
           sizeof(uint32_t) * kSortPasses * 256 * ((size_t)l->sort_tiles_cap + look_groups(l->sort_tiles_cap)));
     alloc((void**)&l->scan, sizeof(uint32_t) * scan_words(l->emit_tiles_cap));
     alloc((void**)&l->leaf_of, 4 * cap);
-    // items and item counts of every merge level (chunk slots = 4 x tiles, then
-    // the groups above: < 6 x tiles in all), the tiles' unit counts (tiles),
-    // the merge tickets (tiles, zero between builds)
-    alloc((void**)&l->items, sizeof(uint2) * 6 * (size_t)kItemCap * l->emit_tiles_cap);
+    // items of every merge level; their counts (< 6 x tiles), the tiles' unit
+    // counts (tiles) and the merge tickets (tiles, zero between builds)
+    alloc((void**)&l->items, sizeof(uint2) * (size_t)kItemCap * merge_slots(l->emit_tiles_cap));
     alloc((void**)&l->item_counts, sizeof(uint32_t) * 8 * (size_t)l->emit_tiles_cap);
     if (e == cudaSuccess) e = cudaMemset(l->counters, 0, sizeof(uint32_t) * 16);
     if (e == cudaSuccess) e = cudaMemset(l->nodes, 0, sizeof(rt_node) * l->num_nodes);
@@ -3055,7 +3064,7 @@ extern "C" rt_status rt_batch_create(rt_ctx* ctx, uint32_t n_scenes, const uint3
     alloc((void**)&b->scan, sizeof(uint32_t) * scan_words(emit_tiles));
     alloc((void**)&b->leaf_of, 4 * n);
     // items and counts of the merge levels, as a single tree's (rt_lbvh_create)
-    alloc((void**)&b->items, sizeof(uint2) * 6 * (size_t)kItemCap * emit_tiles);
+    alloc((void**)&b->items, sizeof(uint2) * (size_t)kItemCap * merge_slots(emit_tiles));
     alloc((void**)&b->item_counts, sizeof(uint32_t) * 8 * (size_t)emit_tiles);
     alloc((void**)&b->cams, sizeof(rt_camera) * n_scenes);
     alloc((void**)&b->lights, sizeof(float) * 3 * n_scenes);

@@ -188,7 +188,7 @@ struct rt_lbvh {
     uint32_t* hist = nullptr;        // 4 x 256 digit histograms
     uint32_t* lookback = nullptr;    // 4 passes x sort tiles x 256 status words
     uint32_t* scan = nullptr;        // emission tiles x 4 (fwd agg, bwd agg, fwd prefix, bwd suffix)
-    uint2* items = nullptr;          // emission items (heap index, mask) of every merge level: 6 x emit tiles x 64
+    uint2* items = nullptr;          // emission items (heap index, mask), 64 for each chunk and group of every merge level
     uint32_t* item_counts = nullptr; // 8 x emit tiles: item counts of every level (6x), tile unit counts, merge tickets
     uint32_t sort_tiles_cap = 0, emit_tiles_cap = 0, bounds_blocks = 0;
     // frame buffers for rt_render_frame_host (grown on demand)

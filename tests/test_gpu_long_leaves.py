@@ -36,3 +36,17 @@ def test_batch(gpu_ctx, oracle_mod):
         onodes, oids, okeys, reached = oracle_mod.lbvh_build(p, 14)
         r = np.nonzero(reached)[0]
         assert np.array_equal(keys, okeys) and np.array_equal(ids, oids) and same_bits(nodes[r], onodes[r])
+
+
+def test_memory_of_a_tree(gpu_ctx):
+    """What a tree of 8 M triangles holds: 36 + 48 bytes of triangles, 16 of codes and ids and their
+    alternates, 4 of leaves, and about 2 of the sort's and the emission's scratch each."""
+    import torch
+    from rtgpu.api import LBVH
+    n = 8 << 20
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    lb = LBVH(gpu_ctx, n, 10)
+    used = before - torch.cuda.mem_get_info()[0]
+    lb.close()
+    assert 104 * n < used < 108 * n
