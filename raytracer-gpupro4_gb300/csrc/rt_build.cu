@@ -366,9 +366,9 @@ __host__ __device__ constexpr uint32_t look_groups(uint32_t tiles) { return (til
 // per SM the look-back costs more than that saves (260,000: 114 us with 4, 113 with
 // 8; 400,000: 140 and 139; 1.2 M: 232 and 208), and above one wave of tiles of 8 keys
 // (four blocks an SM) 16 are faster (2.1 M: 336, 310 and 298 us with 4, 8 and 16).
-constexpr uint32_t kSort4Keys = 152u * 4u * kSortThreads;
-constexpr uint32_t kSort8Keys = 4u * 152u * 8u * kSortThreads;
-int sort_items_of(uint32_t n) { return n <= kSort4Keys ? 4 : n <= kSort8Keys ? 8 : kSortItems; }
+uint32_t sort4_keys(int sms) { return (uint32_t)sms * 4u * kSortThreads; }
+uint32_t sort8_keys(int sms) { return 4u * (uint32_t)sms * 8u * kSortThreads; }
+int sort_items_of(uint32_t n, int sms) { return n <= sort4_keys(sms) ? 4 : n <= sort8_keys(sms) ? 8 : kSortItems; }
 
 template <bool SCENE, bool GROUPED = false, int ITEMS = kSortItems>
 __global__ void __launch_bounds__(kSortThreads, 4) k_onesweep(const uint32_t* __restrict__ keys_in,
@@ -2310,8 +2310,9 @@ extern "C" rt_status rt_lbvh_create(rt_ctx* ctx, uint32_t max_tris, uint32_t dep
     l->cap = max_tris;
     l->depth = depth;
     l->num_nodes = 1u << depth;
-    l->sort_tiles_cap = std::max({ceil_div(max_tris, kSortTile), ceil_div(std::min(max_tris, kSort4Keys), 4 * kSortThreads),
-                                  ceil_div(std::min(max_tris, kSort8Keys), 8 * kSortThreads)});
+    l->num_sms = ctx->num_sms;
+    l->sort_tiles_cap = std::max({ceil_div(max_tris, kSortTile), ceil_div(std::min(max_tris, sort4_keys(l->num_sms)), 4 * kSortThreads),
+                                  ceil_div(std::min(max_tris, sort8_keys(l->num_sms)), 8 * kSortThreads)});
     l->emit_tiles_cap = ceil_div(max_tris, kTreeTile);
     l->bounds_blocks = std::max(1u, std::min(ceil_div(3ull * max_tris, 256), (uint32_t)ctx->num_sms * 4));
     const size_t cap = max_tris;
@@ -2408,7 +2409,7 @@ static rt_status launch_build(rt_ctx* ctx, rt_lbvh* l, const float* d_tris, uint
         return RT_OK;
     }
     const uint32_t emit_tiles = ceil_div(n, kTreeTile);
-    const int sort_items = sort_items_of(n);
+    const int sort_items = sort_items_of(n, l->num_sms);
     const uint32_t sort_tiles = ceil_div(n, kSortThreads * sort_items);
     const uint32_t lb_pass = 256 * (sort_tiles + look_groups(sort_tiles));  // tile words, group words
     const uint32_t lb_words = kSortPasses * lb_pass;
@@ -3027,6 +3028,7 @@ extern "C" rt_status rt_batch_create(rt_ctx* ctx, uint32_t n_scenes, const uint3
     b->S = n_scenes;
     b->depth = depth;
     b->total = (uint32_t)total;
+    b->num_sms = ctx->num_sms;
     b->h_tri_off.resize(n_scenes + 1);
     std::vector<uint32_t> chunks;
     b->h_tri_off[0] = 0;
@@ -3041,7 +3043,7 @@ extern "C" rt_status rt_batch_create(rt_ctx* ctx, uint32_t n_scenes, const uint3
     b->nchunks = (uint32_t)(chunks.size() / 3);
     const size_t n = total;
     const size_t num_nodes = (size_t)n_scenes << depth;
-    const uint32_t sort_tiles = ceil_div(n, kSortThreads * sort_items_of((uint32_t)n)), emit_tiles = ceil_div(n, kTreeTile);
+    const uint32_t sort_tiles = ceil_div(n, kSortThreads * sort_items_of((uint32_t)n, b->num_sms)), emit_tiles = ceil_div(n, kTreeTile);
     cudaError_t e = cudaSuccess;
     auto alloc = [&](void** p, size_t bytes) {
         if (e == cudaSuccess) e = cudaMalloc(p, bytes);
@@ -3095,7 +3097,7 @@ extern "C" rt_status rt_batch_build(rt_ctx* ctx, rt_batch* b, const float* d_tri
     if (!b || !d_tris) return rt_fail(ctx, RT_ERR_INVALID, "rt_batch_build: null argument");
     cudaStream_t st = ctx->stream;
     const uint32_t n = b->total, S = b->S;
-    const int sort_items = sort_items_of(n);
+    const int sort_items = sort_items_of(n, b->num_sms);
     const uint32_t sort_tiles = ceil_div(n, kSortThreads * sort_items), emit_tiles = ceil_div(n, kTreeTile);
     const uint32_t lb_pass = 256 * (sort_tiles + look_groups(sort_tiles)), lb_words = 5 * lb_pass;
     const uint32_t num_nodes = S << b->depth;

@@ -191,6 +191,7 @@ struct rt_lbvh {
     uint2* items = nullptr;          // emission items (heap index, mask), 64 for each chunk and group of every merge level
     uint32_t* item_counts = nullptr; // 8 x emit tiles: item counts of every level (6x), tile unit counts, merge tickets
     uint32_t sort_tiles_cap = 0, emit_tiles_cap = 0, bounds_blocks = 0;
+    int num_sms = 0;                 // of the device, when the scratch was sized
     // frame buffers for rt_render_frame_host (grown on demand)
     rt_hit* f_primary = nullptr;
     rt_hit* f_mirror = nullptr;
@@ -220,6 +221,7 @@ void free_batch(rt_batch* b);
 // of the concatenated soup and heap slots [s << depth, (s + 1) << depth).
 struct rt_batch {
     uint32_t S = 0, depth = 0, total = 0;
+    int num_sms = 0;               // of the device, when the scratch was sized
     uint32_t graph_refs = 0;       // captured frames pointing into the batch (see rt_lbvh)
     bool destroy_pending = false;
     std::vector<uint32_t> h_tri_off;
