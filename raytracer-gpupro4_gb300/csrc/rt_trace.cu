@@ -670,7 +670,7 @@ __device__ __forceinline__ void heavy_closest(const HeavyArgs& a, uint32_t entry
     }
 }
 
-__global__ void __launch_bounds__(kTraceThreads, 7) k_trace_heavy(HeavyArgs a) {
+__global__ void __launch_bounds__(kTraceThreads, 6) k_trace_heavy(HeavyArgs a) {
     grid_dep_wait();
     const uint32_t n = min(*a.count, a.cap);
     const int lane = threadIdx.x & 31;
@@ -696,8 +696,10 @@ __global__ void __launch_bounds__(kTraceThreads, 7) k_trace_heavy(HeavyArgs a) {
 
 // A few closest-hit rays, a warp each from the start: with a lane each they fill
 // a handful of warps, and the call lasts as long as the longest chain of dependent
-// loads: 256 rays over 65 k triangles 70 -> 14 us, 16,384 rays 132 -> 72 us; at
-// 32,768 both take 135 us.
+// loads.  256 rays over 65 k triangles 66 -> 19 us; 16,384 rays at a torus of 65 k triangles, at
+// 260 k and in a soup of 200 k 109, 112 and 114 us (lanes 163, 157 and 173), 24,000 152,
+// 158 and 161 (165, 158 and 180).  Rays along an axis of a mesh are the exception: 18,000 over 260 k
+// triangles 116 us, with lanes 82.
 constexpr uint32_t kFewRays = 16384;
 
 __global__ void __launch_bounds__(kTraceThreads) k_rays_wide(TreeRef tr, const rt_ray* __restrict__ rays, uint32_t n,
@@ -714,7 +716,7 @@ __global__ void __launch_bounds__(kTraceThreads) k_rays_wide(TreeRef tr, const r
 // tests, where a warp per ray leaves the GPU waiting on the longest few.  The closest-hit
 // entries come first, a warp each (a block each: 3 us of 1,400 for the mirror rays of
 // 2.1 M triangles at 1080p).
-__global__ void __launch_bounds__(kTeamThreads) k_trace_heavy_team(HeavyArgs a) {
+__global__ void __launch_bounds__(kTeamThreads, 6) k_trace_heavy_team(HeavyArgs a) {
     grid_dep_wait();
     __shared__ TeamShared ts;
     __shared__ uint32_t s_e;

@@ -835,13 +835,13 @@ struct Walk {
         // a leaf of 32 or more triangles: its exact box, with the bound of now, first (of
         // 5 or more, 330 k triangles at 720p took 9 us a frame longer)
         if ((leaf & kBigLeaf) && !inside) {
-            inside = leaf_entered(tr, leaf & kSlotMask);
+            inside = leaf_entered<POOL_MIN>(tr, leaf & kSlotMask);
             if (!inside) cnt = 0u;
         }
         tests += cnt;
         at_leaf += cnt;
         if (__reduce_max_sync(kFull, cnt) > POOL_MIN) {
-            pooled(tr, leaf, pos, cnt, inside);
+            pooled<POOL_MIN>(tr, leaf, pos, cnt, inside);
         } else {
             while (__any_sync(kFull, cnt != 0u)) {
                 if (cnt != 0u) {
@@ -855,7 +855,7 @@ struct Walk {
                     r.o = o;
                     r.d = d;
                     if (id != exclude && tri_test(r, a, bb, c, &u, &v, &t)) {
-                        if (!accept(tr, leaf, hit_key(t, id), id, t, u, v, inside)) cnt = 0u;
+                        if (!accept<POOL_MIN>(tr, leaf, hit_key(t, id), id, t, u, v, inside)) cnt = 0u;
                     }
                 }
                 __syncwarp();
@@ -882,11 +882,12 @@ struct Walk {
 
     // A candidate hit in `leaf`.  Returns false when the leaf's box rejects it,
     // and so every triangle of the leaf.
+    template <uint32_t POOL_MIN>
     __device__ __forceinline__ bool accept(const TreeRef& tr, uint32_t leaf, uint64_t key, int id, float t, float u,
                                            float v, bool& inside) {
         if (!(key < b.key)) return true;
         const uint32_t h = (leaf & kBigLeaf) ? leaf & kSlotMask : __ldg(tr.leaf_of + tr.tri_base + (leaf & 0x1ffffffu));
-        if (!inside && !leaf_entered(tr, h)) return false;
+        if (!inside && !leaf_entered<POOL_MIN>(tr, h)) return false;
         inside = true;
         b.key = key;
         b.t = t;
@@ -900,6 +901,7 @@ struct Walk {
     // The triangles [pos, pos + cnt) of every lane's leaf, 32 (lane, triangle)
     // pairs at a time (see leaf_phase): a lane's 200 triangles cost 7 steps
     // of the warp instead of 200.
+    template <uint32_t POOL_MIN>
     __device__ __forceinline__ void pooled(const TreeRef& tr, uint32_t leaf, uint32_t pos, uint32_t cnt, bool inside) {
         constexpr uint32_t kFull = 0xffffffffu;
         const int lane = threadIdx.x & 31;
@@ -963,13 +965,16 @@ struct Walk {
             const float hu = __shfl_sync(kFull, ku, hs);
             const float hv = __shfl_sync(kFull, kv, hs);
             if (mine && !rejected && hk != ~0ull)
-                rejected = !accept(tr, leaf, hk, (int)(uint32_t)hk, ht, hu, hv, inside);
+                rejected = !accept<POOL_MIN>(tr, leaf, hk, (int)(uint32_t)hk, ht, hu, hv, inside);
             __syncwarp();
         }
     }
 
     // box_enter of the heap box of leaf h, under the bound of now: the leaf may
     // have been put aside, or its parent expanded, before a nearer hit was found.
+    // (A path's ray divides again even where k holds 1 / d: the choice cost the
+    // 56-register kernels 2 %.)
+    template <uint32_t POOL_MIN>
     __device__ __forceinline__ bool leaf_entered(const TreeRef& tr, uint32_t h) const {
         if (h >= tr.num_heap) {
             atomicOr(tr.err, RT_DEVERR_BOUNDS);
@@ -979,7 +984,7 @@ struct Walk {
         RayState r;
         r.o = o;
         r.inv = k;
-        if (!(sgn & kGeneral)) r.inv = mk3(fdiv(1.0f, d.x), fdiv(1.0f, d.y), fdiv(1.0f, d.z));
+        if (POOL_MIN == kPathPoolMin || !(sgn & kGeneral)) r.inv = mk3(fdiv(1.0f, d.x), fdiv(1.0f, d.y), fdiv(1.0f, d.z));
         float t0;
         return enter(r, nb, b.t, &t0, (sgn & kInfinite) != 0u);
     }
@@ -1021,8 +1026,7 @@ __host__ __device__ constexpr uint32_t wide_stack_entries(uint32_t depth) {
 // Dynamic shared memory of a block running traverse_wide or traverse_ordered with
 // `cap` stack entries per warp: stack nodes and entry distances, then the leaves
 // (and pending hits) of each warp.
-constexpr int kWideScratch = 2432;
-static_assert(kWideQueue * 16 <= kWideScratch, "");
+constexpr int kWideScratch = kWideQueue * 16;
 __host__ __device__ constexpr size_t wide_smem_bytes(uint32_t cap) {
     return (size_t)kWideWarps * (cap * 8u + kWideScratch);
 }
@@ -1255,9 +1259,9 @@ __device__ __forceinline__ Hit traverse_wide(const RayState& r, const TreeRef& t
 // distance of a leaf's box can lie above the distance of a hit inside it, and whether the
 // leaf is still entered depends on the hits found before it, so on the order.  The
 // frontier therefore stays in traverse()'s order, the next node on top:
-//   - a step pops up to 32 entries, the next ones in that order, and puts back in
-//     their places the internal children that are entered and, for the leaves among
-//     the children, a hit (the leaf's entry distance and its closest triangle);
+//   - a step takes up to 32 entries, the next ones in that order, and puts back in their
+//     places a node's entered children and a leaf's hit (the leaf's entry distance and its
+//     closest triangle);
 //   - a hit that comes to the top has everything before it behind it: it is accepted
 //     exactly when traverse() would enter its leaf and accept its triangle;
 //   - an entry is dropped early only for what holds at its turn in any case: the
@@ -1270,14 +1274,22 @@ __device__ __forceinline__ Hit traverse_wide(const RayState& r, const TreeRef& t
 // ray alone.  `known`: the hit of a walk in the same order that was broken off (id
 // < 0: none); going over its part again with that bound changes nothing.  `start`: as in
 // traverse().
-constexpr uint32_t kEntryHit = 1u << 31, kEntryLeaf = 1u << 30, kEntryRight = 1u << 29;
-constexpr int kOrderedLeaves = 64, kOrderedHits = 32;
-static_assert(kOrderedLeaves * 28 + kOrderedHits * 20 <= kWideScratch, "");
+// An entry: an internal node as the slot of its children's pair and whether the near child is
+// the right one; a leaf as its count and position, or by its slot when they do not fit
+// (leaf_word's limits); a pending hit.
+constexpr uint32_t kEntryKind = 3u << 30, kEntryNode = 0u, kEntryLeaf = 1u << 30, kEntryHit = 2u << 30,
+                   kEntrySlot = 3u << 30, kEntryRight = 1u << 29;
+constexpr int kOrderedHits = 32;
+constexpr uint32_t kOrderedOwn = 4;  // leaves of more triangles are tested by the warp together
+static_assert(32 * 28 + kOrderedHits * 20 <= kWideScratch, "");
 
 __device__ __forceinline__ uint32_t ordered_entry(const TreeRef& tr, const RayState& r, uint32_t node, float prim_count,
                                                   float prim_pos) {
     const int pc = __float_as_int(prim_count), field = pc & 3;
-    if (pc & 4) return kEntryLeaf | node;
+    if (pc & 4) {
+        const uint32_t pos = (uint32_t)__float_as_int(prim_pos), cnt = (uint32_t)(pc >> 3);
+        return (cnt < 32u && pos < (1u << 25)) ? kEntryLeaf | (cnt << 25) | pos : kEntrySlot | node;
+    }
     return child_pair(tr, node, prim_pos) | (((r.sgn >> (field == 0 ? 2 : field - 1)) & 1u) ? kEntryRight : 0u);
 }
 
@@ -1303,13 +1315,13 @@ __device__ __forceinline__ Hit traverse_ordered(const RayState& r, const TreeRef
     float* st0 = ws.st0;
     // the leaves of a step, in order
     uint64_t* qbest = reinterpret_cast<uint64_t*>(ws.scratch);
-    uint64_t* pkey = qbest + kOrderedLeaves;  // the pending hits
+    uint64_t* pkey = qbest + 32;  // the pending hits
     float* qt = reinterpret_cast<float*>(pkey + kOrderedHits);
-    float* qu = qt + kOrderedLeaves;
-    float* qv = qu + kOrderedLeaves;
-    int32_t* qpos = reinterpret_cast<int32_t*>(qv + kOrderedLeaves);
-    uint32_t* qincl = reinterpret_cast<uint32_t*>(qpos + kOrderedLeaves);
-    float* pt = reinterpret_cast<float*>(qincl + kOrderedLeaves);
+    float* qu = qt + 32;
+    float* qv = qu + 32;
+    uint32_t* qpos = reinterpret_cast<uint32_t*>(qv + 32);
+    uint32_t* qincl = qpos + 32;
+    float* pt = reinterpret_cast<float*>(qincl + 32);
     float* pu = pt + kOrderedHits;
     float* pv = pu + kOrderedHits;
     const uint64_t init = hit_key(r.tmax, 0);
@@ -1346,8 +1358,8 @@ __device__ __forceinline__ Hit traverse_ordered(const RayState& r, const TreeRef
     while (size > 0 && !alone) {
         {  // a hit on top: its turn
             const uint32_t e = snode[size - 1];
-            if (e & kEntryHit) {
-                const uint32_t q = e & ~kEntryHit;
+            if ((e & kEntryKind) == kEntryHit) {
+                const uint32_t q = e & ~kEntryKind;
                 const uint64_t key = pkey[q];
                 if (key < best && !(st0[size - 1] > key_t(best))) {
                     best = key;
@@ -1369,8 +1381,8 @@ __device__ __forceinline__ Hit traverse_ordered(const RayState& r, const TreeRef
             t0 = st0[size - 1 - lane];
         }
         float bound = key_t(best);  // at this entry's turn it is this at most
-        const bool is_hit = (e & kEntryHit) != 0u;
-        const uint32_t q_hit = e & ~kEntryHit;
+        const bool is_hit = (e & kEntryKind) == kEntryHit;
+        const uint32_t q_hit = e & ~kEntryKind;
         float hit_t = 0.0f;
         if (__any_sync(kFull, is_hit)) {
             if (is_hit) hit_t = key_t(pkey[q_hit]);
@@ -1385,143 +1397,167 @@ __device__ __forceinline__ Hit traverse_ordered(const RayState& r, const TreeRef
         }
         size -= k;
         __syncwarp();
-        // what takes the entry's place: up to two entries, or leaves to test
+        // what takes the entry's place: up to two entries.  A node's children and a leaf's
+        // first triangle are loaded together.
         uint32_t o[2] = {0u, 0u};
         float ot[2] = {0.0f, 0.0f};
-        int pos[2] = {0, 0}, cnt[2] = {0, 0};
-        bool nan = false;
-        if (e && !(t0 > bound)) {
-            if (is_hit) {
-                if (!(hit_t > bound)) {
-                    o[0] = e;
-                    ot[0] = t0;
-                }
-            } else if (e & kEntryLeaf) {
-                const float4 b = load_node(tr_.nodes, e & ~kEntryLeaf).b;
-                pos[0] = __float_as_int(b.w);
-                cnt[0] = __float_as_int(b.z) >> 3;
+        bool live = e != 0u && !(t0 > bound);
+        uint32_t cnt = 0u, pos = 0u;
+        const float4* p = reinterpret_cast<const float4*>(tr_.nodes);
+        if (live && is_hit) {
+            if (!(hit_t > bound)) {
+                o[0] = e;
                 ot[0] = t0;
-            } else {
-                const uint32_t c0 = e & ~kEntryRight;
-                if (c0 + 1 >= tr_.num_nodes) {
-                    atomicOr(tr_.err, RT_DEVERR_BOUNDS);
-                } else {
-                    const float4* p = reinterpret_cast<const float4*>(tr_.nodes + c0);
-                    const float4 l0 = __ldg(p), l1 = __ldg(p + 1), r0 = __ldg(p + 2), r1 = __ldg(p + 3);
-                    float tl, tr;
-                    const bool hl = box_enter<EXACT>(r, l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, bound, &tl);
-                    const bool hr = box_enter<EXACT>(r, r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, bound, &tr);
-                    nan = EXACT && ((hl && isnan(tl)) || (hr && isnan(tr)));
-                    const bool right = (e & kEntryRight) != 0u;
-#pragma unroll
-                    for (int c = 0; c < 2; ++c) {  // the near child, then the far one
-                        const bool rc = right == (c == 0);
-                        if (!(rc ? hr : hl)) continue;
-                        const float pc = rc ? r1.z : l1.z, pp = rc ? r1.w : l1.w;
-                        ot[c] = rc ? tr : tl;
-                        if (__float_as_int(pc) & 4) {
-                            pos[c] = __float_as_int(pp);
-                            cnt[c] = __float_as_int(pc) >> 3;
-                        } else {
-                            o[c] = ordered_entry(tr_, r, c0 + (rc ? 1u : 0u), pc, pp);
-                        }
-                    }
-                }
             }
-#pragma unroll
-            for (int c = 0; c < 2; ++c)
-                if (!leaf_in_range((uint32_t)pos[c], (uint32_t)cnt[c], tr_.n)) {
-                    atomicOr(tr_.err, RT_DEVERR_BOUNDS);
-                    cnt[c] = 0;
-                }
+            live = false;
+        } else if (live && (e & kEntryKind) == kEntryNode) {
+            if ((e & ~kEntryRight) + 1u >= tr_.num_nodes) {
+                atomicOr(tr_.err, RT_DEVERR_BOUNDS);
+                live = false;
+            } else {
+                p += 2 * (size_t)(e & ~kEntryRight);
+            }
+        } else if (live) {
+            pos = e & 0x1ffffffu;
+            cnt = (e >> 25) & 31u;
+            if ((e & kEntryKind) == kEntrySlot) {
+                const float4 b = load_node(tr_.nodes, e & ~kEntryKind).b;
+                pos = (uint32_t)__float_as_int(b.w);
+                cnt = (uint32_t)(__float_as_int(b.z) >> 3);
+            }
+            if (!leaf_in_range(pos, cnt, tr_.n)) {
+                atomicOr(tr_.err, RT_DEVERR_BOUNDS);
+                cnt = 0u;
+            }
+            live = cnt != 0u;
+            if (live) p = tr_.tris + 3 * (size_t)pos;
         }
-        if (EXACT && __any_sync(kFull, nan)) {
-            alone = true;
-            break;
+        float4 x0 = make_float4(0.f, 0.f, 0.f, 0.f), x1 = x0, x2 = x0, x3 = x0;
+        if (live) {
+            x0 = __ldg(p);
+            x1 = __ldg(p + 1);
+            x2 = __ldg(p + 2);
+            x3 = __ldg(p + (cnt ? 2 : 3));
         }
         {  // the hits that were dropped
             const uint32_t gone = __ballot_sync(kFull, is_hit && o[0] == 0u);
             if (gone) used &= ~__reduce_or_sync(kFull, (gone >> lane) & 1u ? 1u << q_hit : 0u);
         }
-        // the leaves, 32 (leaf, triangle) pairs at a time
-        const uint32_t la = __ballot_sync(kFull, cnt[0] > 0), lb = __ballot_sync(kFull, cnt[1] > 0);
-        if (la | lb) {
-            const int q0 = __popc(la & lt) + __popc(lb & lt), q1 = q0 + (cnt[0] > 0 ? 1 : 0);
-            const int nq = __popc(la) + __popc(lb);
-            uint32_t incl = (uint32_t)(cnt[0] + cnt[1]);
-#pragma unroll
-            for (int off = 1; off < 32; off <<= 1) {
-                const uint32_t y = __shfl_up_sync(kFull, incl, off);
-                if (lane >= off) incl += y;
-            }
-            const uint32_t total = __shfl_sync(kFull, incl, 31);
-            if (cnt[0] > 0) {
-                qpos[q0] = pos[0];
-                qincl[q0] = incl - (uint32_t)cnt[1];
-                qbest[q0] = ~0ull;
-            }
-            if (cnt[1] > 0) {
-                qpos[q1] = pos[1];
-                qincl[q1] = incl;
-                qbest[q1] = ~0ull;
-            }
-            __syncwarp();
-            for (uint32_t base = 0; base < total; base += 32 * kWidePairs) {
-                float4 va[kWidePairs], vb[kWidePairs], vc[kWidePairs];
-                int leaf[kWidePairs];
-#pragma unroll
-                for (int q = 0; q < kWidePairs; ++q) {
-                    const uint32_t p = min(base + 32u * q + lane, total - 1u);  // past the end: the last pair again
-                    int lo = 0, hi = nq - 1;  // the first leaf with inclusive prefix > p
-                    while (lo < hi) {
-                        const int mid = (lo + hi) >> 1;
-                        if (qincl[mid] > p) hi = mid; else lo = mid + 1;
+        const uint32_t most = __reduce_max_sync(kFull, cnt);
+        bool nan = false;
+        if (live && cnt == 0u) {
+            float tl, tr;
+            const bool hl = box_enter<EXACT>(r, x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, bound, &tl);
+            const bool hr = box_enter<EXACT>(r, x2.x, x2.y, x2.z, x2.w, x3.x, x3.y, bound, &tr);
+            nan = EXACT && ((hl && isnan(tl)) || (hr && isnan(tr)));
+            const uint32_t c0 = e & ~kEntryRight;
+            const uint32_t l = hl ? ordered_entry(tr_, r, c0, x1.z, x1.w) : 0u;
+            const uint32_t rr = hr ? ordered_entry(tr_, r, c0 + 1u, x3.z, x3.w) : 0u;
+            const bool right = (e & kEntryRight) != 0u;  // the near child, then the far one
+            o[0] = right ? rr : l;
+            ot[0] = right ? tr : tl;
+            o[1] = right ? l : rr;
+            ot[1] = right ? tl : tr;
+        }
+        if (EXACT && __any_sync(kFull, nan)) {
+            alone = true;
+            break;
+        }
+        if (most != 0u) {
+            uint64_t key = ~0ull;
+            float kt = 0.0f, ku = 0.0f, kv = 0.0f;
+            auto test = [&](const float4& va, const float4& vb, const float4& vc) {
+                const int id = __float_as_int(va.w);
+                float u, v, t;
+                if (id != r.exclude && tri_test(r, va, vb, vc, &u, &v, &t)) {
+                    const uint64_t q = hit_key(t, id);
+                    if (q < best && q < key) {
+                        key = q;
+                        kt = t;
+                        ku = u;
+                        kv = v;
                     }
-                    leaf[q] = lo;
-                    const float4* tp = tr_.tris + 3 * (size_t)(qpos[lo] + (int)(p - (lo > 0 ? qincl[lo - 1] : 0u)));
-                    va[q] = __ldg(tp);
-                    vb[q] = __ldg(tp + 1);
-                    vc[q] = __ldg(tp + 2);
                 }
+            };
+            if (most <= kOrderedOwn) {
+                if (cnt) test(x0, x1, x2);
+                for (uint32_t j = 1; j < most; ++j)
+                    if (j < cnt) test(__ldg(p + 3 * j), __ldg(p + 3 * j + 1), __ldg(p + 3 * j + 2));
+            } else {  // 32 (leaf, triangle) pairs at a time
+                const uint32_t m = __ballot_sync(kFull, cnt != 0u);
+                const int q0 = __popc(m & lt), nq = __popc(m);
+                uint32_t incl = cnt;
 #pragma unroll
-                for (int q = 0; q < kWidePairs; ++q) {
-                    const int id = __float_as_int(va[q].w);
-                    float u = 0.0f, v = 0.0f, t = 0.0f;
-                    uint64_t key = ~0ull;
-                    if (id != r.exclude && tri_test(r, va[q], vb[q], vc[q], &u, &v, &t)) key = hit_key(t, id);
-                    const bool in = key < best;
-                    if (!__any_sync(kFull, in)) continue;
-                    if (in) atomicMin(reinterpret_cast<unsigned long long*>(qbest + leaf[q]), (unsigned long long)key);
-                    __syncwarp();
-                    if (in && qbest[leaf[q]] == key) {
-                        qt[leaf[q]] = t;
-                        qu[leaf[q]] = u;
-                        qv[leaf[q]] = v;
+                for (int off = 1; off < 32; off <<= 1) {
+                    const uint32_t y = __shfl_up_sync(kFull, incl, off);
+                    if (lane >= off) incl += y;
+                }
+                const uint32_t total = __shfl_sync(kFull, incl, 31);
+                if (cnt) {
+                    qpos[q0] = pos;
+                    qincl[q0] = incl;
+                    qbest[q0] = ~0ull;
+                }
+                __syncwarp();
+                for (uint32_t base = 0; base < total; base += 32 * kWidePairs) {
+                    float4 va[kWidePairs], vb[kWidePairs], vc[kWidePairs];
+                    int leaf[kWidePairs];
+#pragma unroll
+                    for (int q = 0; q < kWidePairs; ++q) {
+                        const uint32_t pr = min(base + 32u * q + lane, total - 1u);  // past the end: the last pair again
+                        int lo = 0, hi = nq - 1;  // the first leaf with inclusive prefix > pr
+                        while (lo < hi) {
+                            const int mid = (lo + hi) >> 1;
+                            if (qincl[mid] > pr) hi = mid; else lo = mid + 1;
+                        }
+                        leaf[q] = lo;
+                        const float4* tp = tr_.tris + 3 * (size_t)(qpos[lo] + (pr - (lo > 0 ? qincl[lo - 1] : 0u)));
+                        va[q] = __ldg(tp);
+                        vb[q] = __ldg(tp + 1);
+                        vc[q] = __ldg(tp + 2);
                     }
-                    __syncwarp();
+#pragma unroll
+                    for (int q = 0; q < kWidePairs; ++q) {
+                        key = ~0ull;
+                        test(va[q], vb[q], vc[q]);
+                        const bool in = key != ~0ull;
+                        if (!__any_sync(kFull, in)) continue;
+                        if (in) atomicMin(reinterpret_cast<unsigned long long*>(qbest + leaf[q]), (unsigned long long)key);
+                        __syncwarp();
+                        if (in && qbest[leaf[q]] == key) {
+                            qt[leaf[q]] = kt;
+                            qu[leaf[q]] = ku;
+                            qv[leaf[q]] = kv;
+                        }
+                        __syncwarp();
+                    }
+                }
+                key = ~0ull;
+                if (cnt) {
+                    key = qbest[q0];
+                    kt = qt[q0];
+                    ku = qu[q0];
+                    kv = qv[q0];
                 }
             }
-            const uint64_t k0 = cnt[0] > 0 ? qbest[q0] : ~0ull, k1 = cnt[1] > 0 ? qbest[q1] : ~0ull;
-            const bool h0 = k0 != ~0ull && !(key_t(k0) > bound), h1 = k1 != ~0ull && !(key_t(k1) > bound);
-            const uint32_t ha = __ballot_sync(kFull, h0), hb = __ballot_sync(kFull, h1);
-            if (ha | hb) {
-                if (__popc(ha) + __popc(hb) > kOrderedHits - __popc(used)) {
+            const bool found = key != ~0ull && !(key_t(key) > bound);
+            const uint32_t m = __ballot_sync(kFull, found);
+            if (m) {
+                if (__popc(m) > kOrderedHits - __popc(used)) {
                     alone = true;
                     break;
                 }
-                const uint32_t rank = (uint32_t)(__popc(ha & lt) + __popc(hb & lt));
                 uint32_t mine = 0u;
-                auto put = [&](int q, uint64_t key, uint32_t nth) {
-                    const uint32_t slot = __fns(~used, 0, (int)nth + 1);
+                if (found) {
+                    const uint32_t slot = __fns(~used, 0, __popc(m & lt) + 1);
                     pkey[slot] = key;
-                    pt[slot] = qt[q];
-                    pu[slot] = qu[q];
-                    pv[slot] = qv[q];
-                    mine |= 1u << slot;
-                    return kEntryHit | slot;
-                };
-                if (h0) o[0] = put(q0, k0, rank);
-                if (h1) o[1] = put(q1, k1, rank + (h0 ? 1u : 0u));
+                    pt[slot] = kt;
+                    pu[slot] = ku;
+                    pv[slot] = kv;
+                    mine = 1u << slot;
+                    o[0] = kEntryHit | slot;
+                    ot[0] = t0;
+                }
                 used |= __reduce_or_sync(kFull, mine);
             }
         }
