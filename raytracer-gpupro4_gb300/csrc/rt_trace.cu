@@ -175,7 +175,8 @@ __global__ void __launch_bounds__(kTraceThreads, BLOCKS) k_walk_primary(TreeRef 
         if (!valid) i = j = 0;  // lanes past the image edge only help the warp
         int slot = -1;
         w.tests = 0u;
-        w.start(valid, make_ray(mk3(cam.eye[0], cam.eye[1], cam.eye[2]), primary_dir(cam, i, j), 1e16f, -1), tr, 1u, stack);
+        const RayState r = make_ray(mk3(cam.eye[0], cam.eye[1], cam.eye[2]), primary_dir(cam, i, j), 1e16f, -1);
+        w.start(valid, r, tr, 1u, stack, Walk::tile_by_heap(valid, r, tr));
         while (__any_sync(kFull, w.have)) {
             w.round(tr, kPrimSteps, stack);
             if (w.have && budgeted && w.tests > spill.budget) {
@@ -670,16 +671,19 @@ __device__ __forceinline__ void heavy_closest(const HeavyArgs& a, uint32_t entry
     }
 }
 
-__global__ void __launch_bounds__(kTraceThreads, 6) k_trace_heavy(HeavyArgs a) {
+// ANY: the list holds a caller's any-hit rays alone (the ordered walk's registers would cost such
+// calls a block per SM).
+template <bool ANY>
+__global__ void __launch_bounds__(kTraceThreads, ANY ? 7 : 6) k_trace_heavy(HeavyArgs a) {
     grid_dep_wait();
     const uint32_t n = min(*a.count, a.cap);
     const int lane = threadIdx.x & 31;
     for (uint32_t e = next_tile(a.work); e < n; e = next_tile(a.work)) {
         const uint32_t entry = __ldg(a.list + e);
         const uint32_t idx = entry & kHeavyIndexMask;
-        if (!heavy_any_hit(a, entry)) {
+        if (!ANY && !heavy_any_hit(a, entry)) {
             heavy_closest(a, entry);
-        } else if ((entry >> 30) == kHeavyRay) {
+        } else if (ANY || (entry >> 30) == kHeavyRay) {
             const Hit h = trace_wide(load_ray(a.rays, idx, true), a.tr, a.wide_cap);
             if (lane == 0) {
                 store_hit(a.hits + idx, h);
@@ -892,11 +896,11 @@ rt_status launch_heavy(rt_ctx* ctx, const Spill& sp, HeavyArgs a, int kind) {
         return RT_OK;
     }
     const size_t smem = wide_smem_bytes(a.wide_cap);
+    const auto k = kind == 2 && a.any_hit ? k_trace_heavy<true> : k_trace_heavy<false>;
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_trace_heavy, kTraceThreads, smem) != cudaSuccess ||
-        per_sm < 1)
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kTraceThreads, smem) != cudaSuccess || per_sm < 1)
         per_sm = 1;
-    launch_pdl(k_trace_heavy, (uint32_t)per_sm * ctx->num_sms, kTraceThreads, smem, ctx->stream, a);
+    launch_pdl(k, (uint32_t)per_sm * ctx->num_sms, kTraceThreads, smem, ctx->stream, a);
     RT_CHECK_LAUNCH(ctx, "k_trace_heavy");
     return RT_OK;
 }
@@ -1485,8 +1489,8 @@ __device__ __forceinline__ void batch_trace_body(const BatchTraceArgs& a, const 
             uint32_t i, j;
             const bool valid = tile_pixel(tile, lane, a.width, a.height, &i, &j);
             if (!valid) i = j = 0;
-            const f3 d = primary_dir(cam, i, j);
-            w.start(valid, make_ray(mk3(cam.eye[0], cam.eye[1], cam.eye[2]), d, 1e16f, -1), tr, 1u, stack);
+            const RayState r = make_ray(mk3(cam.eye[0], cam.eye[1], cam.eye[2]), primary_dir(cam, i, j), 1e16f, -1);
+            w.start(valid, r, tr, 1u, stack, Walk::tile_by_heap(valid, r, tr));
             while (__any_sync(0xffffffffu, w.have)) w.round(tr, kBatchSteps, stack);
             const Hit h = w.hit();
             const uint32_t leaf = w.b.leaf;

@@ -654,11 +654,28 @@ struct Walk {
                    : box_enter<false>(r, nb.a.x, nb.a.y, nb.a.z, nb.a.w, nb.b.x, nb.b.y, bt, t0);
     }
 
+    // Whether the records of a tree with grid g serve ray r.
+    static __device__ __forceinline__ bool served(const RayState& r, float4 g) {
+        const float E = fabsf(g.w);
+        const f3 k = mk3(fmul(E, r.inv.x), fmul(E, r.inv.y), fmul(E, r.inv.z));
+        const f3 q = mk3(fsub(g.x, r.o.x), fsub(g.y, r.o.y), fsub(g.z, r.o.z));
+        const float kmax = max3(fabsf(k.x), fabsf(k.y), fabsf(k.z)), kmin = min3(fabsf(k.x), fabsf(k.y), fabsf(k.z));
+        return max3(fabsf(q.x), fabsf(q.y), fabsf(q.z)) <= 16.0f * E && kmax < 1e30f && kmin > 1e-30f;
+    }
+    // Whether a tile's rays (one of each lane with take) are walked over the heap: where
+    // one is, as in the centre column and row of an image of odd size, the warp would
+    // otherwise take both kinds of steps one after the other.
+    static __device__ __forceinline__ bool tile_by_heap(bool take, const RayState& r, const TreeRef& tr) {
+        float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (tr.tnodes) g = __ldg(reinterpret_cast<const float4*>(tr.tnodes));
+        return __any_sync(0xffffffffu, take && !served(r, g));
+    }
+
     // Lanes with take begin ray r at heap node `first` (<= 1: the root; see
-    // traverse).  counted: over the heap records whatever the ray, so that every test is
+    // traverse).  by_heap: over the heap records whatever the ray, so that every test is
     // traverse()'s and `at_leaf` its count.
     __device__ __forceinline__ void start(bool take, const RayState& r, const TreeRef& tr, uint32_t first, uint2* stack,
-                                          bool counted = false) {
+                                          bool by_heap = false) {
         if (!take) return;
         o = r.o;
         d = r.d;
@@ -682,8 +699,7 @@ struct Walk {
         k = mk3(fmul(g.w, r.inv.x), fmul(g.w, r.inv.y), fmul(g.w, r.inv.z));
         const f3 q = mk3(fsub(g.x, o.x), fsub(g.y, o.y), fsub(g.z, o.z));
         n = mk3(fmul(q.x, r.inv.x), fmul(q.y, r.inv.y), fmul(q.z, r.inv.z));
-        const float kmax = max3(fabsf(k.x), fabsf(k.y), fabsf(k.z)), kmin = min3(fabsf(k.x), fabsf(k.y), fabsf(k.z));
-        const bool gen = counted || !(max3(fabsf(q.x), fabsf(q.y), fabsf(q.z)) <= 16.0f * g.w && kmax < 1e30f && kmin > 1e-30f);
+        const bool gen = by_heap || !served(r, g);
         if (gen) {
             sgn |= kGeneral;
             k = r.inv;
