@@ -271,8 +271,8 @@ rt_status rt_trace_rays(rt_ctx* ctx, const rt_lbvh* lbvh, const rt_ray* d_rays, 
  * dependence every walk has between two triangles hit within an ulp of each
  * other); a ray leaving a surface near its last hit reaches fewer boxes.  A start of 0 or 1 is the root; any
  * other start must be a node the current build reached, such as a leaf one
- * of these calls reported (1 is reported for a miss, for a ray handed to the
- * warp-per-ray pass, and for every ray when the compact layout is built).
+ * of these calls reported (1 is reported for a miss, for an any-hit ray handed to the
+ * second pass, and for every ray when the compact layout is built).
  * d_leaves / d_mirror_leaves (nullable): the heap node whose triangles gave
  * each closest hit. */
 rt_status rt_trace_primary_leaves(rt_ctx* ctx, const rt_lbvh* lbvh, const rt_camera* cam, rt_hit* d_hits,

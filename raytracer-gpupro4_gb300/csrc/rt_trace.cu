@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(kTraceThreads, BLOCKS) k_walk_primary(TreeRef 
         if (valid) {
             store_hit(hits + p, h);  // of a handed-over ray: the closest hit so far
             if (slot >= 0) spill_record(list, slot, kHeavyPrimary, p);
-            else if (leaves) leaves[p] = leaf;
+            if (leaves) leaves[p] = leaf;
         }
         if (sl.lists) {  // uniform; a handed-over pixel is set up by the warp-per-ray pass
             const int4 ph = make_int4(h.id, __float_as_int(h.u), __float_as_int(h.v), __float_as_int(h.t));
@@ -392,7 +392,7 @@ __global__ void __launch_bounds__(kTraceThreads, BATCH ? 8 : 7) k_walk_shade(
             if (slot >= 0) spill_record(list, slot, shadow ? kHeavyShadow : kHeavyMirror, p);
             if (!shadow) {
                 store_hit(mirror + p, w.hit());  // of a handed-over ray: the closest hit so far
-                if (mirror_leaves && slot < 0) mirror_leaves[p] = tr.compact ? 1u : w.b.leaf;
+                if (mirror_leaves) mirror_leaves[p] = tr.compact ? 1u : w.b.leaf;
             } else if (slot < 0) {
                 vis[p] = vis_code(true, true, w.b.id >= 0);
             }
@@ -483,7 +483,7 @@ __global__ void __launch_bounds__(kTraceThreads, kRayBlocks) k_walk_rays(TreeRef
             } else {
                 store_hit(hits + k, w.hit());
                 if (slot >= 0) spill_record(list, slot, kHeavyRay, k);
-                else if (leaves) leaves[k] = tr.compact ? 1u : w.b.leaf;
+                if (leaves) leaves[k] = tr.compact ? 1u : w.b.leaf;
             }
             live = false;
         }
@@ -571,7 +571,7 @@ __global__ void __launch_bounds__(kTraceThreads) k_trace_rays(TreeRef tr, const 
         if (valid) {
             store_hit(hits + k, h);  // of a handed-over ray: the closest hit so far
             if (slot >= 0) spill_record(list, slot, kHeavyRay, k);
-            else if (leaves) leaves[k] = leaf;
+            if (leaves) leaves[k] = leaf;
             if (STATS) {
                 stats[2 * k] = nb;
                 stats[2 * k + 1] = nt;
@@ -660,14 +660,17 @@ __device__ __forceinline__ void heavy_closest(const HeavyArgs& a, uint32_t entry
         out = a.mirror + idx;
         leaves = a.mirror_leaves;
     }
-    const Hit h = trace_ordered(r, a.tr, a.wide_cap, hit_so_far(out), start);
+    uint32_t leaf = 1u;
+    const Hit h = trace_ordered(r, a.tr, a.wide_cap, hit_so_far(out), start, leaves ? &leaf : nullptr);
+    if (leaves && leaf == 0u) leaf = __ldcg(leaves + idx);  // the first pass's
+    __syncwarp();
     if (lane == 0) {
         store_hit(out, h);
-        if (leaves) leaves[idx] = 1u;  // the root: a valid restart node
+        if (leaves) leaves[idx] = leaf;
     }
     if (kind == kHeavyPrimary && a.sl.lists) {
         const int4 ph = make_int4(h.id, __float_as_int(h.u), __float_as_int(h.v), __float_as_int(h.t));
-        shade_setup_pixel(a.sl, a.cam, ph, lane == 0, idx % a.cam.width, idx / a.cam.width, idx, 1u);
+        shade_setup_pixel(a.sl, a.cam, ph, lane == 0, idx % a.cam.width, idx / a.cam.width, idx, leaf);
     }
 }
 
@@ -711,7 +714,7 @@ __global__ void __launch_bounds__(kTraceThreads) k_rays_wide(TreeRef tr, const r
     grid_dep_wait();
     const uint32_t k = blockIdx.x * kWideWarps + (threadIdx.x >> 5);
     if (k >= n) return;
-    const Hit h = trace_ordered(load_ray(rays, k, true), tr, cap, no_hit(), 1u);
+    const Hit h = trace_ordered(load_ray(rays, k, true), tr, cap, no_hit(), 1u, nullptr);
     if ((threadIdx.x & 31) == 0) store_hit(hits + k, h);
 }
 

@@ -1289,7 +1289,7 @@ __device__ __forceinline__ Hit traverse_wide(const RayState& r, const TreeRef& t
 // face of a box), and when the pending hits or the stack overflow, one lane walks the
 // ray alone.  `known`: the hit of a walk in the same order that was broken off (id
 // < 0: none); going over its part again with that bound changes nothing.  `start`: as in
-// traverse().
+// traverse().  `leaf` (nullable): the hit's leaf, 0 where the known hit stays.
 // An entry: an internal node as the slot of its children's pair and whether the near child is
 // the right one; a leaf as its count and position, or by its slot when they do not fit
 // (leaf_word's limits); a pending hit.
@@ -1297,22 +1297,23 @@ constexpr uint32_t kEntryKind = 3u << 30, kEntryNode = 0u, kEntryLeaf = 1u << 30
                    kEntrySlot = 3u << 30, kEntryRight = 1u << 29;
 constexpr int kOrderedHits = 32;
 constexpr uint32_t kOrderedOwn = 4;  // leaves of more triangles are tested by the warp together
-static_assert(32 * 28 + kOrderedHits * 20 <= kWideScratch, "");
+static_assert(32 * 28 + kOrderedHits * 24 <= kWideScratch, "");
 
 __device__ __forceinline__ uint32_t ordered_entry(const TreeRef& tr, const RayState& r, uint32_t node, float prim_count,
-                                                  float prim_pos) {
+                                                  float prim_pos, bool by_slot) {
     const int pc = __float_as_int(prim_count), field = pc & 3;
     if (pc & 4) {
         const uint32_t pos = (uint32_t)__float_as_int(prim_pos), cnt = (uint32_t)(pc >> 3);
-        return (cnt < 32u && pos < (1u << 25)) ? kEntryLeaf | (cnt << 25) | pos : kEntrySlot | node;
+        return (cnt < 32u && pos < (1u << 25) && !by_slot) ? kEntryLeaf | (cnt << 25) | pos : kEntrySlot | node;
     }
     return child_pair(tr, node, prim_pos) | (((r.sgn >> (field == 0 ? 2 : field - 1)) & 1u) ? kEntryRight : 0u);
 }
 
 // traverse() by one lane of the warp (out of line: rare).
 template <bool EXACT>
-__device__ __noinline__ Hit traverse_alone(const RayState& r, const TreeRef& tr, uint32_t start) {
-    Hit h = traverse<EXACT, false>(r, (threadIdx.x & 31) == 0, tr, false, nullptr, nullptr, nullptr, nullptr, start);
+__device__ __noinline__ Hit traverse_alone(const RayState& r, const TreeRef& tr, uint32_t start, uint32_t* leaf) {
+    Hit h = traverse<EXACT, false>(r, (threadIdx.x & 31) == 0, tr, false, nullptr, nullptr, nullptr, nullptr, start, leaf);
+    *leaf = __shfl_sync(0xffffffffu, *leaf, 0);
     h.id = __shfl_sync(0xffffffffu, h.id, 0);
     h.u = __shfl_sync(0xffffffffu, h.u, 0);
     h.v = __shfl_sync(0xffffffffu, h.v, 0);
@@ -1322,8 +1323,10 @@ __device__ __noinline__ Hit traverse_alone(const RayState& r, const TreeRef& tr,
 
 template <bool EXACT>
 __device__ __forceinline__ Hit traverse_ordered(const RayState& r, const TreeRef& tr_, uint32_t cap, const Hit& known,
-                                                uint32_t start) {
+                                                uint32_t start, uint32_t* leaf) {
     constexpr uint32_t kFull = 0xffffffffu;
+    // leaves by their slots where leaf_of does not name them
+    const bool by_slot = leaf && (!tr_.tnodes || signbit(__ldg(reinterpret_cast<const float4*>(tr_.tnodes)).w));
     const int lane = threadIdx.x & 31;
     const uint32_t lt = (1u << lane) - 1u;
     const WideSmem ws = wide_smem(cap);
@@ -1340,6 +1343,8 @@ __device__ __forceinline__ Hit traverse_ordered(const RayState& r, const TreeRef
     float* pt = reinterpret_cast<float*>(qincl + 32);
     float* pu = pt + kOrderedHits;
     float* pv = pu + kOrderedHits;
+    uint32_t* pleaf = reinterpret_cast<uint32_t*>(pv + kOrderedHits);
+    uint32_t best_leaf = 0u;  // the leaf entry of the best hit (0: known's)
     const uint64_t init = hit_key(r.tmax, 0);
     uint64_t best = known.id >= 0 ? hit_key(known.t, known.id) : init;  // uniform across the warp
     float bu = known.u, bv = known.v, bt = known.t;
@@ -1360,7 +1365,7 @@ __device__ __forceinline__ Hit traverse_ordered(const RayState& r, const TreeRef
             const uint32_t node = lane < D ? (first >> (D - 1 - lane)) ^ 1u : first;
             const NodeBox nb = load_node(tr_.nodes, node);
             if (box_enter<EXACT>(r, nb.a.x, nb.a.y, nb.a.z, nb.a.w, nb.b.x, nb.b.y, key_t(best), &t0))
-                e = ordered_entry(tr_, r, node, nb.b.z, nb.b.w);
+                e = ordered_entry(tr_, r, node, nb.b.z, nb.b.w, by_slot);
         }
         const uint32_t m = __ballot_sync(kFull, e != 0u);
         if (e) {
@@ -1382,6 +1387,7 @@ __device__ __forceinline__ Hit traverse_ordered(const RayState& r, const TreeRef
                     bt = pt[q];
                     bu = pu[q];
                     bv = pv[q];
+                    if (leaf) best_leaf = pleaf[q];
                 }
                 used &= ~(1u << q);
                 --size;
@@ -1467,8 +1473,8 @@ __device__ __forceinline__ Hit traverse_ordered(const RayState& r, const TreeRef
             const bool hr = box_enter<EXACT>(r, x2.x, x2.y, x2.z, x2.w, x3.x, x3.y, bound, &tr);
             nan = EXACT && ((hl && isnan(tl)) || (hr && isnan(tr)));
             const uint32_t c0 = e & ~kEntryRight;
-            const uint32_t l = hl ? ordered_entry(tr_, r, c0, x1.z, x1.w) : 0u;
-            const uint32_t rr = hr ? ordered_entry(tr_, r, c0 + 1u, x3.z, x3.w) : 0u;
+            const uint32_t l = hl ? ordered_entry(tr_, r, c0, x1.z, x1.w, by_slot) : 0u;
+            const uint32_t rr = hr ? ordered_entry(tr_, r, c0 + 1u, x3.z, x3.w, by_slot) : 0u;
             const bool right = (e & kEntryRight) != 0u;  // the near child, then the far one
             o[0] = right ? rr : l;
             ot[0] = right ? tr : tl;
@@ -1570,6 +1576,7 @@ __device__ __forceinline__ Hit traverse_ordered(const RayState& r, const TreeRef
                     pt[slot] = kt;
                     pu[slot] = ku;
                     pv[slot] = kv;
+                    if (leaf) pleaf[slot] = e;
                     mine = 1u << slot;
                     o[0] = kEntryHit | slot;
                     ot[0] = t0;
@@ -1596,7 +1603,17 @@ __device__ __forceinline__ Hit traverse_ordered(const RayState& r, const TreeRef
         size += total;
         __syncwarp();
     }
-    if (alone) return traverse_alone<EXACT>(r, tr_, start);
+    if (alone) {
+        uint32_t l = 1u;
+        const Hit h = traverse_alone<EXACT>(r, tr_, start, &l);
+        if (leaf) *leaf = l;
+        return h;
+    }
+    if (leaf)
+        *leaf = tr_.compact || (best >= init) ? 1u
+                : best_leaf == 0u                                ? 0u
+                : (best_leaf & kEntryKind) == kEntrySlot         ? best_leaf & ~kEntryKind
+                                                                 : __ldg(tr_.leaf_of + (best_leaf & 0x1ffffffu));
     Hit h;
     if (best < init) {
         h.id = (int)(uint32_t)best;
@@ -1890,9 +1907,9 @@ __device__ __forceinline__ Hit trace_wide(const RayState& r, const TreeRef& tr, 
 
 // One closest-hit ray traced by the whole warp; every lane passes the same ray.
 __device__ __forceinline__ Hit trace_ordered(const RayState& r, const TreeRef& tr, uint32_t cap, const Hit& known,
-                                             uint32_t start) {
-    if (r.exact) return traverse_ordered<true>(r, tr, cap, known, start);
-    return traverse_ordered<false>(r, tr, cap, known, start);
+                                             uint32_t start, uint32_t* leaf) {
+    if (r.exact) return traverse_ordered<true>(r, tr, cap, known, start, leaf);
+    return traverse_ordered<false>(r, tr, cap, known, start, leaf);
 }
 
 // Primary ray of pixel (i, j): CSPrimaryRays.hlsl:36-56 with the basis camera.

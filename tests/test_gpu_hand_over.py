@@ -123,15 +123,15 @@ def test_restarted_rays(gpu_ctx, oracle_mod, kind):
     leaf = np.nonzero((reached != 0) & ((nodes["prim_count"] & 4) != 0))[0]
     starts = leaf[np.random.default_rng(1).integers(0, len(leaf), n)].astype(np.uint32)
     tmax, excl = np.full(n, 1e16, np.float32), np.full(n, -1, np.int32)
-    ref = oracle_mod.trace_from(nodes, depth, ids, tris, oracle_mod.rays_array(o, d, tmax, excl), starts)
-    ref = ref[0] if isinstance(ref, tuple) else ref
+    ref, ref_leaves = oracle_mod.trace_from(nodes, depth, ids, tris, oracle_mod.rays_array(o, d, tmax, excl), starts)
     st = torch.from_numpy(starts.view(np.int32)).cuda()
     rt = RayTracer(gpu_ctx)
     try:
         for budget in BUDGETS:
             gpu_ctx.set_trace_budget(budget)
-            got, _ = rt.rays_from(lb, rays_tensor(o, d, tmax, excl, "cuda"), st)
+            got, leaves = rt.rays_from(lb, rays_tensor(o, d, tmax, excl, "cuda"), st)
             assert np.array_equal(hits_to_numpy(got).view(np.int32), ref.view(np.int32)), budget
+            assert np.array_equal(leaves.cpu().numpy().view(np.uint32), ref_leaves), budget
         gpu_ctx.check()
     finally:
         gpu_ctx.set_trace_budget(None)
@@ -140,8 +140,7 @@ def test_restarted_rays(gpu_ctx, oracle_mod, kind):
 @pytest.mark.parametrize("block", [0, 2, 7])
 @pytest.mark.parametrize("kind", ["plane", "tilted"])
 def test_frame(gpu_ctx, oracle_mod, kind, block):
-    """Primary, shadow and mirror rays under every budget: the result without a hand-over,
-    whose primary hits are the oracle's."""
+    """Primary, shadow and mirror rays and their leaves under every budget."""
     import torch
     from rtgpu import scenes
     from rtgpu.api import LBVH, RayTracer, hits_to_numpy
@@ -154,24 +153,22 @@ def test_frame(gpu_ctx, oracle_mod, kind, block):
     walls = np.concatenate([tris, tris[:600] + np.float32(0.02)])  # something to mirror and to cast shadows
     lb = LBVH(gpu_ctx, len(walls), depth).Build(torch.from_numpy(walls).cuda())
     nodes, ids, _, _ = oracle_mod.lbvh_build(walls, depth)
-    ref = oracle_mod.trace(nodes, depth, ids, walls, oracle_mod.primary_rays(cam))
+    ref, ref_leaves = oracle_mod.trace_from(nodes, depth, ids, walls, oracle_mod.primary_rays(cam))
+    ref_vis, ref_mir, ref_ml = oracle_mod.shadow_mirror_from(nodes, depth, ids, walls, cam, light, ref, ref_leaves)
     rt = RayTracer(gpu_ctx)
-    first = None
     gpu_ctx.set_heavy_block(block)
     try:
         for budget in (0, None, 1, 40):
             gpu_ctx.set_trace_budget(budget)
             prim, leaves = rt.primary_leaves(lb, cam)
             assert np.array_equal(hits_to_numpy(prim).view(np.int32), ref.view(np.int32)), budget
-            if first is None:
-                root = leaves
-            # the same start nodes for every budget: a handed-over ray reports the root
-            vis, mir, _ = rt.shadow_mirror_from(lb, cam, light, prim, root)
-            got = (vis.clone(), mir.clone())
-            first = first or got
-            assert torch.equal(got[0], first[0]) and torch.equal(got[1], first[1]), budget
+            assert np.array_equal(leaves.cpu().numpy().view(np.uint32), ref_leaves), budget
+            vis, mir, ml = rt.shadow_mirror_from(lb, cam, light, prim, leaves)
+            assert np.array_equal(vis.cpu().numpy(), ref_vis), budget
+            assert np.array_equal(hits_to_numpy(mir).view(np.int32), ref_mir.view(np.int32)), budget
+            assert np.array_equal(ml.cpu().numpy().view(np.uint32), ref_ml), budget
         gpu_ctx.check()
     finally:
         gpu_ctx.set_trace_budget(None)
         gpu_ctx.set_heavy_block(None)
-    assert (ref["id"] >= 0).mean() > 0.2 and len(first[0].unique()) >= 3
+    assert (ref["id"] >= 0).mean() > 0.2 and len(np.unique(ref_vis)) >= 3 and (ref_mir["id"] >= 0).any()
