@@ -598,8 +598,8 @@ __device__ __forceinline__ void mark_records(const TreeRef& tr) {
 }
 
 constexpr uint32_t kGeneral = 8u;    // Walk::sgn: the records do not serve this ray
-constexpr uint32_t kInfinite = 16u;  // some 1 / d is infinite: the reference's NaN-sensitive min / max
-constexpr uint32_t kBySlot = 32u;    // the tree's leaves are named by their slots
+constexpr uint32_t kInfinite = kLeafFlag;  // some 1 / d is infinite: the reference's NaN-sensitive min / max
+constexpr uint32_t kBySlot = 16u;    // the tree's leaves are named by their slots
 // An internal node in hand of a ray that reads the heap: its slot, and its axis field above.
 constexpr uint32_t kAxisShift = 26u, kSlotMask = (1u << kAxisShift) - 1u;
 static_assert(kMaxDepth <= (int)kAxisShift, "");
@@ -799,7 +799,9 @@ struct Walk {
 
     // Moves every walking lane on: at most `steps` expansions (a lane puts its
     // first leaf aside and goes on; with two or three leaves set aside no
-    // faster), then the leaves: pooled where one is large, else a triangle of
+    // faster), then the leaves (a ray with an infinite 1 / d waits, on an empty leaf's
+    // word: a box that it runs along the face of is entered at NaN, which no later
+    // bound rejects, so nothing may be entered before the leaf has set the bound): pooled where one is large, else a triangle of
     // each lane at a time.  All 32 lanes call.
     // Returns whether the lane tested a leaf.
     template <uint32_t POOL_MIN = kPoolMin>
@@ -812,7 +814,7 @@ struct Walk {
                 if (cur == 0u) pop(stack);
                 if ((int)cur < 0 && !pend) {
                     pend = cur;
-                    cur = 0u;
+                    cur = sgn & kInfinite;  // 0, or the empty leaf
                     at_leaf = tests;
                     more = sp != 0u;
                 }
@@ -877,6 +879,7 @@ struct Walk {
                 __syncwarp();
             }
         }
+        if (cur == kLeafFlag) cur = 0u;  // the wait is over
         if (any_hit && b.id >= 0) cur = sp = 0u;
         have = cur != 0u || sp != 0u;
         return leaf != 0u;
@@ -1288,8 +1291,9 @@ __device__ __forceinline__ Hit traverse_wide(const RayState& r, const TreeRef& t
 // the tests at its ancestors' turns would have; where a NaN breaks that (a ray along a
 // face of a box), and when the pending hits or the stack overflow, one lane walks the
 // ray alone.  `known`: the hit of a walk in the same order that was broken off (id
-// < 0: none); going over its part again with that bound changes nothing.  `start`: as in
-// traverse().  `leaf` (nullable): the hit's leaf, 0 where the known hit stays.
+// < 0: none); going over its part again with that bound changes nothing, unless there are
+// NaN distances, so a ray with an infinite 1 / d begins anew.  `start`: as in traverse().
+// `leaf` (nullable): the hit's leaf, 0 where the known hit stays.
 // An entry: an internal node as the slot of its children's pair and whether the near child is
 // the right one; a leaf as its count and position, or by its slot when they do not fit
 // (leaf_word's limits); a pending hit.
@@ -1346,7 +1350,7 @@ __device__ __forceinline__ Hit traverse_ordered(const RayState& r, const TreeRef
     uint32_t* pleaf = reinterpret_cast<uint32_t*>(pv + kOrderedHits);
     uint32_t best_leaf = 0u;  // the leaf entry of the best hit (0: known's)
     const uint64_t init = hit_key(r.tmax, 0);
-    uint64_t best = known.id >= 0 ? hit_key(known.t, known.id) : init;  // uniform across the warp
+    uint64_t best = !EXACT && known.id >= 0 ? hit_key(known.t, known.id) : init;  // uniform across the warp
     float bu = known.u, bv = known.v, bt = known.t;
     uint32_t used = 0u;  // pending hits in use (uniform)
     int size = 0;        // uniform

@@ -172,3 +172,42 @@ def test_frame(gpu_ctx, oracle_mod, kind, block):
         gpu_ctx.set_trace_budget(None)
         gpu_ctx.set_heavy_block(None)
     assert (ref["id"] >= 0).mean() > 0.2 and len(np.unique(ref_vis)) >= 3 and (ref_mir["id"] >= 0).any()
+
+
+@pytest.mark.parametrize("n", [9000, 60000])
+@pytest.mark.parametrize("scale,offset,stretch", [(1e-18, 1e5, (1, 1, 1)), (1e4, 1e7, (1, 1e-7, 1e3)), (1e4, 1e5, (1, 1e-3, 1)),
+                                                  (1.0, 0.0, (1, 1, 0))])
+def test_rays_along_faces(gpu_ctx, oracle_mod, scale, offset, stretch, n):
+    """Far from the origin of coordinates few values are left between the triangles, and rays in a
+    plane x = const run along the faces of many boxes."""
+    import torch
+    from rtgpu import scenes
+    from rtgpu.api import LBVH, RayTracer, hits_to_numpy, rays_tensor
+    tris = scenes.random_soup(6000, 7, 0.01, 0.1).reshape(-1, 3) * np.array(stretch) + offset
+    tris = tris * scale
+    tris = np.ascontiguousarray(tris.reshape(-1, 9), np.float32)
+    rng = np.random.default_rng(n)
+    size = float((tris.reshape(-1, 3).max(0) - tris.reshape(-1, 3).min(0)).max())
+    t = tris[rng.integers(0, len(tris), n)].reshape(n, 3, 3).mean(1).astype(np.float64)
+    d = rng.normal(size=(n, 3))
+    d[:, 0] = 0.0
+    d[::5, 1] = 0.0
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    o = (t - d * size * rng.choice([0.0, 0.01, 0.5, 14.0, 1e3], n)[:, None]).astype(np.float32)
+    d = d.astype(np.float32)
+    lb = LBVH(gpu_ctx, len(tris), 16).Build(torch.from_numpy(tris).cuda())
+    nodes, ids, _, _ = oracle_mod.lbvh_build(tris, 16)
+    tmax, excl = np.full(n, 1e16, np.float32), np.full(n, -1, np.int32)
+    rays = oracle_mod.rays_array(o, d, tmax, excl)
+    ref = oracle_mod.trace(nodes, 16, ids, tris, rays)
+    any_ref = oracle_mod.trace(nodes, 16, ids, tris, rays, any_hit=True)
+    rt, dev = RayTracer(gpu_ctx), rays_tensor(o, d, tmax, excl, "cuda")
+    try:
+        for budget in BUDGETS:
+            gpu_ctx.set_trace_budget(budget)
+            assert np.array_equal(hits_to_numpy(rt.rays(lb, dev)).view(np.int32), ref.view(np.int32)), budget
+            assert np.array_equal(hits_to_numpy(rt.rays(lb, dev, any_hit=True))["id"] >= 0, any_ref["id"] >= 0), budget
+        gpu_ctx.check()
+    finally:
+        gpu_ctx.set_trace_budget(None)
+    assert (ref["id"] >= 0).mean() > 0.2
