@@ -278,7 +278,7 @@ __global__ void __launch_bounds__(kPtThreads, BLOCKS) k_pathtrace(
                 continue;
             }
         }
-        w.round<kPathPoolMin>(tr, kPtSteps, stack);
+        w.round<kPathPoolMin, false>(tr, kPtSteps, stack);
     }
 }
 
@@ -474,7 +474,7 @@ __global__ void __launch_bounds__(kPtThreads, kPtBlocks) k_pathtrace_adjoint(
                 continue;
             }
         }
-        w.round<kPathPoolMin>(tr, kPtSteps, stack);
+        w.round<kPathPoolMin, false>(tr, kPtSteps, stack);
     }
     // emitter gradient: warp and block sums, one atomic per block and channel (one per
     // warp rounds as often again as there are warps in a block)

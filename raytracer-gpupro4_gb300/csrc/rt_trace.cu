@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(kTraceThreads, BATCH ? 8 : 7) k_walk_shade(
             if (drained) break;
             continue;
         }
-        w.round(tr, kWalkSteps, stack, shadow);
+        w.round<kPoolMin, !BATCH>(tr, kWalkSteps, stack, shadow);
         int slot = -1;
         if (live && w.have && budgeted && w.tests > spill.budget) {
             const uint32_t e = atomicAdd(spill.count, 1u);
@@ -1494,7 +1494,7 @@ __device__ __forceinline__ void batch_trace_body(const BatchTraceArgs& a, const 
             if (!valid) i = j = 0;
             const RayState r = make_ray(mk3(cam.eye[0], cam.eye[1], cam.eye[2]), primary_dir(cam, i, j), 1e16f, -1);
             w.start(valid, r, tr, 1u, stack, Walk::tile_by_heap(valid, r, tr));
-            while (__any_sync(0xffffffffu, w.have)) w.round(tr, kBatchSteps, stack);
+            while (__any_sync(0xffffffffu, w.have)) w.round<kPoolMin, false>(tr, kBatchSteps, stack);
             const Hit h = w.hit();
             const uint32_t leaf = w.b.leaf;
             const size_t p = (size_t)j * a.width + i;
@@ -1511,7 +1511,7 @@ __device__ __forceinline__ void batch_trace_body(const BatchTraceArgs& a, const 
                                                 __ldg(a.lights + 3 * s + 1), __ldg(a.lights + 3 * s + 2), ph, valid, i, j,
                                                 false);
                 w.start(valid && sr.cast, sr.shadow, tr, h.id >= 0 ? leaf : 1u, stack);
-                while (__any_sync(0xffffffffu, w.have)) w.round(tr, kBatchSteps, stack, true);
+                while (__any_sync(0xffffffffu, w.have)) w.round<kPoolMin, false>(tr, kBatchSteps, stack, true);
                 if (valid) a.vis[s * px + p] = vis_code(sr.has, sr.cast, sr.cast && w.b.id >= 0);
             }
         }

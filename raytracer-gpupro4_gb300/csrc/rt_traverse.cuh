@@ -804,7 +804,7 @@ struct Walk {
     // bound rejects, so nothing may be entered before the leaf has set the bound): pooled where one is large, else a triangle of
     // each lane at a time.  All 32 lanes call.
     // Returns whether the lane tested a leaf.
-    template <uint32_t POOL_MIN = kPoolMin>
+    template <uint32_t POOL_MIN = kPoolMin, bool HELD = true>
     __device__ __forceinline__ bool round(const TreeRef& tr, int steps, uint2* stack, bool any_hit = false) {
         constexpr uint32_t kFull = 0xffffffffu;
         for (int s = 0; s < steps; ++s) {
@@ -849,17 +849,17 @@ struct Walk {
             pos += tr.tri_base;
         }
         // the heap's boxes were tested exactly, under this bound while there is no hit
-        bool inside = POOL_MIN == kPoolMin && (sgn & kGeneral) && b.id < 0;
+        bool inside = HELD && (sgn & kGeneral) && b.id < 0;
         // a leaf of 32 or more triangles: its exact box, with the bound of now, first (of
         // 5 or more, 330 k triangles at 720p took 9 us a frame longer)
         if ((leaf & kBigLeaf) && !inside) {
-            inside = leaf_entered<POOL_MIN>(tr, leaf & kSlotMask);
+            inside = leaf_entered<HELD>(tr, leaf & kSlotMask);
             if (!inside) cnt = 0u;
         }
         tests += cnt;
         at_leaf += cnt;
         if (__reduce_max_sync(kFull, cnt) > POOL_MIN) {
-            pooled<POOL_MIN>(tr, leaf, pos, cnt, inside);
+            pooled<HELD>(tr, leaf, pos, cnt, inside);
         } else {
             while (__any_sync(kFull, cnt != 0u)) {
                 if (cnt != 0u) {
@@ -873,7 +873,7 @@ struct Walk {
                     r.o = o;
                     r.d = d;
                     if (id != exclude && tri_test(r, a, bb, c, &u, &v, &t)) {
-                        if (!accept<POOL_MIN>(tr, leaf, hit_key(t, id), id, t, u, v, inside)) cnt = 0u;
+                        if (!accept<HELD>(tr, leaf, hit_key(t, id), id, t, u, v, inside)) cnt = 0u;
                     }
                 }
                 __syncwarp();
@@ -901,12 +901,12 @@ struct Walk {
 
     // A candidate hit in `leaf`.  Returns false when the leaf's box rejects it,
     // and so every triangle of the leaf.
-    template <uint32_t POOL_MIN>
+    template <bool HELD>
     __device__ __forceinline__ bool accept(const TreeRef& tr, uint32_t leaf, uint64_t key, int id, float t, float u,
                                            float v, bool& inside) {
         if (!(key < b.key)) return true;
         const uint32_t h = (leaf & kBigLeaf) ? leaf & kSlotMask : __ldg(tr.leaf_of + tr.tri_base + (leaf & 0x1ffffffu));
-        if (!inside && !leaf_entered<POOL_MIN>(tr, h)) return false;
+        if (!inside && !leaf_entered<HELD>(tr, h)) return false;
         inside = true;
         b.key = key;
         b.t = t;
@@ -920,7 +920,7 @@ struct Walk {
     // The triangles [pos, pos + cnt) of every lane's leaf, 32 (lane, triangle)
     // pairs at a time (see leaf_phase): a lane's 200 triangles cost 7 steps
     // of the warp instead of 200.
-    template <uint32_t POOL_MIN>
+    template <bool HELD>
     __device__ __forceinline__ void pooled(const TreeRef& tr, uint32_t leaf, uint32_t pos, uint32_t cnt, bool inside) {
         constexpr uint32_t kFull = 0xffffffffu;
         const int lane = threadIdx.x & 31;
@@ -984,16 +984,16 @@ struct Walk {
             const float hu = __shfl_sync(kFull, ku, hs);
             const float hv = __shfl_sync(kFull, kv, hs);
             if (mine && !rejected && hk != ~0ull)
-                rejected = !accept<POOL_MIN>(tr, leaf, hk, (int)(uint32_t)hk, ht, hu, hv, inside);
+                rejected = !accept<HELD>(tr, leaf, hk, (int)(uint32_t)hk, ht, hu, hv, inside);
             __syncwarp();
         }
     }
 
     // box_enter of the heap box of leaf h, under the bound of now: the leaf may
     // have been put aside, or its parent expanded, before a nearer hit was found.
-    // (A path's ray divides again even where k holds 1 / d: the choice cost the
-    // 56-register kernels 2 %.)
-    template <uint32_t POOL_MIN>
+    // HELD: take 1 / d from k where it holds it; the choice costs the kernels of 48 and 56
+    // registers (batches, paths) 1 to 2 %.
+    template <bool HELD>
     __device__ __forceinline__ bool leaf_entered(const TreeRef& tr, uint32_t h) const {
         if (h >= tr.num_heap) {
             atomicOr(tr.err, RT_DEVERR_BOUNDS);
@@ -1003,7 +1003,7 @@ struct Walk {
         RayState r;
         r.o = o;
         r.inv = k;
-        if (POOL_MIN == kPathPoolMin || !(sgn & kGeneral)) r.inv = mk3(fdiv(1.0f, d.x), fdiv(1.0f, d.y), fdiv(1.0f, d.z));
+        if (!HELD || !(sgn & kGeneral)) r.inv = mk3(fdiv(1.0f, d.x), fdiv(1.0f, d.y), fdiv(1.0f, d.z));
         float t0;
         return enter(r, nb, b.t, &t0, (sgn & kInfinite) != 0u);
     }
