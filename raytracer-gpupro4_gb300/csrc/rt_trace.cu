@@ -710,11 +710,12 @@ __global__ void __launch_bounds__(kTraceThreads, ANY ? 7 : 6) k_trace_heavy(Heav
 constexpr uint32_t kFewRays = 16384;
 
 __global__ void __launch_bounds__(kTraceThreads) k_rays_wide(TreeRef tr, const rt_ray* __restrict__ rays, uint32_t n,
+                                                             const uint32_t* __restrict__ starts,
                                                              rt_hit* __restrict__ hits, uint32_t cap) {
     grid_dep_wait();
     const uint32_t k = blockIdx.x * kWideWarps + (threadIdx.x >> 5);
     if (k >= n) return;
-    const Hit h = trace_ordered(load_ray(rays, k, true), tr, cap, no_hit(), 1u, nullptr);
+    const Hit h = trace_ordered(load_ray(rays, k, true), tr, cap, no_hit(), starts ? __ldg(starts + k) : 1u, nullptr);
     if ((threadIdx.x & 31) == 0) store_hit(hits + k, h);
 }
 
@@ -1086,7 +1087,7 @@ rt_status trace_rays(rt_ctx* ctx, const rt_lbvh* l, const rt_ray* d_rays, uint32
     if (!d_stats && !any_hit && !d_leaves && n <= kFewRays) {
         const uint32_t cap = wide_stack_entries(l->depth);
         launch_pdl(k_rays_wide, (n + kWideWarps - 1) / kWideWarps, kTraceThreads, wide_smem_bytes(cap), ctx->stream,
-                   tree_ref(ctx, l), d_rays, n, d_hits, cap);
+                   tree_ref(ctx, l), d_rays, n, d_starts, d_hits, cap);
         RT_CHECK_LAUNCH(ctx, "k_rays_wide");
         return RT_OK;
     }

@@ -114,7 +114,10 @@ def test_rays(gpu_ctx, oracle_mod, kind, n):
 @pytest.mark.parametrize("kind", ["plane", "tilted", "down"])
 def test_restarted_rays(gpu_ctx, oracle_mod, kind):
     """The order of a restarted walk begins at its start node."""
+    import ctypes as C
+
     import torch
+    from rtgpu import _lib as L
     from rtgpu.api import LBVH, RayTracer, hits_to_numpy, rays_tensor
     n = 20000
     tris, depth, (o, d) = case(kind, n)
@@ -132,6 +135,12 @@ def test_restarted_rays(gpu_ctx, oracle_mod, kind):
             got, leaves = rt.rays_from(lb, rays_tensor(o, d, tmax, excl, "cuda"), st)
             assert np.array_equal(hits_to_numpy(got).view(np.int32), ref.view(np.int32)), budget
             assert np.array_equal(leaves.cpu().numpy().view(np.uint32), ref_leaves), budget
+            for m in (9000, n):  # a warp a ray or a lane, without leaves
+                hits = torch.empty((m, 4), dtype=torch.int32, device="cuda")
+                ptr = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+                dev = rays_tensor(o[:m], d[:m], tmax[:m], excl[:m], "cuda")
+                assert L.lib().rt_trace_rays_from(gpu_ctx.h, lb.h, ptr(dev), m, 0, ptr(st), ptr(hits), None, None) == L.RT_OK
+                assert np.array_equal(hits_to_numpy(hits).view(np.int32), ref[:m].view(np.int32)), (budget, m)
         gpu_ctx.check()
     finally:
         gpu_ctx.set_trace_budget(None)
