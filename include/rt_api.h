@@ -91,18 +91,22 @@ rt_status rt_ctx_destroy(rt_ctx* ctx);
 rt_status rt_ctx_set_stream(rt_ctx* ctx, void* stream);
 /* Work budget of the camera, shading and generic ray traces: a ray that has
  * spent more than `budget` box + triangle tests in the per-lane traversal is
- * handed to a second kernel that traces it with a whole warp (same hit).
+ * handed to a second kernel that traces it with a whole warp (same closest hit
+ * and leaf whatever the budget; an any-hit ray may report another hit).
  * 0 turns the hand-over off.  rt_ctx_set_trace_budget sets every kind;
  * rt_ctx_set_trace_budget_kind one (0 primary rays, 1 shadow / mirror rays,
  * 2 rt_trace_rays).  Defaults: 384, 768, 384 (the fastest on a 2.1 M-triangle
- * frame).  Path tracing never hands over. */
+ * frame).  Path tracing never hands over, and neither do rt_trace_rays(_from)
+ * calls of at most 16,384 closest-hit rays without leaves: each of those rays has a
+ * warp from the start. */
 rt_status rt_ctx_set_trace_budget(rt_ctx* ctx, uint32_t budget);
 rt_status rt_ctx_set_trace_budget_kind(rt_ctx* ctx, uint32_t kind, uint32_t budget);
-/* How the handed-over rays are traced, per trace kind in `kinds` (bit 0
+/* How the handed-over any-hit rays are traced, per trace kind in `kinds` (bit 0
  * primary rays, bit 1 shadow / mirror rays, bit 2 rt_trace_rays): a set bit
  * traces each with a whole block of 128 threads (suits a few hundred very
- * long rays), a clear bit with a warp (suits thousands).  Same hits either
- * way.  Default 2 (the shading rays a block per ray: the fastest on a
+ * long rays), a clear bit with a warp (suits thousands).  Closest-hit
+ * rays always have a warp each; of an any-hit ray the visibility does not depend on it,
+ * the reported hit may.  Default 2 (the shading rays a block per ray: the fastest on a
  * 2.1 M-triangle frame). */
 rt_status rt_ctx_set_heavy_block(rt_ctx* ctx, uint32_t kinds);
 /* Heavy-first tile order: for each trace kind in `kinds` (bit 0 primary

@@ -1060,7 +1060,7 @@ __global__ void __launch_bounds__(256) k_emit_refit(const uint32_t* __restrict__
 //      a warp takes 32 consecutive elements at a time: they leave through a
 //      per-warp staging buffer as 512-byte runs, and their boxes go to
 //      shared memory;
-//   2. the boxes folded per leaf, each thread over its own eight consecutive
+//   2. the boxes folded per leaf, each thread over its own two consecutive
 //      elements (a segmented scan carries a leaf that spans threads, with its
 //      head); the leaf records are stored;
 //   3. a leaf that began in an earlier tile and ends in this one is finished
@@ -1106,7 +1106,7 @@ constexpr int kUnitCap = kMergeGroup * kItemCap;  // units of one CTA of the mer
 constexpr size_t kUnitSmem = (size_t)kUnitWords * kUnitCap * sizeof(uint32_t) + 16;
 constexpr size_t kChunkSmem = (size_t)kUnitWords * kTreeTile * sizeof(uint32_t) + 16;
 // k_emit_units: the tile's triangle boxes, six planes of kBoxStride floats
-// (element e at e + e / 32, so that a warp reading eight consecutive
+// (element e at e + e / 32, so that a warp reading two consecutive
 // elements per lane hits 32 different banks), then one staging buffer of
 // 32 triangles (96 float4) per warp
 constexpr int kBoxStride = kTreeTile + kTreeTile / 32;

@@ -153,7 +153,7 @@ struct rt_ctx {
     // hand-over budget per trace kind (0 primary, 1 shading, 2 generic rays); 0: no hand-over
     uint32_t trace_budget[3] = {kDefaultTraceBudget, kDefaultShadeBudget, kDefaultTraceBudget};
     // per trace kind (bit 0 primary, 1 shading, 2 generic rays): the handed-over
-    // rays are traced a block per ray (k_trace_heavy_team) instead of a warp
+    // any-hit rays are traced a block per ray (k_trace_heavy_team) instead of a warp
     uint32_t heavy_team = kDefaultHeavyTeam;
     uint32_t tile_order = 1u;  // heavy-first tile order per kind: bit 0 primary, 1 shading, 2 generic rays
     int num_sms = 0;

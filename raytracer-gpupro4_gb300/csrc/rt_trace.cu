@@ -146,7 +146,7 @@ constexpr int kPrimSteps = 3;
 // Blocks per SM: with few tiles a warp the image lasts as long as its slowest tiles,
 // and 72 registers (no spills) move a lane faster; with many, 64 registers and
 // another block per SM hide more latency (65 k triangles at 512 x 512 275 us a frame with
-// eight blocks and 272 with seven, 330 k at 720p 583 and 576, 2.1 M at 1080p
+// eight blocks and 272 with seven, 260 k at 720p 583 and 576, 2.1 M at 1080p
 // 1,404 and 1,412).
 constexpr uint32_t kPrimWarps = 8u * kTraceThreads / 32u;  // warps an SM
 uint32_t prim_blocks(const rt_ctx* ctx, uint32_t tiles) {
@@ -303,7 +303,7 @@ __device__ __forceinline__ RayState load_ray(const rt_ray* __restrict__ rays, ui
 // scene g / px, and a warp's lanes may walk different scenes.
 // 16 idle lanes and 4 expansions a round were the fastest of 12 to 24 and 3 to 10:
 // 650 -> 545 us a frame of 2.1 M triangles at 1080p.  A frame's rays take 72 registers
-// (seven blocks an SM; five to eight at 330 k triangles and 720p: 570, 561, 555 and 565 us,
+// (seven blocks an SM; five to eight at 260 k triangles and 720p: 570, 561, 555 and 565 us,
 // at 2.1 M and 1080p 1,509, 1,446, 1,410 and 1,404), a batch's many scenes 64.
 constexpr int kWalkRefill = 16;
 constexpr int kWalkSteps = 4;

@@ -451,7 +451,8 @@ __device__ __forceinline__ bool start_walk(const RayState& r, const TreeRef& tr_
 // Hand-over of rays that exceed a work budget.  A lane whose ray has spent
 // more than `budget` box + triangle tests takes a slot of the heavy-ray list
 // (atomicAdd on *count) and stops; the caller records the ray in that slot,
-// and a second kernel traces it with a whole warp (traverse_wide).  When the
+// and a second kernel traces it with a whole warp: traverse_ordered for a closest hit,
+// traverse_wide (or a block, traverse_team) for an any-hit ray.  When the
 // list is full the lane keeps going.  count == nullptr: no budget.
 struct Spill {
     uint32_t* count;
@@ -604,7 +605,7 @@ constexpr uint32_t kBySlot = 16u;    // the tree's leaves are named by their slo
 constexpr uint32_t kAxisShift = 26u, kSlotMask = (1u << kAxisShift) - 1u;
 static_assert(kMaxDepth <= (int)kAxisShift, "");
 // A leaf of more triangles makes the warp pool its leaves: 2 for rays that stay
-// neighbours (330 k triangles at 720p 561 us a frame with 3, 538 with 2; 1: the same), 3
+// neighbours (260 k triangles at 720p 561 us a frame with 3, 538 with 2; 1: the same), 3
 // for paths (24.2 ms with 3, 24.5 with 2, 25.9 with 1).
 constexpr uint32_t kPoolMin = 2u;
 constexpr uint32_t kPathPoolMin = 3u;
@@ -851,7 +852,7 @@ struct Walk {
         // the heap's boxes were tested exactly, under this bound while there is no hit
         bool inside = HELD && (sgn & kGeneral) && b.id < 0;
         // a leaf of 32 or more triangles: its exact box, with the bound of now, first (of
-        // 5 or more, 330 k triangles at 720p took 9 us a frame longer)
+        // 5 or more, 260 k triangles at 720p took 9 us a frame longer)
         if ((leaf & kBigLeaf) && !inside) {
             inside = leaf_entered<HELD>(tr, leaf & kSlotMask);
             if (!inside) cnt = 0u;
