@@ -973,9 +973,9 @@ def run_pt(args, dist: Dist, adjoint: bool = False):
            "roofline": roofline,
            "clocks": clk.summary(),
            # per step: the build's kernels; k_reset_words (which also makes the trace records),
-           # k_pathtrace and, with several samples, k_fold_terms; k_reset_words and
-           # k_pathtrace_adjoint
-           "gpu_launches": (build_launches(n) + (3 if spp > 1 else 2) + (2 if adjoint else 0)) * args.steps}
+           # k_pathtrace and, with several samples, k_fold_terms; k_reset_words,
+           # k_pathtrace_adjoint and k_fold_emitter
+           "gpu_launches": (build_launches(n) + (3 if spp > 1 else 2) + (3 if adjoint else 0)) * args.steps}
     if adjoint:
         out["components"]["backward_ms"] = round(bwd_ms, 4)
         out["components"]["backward_over_forward"] = round(bwd_ms / fwd_ms, 3)

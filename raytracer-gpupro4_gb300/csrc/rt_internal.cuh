@@ -126,6 +126,8 @@ constexpr uint32_t kMaxTris = (1u << 29);
 constexpr uint32_t kSpillCap = 1u << 20;
 constexpr int kTeamClaims = 38;  // ctx->d_words: claims of the block-per-ray passes (two)
 constexpr int kDoubtCount = 36;  // ctx->d_words: length of the any-hit rays' second list, its claim counter
+constexpr int kEmitterSum = 54;  // ctx->d_words: a call's emitter gradient, three FP64 words
+static_assert(kEmitterSum % 2 == 0 && kEmitterSum + 6 <= 64, "");
 constexpr uint32_t kDefaultHeavyTeam = 2u;
 constexpr uint32_t kDefaultTraceBudget = 384;
 constexpr uint32_t kDefaultShadeBudget = 768;
@@ -346,5 +348,5 @@ inline rt_status reset_work(rt_ctx* ctx, int slot) {
     return RT_OK;
 }
 // The same, and the trace records of l if they are not valid.
-rt_status reset_work_and_records(rt_ctx* ctx, int slot, const rt_lbvh* l);
+rt_status reset_work_and_records(rt_ctx* ctx, int slot, const rt_lbvh* l, uint64_t words = 0);
 

@@ -1138,8 +1138,8 @@ rt_status begin_bounce(rt_ctx* ctx, const rt_lbvh* l, const Spill& shadow, std::
     return reset_words(ctx, mask, records_of(ctx, l));
 }
 
-rt_status reset_work_and_records(rt_ctx* ctx, int slot, const rt_lbvh* l) {
-    return reset_words(ctx, word_bit(ctx, ctx->d_work + slot), records_of(ctx, l));
+rt_status reset_work_and_records(rt_ctx* ctx, int slot, const rt_lbvh* l, uint64_t words) {
+    return reset_words(ctx, words | word_bit(ctx, ctx->d_work + slot), records_of(ctx, l));
 }
 
 extern "C" rt_status rt_trace_primary(rt_ctx* ctx, const rt_lbvh* l, const rt_camera* cam, rt_hit* d_hits,
